@@ -85,12 +85,13 @@ struct Variant {
   int planes;  // 1: bit-sliced kernel over bit-plane rows (R = words per thread)
   int slot;    // > 0: kernel compiled for exactly this slot width (words)
   int pairs = 0;  // 1: 2-bit channel-pair kernel over pair-sum rows (three planes)
+  double rate = 0.0;  // float32 shapes: measured rate relative to the fastest
 };
 
 template <int NB, int R, int DW, int TW, int SLAB, int STAGES, int ACC>
-static Variant mk(int single) {
+static Variant mk(int single, double rate = 0.0) {
   return Variant{NB, ACC, R, DW, TW, SLAB, STAGES, &k_dmt<NB, R, DW, TW, SLAB, STAGES, ACC>,
-                 single, 0, 0};
+                 single, 0, 0, 0, rate};
 }
 
 // Bit-sliced counters hold sums below 2^bit_levels(nbits).
@@ -162,13 +163,16 @@ static const std::vector<Variant>& variants() {
       mk<32, 16, 4, 1, 16, 2, SPP_ACC_KAHAN32>(0),
       mk<32, 8, 2, 1, 16, 2, SPP_ACC_KAHAN32>(0),
       mk<32, 16, 2, 1, 16, 2, SPP_ACC_KAHAN32>(0),
-      // float32 input, fp64 accumulator (channel-ordered sums: the reference's)
-      mk<32, 16, 4, 1, 16, 2, SPP_ACC_F64>(0),
-      mk<32, 16, 2, 1, 16, 2, SPP_ACC_F64>(0),
-      mk<32, 8, 2, 1, 16, 2, SPP_ACC_F64>(0),
-      mk<32, 8, 8, 1, 32, 2, SPP_ACC_F64>(0),
-      mk<32, 4, 8, 2, 32, 2, SPP_ACC_F64>(0),
-      mk<32, 8, 4, 1, 16, 2, SPP_ACC_F64>(0),
+      // float32 input, fp64 accumulator (channel-ordered sums: the reference's).
+      // The argument is the shape's measured rate with the SMs full, relative to
+      // the first (1024 channels, 256 trials to DM 500, 57444 outputs: 2.95 ms;
+      // 16 words x 4 trials, the choice before, 4.14 ms: three CTAs of four
+      // warps per SM leave the adders waiting on slab hand-overs); wide delay
+      // spreads fit only the small tiles
+      mk<32, 16, 8, 2, 16, 2, SPP_ACC_F64>(0, 1.0), mk<32, 16, 5, 3, 16, 2, SPP_ACC_F64>(0, 0.99),
+      mk<32, 8, 8, 2, 16, 2, SPP_ACC_F64>(0, 0.97), mk<32, 8, 4, 2, 16, 2, SPP_ACC_F64>(0, 0.85),
+      mk<32, 8, 4, 1, 16, 2, SPP_ACC_F64>(0, 0.94), mk<32, 16, 4, 1, 16, 2, SPP_ACC_F64>(0, 0.8),
+      mk<32, 16, 2, 1, 16, 2, SPP_ACC_F64>(0, 0.6), mk<32, 8, 2, 1, 16, 2, SPP_ACC_F64>(0, 0.75),
       mk<32, 4, 1, 4, 32, 2, SPP_ACC_F64>(1),
       mk<32, 2, 1, 4, 32, 2, SPP_ACC_F64>(1),
   };
@@ -728,6 +732,30 @@ static void free_pair_tables(spp_dmt_plan* p) {
   p->d_pair_src = nullptr;
 }
 
+// The float32 shape a plan starts from (without autotuning).
+static int first_float_choice(const spp_dmt_plan* p) {
+  const int64_t nvalid = std::max<int64_t>(1, plan_nvalid(p, p->nsamps_max));
+  // float64 sums: waves of the CTAs an SM holds (shared memory, 64 warps)
+  // times a tile's adds over its rate, which falls below 12 adding warps per SM
+  int pick = 0;
+  double best = 0.0;
+  for (int i = 0; i < (int)p->cands.size(); ++i) {
+    const Variant& v = variants()[p->cands[i]];
+    if (v.rate <= 0.0) continue;
+    const int64_t smem = smem_bytes(v, slot_words(v, p->spans[i])) + 1024;
+    const int64_t per_sm = std::min<int64_t>((228 << 10) / smem, 64 / (v.DW * v.TW + 1));
+    const int64_t ctas = ceil_div(p->ndm, v.DW) * ceil_div(nvalid, tile_T(v));
+    const double full = std::min(1.0, (double)(per_sm * v.DW * v.TW) / 12.0);
+    const double t =
+        (double)(ceil_div(ctas, 148 * per_sm) * per_sm * v.DW * tile_T(v)) / (v.rate * full);
+    if (best == 0.0 || t < best) {
+      best = t;
+      pick = i;
+    }
+  }
+  return pick;
+}
+
 extern "C" {
 
 int spp_dmt_plan_create(spp_dmt_plan** plan, int nbits, int bitorder, int64_t nchans,
@@ -918,6 +946,7 @@ int spp_dmt_plan_create(spp_dmt_plan** plan, int nbits, int bitorder, int64_t nc
     if (p->nprows * 3 * g.pitch_w * 4 <= kPairDefaultBytes) p->cur = (int)i;
     break;
   }
+  if (nbits == 32) p->cur = first_float_choice(p);
   const int trc = ensure_pair_tables(p, p->cur);
   if (trc != SPP_OK) {
     free_pair_tables(p);

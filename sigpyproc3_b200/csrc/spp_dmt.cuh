@@ -14,6 +14,8 @@
 // compensated fp32 / fp64 (float input).  All waits are bounded.
 #pragma once
 
+#include <type_traits>
+
 #include "spp_common.cuh"
 
 namespace spp {
@@ -138,21 +140,21 @@ k_corner_turn_int(const uint8_t* __restrict__ raw, int64_t nchans, int64_t nsamp
   }
 }
 
-// IEEE-754 binary32 -> binary64 for normal numbers by field arithmetic:
-// (-1)^s 2^(e-127) (1 + m 2^-23) is the binary64 number with the same sign,
-// biased exponent e - 127 + 1023 = e + 896 and significand m followed by 29
-// zero bits.  The high word is sign | (e + 896) << 20 | m >> 3, i.e.
-// ((|u| >> 3) + (896 << 20)) | sign, and the low word m << 29 = u << 29.
-// Integer-pipe work, so it runs beside the conversion unit's F2F; zero,
-// subnormals, infinities and NaN are not handled (the caller checks
-// f32_is_normal over its data first).
-__device__ __forceinline__ bool f32_is_normal(float x) {
-  return ((__float_as_uint(x) & 0x7fffffffu) - 0x00800000u) < 0x7f000000u;  // 1 <= e <= 254
+// Adds a finite float32 to a float64 sum without the conversion unit.  The
+// float's sign, exponent and significand fields moved to the places they have
+// in a binary64 (high word: sign, then the other 31 bits >> 3; low word: the
+// three bits left over) read as x * 2^(127 - 1023), for normal numbers, zeros
+// and subnormals alike; the fused multiply-add scales by 2^896 exactly and
+// rounds once, as adding the converted float does.  Infinities and NaN are not
+// handled (the caller checks f32_is_finite over its data first).
+__device__ __forceinline__ bool f32_is_finite(float x) {
+  return (__float_as_uint(x) & 0x7f800000u) != 0x7f800000u;
 }
-__device__ __forceinline__ double f64_of_normal_f32(float x) {
+__device__ __forceinline__ double add_finite_f32(double acc, float x) {
   const uint32_t u = __float_as_uint(x);
-  const uint32_t hi = (((u & 0x7fffffffu) >> 3) + (896u << 20)) | (u & 0x80000000u);
-  return __hiloint2double((int)hi, (int)(u << 29));
+  const uint32_t hi = (uint32_t)((int32_t)u >> 3) & 0x8fffffffu;
+  const double scaled = __hiloint2double((int)hi, (int)(u << 29));
+  return __fma_rn(scaled, __longlong_as_double((1023ll + 896ll) << 52), acc);
 }
 
 // Corner turn for float32 data, optionally fused with zero-DM subtraction
@@ -160,7 +162,7 @@ __device__ __forceinline__ double f64_of_normal_f32(float x) {
 //   y = f32((f64(x) - zdm[t] * f64(chanwts[c])) + f64(bpass[c]))
 // computed with round-to-nearest intrinsics (no contraction).  `special`
 // (optional): set to 1 when any sample taken from the block (after zero-DM)
-// is not a normal float32.
+// is not finite.
 static __global__ void __launch_bounds__(256)
 k_corner_turn_f32(const float* __restrict__ raw, int64_t nchans, int64_t nsamps,
                   int64_t halo, float* __restrict__ planar, int64_t pitch,
@@ -170,7 +172,7 @@ k_corner_turn_f32(const float* __restrict__ raw, int64_t nchans, int64_t nsamps,
   const int64_t c0 = (int64_t)blockIdx.x * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
   const int64_t nty = (pitch + 31) / 32;
-  bool odd = false;  // a sample from the block that is not a normal float32
+  bool odd = false;  // a sample from the block that is not finite
   for (int64_t by = blockIdx.y; by < nty; by += gridDim.y) {
     const int64_t p0 = by * 32;  // planar column (sample + halo)
     for (int i = ty; i < 32; i += 8) {
@@ -184,7 +186,7 @@ k_corner_turn_f32(const float* __restrict__ raw, int64_t nchans, int64_t nsamps,
           const double t2 = __dsub_rn((double)v, t1);
           v = (float)__dadd_rn(t2, (double)bpass[c]);
         }
-        odd |= !f32_is_normal(v);
+        odd |= !f32_is_finite(v);
       }
       tile[i][tx] = v;
     }
@@ -313,7 +315,7 @@ struct DmtArgs {
   int64_t nvalid;
   uint32_t* status;
   // float64 accumulation of float32 rows: a word that is 0 when every sample
-  // of the block is a normal float32 (set by the corner turn); then part of
+  // of the block is a finite float32 (set by the corner turn); then part of
   // the conversions run on the integer pipe.  nullptr: conversion unit only.
   const uint32_t* special;
   // channel-pair kernels (2-bit data): `planar` holds pair-sum rows of three
@@ -439,11 +441,12 @@ k_dmt(const DmtArgs a) {
     double d_acc[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) { s_acc[r] = 0.f; c_acc[r] = 0.f; d_acc[r] = 0.0; }
-    // all samples normal: one word in four converts by field arithmetic
-    // (integer pipe), the rest by F2F (conversion unit): exactly the same
-    // values.  F2F alone keeps the conversion unit near full; the field
-    // conversion costs ~6 issue slots, so half and half made the kernel
-    // issue-bound at the same speed and one in four is the balance measured.
+    // all samples finite: every second word is added through the integer pipe,
+    // the others through F2F (conversion unit, 16 per clock and SM): exactly the
+    // same sums.  Of 8 words 3 on the integer pipe measured 2.89-3.01 ms over
+    // the best shapes, 4 of 8 2.90, 5 and 6 slower (1024 channels, 256 trials,
+    // 57444 outputs); 2 of 8 with a longer conversion for normal numbers alone
+    // was the balance before.
     const bool split = ACC == SPP_ACC_F64 && a.special != nullptr && *a.special == 0u;
     for (int k = 0; k < nslab; ++k) {
       const int s = k % STAGES;
@@ -456,28 +459,31 @@ k_dmt(const DmtArgs a) {
       float p_acc[R];
 #pragma unroll
       for (int r = 0; r < R; ++r) p_acc[r] = 0.f;
-      if (ACC == SPP_ACC_F64 && split) {
-#pragma unroll 4
-        for (int j = 0; j < nc; ++j) {
-          const float* row = sd + j * a.slot_w + (wbase + dl[j]);
+      auto add_slab = [&](auto sp) {
+        auto add_row = [&](const float* row) {
 #pragma unroll
           for (int r = 0; r < R; ++r) {
             const float x = row[32 * r];
-            d_acc[r] += (r % 4 == 3) ? f64_of_normal_f32(x) : (double)x;
+            if (ACC != SPP_ACC_F64) p_acc[r] = __fadd_rn(p_acc[r], x);
+            else if (decltype(sp)::value && (r & 1)) d_acc[r] = add_finite_f32(d_acc[r], x);
+            else d_acc[r] += (double)x;
           }
+        };
+        // four channels' offsets at a time; a short last slab one by one
+        int j = 0;
+#pragma unroll 1
+        for (; j + 4 <= nc; j += 4) {
+          const int4 o = *reinterpret_cast<const int4*>(dl + j);
+          const float* row = sd + j * a.slot_w + wbase;
+          add_row(row + o.x);
+          add_row(row + a.slot_w + o.y);
+          add_row(row + 2 * a.slot_w + o.z);
+          add_row(row + 3 * a.slot_w + o.w);
         }
-      } else {
-#pragma unroll 4
-        for (int j = 0; j < nc; ++j) {
-          const float* row = sd + j * a.slot_w + (wbase + dl[j]);
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            const float x = row[32 * r];
-            if (ACC == SPP_ACC_F64) d_acc[r] += (double)x;
-            else p_acc[r] = __fadd_rn(p_acc[r], x);
-          }
-        }
-      }
+        for (; j < nc; ++j) add_row(sd + j * a.slot_w + (wbase + dl[j]));
+      };
+      if (split) add_slab(std::true_type{});
+      else add_slab(std::false_type{});
       if (ACC != SPP_ACC_F64) {
 #pragma unroll
         for (int r = 0; r < R; ++r) {
