@@ -11,6 +11,7 @@
 
 #include "spp_common.cuh"
 #include "spp_dmt.cuh"
+#include "spp_ilv.h"
 
 namespace spp {
 
@@ -84,14 +85,13 @@ struct Variant {
   int single;  // 1: meant for one DM (time-split warps)
   int planes;  // 1: bit-sliced kernel over bit-plane rows (R = words per thread)
   int slot;    // > 0: kernel compiled for exactly this slot width (words)
-  int pairs = 0;  // 1: 2-bit channel-pair kernel over pair-sum rows (three planes)
   double rate = 0.0;  // float32 shapes: measured rate relative to the fastest
 };
 
 template <int NB, int R, int DW, int TW, int SLAB, int STAGES, int ACC>
 static Variant mk(int single, double rate = 0.0) {
   return Variant{NB, ACC, R, DW, TW, SLAB, STAGES, &k_dmt<NB, R, DW, TW, SLAB, STAGES, ACC>,
-                 single, 0, 0, 0, rate};
+                 single, 0, 0, rate};
 }
 
 // Bit-sliced counters hold sums below 2^bit_levels(nbits).
@@ -107,50 +107,25 @@ static Variant mkb() {
   return Variant{NB, 0, P, DW, TW, SLAB, STAGES, fn, 0, 1, SLOT};
 }
 
-// Channel-pair kernels (2-bit data): SLAB pairs per slab, two staged rows
-// per pair.
-template <int P, int DW, int TW, int STAGES, int SLAB, int SLOT = 0, int MINB = 0>
-static Variant mkp() {
-  constexpr int L = BitsLevels<3>::kLevels;
-  void (*fn)(const DmtArgs) = &k_dmt_pairs<P, DW, TW, STAGES, L, SLAB, SLOT>;
-  if constexpr (MINB > 0) fn = &k_dmt_pairs_minb<P, DW, TW, STAGES, L, SLAB, SLOT, MINB>;
-  Variant v{2, 0, P, DW, TW, SLAB, STAGES, fn, 0, 1, SLOT};
-  v.pairs = 1;
-  return v;
-}
-
 #define SPP_INT_VARIANTS(NB)                    \
   mk<NB, 2, 8, 1, 64, 3, 0>(0), mk<NB, 1, 8, 1, 64, 3, 0>(0), mk<NB, 2, 4, 2, 64, 3, 0>(0), \
-      mk<NB, 1, 16, 1, 64, 3, 0>(0), mk<NB, 2, 1, 4, 64, 3, 0>(1), mk<NB, 1, 1, 4, 64, 3, 0>(1)
+      mk<NB, 2, 1, 4, 64, 3, 0>(1), mk<NB, 1, 1, 4, 64, 3, 0>(1)
 
 static const std::vector<Variant>& variants() {
   static const std::vector<Variant> v = {
-      // bit-sliced (1- and 2-bit data)
-      // fixed slot widths first: 32-channel slabs keep 3-4 CTAs resident per SM
-      mkb<2, 2, 8, 1, 2, 32, 80, 4>(), mkb<2, 2, 8, 1, 2, 32, 80>(), mkb<2, 2, 8, 1, 3, 32, 80>(),
-      mkb<2, 2, 8, 1, 2, 32, 96>(), mkb<2, 2, 8, 1, 2, 32, 128>(),
-      mkb<2, 2, 8, 1, 2, 64, 80>(), mkb<2, 2, 8, 1, 2, 64, 96>(),
-      mkb<2, 3, 8, 1, 2, 32, 112, 3>(), mkb<2, 3, 8, 1, 2, 32, 112, 2>(),
-      mkb<2, 2, 8, 1, 2>(), mkb<2, 2, 8, 1, 3, 32>(), mkb<2, 2, 8, 1, 2, 32>(),
-      mkb<2, 4, 8, 1, 2, 32>(), mkb<2, 2, 16, 1, 2, 32>(), mkb<2, 1, 8, 1, 3>(),
-      // channel pairs summed once per relative delay (2-bit DM grids whose
-      // adjacent channels differ by few distinct delays)
-      mkp<3, 8, 1, 2, 8, 112, 3>(), mkp<3, 8, 1, 3, 8, 112, 3>(), mkp<3, 8, 1, 2, 16, 112, 2>(),
-      mkp<2, 8, 1, 2, 16, 80, 3>(), mkp<3, 8, 1, 2, 16>(), mkp<2, 8, 1, 3, 8>(),
-      mkb<1, 2, 8, 1, 2, 32, 80>(), mkb<1, 2, 8, 1, 2, 32, 128>(),
-      mkb<1, 2, 8, 1, 2>(), mkb<1, 2, 8, 1, 3, 32>(), mkb<1, 4, 8, 1, 2, 32>(),
+      // bit-sliced, 32 consecutive samples per word: blocks or tables that the
+      // interleaved layout (spp_ilv.cu) does not take, fixed slot widths first
+      mkb<2, 2, 8, 1, 2, 32, 80, 4>(), mkb<2, 2, 8, 1, 2, 32, 128>(), mkb<2, 2, 8, 1, 2, 32>(),
+      mkb<2, 4, 8, 1, 2, 32>(),
+      mkb<1, 2, 8, 1, 2, 32, 80>(), mkb<1, 2, 8, 1, 2, 32, 128>(), mkb<1, 2, 8, 1, 3, 32>(),
       SPP_INT_VARIANTS(1),
       SPP_INT_VARIANTS(2),
-      // bit-sliced 4-bit (four plane rows per channel; 16-channel slabs keep
-      // a stage's planes within a third of shared memory): 1.8-2.3x the SIMD
-      // kernels' adds/s, so they come first for 4-bit data
-      mkb<4, 2, 8, 1, 2, 16, 96, 3>(), mkb<4, 2, 8, 1, 2, 16>(), mkb<4, 3, 8, 1, 2, 16, 112, 2>(),
-      mkb<4, 2, 8, 1, 2, 32>(), mkb<4, 1, 8, 1, 3, 16>(),
+      // four plane rows per channel; 16-channel slabs keep a stage's planes
+      // within a third of shared memory
+      mkb<4, 2, 8, 1, 2, 16, 96, 3>(), mkb<4, 2, 8, 1, 2, 16>(),
       SPP_INT_VARIANTS(4),
-      // bit-sliced 8-bit (eight plane rows per channel, 20-level counters):
-      // 1.6-2.8x the SIMD byte-lane kernels, so they come first for 8-bit data
+      // eight plane rows per channel, 20-level counters
       mkb<8, 2, 8, 1, 2, 16, 96, 2>(), mkb<8, 2, 8, 1, 2, 16, 0, 2>(), mkb<8, 1, 8, 1, 2, 16>(),
-      mkb<8, 1, 8, 1, 3, 16>(),
       SPP_INT_VARIANTS(8),
       mk<8, 4, 1, 4, 16, 3, 0>(1),
       // float32 input, compensated fp32
@@ -165,14 +140,16 @@ static const std::vector<Variant>& variants() {
       mk<32, 16, 2, 1, 16, 2, SPP_ACC_KAHAN32>(0),
       // float32 input, fp64 accumulator (channel-ordered sums: the reference's).
       // The argument is the shape's measured rate with the SMs full, relative to
-      // the first (1024 channels, 256 trials to DM 500, 57444 outputs: 2.95 ms;
+      // the first (1024 channels, 256 trials to DM 500, 57444 outputs: 2.98 ms;
       // 16 words x 4 trials, the choice before, 4.14 ms: three CTAs of four
-      // warps per SM leave the adders waiting on slab hand-overs); wide delay
-      // spreads fit only the small tiles
-      mk<32, 16, 8, 2, 16, 2, SPP_ACC_F64>(0, 1.0), mk<32, 16, 5, 3, 16, 2, SPP_ACC_F64>(0, 0.99),
-      mk<32, 8, 8, 2, 16, 2, SPP_ACC_F64>(0, 0.97), mk<32, 8, 4, 2, 16, 2, SPP_ACC_F64>(0, 0.85),
-      mk<32, 8, 4, 1, 16, 2, SPP_ACC_F64>(0, 0.94), mk<32, 16, 4, 1, 16, 2, SPP_ACC_F64>(0, 0.8),
-      mk<32, 16, 2, 1, 16, 2, SPP_ACC_F64>(0, 0.6), mk<32, 8, 2, 1, 16, 2, SPP_ACC_F64>(0, 0.75),
+      // warps per SM leave the adders waiting on slab hand-overs).  16 words per
+      // thread leave few registers for loads in flight: 8 trials x 2 warps of
+      // them took 2.9 to 4.1 ms from one build to the next and are not used.
+      // Wide delay spreads fit only the small tiles.
+      mk<32, 8, 8, 2, 16, 2, SPP_ACC_F64>(0, 1.0), mk<32, 16, 5, 3, 16, 2, SPP_ACC_F64>(0, 0.97),
+      mk<32, 8, 4, 1, 16, 2, SPP_ACC_F64>(0, 0.95), mk<32, 8, 4, 2, 16, 2, SPP_ACC_F64>(0, 0.9),
+      mk<32, 16, 4, 1, 16, 2, SPP_ACC_F64>(0, 0.8), mk<32, 16, 2, 1, 16, 2, SPP_ACC_F64>(0, 0.6),
+      mk<32, 8, 2, 1, 16, 2, SPP_ACC_F64>(0, 0.75),
       mk<32, 4, 1, 4, 32, 2, SPP_ACC_F64>(1),
       mk<32, 2, 1, 4, 32, 2, SPP_ACC_F64>(1),
   };
@@ -194,9 +171,6 @@ static int slot_words(const Variant& v, int32_t span) {
 }
 
 static int64_t smem_bytes(const Variant& v, int slot_w) {
-  if (v.pairs)
-    return v.STAGES * pair_stage_bytes(v.SLAB, slot_w, v.DW) + 8 + 2 * v.STAGES * 8 +
-           pair_hi_bytes(v.R, v.DW * v.TW);
   if (v.planes) return v.STAGES * bits_stage_bytes(v.nb, v.SLAB, slot_w, v.DW) + 8 + 2 * v.STAGES * 8;
   return v.STAGES * dmt_stage_bytes(v.SLAB, slot_w, v.DW) + 8 + 2 * v.STAGES * 8;
 }
@@ -618,19 +592,26 @@ struct spp_dmt_plan {
   std::vector<int> cands;      // candidate variant indices
   std::vector<int32_t> spans;  // span per candidate
   int cur = 0;                 // index into cands
-  // channel pairs (2-bit): rows (pair k, relative offset r) and each DM's row
-  // per pair; empty when the table has too many distinct offsets
-  int64_t nprows = 0;
-  int2* d_pair_src = nullptr;      // device, nprows x (k, r)
-  std::vector<int32_t> pair_rows;  // host, ndm x nchans/2
-  std::vector<int32_t> delays_h;   // host copy of the table while pair kernels are offered
-  // per candidate (nullptr until a pair kernel is first selected): staging tables
-  std::vector<int2*> pair_off, pair_ent;
+  // interleaved bit-plane kernels: rows of channels and of channel pairs, and
+  // per kernel shape the staging tables (sized at creation, built when first
+  // selected)
+  IlvRows ilv_rows[2];
+  std::vector<IlvTables> ilv_tabs;
   // optional per-kernel timing: events (start, after corner turn, end) per execute
   bool timing = false;
   std::vector<cudaEvent_t> evpool;
   size_t evused = 0;
 };
+
+// Candidate codes at or above this name an interleaved bit-plane shape.
+constexpr int kIlvCode = 1 << 20;
+static int ilv_index(const spp_dmt_plan* p, int cand) {
+  return p->cands[cand] >= kIlvCode ? p->cands[cand] - kIlvCode : -1;
+}
+static int plan_sign(const spp_dmt_plan* p) { return p->mode == SPP_MODE_ROLL ? -1 : 1; }
+static IlvDelays ilv_delays(const spp_dmt_plan* p) {
+  return IlvDelays{p->d_delays, p->ndm, p->nchans, plan_sign(p)};
+}
 
 static cudaEvent_t plan_event(spp_dmt_plan* p) {
   if (p->evused == p->evpool.size()) {
@@ -641,116 +622,129 @@ static cudaEvent_t plan_event(spp_dmt_plan* p) {
   return p->evpool[p->evused++];
 }
 
-static int plan_sign(const spp_dmt_plan* p) { return p->mode == SPP_MODE_ROLL ? -1 : 1; }
-
 static int64_t plan_nvalid(const spp_dmt_plan* p, int64_t nsamps) {
   return p->mode == SPP_MODE_ROLL ? nsamps : nsamps - p->maxabs;
 }
 
-// Staging tables of a pair kernel with DW trials per tile, SLAB pairs per
-// slab and slot_w words per staged row.  Per (tile, slab): the DW x SLAB
-// decoded offsets (staged row x 3 x slot_w + word, bit shift) and the
-// 2 x SLAB staged rows (pair-sum row, window start word relative to the time
-// tile; -1: unused).  The window of pair k starts at the 4-word boundary at
-// or below the tile's smallest offset of channel 2k; tiles are multiples of
-// 128 samples, so the same tables serve every time tile.
-static int pair_tables(spp_dmt_plan* p, const int32_t* delays_host, int dw, int slab, int slot_w,
-                       int2** d_off, int2** d_ent) {
-  const int64_t np = p->nchans / 2, ndm = p->ndm;
-  const int64_t ntile = ceil_div(ndm, dw), nslab = ceil_div(np, slab);
-  const int sign = plan_sign(p);
-  const int64_t halo = round_up(std::max<int64_t>(0, -(int64_t)p->omin), 128);
-  std::vector<int2> off((size_t)(ntile * nslab * dw * slab), make_int2(0, 0));
-  std::vector<int2> ent((size_t)(ntile * nslab * 2 * slab), make_int2(-1, 0));
-  for (int64_t t = 0; t < ntile; ++t) {
-    for (int64_t k = 0; k < nslab; ++k) {
-      const int64_t blk = t * nslab + k;
-      int e = 0;
-      for (int64_t j = 0; j < slab && k * slab + j < np; ++j) {
-        const int64_t pr = k * slab + j;
-        int32_t dv[64], rv[64], u[3];
-        int nu = 0;
-        int32_t mn = INT32_MAX;
-        for (int i = 0; i < dw; ++i) {
-          const int64_t dm = std::min<int64_t>(t * dw + i, ndm - 1);
-          dv[i] = sign * delays_host[dm * p->nchans + 2 * pr];
-          rv[i] = p->pair_rows[dm * np + pr];
-          mn = std::min(mn, dv[i]);
-          bool seen = false;
-          for (int m = 0; m < nu; ++m) seen = seen || u[m] == rv[i];
-          if (!seen) {
-            if (nu == 3) return fail(SPP_ERR_UNSUPPORTED, "pair %lld: more than 3 rows in a tile", (long long)pr);
-            u[nu++] = rv[i];
-          }
-        }
-        if (e + nu > 2 * slab) return fail(SPP_ERR_UNSUPPORTED, "pair slab needs more than %d rows", 2 * slab);
-        std::sort(u, u + nu);
-        const int64_t wsrel = ((mn + halo) / 32) & ~int64_t(3);  // mn + halo >= 0
-        const int64_t base = wsrel * 32 - halo;
-        for (int m = 0; m < nu; ++m) ent[blk * 2 * slab + e + m] = make_int2(u[m], (int)wsrel);
-        for (int i = 0; i < dw; ++i) {
-          int m = 0;
-          while (u[m] != rv[i]) ++m;
-          const int64_t o = dv[i] - base;
-          off[(blk * dw + i) * slab + j] =
-              make_int2((int)((e + m) * 3 * slot_w + (o >> 5)), (int)(o & 31));
-        }
-        e += nu;
+// Staging tables of candidate i, built the first time it is selected (plan
+// creation for the initial choice, else set_variant).
+static int ensure_tables(spp_dmt_plan* p, int i) {
+  const int iv = ilv_index(p, i);
+  if (iv < 0) return SPP_OK;
+  const IlvCfg& c = ilv_cfgs()[iv];
+  return ilv_build_tables(c, ilv_delays(p), p->ilv_rows[c.G - 1], &p->ilv_tabs[iv]);
+}
+
+static void free_device(spp_dmt_plan* p) {
+  for (IlvTables& t : p->ilv_tabs) ilv_free_tables(&t);
+  if (p->d_delays) cudaFree(p->d_delays);
+  p->d_delays = nullptr;
+}
+
+// Pair rows a plan may hold, per channel.
+constexpr int64_t kPairRowsPerChan = 12;
+
+// Interleaved bit-plane shapes this table and sample width can use.  `words`:
+// plan-owned device words after the delay table.
+static int add_ilv_candidates(spp_dmt_plan* p, int32_t* words) {
+  const auto& cfgs = ilv_cfgs();
+  p->ilv_tabs.resize(cfgs.size());
+  const IlvDelays d = ilv_delays(p);
+  const int64_t max_rows = kPairRowsPerChan * p->nchans;
+  IlvArena ar{words + 2 * p->nchans + 2 * max_rows + 64, words};
+  std::vector<int> which;
+  for (int i = 0; i < (int)cfgs.size(); ++i) {
+    const IlvCfg& c = cfgs[i];
+    if (c.nb != p->nbits || p->nchans % c.G) continue;
+    if (p->nchans * ((1ll << c.nb) - 1) >= (1ll << c.levels)) continue;
+    for (int G = 1; G <= c.G; ++G) {
+      IlvRows& r = p->ilv_rows[G - 1];
+      if (r.G != 0) continue;
+      const int rc = ilv_make_rows(d, G, max_rows, &ar, &r);
+      r.G = G;
+      if (rc == SPP_ERR_UNSUPPORTED) continue;  // no rows: shapes of this grouping are skipped
+      if (rc) return rc;
+    }
+    if (p->ilv_rows[0].nrows == 0 || p->ilv_rows[c.G - 1].nrows == 0) continue;
+    which.push_back(i);
+  }
+  if (which.empty()) return SPP_OK;
+  const int rc = ilv_size_tables(which, d, p->ilv_rows, &ar, &p->ilv_tabs);
+  if (rc) return rc;
+  for (int i : which) {
+    if (p->ilv_tabs[i].stages == 0) continue;
+    p->cands.push_back(kIlvCode + i);
+    p->spans.push_back(0);
+  }
+  return SPP_OK;
+}
+
+// The shape a plan starts from (without autotuning): the least estimated time
+// at nsamps_max.  An interleaved shape takes, per wave of 148 CTAs, a fixed
+// part (start, first copies, stores) and a part per group of channels, both
+// measured per shape (IlvCfg::us_wave, ns_group: within 4 % of 20 measured
+// geometries of 256-4096 channels and 64-1024 trials), plus 0.3 us per MB of
+// what its rows hold beyond the block itself.  The kernels over 32 consecutive
+// samples per word run at the rates below (channel-adds per us on fine trial
+// grids); coarse grids and short blocks cost them half as much again and a
+// launch (8-bit, 1024 channels, 64 trials to DM 600, 40289 outputs: 0.56 ms
+// against 0.40 ms interleaved; 2-bit, 100 trials to DM 1500, 35724 outputs:
+// 0.18 against 0.22 ms).  Rows above kIlvDefaultBytes leave a shape to explicit
+// choice: they grow with the block and the delay range.
+// 2-bit grids so fine that a pair row serves 100 trials or more start from
+// pairs at every block length, so that the blocks of one observation run one
+// kernel (4096 channels, 1024 trials to DM 2000: 45.9 ms against 52.6 ms
+// without pairs at 1016174 outputs, 3.5 against 3.7 ms at 65536, 1.3 against
+// 1.0 ms at 16384).
+static int first_choice(const spp_dmt_plan* p) {
+  constexpr int64_t kIlvDefaultBytes = 16ll << 30;
+  const int64_t nvalid = std::max<int64_t>(1, plan_nvalid(p, p->nsamps_max));
+  if (p->nbits == 32) {
+    // float64 sums: waves of the CTAs an SM holds (shared memory, 64 warps)
+    // times a tile's adds over its rate, which falls below 12 adding warps per SM
+    int pick = 0;
+    double best = 0.0;
+    for (int i = 0; i < (int)p->cands.size(); ++i) {
+      const Variant& v = variants()[p->cands[i]];
+      if (v.rate <= 0.0) continue;
+      const int64_t smem = smem_bytes(v, slot_words(v, p->spans[i])) + 1024;
+      const int64_t per_sm = std::min<int64_t>((228 << 10) / smem, 64 / (v.DW * v.TW + 1));
+      const int64_t ctas = ceil_div(p->ndm, v.DW) * ceil_div(nvalid, tile_T(v));
+      const double full = std::min(1.0, (double)(per_sm * v.DW * v.TW) / 12.0);
+      const double t =
+          (double)(ceil_div(ctas, 148 * per_sm) * per_sm * v.DW * tile_T(v)) / (v.rate * full);
+      if (best == 0.0 || t < best) {
+        best = t;
+        pick = i;
       }
     }
+    return pick;
   }
-  cudaError_t err = cudaMalloc(d_off, sizeof(int2) * off.size());
-  if (err == cudaSuccess) err = cudaMalloc(d_ent, sizeof(int2) * ent.size());
-  if (err == cudaSuccess)
-    err = cudaMemcpy(*d_off, off.data(), sizeof(int2) * off.size(), cudaMemcpyHostToDevice);
-  if (err == cudaSuccess)
-    err = cudaMemcpy(*d_ent, ent.data(), sizeof(int2) * ent.size(), cudaMemcpyHostToDevice);
-  if (err != cudaSuccess) {  // leave both unset so a later selection retries
-    if (*d_off) cudaFree(*d_off);
-    if (*d_ent) cudaFree(*d_ent);
-    *d_off = nullptr;
-    *d_ent = nullptr;
-  }
-  return cuda_status(err, "pair staging tables");
-}
-
-// Staging tables of candidate i, built the first time a pair kernel is
-// selected (plan creation for the initial choice, else set_variant).
-static int ensure_pair_tables(spp_dmt_plan* p, int i) {
-  const Variant& v = variants()[p->cands[i]];
-  if (!v.pairs || p->pair_off[i]) return SPP_OK;
-  return pair_tables(p, p->delays_h.data(), v.DW, v.SLAB, slot_words(v, p->spans[i]),
-                     &p->pair_off[i], &p->pair_ent[i]);
-}
-
-static void free_pair_tables(spp_dmt_plan* p) {
-  for (int2* q : p->pair_off) if (q) cudaFree(q);
-  for (int2* q : p->pair_ent) if (q) cudaFree(q);
-  p->pair_off.clear();
-  p->pair_ent.clear();
-  if (p->d_pair_src) cudaFree(p->d_pair_src);
-  p->d_pair_src = nullptr;
-}
-
-// The float32 shape a plan starts from (without autotuning).
-static int first_float_choice(const spp_dmt_plan* p) {
-  const int64_t nvalid = std::max<int64_t>(1, plan_nvalid(p, p->nsamps_max));
-  // float64 sums: waves of the CTAs an SM holds (shared memory, 64 warps)
-  // times a tile's adds over its rate, which falls below 12 adding warps per SM
+  const double adds_per_us = p->nbits == 1 ? 8.2e7 : p->nbits == 2 ? 5.0e7 : p->nbits == 4 ? 2.2e7 : 1.0e7;
+  double best = 1.5 * (double)p->ndm * nvalid * p->nchans / adds_per_us + 20.0;
+  const int64_t prows = p->ilv_rows[1].nrows;
+  const bool shared_pairs = p->nbits == 2 && prows > 0 && p->ndm * (p->nchans / 2) >= 100 * prows;
   int pick = 0;
-  double best = 0.0;
+  bool any = p->cands[0] < kIlvCode;  // candidate 0 is taken unless a better one follows
+  bool paired = false;
   for (int i = 0; i < (int)p->cands.size(); ++i) {
-    const Variant& v = variants()[p->cands[i]];
-    if (v.rate <= 0.0) continue;
-    const int64_t smem = smem_bytes(v, slot_words(v, p->spans[i])) + 1024;
-    const int64_t per_sm = std::min<int64_t>((228 << 10) / smem, 64 / (v.DW * v.TW + 1));
-    const int64_t ctas = ceil_div(p->ndm, v.DW) * ceil_div(nvalid, tile_T(v));
-    const double full = std::min(1.0, (double)(per_sm * v.DW * v.TW) / 12.0);
-    const double t =
-        (double)(ceil_div(ctas, 148 * per_sm) * per_sm * v.DW * tile_T(v)) / (v.rate * full);
-    if (best == 0.0 || t < best) {
+    const int iv = ilv_index(p, i);
+    if (iv < 0) continue;
+    const IlvCfg& c = ilv_cfgs()[iv];
+    const IlvRows& rows = p->ilv_rows[c.G - 1];
+    const IlvGeom g = ilv_geometry(c, p->ilv_rows[0], rows, p->nchans, nvalid);
+    if (g.chan_bytes + g.row_bytes > kIlvDefaultBytes && any) continue;
+    const int64_t ctas = ceil_div(p->ndm, c.DW) * ceil_div(g.M, c.words());
+    const double ng = (double)round_up(p->nchans / c.G, 4 * c.nq);
+    double t = (double)ceil_div(ctas, 148) * (c.us_wave + ng * c.ns_group * 1e-3);
+    t += (double)(g.chan_bytes - p->nchans * g.M * c.nb * 4 + g.row_bytes) * 3e-7;
+    const bool first_pair = shared_pairs && c.G == 2 && !paired;
+    if (shared_pairs && paired && c.G == 1) continue;
+    if (t < best || !any || first_pair) {
       best = t;
       pick = i;
+      any = true;
+      paired = paired || c.G == 2;
     }
   }
   return pick;
@@ -817,82 +811,9 @@ int spp_dmt_plan_create(spp_dmt_plan** plan, int nbits, int bitorder, int64_t nc
     span_of_dw.emplace_back(dw, span);
     return span;
   };
-  // Channel pairs (2-bit data): pair k = channels (2k, 2k+1) summed at the
-  // relative offset r = o(2k+1) - o(2k), one row per (k, r) over all DMs
-  // (at most 12 rows per channel, else the pair kernels are not offered).
-  std::vector<int2> pair_src;
-  if (nbits == 2) {
-    const int64_t np = nchans / 2;
-    std::vector<int32_t> rlo(np, INT32_MAX), rhi(np, INT32_MIN);
-    for (int64_t d = 0; d < ndm; ++d) {
-      const int32_t* row = delays_host + d * nchans;
-      for (int64_t k = 0; k < np; ++k) {
-        const int32_t r = sign * (row[2 * k + 1] - row[2 * k]);
-        rlo[k] = std::min(rlo[k], r);
-        rhi[k] = std::max(rhi[k], r);
-      }
-    }
-    std::vector<int64_t> rbase(np);
-    int64_t nrows = 0;
-    for (int64_t k = 0; k < np; ++k) {
-      rbase[k] = nrows;
-      nrows += (int64_t)rhi[k] - rlo[k] + 1;
-    }
-    if (nrows <= 12 * nchans) {
-      pair_src.resize(nrows);
-      for (int64_t k = 0; k < np; ++k)
-        for (int32_t r = rlo[k]; r <= rhi[k]; ++r)
-          pair_src[rbase[k] + (r - rlo[k])] = make_int2((int)k, r);
-      p->pair_rows.resize(ndm * np);
-      for (int64_t d = 0; d < ndm; ++d) {
-        const int32_t* row = delays_host + d * nchans;
-        for (int64_t k = 0; k < np; ++k) {
-          const int32_t r = sign * (row[2 * k + 1] - row[2 * k]);
-          p->pair_rows[d * np + k] = (int32_t)(rbase[k] + (r - rlo[k]));
-        }
-      }
-      p->nprows = nrows;
-    }
-  }
-  // a pair kernel's stage holds 2 x slab rows: in every DM tile each pair
-  // may use up to three distinct rows, and each slab's pairs together at
-  // most 2 x slab
-  std::vector<std::pair<int64_t, bool>> pairs_of_shape;
-  auto pairs_fit = [&](int dw, int slab) -> bool {
-    if (p->nprows == 0) return false;
-    const int64_t key = (int64_t)dw << 16 | slab;
-    for (auto& e : pairs_of_shape)
-      if (e.first == key) return e.second;
-    const int64_t np = nchans / 2;
-    bool fit = true;
-    for (int64_t d0 = 0; d0 < ndm && fit; d0 += dw) {
-      const int64_t d1 = std::min<int64_t>(ndm, d0 + dw);
-      int64_t used = 0;
-      for (int64_t k = 0; k < np && fit; ++k) {
-        int32_t u[3];
-        int n = 0;
-        for (int64_t d = d0; d < d1 && fit; ++d) {
-          const int32_t r = p->pair_rows[d * np + k];
-          bool seen = false;
-          for (int i = 0; i < n; ++i) seen = seen || u[i] == r;
-          if (seen) continue;
-          if (n == 3) fit = false;
-          else u[n++] = r;
-        }
-        used += n;
-        if ((k + 1) % slab == 0 || k + 1 == np) {
-          if (used > 2 * slab) fit = false;
-          used = 0;
-        }
-      }
-    }
-    pairs_of_shape.emplace_back(key, fit);
-    return fit;
-  };
   for (int i = 0; i < (int)vs.size(); ++i) {
     const Variant& v = vs[i];
     if (v.nb != nbits || (nbits == 32 && v.acc != acc)) continue;
-    if (v.pairs && !pairs_fit(v.DW, v.SLAB)) continue;
     if (ndm == 1 ? !v.single : v.single) continue;
     if (v.planes && nchans * ((1 << nbits) - 1) >= (1 << bit_levels(nbits))) continue;
     const int32_t span = tile_span(v.DW);
@@ -901,58 +822,24 @@ int spp_dmt_plan_create(spp_dmt_plan** plan, int nbits, int bitorder, int64_t nc
     p->cands.push_back(i);
     p->spans.push_back(span);
   }
-  if (p->cands.empty()) {
-    delete p;
-    return fail(SPP_ERR_UNSUPPORTED, "no kernel variant fits this delay table");
-  }
   p->dpitch = nchans;
-  cudaError_t e = cudaMalloc(&p->d_delays, sizeof(int32_t) * ndm * nchans);
+  const bool ilv = ndm > 1 && nbits <= 8;
+  const int64_t more = ilv ? ilv_plan_words(nchans, kPairRowsPerChan * nchans) : 0;
+  cudaError_t e = cudaMalloc(&p->d_delays, sizeof(int32_t) * (ndm * nchans + more));
   if (e != cudaSuccess) { delete p; return cuda_status(e, "plan cudaMalloc"); }
   e = cudaMemcpy(p->d_delays, delays_host, sizeof(int32_t) * ndm * nchans, cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) { cudaFree(p->d_delays); delete p; return cuda_status(e, "plan upload"); }
-  bool use_pairs = false;
-  for (int c : p->cands) use_pairs = use_pairs || vs[c].pairs;
-  p->pair_off.assign(p->cands.size(), nullptr);
-  p->pair_ent.assign(p->cands.size(), nullptr);
-  if (use_pairs) {
-    e = cudaMalloc(&p->d_pair_src, sizeof(int2) * pair_src.size());
-    if (e == cudaSuccess)
-      e = cudaMemcpy(p->d_pair_src, pair_src.data(), sizeof(int2) * pair_src.size(),
-                     cudaMemcpyHostToDevice);
-    const int rc = cuda_status(e, "plan pair rows");
-    if (rc != SPP_OK) {
-      free_pair_tables(p);
-      cudaFree(p->d_delays);
-      delete p;
-      return rc;
-    }
-    p->delays_h.assign(delays_host, delays_host + ndm * nchans);
-  } else {
-    p->pair_rows.clear();
-    p->pair_rows.shrink_to_fit();
+  int rc = cuda_status(e, "plan upload");
+  if (rc == SPP_OK && ilv) rc = add_ilv_candidates(p, p->d_delays + ndm * nchans);
+  if (rc == SPP_OK && p->cands.empty())
+    rc = fail(SPP_ERR_UNSUPPORTED, "no kernel variant fits this delay table");
+  if (rc == SPP_OK) {
+    p->cur = first_choice(p);
+    rc = ensure_tables(p, p->cur);
   }
-  // without autotuning, start from the first fixed-slot pair kernel when the
-  // table admits one (config 2: 17.1 ms against 22.1 ms for the first
-  // per-channel kernel at 2^18 outputs) and its pair rows at nsamps_max stay
-  // within kPairDefaultBytes (longer blocks keep the pair kernels for explicit
-  // choice only: their rows grow with the block)
-  constexpr int64_t kPairDefaultBytes = 16ll << 30;
-  for (size_t i = 0; i < p->cands.size(); ++i) {
-    const Variant& v = vs[p->cands[i]];
-    if (!v.pairs || v.slot <= 0) continue;
-    const int slot = slot_words(v, p->spans[i]);
-    const Geometry g = geometry(v, nchans, nsamps_max, plan_nvalid(p, nsamps_max), p->omin,
-                                p->omax, slot);
-    if (p->nprows * 3 * g.pitch_w * 4 <= kPairDefaultBytes) p->cur = (int)i;
-    break;
-  }
-  if (nbits == 32) p->cur = first_float_choice(p);
-  const int trc = ensure_pair_tables(p, p->cur);
-  if (trc != SPP_OK) {
-    free_pair_tables(p);
-    cudaFree(p->d_delays);
+  if (rc != SPP_OK) {
+    free_device(p);
     delete p;
-    return trc;
+    return rc;
   }
   *plan = p;
   return SPP_OK;
@@ -963,7 +850,8 @@ int spp_dmt_plan_destroy(spp_dmt_plan* p) {
   int rc = SPP_OK;
   for (cudaEvent_t e : p->evpool) cudaEventDestroy(e);
   if (p->d_delays) rc = cuda_status(cudaFree(p->d_delays), "plan cudaFree");
-  free_pair_tables(p);
+  p->d_delays = nullptr;
+  free_device(p);
   delete p;
   return rc;
 }
@@ -978,7 +866,7 @@ int spp_dmt_plan_num_variants(const spp_dmt_plan* p) { return p ? (int)p->cands.
 int spp_dmt_plan_set_variant(spp_dmt_plan* p, int variant) {
   if (!p) return fail(SPP_ERR_ARG, "null plan");
   if (variant < 0 || variant >= (int)p->cands.size()) return fail(SPP_ERR_ARG, "bad variant %d", variant);
-  const int rc = ensure_pair_tables(p, variant);
+  const int rc = ensure_tables(p, variant);
   if (rc != SPP_OK) return rc;
   p->cur = variant;
   return SPP_OK;
@@ -986,9 +874,19 @@ int spp_dmt_plan_set_variant(spp_dmt_plan* p, int variant) {
 
 int spp_dmt_plan_describe(const spp_dmt_plan* p, int32_t* cfg) {
   if (!p || !cfg) return fail(SPP_ERR_ARG, "null pointer");
+  const int iv = ilv_index(p, p->cur);
+  if (iv >= 0) {
+    const IlvCfg& c = ilv_cfgs()[iv];
+    const IlvTables& t = p->ilv_tabs[iv];
+    cfg[0] = c.nb | (1 << 8) | ((c.G == 2) << 9);
+    cfg[1] = c.P; cfg[2] = c.DW; cfg[3] = c.TW; cfg[4] = 4 * c.nq; cfg[5] = t.stages;
+    cfg[6] = 32 * c.words();
+    cfg[7] = (int32_t)t.smem;
+    return SPP_OK;
+  }
   const Variant& v = variants()[p->cands[p->cur]];
   const int slot = slot_words(v, p->spans[p->cur]);
-  cfg[0] = v.nb | (v.planes << 8) | (v.pairs << 9); cfg[1] = v.R; cfg[2] = v.DW; cfg[3] = v.TW; cfg[4] = v.SLAB;
+  cfg[0] = v.nb | (v.planes << 8); cfg[1] = v.R; cfg[2] = v.DW; cfg[3] = v.TW; cfg[4] = v.SLAB;
   cfg[5] = v.STAGES;
   cfg[6] = (int32_t)tile_T(v);
   cfg[7] = (int32_t)smem_bytes(v, slot);
@@ -1001,36 +899,74 @@ static Geometry plan_geometry(const spp_dmt_plan* p, int64_t nsamps, int* slot) 
   return geometry(v, p->nchans, nsamps, plan_nvalid(p, nsamps), p->omin, p->omax, *slot);
 }
 
-// pair-sum rows follow the channel rows in the workspace
-static int64_t pair_bytes(const spp_dmt_plan* p, const Geometry& g) {
-  return variants()[p->cands[p->cur]].pairs ? p->nprows * 3 * g.pitch_w * 4 : 0;
+static IlvGeom plan_ilv_geometry(const spp_dmt_plan* p, int iv, int64_t nsamps) {
+  const IlvCfg& c = ilv_cfgs()[iv];
+  return ilv_geometry(c, p->ilv_rows[0], p->ilv_rows[c.G - 1], p->nchans, plan_nvalid(p, nsamps));
 }
 
 int64_t spp_dmt_plan_workspace_bytes(const spp_dmt_plan* p, int64_t nsamps) {
   if (!p) return -1;
+  const int iv = ilv_index(p, p->cur);
+  if (iv >= 0) {
+    const IlvGeom g = plan_ilv_geometry(p, iv, nsamps);
+    return kStatusBytes + g.chan_bytes + g.row_bytes;
+  }
   int slot;
   Geometry g = plan_geometry(p, nsamps, &slot);
-  return kStatusBytes + g.bytes + pair_bytes(p, g);
+  return kStatusBytes + g.bytes;
+}
+
+// The transform by an interleaved bit-plane shape (arguments checked by dmt_run).
+static int ilv_run(const spp_dmt_plan* p, int iv, const void* in, int64_t nsamps, void* out,
+                   int64_t out_stride, int64_t out_start, uint8_t* ws, int64_t ws_bytes,
+                   cudaStream_t st) {
+  const int64_t nvalid = plan_nvalid(p, nsamps);
+  const IlvCfg& c = ilv_cfgs()[iv];
+  const IlvRows &chan = p->ilv_rows[0], &rows = p->ilv_rows[c.G - 1];
+  const IlvGeom g = plan_ilv_geometry(p, iv, nsamps);
+  const int64_t need = kStatusBytes + g.chan_bytes + g.row_bytes;
+  if (ws_bytes < need)
+    return fail(SPP_ERR_SIZE, "workspace %lld B < required %lld B", (long long)ws_bytes, (long long)need);
+  spp_dmt_plan* pm = const_cast<spp_dmt_plan*>(p);
+  cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
+  if (p->timing) {
+    for (int i = 0; i < 3; ++i) {
+      ev[i] = plan_event(pm);
+      if (!ev[i]) return fail(SPP_ERR_CUDA, "cudaEventCreate failed");
+    }
+    cudaEventRecord(ev[0], st);
+  }
+  uint8_t* data = ws + kStatusBytes;
+  int rc = ilv_corner_turn(c, chan, g, in, p->bitorder, p->nchans, nsamps, data, st);
+  if (!rc) rc = ilv_group_rows(c, chan, rows, g, p->nchans, data, st);
+  if (p->timing) cudaEventRecord(ev[1], st);
+  if (!rc)
+    rc = ilv_launch(c, p->ilv_tabs[iv], rows, g, p->nchans / c.G, p->ndm, data, out, p->out_kind,
+                    out_stride, out_start, nvalid, reinterpret_cast<uint32_t*>(ws), st);
+  if (p->timing) cudaEventRecord(ev[2], st);
+  return rc;
 }
 
 static int dmt_run(const spp_dmt_plan* p, const void* in, int64_t nsamps, void* out,
                    int64_t out_stride, int64_t out_start, uint8_t* ws, int64_t ws_bytes,
                    cudaStream_t st, const float* zd_bpass = nullptr,
                    const float* zd_chanwts = nullptr, double* zd_rows = nullptr) {
-  int slot;
-  Geometry g = plan_geometry(p, nsamps, &slot);
-  if (g.nvalid <= 0) return SPP_OK;
+  const int64_t nvalid = plan_nvalid(p, nsamps);
+  if (nvalid <= 0) return SPP_OK;
   if (p->mode == SPP_MODE_ROLL && p->maxabs >= nsamps)
     return fail(SPP_ERR_DELAY, "roll mode needs |delay| < nsamps");
   if (-(int64_t)p->omin > nsamps)
     return fail(SPP_ERR_DELAY, "negative offset %d reaches before the block", p->omin);
-  const int64_t pb = pair_bytes(p, g);
-  if (ws_bytes < kStatusBytes + g.bytes + pb)
-    return fail(SPP_ERR_SIZE, "workspace %lld B < required %lld B", (long long)ws_bytes,
-                (long long)(kStatusBytes + g.bytes + pb));
-  if (out_start < 0 || (p->ndm > 1 && out_stride < out_start + g.nvalid))
+  if (out_start < 0 || (p->ndm > 1 && out_stride < out_start + nvalid))
     return fail(SPP_ERR_SIZE, "out_stride %lld < out_start %lld + nvalid %lld",
-                (long long)out_stride, (long long)out_start, (long long)g.nvalid);
+                (long long)out_stride, (long long)out_start, (long long)nvalid);
+  const int iv = ilv_index(p, p->cur);
+  if (iv >= 0) return ilv_run(p, iv, in, nsamps, out, out_stride, out_start, ws, ws_bytes, st);
+  int slot;
+  Geometry g = plan_geometry(p, nsamps, &slot);
+  if (ws_bytes < kStatusBytes + g.bytes)
+    return fail(SPP_ERR_SIZE, "workspace %lld B < required %lld B", (long long)ws_bytes,
+                (long long)(kStatusBytes + g.bytes));
   if (g.ntiles_t > 65535)
     return fail(SPP_ERR_UNSUPPORTED, "%lld time tiles exceed the grid limit", (long long)g.ntiles_t);
   const Variant& v = variants()[p->cands[p->cur]];
@@ -1052,7 +988,7 @@ static int dmt_run(const spp_dmt_plan* p, const void* in, int64_t nsamps, void* 
     if (rc) return rc;
   }
   // float64 sums of float32 rows: the corner turn flags samples that are not
-  // normal floats (word kSpecialWord of the status block, cleared here)
+  // finite floats (word kSpecialWord of the status block, cleared here)
   uint32_t* special = nullptr;
   if (p->nbits == 32 && v.acc == SPP_ACC_F64) {
     special = reinterpret_cast<uint32_t*>(ws) + kSpecialWord;
@@ -1062,19 +998,6 @@ static int dmt_run(const spp_dmt_plan* p, const void* in, int64_t nsamps, void* 
   rc = launch_corner_turn(p->nbits, in, p->bitorder, p->nchans, nsamps, g, planar, st, zd_rows,
                           zd_chanwts, zd_bpass, special);
   if (rc) return rc;
-  if (v.pairs) {
-    // pair-sum rows from the channel planes: one row per (pair, offset)
-    uint32_t* pp = reinterpret_cast<uint32_t*>(ws + kStatusBytes + g.bytes);
-    const int64_t gy = ceil_div(g.pitch_w, 4 * 256);
-    if (gy > 65535 || p->nprows > INT32_MAX)
-      return fail(SPP_ERR_UNSUPPORTED, "pair rows: %lld words x %lld rows", (long long)g.pitch_w,
-                  (long long)p->nprows);
-    k_pair_sums2<<<dim3((unsigned)p->nprows, (unsigned)gy), 256, 0, st>>>(
-        static_cast<const uint32_t*>(planar), g.pitch_w, p->d_pair_src, pp);
-    rc = cuda_status(cudaGetLastError(), "pair sums launch");
-    if (rc) return rc;
-    planar = pp;
-  }
   if (p->timing) cudaEventRecord(ev[1], st);
   DmtArgs a{};
   a.planar = planar;
@@ -1096,9 +1019,6 @@ static int dmt_run(const spp_dmt_plan* p, const void* in, int64_t nsamps, void* 
   a.nvalid = g.nvalid;
   a.status = reinterpret_cast<uint32_t*>(ws);
   a.special = special;
-  a.pair_off = p->pair_off[p->cur];
-  a.pair_ent = p->pair_ent[p->cur];
-  a.npairs = (int32_t)(p->nchans / 2);
   rc = launch_dmt(v, a, g.ntiles_t, p->ndm, st);
   if (rc) return rc;
   if (p->timing) cudaEventRecord(ev[2], st);

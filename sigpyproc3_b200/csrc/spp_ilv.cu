@@ -1,0 +1,1032 @@
+// DM-time transform over interleaved bit planes (integer data, 1-8 bit).
+//
+// Layout.  An output row of nvalid samples is cut into 32 runs of M words:
+// bit i of word w stands for sample i * M + w.  A channel's row holds, for
+// every word w in [lo, lo + M + ext), the NB bit planes of samples
+// i * M + w (i = 0..31), plane words next to each other.  A trial that shifts
+// the channel by o samples then reads word w + o: the shift is an address
+// offset, so the bit-sliced adders take the loaded words as they are.  (With
+// 32 consecutive samples per word every plane word needs a funnel shift,
+// which runs at half the rate of the logic that adds it and takes a second
+// shared load for the neighbouring word.)  The price is that a row is longer
+// than M words by the range of the channel's delays over the trials (ext).
+//
+// Rows may hold sums of two channels (2k, 2k+1) at one relative offset r:
+// S[w] = x[2k][w] + x[2k+1][w + r], NB + 1 planes, shared by every trial whose
+// delays differ by r there.
+//
+// k_ilv: one CTA = DW trials x W words (32 W samples).  A producer warp copies,
+// per slab of 4 NQ groups, the distinct rows the tile's trials read (bulk
+// copies, mbarrier ring); where each trial reads inside them does not depend
+// on the word tile, so the plan tabulates it once.  Consumer warps (one trial,
+// 32 P words each) run the carry-save network of spp_dmt.cuh and write 32
+// samples per word as 32 coalesced stores.
+#include <algorithm>
+#include <climits>
+
+#include "spp_dmt.cuh"
+#include "spp_ilv.h"
+
+namespace spp {
+
+namespace {
+
+constexpr int kIlvMaxEnt = 32;   // staged rows per slab: one producer lane each
+constexpr int64_t kIlvMaxSmem = 227 * 1024;
+
+struct IlvArgs {
+  const uint32_t* rows;   // rows of NP-plane words
+  const uint32_t* zero;   // W zero words (NP planes), for absent groups
+  int64_t mp;             // words per row without its extra words
+  int64_t M;              // output words
+  const int32_t* off;
+  const int4* ent;
+  int32_t emax, nslab, stages, stage_bytes;
+  int32_t ndt, njt, db;   // trial tiles, word tiles, trial tiles per block of the CTA order
+  int32_t ndm;
+  void* out;
+  int32_t out_kind;
+  int64_t out_stride, out_start, nvalid;
+  uint32_t* status;
+};
+
+// Levels of the network: a quad of NP-plane rows leaves one carry of weight
+// 2^ilv_quad(NP) (4 x (2^NP - 1) < 2^(NP + 2); two levels for one plane).
+__host__ __device__ constexpr int ilv_quad(int np) { return np == 1 ? 2 : np + 2; }
+
+// Where a thread reads one row: its word's address, and for NP = 8 that of the
+// word's second 16 bytes.  Even plane counts use 8- or 16-byte loads; a warp's
+// 32 consecutive words are conflict-free for every NP (for NP = 8 the two
+// 16-byte halves of a word are swapped in every second group of four words,
+// which keeps eight lanes on distinct banks).  The words 32 apart that a thread
+// owns are reached by load immediates.
+template <int NP>
+struct IlvRow {
+  static constexpr int kStep = NP == 8 ? 4 : NP;  // planes fetched at a time
+  const unsigned char* p[NP == 8 ? 2 : 1];
+  __device__ __forceinline__ void set(const unsigned char* stage, uint32_t a) {
+    if constexpr (NP == 8) {
+      const uint32_t z = a ^ ((a >> 3) & 16u);
+      p[0] = stage + z;
+      p[1] = stage + (z ^ 16u);
+    } else {
+      p[0] = stage + a;
+    }
+  }
+  template <int H>
+  __device__ __forceinline__ void load(int imm, uint32_t (&x)[kStep]) const {
+    const unsigned char* q = p[H] + imm;
+    if constexpr (NP % 4 == 0) {
+      const uint4 v = *reinterpret_cast<const uint4*>(q);
+      x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+    } else if constexpr (NP % 2 == 0) {
+#pragma unroll
+      for (int b = 0; b < NP; b += 2) {
+        const uint2 v = *reinterpret_cast<const uint2*>(q + 4 * b);
+        x[b] = v.x; x[b + 1] = v.y;
+      }
+    } else {
+#pragma unroll
+      for (int b = 0; b < NP; ++b) x[b] = *reinterpret_cast<const uint32_t*>(q + 4 * b);
+    }
+  }
+};
+
+// Level B of a quad of rows: the four plane-B words and the carries of the
+// level below, added into A[B] in pairs (an odd one through a half adder).
+// Planes are fetched kStep at a time, when their first level is reached.
+template <int NP, int B, int NCIN>
+struct IlvLevel {
+  template <int LR>
+  __device__ __forceinline__ static void run(uint32_t (&A)[LR], const IlvRow<NP> (&r)[4], int imm,
+                                             uint32_t (&x)[4][IlvRow<NP>::kStep],
+                                             const uint32_t* cin, uint32_t& out) {
+    constexpr int KS = IlvRow<NP>::kStep;
+    if constexpr (B < NP && B % KS == 0) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) r[q].template load<B / KS>(imm, x[q]);
+    }
+    constexpr int NPL = B < NP ? 4 : 0;
+    constexpr int NIN = NPL + NCIN;
+    constexpr int NOUT = (NIN + 1) / 2;
+    uint32_t w[NIN], co[NOUT];
+#pragma unroll
+    for (int q = 0; q < NPL; ++q) w[q] = x[q][B % KS];
+#pragma unroll
+    for (int k = 0; k < NCIN; ++k) w[NPL + k] = cin[k];
+#pragma unroll
+    for (int k = 0; k < NIN / 2; ++k) csa(A[B], w[2 * k], w[2 * k + 1], co[k]);
+    if constexpr (NIN & 1) half(A[B], w[NIN - 1], co[NOUT - 1]);
+    if constexpr (NOUT == 1 && B + 1 >= NP) {
+      static_assert(B + 1 == ilv_quad(NP), "quad carry level");
+      out = co[0];
+    } else {
+      IlvLevel<NP, B + 1, NOUT>::run(A, r, imm, x, co, out);
+    }
+  }
+};
+
+// 16 x 16 bit transposes of both half-words at once: v[l] bit i -> v[i] bit l
+// (i < 16, and i - 16 in the upper half).
+__device__ __forceinline__ void transpose16x2(uint32_t (&v)[16]) {
+#pragma unroll
+  for (int s = 8; s >= 1; s >>= 1) {
+    const uint32_t m = s == 8 ? 0x00FF00FFu : s == 4 ? 0x0F0F0F0Fu : s == 2 ? 0x33333333u : 0x55555555u;
+#pragma unroll
+    for (int l = 0; l < 16; ++l) {
+      if (l & s) continue;
+      const uint32_t a = v[l], b = v[l + s];
+      v[l] = (a & m) | ((b & m) << s);
+      v[l + s] = ((a >> s) & m) | (b & ~m);
+    }
+  }
+}
+
+template <int NP, int P, int DW, int TW, int NQ, int L, int LR>
+__device__ __forceinline__ void ilv_body(const IlvArgs& a) {
+  constexpr int NWC = DW * TW;
+  constexpr int W = TW * 32 * P;
+  constexpr int LQ = ilv_quad(NP);
+  constexpr int LS = NQ == 1 ? 0 : NQ == 2 ? 1 : 2;  // folds within a slab
+  constexpr int LF = LQ + LS;                        // level of a slab's one carry
+  static_assert(LR <= L && LF + 2 <= LR, "register levels hold the folded carries");
+
+  extern __shared__ __align__(256) unsigned char smem[];
+  constexpr int nq4 = 4 * NQ;
+  int32_t* soff = reinterpret_cast<int32_t*>(smem + (int64_t)a.stages * a.stage_bytes);
+  uint32_t* shi = reinterpret_cast<uint32_t*>(soff + a.stages * DW * nq4);
+  uint64_t* full = reinterpret_cast<uint64_t*>(shi + (L - LR) * P * NWC * 32);
+  uint64_t* empty = full + a.stages;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // CTA order: blocks of db trial tiles sweep the word tiles together, so that
+  // the windows of neighbouring trials overlap in L2
+  const int blk = blockIdx.x / (a.db * a.njt);
+  const int rem = blockIdx.x - blk * a.db * a.njt;
+  const int dcnt = min(a.db, a.ndt - blk * a.db);
+  const int jt = rem / dcnt;
+  const int dt = blk * a.db + (rem - jt * dcnt);
+  const int64_t j0 = (int64_t)jt * W;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < a.stages; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], NWC);
+    }
+    fence_mbar_init();
+  }
+  __syncthreads();
+
+  if (warp == NWC) {
+    // producer: lane e copies row entry e of the slab
+    const int32_t* toff = a.off + (int64_t)dt * a.nslab * DW * nq4;
+    const int4* tent = a.ent + (int64_t)dt * a.nslab * a.emax;
+    int s = 0;
+    uint32_t ph = 1;  // parity of the phase before the first: passes at once
+    for (int k = 0; k < a.nslab; ++k) {
+      const int4 en = lane < a.emax ? __ldg(tent + (int64_t)k * a.emax + lane) : make_int4(-1, 0, 0, 0);
+      const uint32_t bytes = en.x == -1 ? 0u : (uint32_t)en.z * (NP * 4);
+      const uint32_t total = __reduce_add_sync(0xffffffffu, bytes);
+      if (k >= a.stages && !mbar_wait(&empty[s], ph, a.status)) break;
+      if (lane == 0) {
+        mbar_arrive_expect_tx(&full[s], total + (uint32_t)(DW * nq4 * 4));
+        bulk_g2s(soff + s * DW * nq4, toff + (int64_t)k * DW * nq4, DW * nq4 * 4, &full[s]);
+      }
+      __syncwarp();
+      if (bytes) {
+        const uint32_t* src = en.x < 0 ? a.zero : a.rows + ((int64_t)en.x * a.mp + en.y + j0) * NP;
+        bulk_g2s(smem + (int64_t)s * a.stage_bytes + (int64_t)en.w * 4, src, bytes, &full[s]);
+      }
+      if (++s == a.stages) { s = 0; ph ^= 1; }
+    }
+    return;
+  }
+
+  // consumers: warp (trial dmw, word group tw); thread words 32 p + lane
+  const int dmw = warp / TW, tw = warp % TW;
+  const int dm = dt * DW + dmw;
+  const int wl = tw * 32 * P + lane;
+  const uint32_t wb = (uint32_t)wl * (NP * 4);
+  const int ct = threadIdx.x;
+  auto hi = [&](int l, int p) -> uint32_t& { return shi[((l - LR) * P + p) * (NWC * 32) + ct]; };
+#pragma unroll
+  for (int l = LR; l < L; ++l)
+#pragma unroll
+    for (int p = 0; p < P; ++p) hi(l, p) = 0u;
+  uint32_t A[P][LR];
+#pragma unroll
+  for (int p = 0; p < P; ++p)
+#pragma unroll
+    for (int l = 0; l < LR; ++l) A[p][l] = 0u;
+  auto ripple = [&](int p, int l0, uint32_t c) {
+#pragma unroll
+    for (int l = 0; l < LR; ++l) {
+      if (l < l0) continue;
+      uint32_t nc;
+      half(A[p][l], c, nc);
+      c = nc;
+    }
+#pragma unroll
+    for (int l = LR; l < L; ++l) {
+      if (c == 0u) break;
+      uint32_t& h = hi(l, p);
+      const uint32_t nc = h & c;
+      h ^= c;
+      c = nc;
+    }
+  };
+  // quad carries are folded in pairs: log2(NQ) levels within a slab, two more
+  // over slabs, then one ripple per four slabs
+  uint32_t h0[P], h1[P];
+  bool ok = true;
+  int s = 0;
+  uint32_t ph = 0;
+  for (int k = 0; k < a.nslab; ++k) {
+    if (!mbar_wait(&full[s], ph, a.status)) { ok = false; break; }
+    const unsigned char* base = smem + s * a.stage_bytes;
+    const int4* off = reinterpret_cast<const int4*>(soff + (s * DW + dmw) * nq4);
+    int4 o[NQ];
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) o[i] = off[i];
+    uint32_t c0[P], c1[P];
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+      IlvRow<NP> r[4];
+      r[0].set(base, (uint32_t)o[i].x + wb);
+      r[1].set(base, (uint32_t)o[i].y + wb);
+      r[2].set(base, (uint32_t)o[i].z + wb);
+      r[3].set(base, (uint32_t)o[i].w + wb);
+#pragma unroll
+      for (int p = 0; p < P; ++p) {
+        uint32_t x[4][IlvRow<NP>::kStep], cq;
+        IlvLevel<NP, 0, 0>::run(A[p], r, p * 32 * NP * 4, x, nullptr, cq);
+        if (i % 2 == 0) {
+          c0[p] = cq;
+        } else {
+          csa(A[p][LQ], c0[p], cq, c0[p]);
+          if (i == 1) c1[p] = c0[p];
+          else if (i == 3) csa(A[p][LQ + 1], c1[p], c0[p], c0[p]);
+        }
+      }
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[s]);
+    if (++s == a.stages) { s = 0; ph ^= 1; }
+    if (!(k & 1)) {
+#pragma unroll
+      for (int p = 0; p < P; ++p) h0[p] = c0[p];
+    } else {
+#pragma unroll
+      for (int p = 0; p < P; ++p) csa(A[p][LF], h0[p], c0[p], c0[p]);
+      if (!(k & 2)) {
+#pragma unroll
+        for (int p = 0; p < P; ++p) h1[p] = c0[p];
+      } else {
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+          uint32_t c2;
+          csa(A[p][LF + 1], h1[p], c0[p], c2);
+          ripple(p, LF + 2, c2);
+        }
+      }
+    }
+  }
+  if (!ok || dm >= a.ndm) return;
+#pragma unroll
+  for (int p = 0; p < P; ++p) {
+    if (a.nslab & 1) ripple(p, LF, h0[p]);
+    if (a.nslab & 2) ripple(p, LF + 1, h1[p]);
+  }
+  // sample i * M + j of word j = bit i: 32 stores per word, each a warp's
+  // consecutive samples
+  const int64_t obase = (int64_t)dm * a.out_stride + a.out_start;
+#pragma unroll 1
+  for (int p = 0; p < P; ++p) {
+    const int64_t j = j0 + wl + 32 * p;
+    if (j >= a.M) break;
+    uint32_t v[16], up[L > 16 ? L - 16 : 1];
+#pragma unroll
+    for (int pp = 0; pp < P; ++pp) {  // register arrays need a static index
+      if (pp != p) continue;
+#pragma unroll
+      for (int l = 0; l < 16; ++l) v[l] = l < LR ? A[pp][l < LR ? l : 0] : l < L ? hi(l, pp) : 0u;
+#pragma unroll
+      for (int l = 16; l < L; ++l) up[l - 16] = l < LR ? A[pp][l < LR ? l : 0] : hi(l, pp);
+    }
+    transpose16x2(v);
+    // the first `cnt` of the word's 32 samples lie inside the row
+    const int cnt = j < a.nvalid ? (int)((a.nvalid - 1 - j) / a.M) + 1 : 0;
+    auto emit = [&](auto* dst, auto conv) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        uint32_t c = i < 16 ? (v[i & 15] & 0xFFFFu) : (v[i & 15] >> 16);
+#pragma unroll
+        for (int l = 16; l < L; ++l) c |= ((up[l - 16] >> i) & 1u) << l;
+        if (i < cnt) *dst = conv(c);
+        dst += a.M;
+      }
+    };
+    if (a.out_kind == SPP_OUT_I32)
+      emit(static_cast<int32_t*>(a.out) + obase + j, [](uint32_t c) { return (int32_t)c; });
+    else
+      emit(static_cast<float*>(a.out) + obase + j, [](uint32_t c) { return (float)c; });
+  }
+}
+
+template <int NP, int P, int DW, int TW, int NQ, int L, int LR, int MINB>
+__global__ void __launch_bounds__((DW * TW + 1) * 32, MINB)
+k_ilv(const IlvArgs a) {
+  ilv_body<NP, P, DW, TW, NQ, L, LR>(a);
+}
+
+// ---------------------------------------------------------------------------
+// Raw block -> channel rows.  A CTA owns 256 / NB channels (32 bytes of a raw
+// row) and walks tiles of 8 words w in [lo, lo + M): it loads the raw rows
+// i * M + w (whole 32-byte sectors, the next tile's loads in flight during this
+// one) and bit-transposes 32 rows x 32 bits per warp step, which gives the
+// words of i = 0..31 (block 0) and, where rows run past M words, of
+// i = 32..63 (block 1) and so on.  Word w + q M is block q / 32 and the next
+// one funnel-shifted by q mod 32, so every raw row is read and transposed once
+// however long the rows are.  Each channel's 8 words x NB planes leave as one
+// contiguous run.  Bound by the transposes (shuffles and logic) and the row
+// stores.
+// ---------------------------------------------------------------------------
+template <int NB>
+__global__ void __launch_bounds__(256)
+k_ilv_turn(const uint8_t* __restrict__ raw, int64_t nchans, int64_t nsamps, int bitorder,
+           int64_t M, int64_t mp, const int32_t* __restrict__ lo, const int32_t* __restrict__ ext,
+           uint32_t* __restrict__ rows) {
+  constexpr int CC = planes_ct_chans(NB);
+  constexpr int RT = 256;
+  constexpr int SBP = 36;
+  constexpr int OP = 8 * NB + 4;  // words per channel in s_out
+  __shared__ __align__(16) uint8_t s_raw[2][RT * SBP];
+  __shared__ __align__(16) uint32_t s_out[2][CC * OP];
+  __shared__ int s_rng[2];
+  const int64_t c0 = (int64_t)blockIdx.x * CC;
+  const int nc = (int)((nchans - c0) < CC ? (nchans - c0) : CC);
+  const int seg = (nc * NB + 7) / 8;
+  const int64_t rowbytes = nchans * NB / 8;
+  const int64_t segstart = c0 * NB / 8;
+  const bool vec16 = seg == 32 && (rowbytes & 15) == 0 && (reinterpret_cast<uintptr_t>(raw) & 15) == 0;
+  if (threadIdx.x == 0) { s_rng[0] = INT_MAX; s_rng[1] = INT_MIN; }
+  __syncthreads();
+  for (int c = threadIdx.x; c < nc; c += blockDim.x) {
+    const int l = lo[c0 + c];
+    atomicMin(&s_rng[0], l);
+    atomicMax(&s_rng[1], l + ext[c0 + c + 1] - ext[c0 + c]);
+  }
+  __syncthreads();
+  const int64_t wlo = s_rng[0];
+  const int64_t xw = s_rng[1] - wlo;  // words past M in the widest row of the group
+  const int64_t ntile = M / 8;
+  // each thread's two 16-byte output units: fixed channel, fixed place in the run
+  int64_t odst[2];
+  int64_t olo[2], ohi[2];
+  int osrc[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int idx = threadIdx.x + u * 256;
+    const int c = idx / (2 * NB), k = idx % (2 * NB);
+    osrc[u] = c * OP + 4 * k;
+    if (c < nc) {
+      olo[u] = lo[c0 + c];
+      ohi[u] = olo[u] + M + ext[c0 + c + 1] - ext[c0 + c];
+      odst[u] = ((c0 + c) * mp + ext[c0 + c] - olo[u]) * NB + 4 * k;
+    } else {
+      olo[u] = INT_MAX; ohi[u] = INT_MIN; odst[u] = 0;
+    }
+  }
+  const int lane = threadIdx.x & 31;
+  const int bi = lane >> 3, bb = lane & 7;
+  const int qc = (bitorder == SPP_BITORDER_BIG) ? (7 - bb) / NB : bb / NB;
+  const int lc = bi * (8 / NB) + qc, lb = bb % NB;  // channel within the byte group, plane
+  // tile row r = 32 w + i of block b holds raw row (32 b + i) * M + w; of block
+  // b only the first `ni` rows are wanted
+  auto fetch = [&](uint4 (&pre)[2], int64_t w0, int64_t b, int ni) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int idx = threadIdx.x + u * 256;
+      const int r = idx >> 1, k = idx & 1;
+      pre[u] = make_uint4(0u, 0u, 0u, 0u);
+      if ((r & 31) >= ni) continue;
+      const int64_t row = wrap_row((32 * b + (r & 31)) * M + w0 + (r >> 5), nsamps);
+      if (row >= 0) pre[u] = __ldg(reinterpret_cast<const uint4*>(raw + row * rowbytes + segstart) + k);
+    }
+  };
+  auto put = [&](const uint4 (&pre)[2], uint8_t* dst) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int idx = threadIdx.x + u * 256;
+      uint32_t* d = reinterpret_cast<uint32_t*>(dst + (idx >> 1) * SBP + 16 * (idx & 1));
+      d[0] = pre[u].x; d[1] = pre[u].y; d[2] = pre[u].z; d[3] = pre[u].w;
+    }
+  };
+  auto fill = [&](uint8_t* dst, int64_t w0, int64_t b, int ni) {  // any alignment
+    for (int idx = threadIdx.x; idx < RT * 32; idx += blockDim.x) {
+      const int r = idx >> 5, k = idx & 31;
+      uint8_t v = 0;
+      if (k < seg && (r & 31) < ni) {
+        const int64_t row = wrap_row((32 * b + (r & 31)) * M + w0 + (r >> 5), nsamps);
+        if (row >= 0) v = __ldg(raw + row * rowbytes + segstart + k);
+      }
+      dst[r * SBP + k] = v;
+    }
+  };
+  auto turn = [&](const uint8_t* src, uint32_t* dst) {  // warp = word, loop over 4-byte column groups
+    const int w = threadIdx.x >> 5;
+    // NB = 8: 16-byte halves swapped in every second group of four words
+    const int b = NB == 8 ? lb ^ (w & 4) : lb;
+#pragma unroll
+    for (int g = 0; g < 8; ++g) {
+      uint32_t x = *reinterpret_cast<const uint32_t*>(src + (w * 32 + lane) * SBP + 4 * g);
+      x = warp_transpose32(x, lane);
+      dst[(4 * g * (8 / NB) + lc) * OP + w * NB + b] = x;
+    }
+  };
+  // words past M of the tile at w0: q = 0..nq(w0), i.e. w0 + q M < wlo + M + xw
+  const int m32 = (int)M, x32 = (int)xw;
+  auto qmax = [&](int64_t w0) { return (m32 + x32 - 1 - (int)(w0 - wlo)) / m32; };
+  auto rows_of = [&](int q, int b) {  // rows of block b that q <= qmax reaches
+    return min(max(q - 32 * (b - 1), 0), 32);
+  };
+  uint4 pre0[2], pre1[2];
+  if (vec16 && blockIdx.y < ntile) {
+    const int64_t w0 = wlo + 8 * (int64_t)blockIdx.y;
+    fetch(pre0, w0, 0, 32);
+    fetch(pre1, w0, 1, rows_of(qmax(w0), 1));
+  }
+  for (int64_t tile = blockIdx.y; tile < ntile; tile += gridDim.y) {
+    const int64_t w0 = wlo + 8 * tile;
+    const int qm = qmax(w0);
+    if (vec16) {
+      put(pre0, s_raw[0]);
+      if (qm > 0) put(pre1, s_raw[1]);
+    } else {
+      fill(s_raw[0], w0, 0, 32);
+      if (qm > 0) fill(s_raw[1], w0, 1, rows_of(qm, 1));
+    }
+    __syncthreads();
+    if (vec16 && tile + gridDim.y < ntile) {
+      const int64_t w1 = w0 + 8 * (int64_t)gridDim.y;
+      fetch(pre0, w1, 0, 32);
+      fetch(pre1, w1, 1, rows_of(qmax(w1), 1));
+    }
+    turn(s_raw[0], s_out[0]);
+    if (qm > 0) turn(s_raw[1], s_out[1]);
+    __syncthreads();
+    for (int b = 0;; ++b) {
+      const uint32_t* sa = s_out[b & 1];
+      const uint32_t* sb = s_out[(b + 1) & 1];
+      const int q1 = min(qm, 32 * b + 31);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        if (olo[u] >= ohi[u]) continue;
+        const uint4 x = *reinterpret_cast<const uint4*>(sa + osrc[u]);
+        const uint4 y = *reinterpret_cast<const uint4*>(sb + osrc[u]);
+        for (int q = 32 * b; q <= q1; ++q) {
+          const int64_t w = w0 + q * M;
+          if (w < olo[u] || w >= ohi[u]) continue;
+          const int sh = q & 31;
+          uint4 v;
+          v.x = __funnelshift_r(x.x, y.x, sh);
+          v.y = __funnelshift_r(x.y, y.y, sh);
+          v.z = __funnelshift_r(x.z, y.z, sh);
+          v.w = __funnelshift_r(x.w, y.w, sh);
+          *reinterpret_cast<uint4*>(rows + odst[u] + w * NB) = v;
+        }
+      }
+      if (qm < 32 * (b + 1)) break;
+      // rows longer than 32 M words: the next block of 32 raw rows per word
+      __syncthreads();
+      fill(s_raw[0], w0, b + 2, rows_of(qm, b + 2));
+      __syncthreads();
+      turn(s_raw[0], s_out[b & 1]);
+      __syncthreads();
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Pair rows: S[w] = x[2k][w] + x[2k+1][w + r] (ripple add of NB planes into
+// NB + 1).  A CTA takes one pair and 512 words and makes all of the pair's rows
+// there: channel 2k's words stay in registers (two per thread), channel
+// 2k+1's window in shared memory, so the channel rows are read once per pair
+// and not once per row.  Each warp gathers its 64 words in shared memory to
+// store whole 16-byte units in order.  Bound by the row stores.
+// ---------------------------------------------------------------------------
+template <int NB>
+__device__ __forceinline__ void load_planes(const uint32_t* __restrict__ row, int64_t w, uint32_t (&x)[NB]) {
+  if constexpr (NB == 8) {
+    const uint4* p = reinterpret_cast<const uint4*>(row + w * 8);
+    const int h = (int)(w >> 2) & 1;
+    const uint4 a = __ldg(p + h), b = __ldg(p + (1 - h));
+    x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
+    x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+  } else if constexpr (NB == 4) {
+    const uint4 a = __ldg(reinterpret_cast<const uint4*>(row + w * 4));
+    x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
+  } else if constexpr (NB == 2) {
+    const uint2 a = __ldg(reinterpret_cast<const uint2*>(row + w * 2));
+    x[0] = a.x; x[1] = a.y;
+  } else {
+    x[0] = __ldg(row + w);
+  }
+}
+
+constexpr int kPairWords = 512;     // words per CTA: two per thread
+constexpr int kPairMaxOffsets = 512;  // distinct relative offsets of one pair, most
+template <int NB>
+__device__ __forceinline__ void load_planes_shared(const uint32_t* row, int w, uint32_t (&x)[NB]) {
+  if constexpr (NB == 8) {
+    const uint4* p = reinterpret_cast<const uint4*>(row + w * 8);
+    const int h = (w >> 2) & 1;
+    const uint4 a = p[h], b = p[1 - h];
+    x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
+    x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+  } else if constexpr (NB == 4) {
+    const uint4 a = *reinterpret_cast<const uint4*>(row + w * 4);
+    x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
+  } else if constexpr (NB == 2) {
+    const uint2 a = *reinterpret_cast<const uint2*>(row + w * 2);
+    x[0] = a.x; x[1] = a.y;
+  } else {
+    x[0] = row[w];
+  }
+}
+
+template <int NB>
+__global__ void __launch_bounds__(256)
+k_ilv_pairs(const uint32_t* __restrict__ chan, int64_t mpc, const int32_t* __restrict__ clo,
+            const int32_t* __restrict__ cext, int64_t M, const int32_t* __restrict__ rbase,
+            const int32_t* __restrict__ roff, int64_t mpr, const int32_t* __restrict__ rlo,
+            const int32_t* __restrict__ rext, uint32_t* __restrict__ rows) {
+  constexpr int NP = NB + 1;
+  extern __shared__ __align__(16) uint32_t sm[];
+  uint32_t* st = sm + (threadIdx.x >> 5) * 64 * NP;  // this warp's 64 words
+  uint32_t* sy = sm + kPairWords * NP;               // channel 2k+1's window
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int k = blockIdx.x, c = 2 * k;
+  const int e0 = rbase[k], e1 = rbase[k + 1];
+  const int r0 = roff[k];
+  const int64_t alo = clo[c], alen = M + cext[c + 1] - cext[c];
+  const int64_t blo = clo[c + 1], blen = M + cext[c + 2] - cext[c + 1];
+  // words [w0, w0 + 512) of channel 2k's grid; all offsets lie in its row
+  const int64_t w0 = alo + (int64_t)blockIdx.y * kPairWords;
+  if (w0 >= alo + alen) return;
+  const uint32_t* a = chan + ((int64_t)c * mpc + cext[c]) * NB;
+  const uint32_t* b = chan + ((int64_t)(c + 1) * mpc + cext[c + 1]) * NB;
+  // window of channel 2k+1: from the 8-word group holding w0 + r0
+  const int64_t y0 = (w0 + r0) & ~int64_t(7);
+  const int yn = (int)((w0 + kPairWords + r0 + (e1 - e0) - y0 + 7) & ~int64_t(7));
+  for (int u = threadIdx.x; u < yn * NB / 4; u += 256) {
+    const int64_t w = y0 - blo + u * 4 / NB;  // word of the unit's first value (in its row)
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (w >= 0 && w < blen) v = __ldg(reinterpret_cast<const uint4*>(b + (y0 - blo) * NB) + u);
+    reinterpret_cast<uint4*>(sy)[u] = v;
+  }
+  uint32_t x[2][NB];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int64_t w = w0 - alo + warp * 64 + 32 * i + lane;
+    if (w < alen) {
+      load_planes<NB>(a, w, x[i]);
+    } else {
+#pragma unroll
+      for (int q = 0; q < NB; ++q) x[i][q] = 0u;
+    }
+  }
+  __syncthreads();
+  const int64_t ww = w0 + warp * 64;  // this warp's first word
+  for (int e = e0; e < e1; ++e) {
+    const int64_t lo = rlo[e], hi = lo + M + rext[e + 1] - rext[e];
+    if (lo >= ww + 64 || hi <= ww) continue;
+    const int ys = (int)(ww + r0 + (e - e0) - y0);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      uint32_t y[NB], o[NP];
+      load_planes_shared<NB>(sy, ys + 32 * i + lane, y);
+      uint32_t cy = 0u;
+#pragma unroll
+      for (int q = 0; q < NB; ++q) {
+        o[q] = x[i][q] ^ y[q] ^ cy;
+        cy = (x[i][q] & y[q]) | (x[i][q] & cy) | (y[q] & cy);
+      }
+      o[NB] = cy;
+#pragma unroll
+      for (int q = 0; q < NP; ++q) st[(lane + 32 * i) * NP + q] = o[q];
+    }
+    __syncwarp();
+    // row bounds are multiples of 8 words = 2 NP units
+    uint4* dst = reinterpret_cast<uint4*>(rows + (e * mpr + rext[e] + ww - lo) * NP);
+    for (int u = lane; u < 16 * NP; u += 32) {
+      const int64_t w = ww + 8 * (u / (2 * NP));
+      if (w >= lo && w < hi) dst[u] = reinterpret_cast<const uint4*>(st)[u];
+    }
+    __syncwarp();
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Plan tables, from the delay table on the device.
+// ---------------------------------------------------------------------------
+// Smallest and largest signed offset of every channel; for pairs the same of
+// the relative offsets.  A CTA takes 32 groups, its eight warps the trials.
+__global__ void __launch_bounds__(256)
+k_ilv_ranges(IlvDelays d, int G, int2* __restrict__ out) {
+  __shared__ int2 red[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t g = (int64_t)blockIdx.x * 32 + lane;
+  int mn = INT_MAX, mx = INT_MIN;
+  if (g < d.nchans / G) {
+#pragma unroll 4
+    for (int64_t i = warp; i < d.ndm; i += 8) {
+      const int32_t* row = d.d_delays + i * d.nchans;
+      const int o = G == 1 ? d.sign * row[g] : d.sign * (row[2 * g + 1] - row[2 * g]);
+      mn = min(mn, o);
+      mx = max(mx, o);
+    }
+  }
+  red[warp][lane] = make_int2(mn, mx);
+  __syncthreads();
+  if (warp == 0 && g < d.nchans / G) {
+    for (int w = 1; w < 8; ++w) {
+      mn = min(mn, red[w][lane].x);
+      mx = max(mx, red[w][lane].y);
+    }
+    out[g] = make_int2(mn, mx);
+  }
+}
+
+__device__ __forceinline__ int ilv_row_of(const IlvDelays& d, int G, const int32_t* rbase,
+                                          const int32_t* rlo, int64_t dm, int64_t g, int* o) {
+  const int32_t* row = d.d_delays + dm * d.nchans;
+  if (G == 1) {
+    *o = d.sign * row[g];
+    return (int)g;
+  }
+  *o = d.sign * row[2 * g];
+  return rbase[g] + (d.sign * row[2 * g + 1] - *o) - rlo[g];
+}
+
+// Offset range of every pair row over the trials that read it.
+__global__ void k_ilv_row_ranges(IlvDelays d, const int32_t* __restrict__ rbase,
+                                 const int32_t* __restrict__ rlo, int32_t* __restrict__ mn,
+                                 int32_t* __restrict__ mx) {
+  const int64_t np = d.nchans / 2;
+  const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= np) return;
+  for (int64_t dm = blockIdx.y; dm < d.ndm; dm += gridDim.y) {
+    int o;
+    const int r = ilv_row_of(d, 2, rbase, rlo, dm, g, &o);
+    atomicMin(mn + r, o);
+    atomicMax(mx + r, o);
+  }
+}
+
+// Staging tables: one thread per (trial tile, slab).  Without `off` only the
+// largest entry count and stage size are taken (stats[0], stats[1] in words).
+__global__ void k_ilv_tables(IlvDelays d, int G, int np, int DW, int W, int nq, int emax,
+                             int64_t ntile, int64_t nslab, const int32_t* __restrict__ lo,
+                             const int32_t* __restrict__ ext, const int32_t* __restrict__ rbase,
+                             const int32_t* __restrict__ rlo, int32_t* __restrict__ off,
+                             int4* __restrict__ ent, int* __restrict__ stats) {
+  const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (id >= ntile * nslab) return;
+  const int64_t tile = id / nslab, k = id - tile * nslab;
+  const int64_t ng = d.nchans / G;
+  int pos = 0, e = 0, zpos = -1;
+  for (int j = 0; j < 4 * nq; ++j) {
+    const int64_t g = k * 4 * nq + j;
+    if (g >= ng) {
+      if (zpos < 0) {
+        zpos = pos;
+        if (ent && e < emax) ent[id * emax + e] = make_int4(-2, 0, W, pos);
+        ++e;
+        pos += W * np;
+      }
+      if (off) for (int i = 0; i < DW; ++i) off[(id * DW + i) * 4 * nq + j] = zpos * 4;
+      continue;
+    }
+    int o[16], rr[16];
+    uint32_t left = 0;
+    for (int i = 0; i < DW; ++i) {
+      const int64_t dm = min(tile * DW + i, d.ndm - 1);
+      rr[i] = ilv_row_of(d, G, rbase, rlo, dm, g, &o[i]);
+      left |= 1u << i;
+    }
+    while (left) {
+      const int f = __ffs(left) - 1;
+      const int r = rr[f];
+      uint32_t same = 0;
+      int mn = INT_MAX, mx = INT_MIN;
+      for (int i = f; i < DW; ++i) {
+        if (rr[i] != r) continue;
+        same |= 1u << i;
+        mn = min(mn, o[i]);
+        mx = max(mx, o[i]);
+      }
+      left &= ~same;
+      const int start = (mn - lo[r]) & ~7;  // words from the row's first, 8-word groups
+      const int len = (W + (mx - lo[r] - start) + 7) & ~7;
+      if (ent && e < emax) ent[id * emax + e] = make_int4(r, ext[r] + start, len, pos);
+      if (off)
+        for (int i = f; i < DW; ++i)
+          if (same >> i & 1) off[(id * DW + i) * 4 * nq + j] = (pos + (o[i] - lo[r] - start) * np) * 4;
+      ++e;
+      // a spread no stage can hold: stop before the sum overflows
+      pos = min(pos, 1 << 28) + min(len, 1 << 20) * np;
+    }
+  }
+  if (ent)
+    for (; e < emax; ++e) ent[id * emax + e] = make_int4(-1, 0, 0, 0);
+  if (stats) {
+    atomicMax(&stats[0], e);
+    atomicMax(&stats[1], pos);
+  }
+}
+
+template <int NB, int G, int P, int DW, int TW, int NQ, int LR, int MINB>
+IlvCfg mki(double us_wave, double ns_group) {
+  constexpr int NP = NB + (G == 2 ? 1 : 0);
+  constexpr int L = NB == 8 ? 20 : NB == 4 ? 16 : 14;
+  static_assert(DW <= 16, "trials per tile");
+  static_assert((L - LR) * P * DW * TW * 32 * 4 % 8 == 0, "barriers follow the upper levels");
+  IlvCfg c{};
+  c.nb = NB; c.G = G; c.np = NP; c.P = P; c.DW = DW; c.TW = TW; c.nq = NQ;
+  c.levels = L;
+  c.threads = (DW * TW + 1) * 32;
+  c.hi_bytes = (int64_t)(L - LR) * P * DW * TW * 32 * 4;
+  c.us_wave = us_wave;
+  c.ns_group = ns_group;
+  c.fn = reinterpret_cast<const void*>(&k_ilv<NP, P, DW, TW, NQ, L, LR, MINB>);
+  return c;
+}
+
+}  // namespace
+
+const std::vector<IlvCfg>& ilv_cfgs() {
+  static const std::vector<IlvCfg> v = {
+      // <NB, G, P, DW, TW, NQ, register levels, CTAs per SM>(us per wave, ns per group).
+      // One CTA per SM of 15 or 18 trial-warps (16 or 20 warps allocated: 128 or
+      // 96 registers each): two thirds of the registers hold the counters, and
+      // fewer, larger slabs of groups matter more than warps (2-bit pairs, 2^18 x
+      // 1024 trials: slabs of 4 groups 14.4 ms, of 8 11.0 ms).  3 x 5 warps:
+      // coarse trial grids, whose tiles of more trials would not fit the stages.
+      mki<1, 1, 4, 11, 2, 4, 10, 1>(32, 97), mki<1, 1, 4, 9, 2, 4, 14, 1>(29, 86),
+      mki<1, 1, 4, 15, 1, 4, 14, 1>(19, 81), mki<1, 1, 4, 3, 5, 4, 14, 1>(22, 83),
+      mki<1, 1, 4, 3, 5, 2, 14, 1>(22, 95),
+      mki<2, 2, 4, 9, 2, 2, 14, 1>(44, 195), mki<2, 2, 4, 15, 1, 2, 14, 1>(72, 148),
+      mki<2, 2, 4, 7, 2, 2, 14, 1>(26, 164),
+      mki<2, 1, 4, 15, 1, 4, 14, 1>(30, 101), mki<2, 1, 4, 9, 2, 4, 14, 1>(33, 141),
+      mki<2, 1, 4, 3, 5, 4, 14, 1>(21, 103), mki<2, 1, 4, 3, 5, 2, 14, 1>(21, 115),
+      mki<4, 2, 3, 7, 2, 2, 16, 1>(18, 174), mki<4, 2, 4, 9, 2, 1, 13, 1>(40, 312),
+      mki<4, 2, 4, 15, 1, 1, 16, 1>(38, 254),
+      mki<4, 1, 4, 15, 1, 2, 16, 1>(37, 174), mki<4, 1, 4, 7, 2, 2, 16, 1>(29, 181),
+      mki<4, 1, 4, 3, 5, 2, 16, 1>(27, 184), mki<4, 1, 4, 3, 5, 1, 16, 1>(27, 200),
+      mki<8, 2, 3, 7, 2, 1, 20, 1>(22, 307), mki<8, 2, 2, 9, 2, 1, 20, 1>(22, 273),
+      mki<8, 2, 2, 3, 5, 1, 20, 1>(17, 247),
+      mki<8, 1, 4, 15, 1, 1, 16, 1>(20, 363), mki<8, 1, 3, 7, 2, 2, 16, 1>(23, 258),
+      mki<8, 1, 3, 15, 1, 1, 20, 1>(15, 279), mki<8, 1, 3, 3, 5, 1, 20, 1>(22, 284),
+  };
+  return v;
+}
+
+void ilv_free_tables(IlvTables* t) {
+  cudaFree(t->d_off);
+  t->d_off = nullptr;
+  t->d_ent = nullptr;
+}
+
+// Device words a plan keeps beside its delay table: the rows of both
+// groupings, and scratch for the range passes and table sizes.
+int64_t ilv_plan_words(int64_t nchans, int64_t max_rows) {
+  return 2 * (nchans + 1) + 2 * (max_rows + 1) + (nchans + 2) + 2 * nchans + 2 * max_rows + 64;
+}
+
+int ilv_make_rows(const IlvDelays& d, int G, int64_t max_rows, IlvArena* ar, IlvRows* out) {
+  const int64_t ng = d.nchans / G;
+  if (d.nchans % G || ng <= 0) return SPP_ERR_UNSUPPORTED;
+  IlvRows r{};
+  r.G = G;
+  int32_t* scratch = ar->scratch;
+  int rc = SPP_OK;
+  auto up = [&](void* dst, const void* s, int64_t words) {
+    if (!rc) rc = cuda_status(cudaMemcpy(dst, s, 4 * words, cudaMemcpyHostToDevice), "row table upload");
+  };
+  auto down = [&](void* dst, const void* s, int64_t words) {
+    if (!rc) rc = cuda_status(cudaMemcpy(dst, s, 4 * words, cudaMemcpyDeviceToHost), "row ranges");
+  };
+  std::vector<int2> rng(ng);
+  k_ilv_ranges<<<(unsigned)ceil_div(ng, 32), 256>>>(d, G, reinterpret_cast<int2*>(scratch));
+  down(rng.data(), scratch, 2 * ng);
+  if (rc) return rc;
+  std::vector<int32_t> mn, mx;
+  if (G == 1) {
+    r.nrows = ng;
+    mn.resize(ng); mx.resize(ng);
+    for (int64_t i = 0; i < ng; ++i) { mn[i] = rng[i].x; mx[i] = rng[i].y; }
+  } else {
+    std::vector<int32_t> head(2 * ng + 1);  // first row of each pair (and the end), smallest offset
+    int64_t n = 0;
+    for (int64_t k = 0; k < ng; ++k) {
+      head[k] = (int32_t)n;
+      head[ng + 1 + k] = rng[k].x;
+      const int64_t cnt = (int64_t)rng[k].y - rng[k].x + 1;
+      n += cnt;
+      if (n > max_rows || cnt > kPairMaxOffsets) return SPP_ERR_UNSUPPORTED;
+      r.max_offsets = std::max(r.max_offsets, (int)cnt);
+    }
+    head[ng] = (int32_t)n;
+    r.nrows = n;
+    r.d_rbase = ar->take(2 * ng + 1);
+    r.d_rlo = r.d_rbase + ng + 1;
+    up(r.d_rbase, head.data(), 2 * ng + 1);
+    mn.assign(2 * n, INT_MAX);
+    std::fill(mn.begin() + n, mn.end(), INT_MIN);
+    up(scratch, mn.data(), 2 * n);
+    if (rc) return rc;
+    k_ilv_row_ranges<<<dim3((unsigned)ceil_div(ng, 128), (unsigned)std::min<int64_t>(d.ndm, 64)), 128>>>(
+        d, r.d_rbase, r.d_rlo, scratch, scratch + n);
+    down(mn.data(), scratch, 2 * n);
+    if (rc) return rc;
+    mx.assign(mn.begin() + n, mn.end());
+  }
+  std::vector<int32_t> tab(2 * r.nrows + 1);  // first word of each row, then prefix sums of the extra words
+  int32_t* lo = tab.data();
+  int32_t* ext = tab.data() + r.nrows;
+  int64_t total = 0;
+  for (int64_t i = 0; i < r.nrows; ++i) {
+    ext[i] = (int32_t)total;
+    if (mn[i] > mx[i]) {  // an offset between two used ones that no trial has: never made
+      lo[i] = 1 << 30;
+      continue;
+    }
+    lo[i] = mn[i] & ~7;
+    const int64_t w = round_up((int64_t)mx[i] - lo[i] + 1, 8);
+    total += w;
+    r.max_ext = std::max(r.max_ext, w);
+    if (total > (1 << 30)) return SPP_ERR_UNSUPPORTED;
+  }
+  ext[r.nrows] = (int32_t)total;
+  r.ext_total = total;
+  r.d_lo = ar->take(2 * r.nrows + 1);
+  r.d_ext = r.d_lo + r.nrows;
+  up(r.d_lo, tab.data(), 2 * r.nrows + 1);
+  if (rc) return rc;
+  *out = r;
+  return SPP_OK;
+}
+
+static int table_pass(const IlvCfg& c, const IlvDelays& d, const IlvRows& r, int emax, int32_t* off,
+                      int4* ent, int* stats) {
+  const int64_t ntile = ceil_div(d.ndm, c.DW), nslab = ceil_div(d.nchans / c.G, 4 * c.nq);
+  k_ilv_tables<<<(unsigned)ceil_div(ntile * nslab, 64), 64>>>(d, c.G, c.np, c.DW, c.words(), c.nq, emax, ntile,
+                                                             nslab, r.d_lo, r.d_ext, r.d_rbase,
+                                                             r.d_rlo, off, ent, stats);
+  return cuda_status(cudaGetLastError(), "staging tables");
+}
+
+int ilv_size_tables(const std::vector<int>& which, const IlvDelays& d, const IlvRows* rows,
+                    IlvArena* ar, std::vector<IlvTables>* tabs) {
+  const int n = (int)which.size();
+  std::vector<int> st(2 * n + 1, 0);
+  int rc = cuda_status(cudaMemset(ar->scratch, 0, sizeof(int) * 2 * n), "stats clear");
+  for (int i = 0; i < n && !rc; ++i) {
+    const IlvCfg& c = ilv_cfgs()[which[i]];
+    rc = table_pass(c, d, rows[c.G - 1], kIlvMaxEnt, nullptr, nullptr, ar->scratch + 2 * i);
+  }
+  if (!rc) rc = cuda_status(cudaMemcpy(st.data(), ar->scratch, sizeof(int) * 2 * n, cudaMemcpyDeviceToHost), "stats");
+  if (rc) return rc;
+  for (int i = 0; i < n; ++i) {
+    const IlvCfg& c = ilv_cfgs()[which[i]];
+    IlvTables& t = (*tabs)[which[i]];
+    t.stages = 0;  // does not fit
+    if (st[2 * i] > kIlvMaxEnt || st[2 * i + 1] >= 1 << 18) continue;
+    const int64_t stage = round_up((int64_t)st[2 * i + 1] * 4, 256);
+    const int64_t per = stage + (int64_t)c.DW * 4 * c.nq * 4 + 16;
+    const int64_t avail = kIlvMaxSmem - c.hi_bytes - 16;
+    const int64_t stages = std::min<int64_t>(4, avail / per);
+    if (stages < 2) continue;
+    t.emax = st[2 * i];
+    t.stage_bytes = stage;
+    t.stages = (int)stages;
+    t.smem = stages * per + c.hi_bytes + 16;
+  }
+  return SPP_OK;
+}
+
+int ilv_build_tables(const IlvCfg& c, const IlvDelays& d, const IlvRows& r, IlvTables* t) {
+  if (t->d_off) return SPP_OK;
+  const int64_t n = ceil_div(d.ndm, c.DW) * ceil_div(d.nchans / c.G, 4 * c.nq);
+  const int64_t off_bytes = round_up(n * c.DW * 4 * c.nq * 4, 256);
+  void* p = nullptr;
+  int rc = cuda_status(cudaMalloc(&p, (size_t)(off_bytes + n * t->emax * (int64_t)sizeof(int4))), "plan table alloc");
+  if (rc) return rc;
+  t->d_off = static_cast<int32_t*>(p);
+  t->d_ent = reinterpret_cast<int4*>(static_cast<uint8_t*>(p) + off_bytes);
+  rc = table_pass(c, d, r, t->emax, t->d_off, t->d_ent, nullptr);
+  if (!rc) rc = cuda_status(cudaStreamSynchronize(nullptr), "staging tables");
+  if (rc) ilv_free_tables(t);
+  return rc;
+}
+
+IlvGeom ilv_geometry(const IlvCfg& c, const IlvRows& chan, const IlvRows& rows, int64_t nchans,
+                     int64_t nvalid) {
+  IlvGeom g{};
+  g.M = round_up(ceil_div(std::max<int64_t>(nvalid, 1), 32), 8);
+  g.mp = ceil_div(g.M, c.words()) * c.words() + 8;
+  const int64_t zero = (int64_t)c.words() * c.np * 4;
+  g.chan_bytes = round_up((nchans * g.mp + chan.ext_total) * c.nb * 4 + (c.G == 1 ? zero : 0), 256);
+  g.row_bytes = c.G == 1 ? 0 : round_up((rows.nrows * g.mp + rows.ext_total) * c.np * 4 + zero, 256);
+  return g;
+}
+
+int ilv_corner_turn(const IlvCfg& c, const IlvRows& chan, const IlvGeom& g, const void* in,
+                    int bitorder, int64_t nchans, int64_t nsamps, void* ws, cudaStream_t st) {
+  const int64_t nblk = ceil_div(nchans, planes_ct_chans(c.nb));
+  dim3 grid((unsigned)nblk, (unsigned)std::min<int64_t>(std::max<int64_t>(1, ceil_div(148 * 8 * 4, nblk)),
+                                                        ceil_div(g.M, 8)));
+  const uint8_t* raw = static_cast<const uint8_t*>(in);
+  uint32_t* rows = static_cast<uint32_t*>(ws);
+  switch (c.nb) {
+    case 1: k_ilv_turn<1><<<grid, 256, 0, st>>>(raw, nchans, nsamps, bitorder, g.M, g.mp, chan.d_lo, chan.d_ext, rows); break;
+    case 2: k_ilv_turn<2><<<grid, 256, 0, st>>>(raw, nchans, nsamps, bitorder, g.M, g.mp, chan.d_lo, chan.d_ext, rows); break;
+    case 4: k_ilv_turn<4><<<grid, 256, 0, st>>>(raw, nchans, nsamps, bitorder, g.M, g.mp, chan.d_lo, chan.d_ext, rows); break;
+    default: k_ilv_turn<8><<<grid, 256, 0, st>>>(raw, nchans, nsamps, bitorder, g.M, g.mp, chan.d_lo, chan.d_ext, rows); break;
+  }
+  return cuda_status(cudaGetLastError(), "interleaved corner turn launch");
+}
+
+int ilv_group_rows(const IlvCfg& c, const IlvRows& chan, const IlvRows& rows, const IlvGeom& g,
+                   int64_t nchans, void* ws, cudaStream_t st) {
+  if (c.G == 1) return SPP_OK;
+  const uint32_t* ch = static_cast<const uint32_t*>(ws);
+  uint32_t* out = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(ws) + g.chan_bytes);
+  const int64_t gy = ceil_div(g.M + chan.max_ext, kPairWords), ng = nchans / 2;
+  if (gy > 65535) return fail(SPP_ERR_UNSUPPORTED, "pair rows of %lld words", (long long)g.M);
+  dim3 grid((unsigned)ng, (unsigned)gy);
+  const int64_t smem = (int64_t)kPairWords * c.np * 4 + (int64_t)(kPairWords + rows.max_offsets + 16) * c.nb * 4;
+  int rc = SPP_OK;
+#define SPP_ILV_PAIRS(NB)                                                                          \
+  if (smem > 48 * 1024) rc = set_smem_attr(reinterpret_cast<const void*>(&k_ilv_pairs<NB>), smem); \
+  if (rc) return rc;                                                                               \
+  k_ilv_pairs<NB><<<grid, 256, smem, st>>>(ch, g.mp, chan.d_lo, chan.d_ext, g.M, rows.d_rbase,     \
+                                           rows.d_rlo, g.mp, rows.d_lo, rows.d_ext, out)
+  switch (c.nb) {
+    case 1: SPP_ILV_PAIRS(1); break;
+    case 2: SPP_ILV_PAIRS(2); break;
+    case 4: SPP_ILV_PAIRS(4); break;
+    default: SPP_ILV_PAIRS(8); break;
+  }
+#undef SPP_ILV_PAIRS
+  return cuda_status(cudaGetLastError(), "pair rows launch");
+}
+
+int ilv_launch(const IlvCfg& c, const IlvTables& t, const IlvRows& rows, const IlvGeom& g,
+               int64_t ngroups, int64_t ndm, const void* ws, void* out, int out_kind,
+               int64_t out_stride, int64_t out_start, int64_t nvalid, uint32_t* status,
+               cudaStream_t st) {
+  const uint8_t* base = static_cast<const uint8_t*>(ws) + (c.G == 1 ? 0 : g.chan_bytes);
+  const int64_t nwords = rows.nrows * g.mp + rows.ext_total;
+  IlvArgs a{};
+  a.rows = reinterpret_cast<const uint32_t*>(base);
+  a.zero = a.rows + nwords * c.np;
+  if (ngroups % (4 * c.nq)) {
+    const int rc = cuda_status(cudaMemsetAsync(const_cast<uint32_t*>(a.zero), 0,
+                                               (size_t)c.words() * c.np * 4, st), "zero row");
+    if (rc) return rc;
+  }
+  a.mp = g.mp;
+  a.M = g.M;
+  a.off = t.d_off;
+  a.ent = t.d_ent;
+  a.emax = t.emax;
+  a.stages = t.stages;
+  a.stage_bytes = (int32_t)t.stage_bytes;
+  a.nslab = (int32_t)ceil_div(ngroups, 4 * c.nq);
+  a.ndt = (int32_t)ceil_div(ndm, c.DW);
+  a.njt = (int32_t)ceil_div(g.M, c.words());
+  // 13 trial tiles per block: their windows of one row overlap, and the rows
+  // the blocks in flight read stay near L2's size (2-bit, 4096 channels, 1024
+  // trials, 2^20 samples: 46.0 ms; 2 per block 46.6, all 114: 46.9)
+  a.db = std::min(a.ndt, 13);
+  a.ndm = (int32_t)ndm;
+  a.out = out;
+  a.out_kind = out_kind;
+  a.out_stride = out_stride;
+  a.out_start = out_start;
+  a.nvalid = nvalid;
+  a.status = status;
+  if (t.smem > 48 * 1024) {
+    const int rc = set_smem_attr(c.fn, t.smem);
+    if (rc) return rc;
+  }
+  const int64_t grid = (int64_t)a.ndt * a.njt;
+  if (grid > INT32_MAX) return fail(SPP_ERR_UNSUPPORTED, "too many tiles");
+  void* args[] = {&a};
+  return cuda_status(cudaLaunchKernel(c.fn, dim3((unsigned)grid), dim3((unsigned)c.threads), args,
+                                      (size_t)t.smem, st), "interleaved DM-time launch");
+}
+
+}  // namespace spp

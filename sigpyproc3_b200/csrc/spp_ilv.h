@@ -1,0 +1,100 @@
+// Host interface of the interleaved bit-plane DM-time kernels (spp_ilv.cu),
+// used by the DM plans in spp_core.cu.
+#pragma once
+
+#include <vector>
+
+#include "spp_common.cuh"
+
+namespace spp {
+
+// One kernel shape: rows of `G` summed channels (NP bit planes), DW trials x
+// W words per CTA.
+struct IlvCfg {
+  int nb;       // sample width, bits
+  int G;        // channels summed per row
+  int np;       // bit planes per row
+  int P;        // words per thread
+  int DW, TW;   // trials per CTA, warps per trial
+  int nq;       // quads of groups per slab
+  int levels;   // counter levels
+  int threads;
+  int64_t hi_bytes;  // counter levels kept in shared memory
+  const void* fn;
+  double us_wave, ns_group;  // measured time of one wave of CTAs: us_wave + groups x ns_group
+  int words() const { return TW * 32 * P; }  // words per CTA tile
+};
+const std::vector<IlvCfg>& ilv_cfgs();
+
+// Rows of one grouping (G channels) of a delay table: row e of group g covers
+// the words [lo, lo + words + ext) of its first channel's grid.
+struct IlvRows {
+  int G = 0;
+  int64_t nrows = 0;       // rows over all groups
+  int64_t ext_total = 0;   // words beyond the common row length, all rows
+  int64_t max_ext = 0;     // the same, widest row
+  int32_t* d_lo = nullptr;     // device, nrows: first word of the row (multiple of 8)
+  int32_t* d_ext = nullptr;    // device, nrows + 1: prefix sums of the extra words
+  int max_offsets = 0;         // G = 2: relative offsets of one pair, most
+  int32_t* d_rbase = nullptr;  // device, G = 2, pairs + 1: first row of each pair
+  int32_t* d_rlo = nullptr;    // device, G = 2: smallest relative offset of each pair
+};
+
+// Staging tables of one kernel shape for one delay table.
+struct IlvTables {
+  int emax = 0;          // staged rows per slab, most
+  int64_t stage_bytes = 0;
+  int stages = 0;
+  int64_t smem = 0;
+  int32_t* d_off = nullptr;  // (tile, slab, trial, group): byte offset in the stage (owns both)
+  int4* d_ent = nullptr;     // (tile, slab, entry): row, word offset, words, stage position
+};
+
+// A delay table on the device.
+struct IlvDelays {
+  const int32_t* d_delays;  // ndm x nchans
+  int64_t ndm, nchans;
+  int sign;
+};
+
+// Plan-owned device words (beside the delay table): rows are taken from it,
+// `scratch` serves the passes that make them.
+struct IlvArena {
+  int32_t* next = nullptr;
+  int32_t* scratch = nullptr;
+  int32_t* take(int64_t words) {
+    int32_t* p = next;
+    next += words;
+    return p;
+  }
+};
+int64_t ilv_plan_words(int64_t nchans, int64_t max_rows);
+
+void ilv_free_tables(IlvTables* t);
+// Rows of grouping G (1 or 2); more than `max_rows` pair rows:
+// SPP_ERR_UNSUPPORTED.
+int ilv_make_rows(const IlvDelays& d, int G, int64_t max_rows, IlvArena* ar, IlvRows* out);
+// Sizes the staging of the shapes `which` (stages = 0: the table's spreads do
+// not fit) from the rows of G = 1 and 2.
+int ilv_size_tables(const std::vector<int>& which, const IlvDelays& d, const IlvRows* rows,
+                    IlvArena* ar, std::vector<IlvTables>* tabs);
+int ilv_build_tables(const IlvCfg& c, const IlvDelays& d, const IlvRows& r, IlvTables* t);
+
+struct IlvGeom {
+  int64_t M;        // words per row that carry outputs (32 * M >= nvalid)
+  int64_t mp;       // words of a row without its extra words
+  int64_t chan_bytes, row_bytes;  // channel rows, pair rows (0 for G = 1)
+};
+IlvGeom ilv_geometry(const IlvCfg& c, const IlvRows& chan, const IlvRows& rows, int64_t nchans,
+                     int64_t nvalid);
+// Raw block -> channel rows (and pair rows) in `ws`.
+int ilv_corner_turn(const IlvCfg& c, const IlvRows& chan, const IlvGeom& g, const void* in,
+                    int bitorder, int64_t nchans, int64_t nsamps, void* ws, cudaStream_t st);
+int ilv_group_rows(const IlvCfg& c, const IlvRows& chan, const IlvRows& rows, const IlvGeom& g,
+                   int64_t nchans, void* ws, cudaStream_t st);
+int ilv_launch(const IlvCfg& c, const IlvTables& t, const IlvRows& rows, const IlvGeom& g,
+               int64_t ngroups, int64_t ndm, const void* ws, void* out, int out_kind,
+               int64_t out_stride, int64_t out_start, int64_t nvalid, uint32_t* status,
+               cudaStream_t st);
+
+}  // namespace spp

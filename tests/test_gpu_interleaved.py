@@ -1,0 +1,101 @@
+"""Interleaved bit-plane DM-time kernels (bit i of word w = sample i * M + w).
+
+Each case sits where the layout's arithmetic can go wrong: output lengths that
+leave the last of the 32 runs short or the last word tile partly filled, trial
+counts around a tile's, channel counts that do not fill a slab of groups (zero
+rows), odd channel counts (no pairs), delay ranges many times the block (rows
+of more than 32 runs), negative offsets and roll mode.  The sums are integers,
+so every variant must equal the oracle's restatement of kernels.dedisperse /
+kernels.dmt_block (src/sigpyproc/core/kernels.py:340-362, :1155-1168) exactly.
+"""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _pack(vals, nbits):
+    if nbits == 8:
+        return vals
+    per = 8 // nbits
+    v = vals.reshape(-1, per)
+    out = np.zeros(v.shape[0], dtype=np.uint8)
+    for k in range(per):
+        out |= (v[:, k] << ((8 - (k + 1) * nbits) if nbits > 1 else k)).astype(np.uint8)
+    return out
+
+
+def _run(orc, nbits, d, nchans, nsamps, mode="dedisperse", seed=0, ref_vals=None):
+    import torch
+
+    from sigpyproc3_b200.dedisp import DMTPlan
+
+    rng = np.random.default_rng(seed)
+    vals = rng.integers(0, 1 << nbits, size=nsamps * nchans, dtype=np.uint8)
+    vals[: nsamps * nchans // 3] = (1 << nbits) - 1  # saturated stretch: the top counter levels
+    if mode == "roll":
+        expect = orc.dmt_roll(vals.astype(np.float32), d, nchans, nsamps).astype(np.int64)
+    else:
+        expect = orc.dmt(vals, d, nchans, nsamps).astype(np.int64)
+    raw = torch.from_numpy(_pack(vals, nbits)).cuda()
+    seen = 0
+    for dtype in (torch.int32, torch.float32):
+        plan = DMTPlan(d, nchans, nsamps, nbits=nbits, bitorder="little" if nbits == 1 else "big",
+                       mode=mode, out_dtype=dtype)
+        for v in range(plan.num_variants):
+            plan.set_variant(v)
+            desc = plan.describe()
+            if desc["R"] * 32 * desc["TW"] * 32 != desc["T"] or not desc["bit_sliced"]:
+                continue
+            seen += 1
+            out = plan.execute(raw, nsamps, check=True).cpu().numpy()
+            np.testing.assert_array_equal(out.astype(np.int64), expect, err_msg=str(desc))
+        plan.close()
+    return seen
+
+
+def _delays(nchans, dm, ndm, fch1=1500.0, bw=300.0, ref="fch1"):
+    from sigpyproc3_b200.header import Header
+
+    h = Header(nchans=nchans, fch1=fch1, foff=-bw / nchans, tsamp=64e-6)
+    return np.atleast_2d(h.get_dmdelays(np.linspace(0.0, dm, ndm), ref)).astype(np.int32)
+
+
+@pytest.mark.parametrize("nbits", [1, 2, 4, 8])
+@pytest.mark.parametrize("nvalid,ndm", [(1, 2), (31 * 256 + 5, 16), (32 * 256, 15), (32 * 264 + 1, 19)])
+def test_tile_edges(orc, nbits, nvalid, ndm):
+    """Last run short, one full word tile, one word past it; trials 16 = one
+    past a 15-trial tile, 19 = one past two of nine."""
+    nchans = 64
+    d = _delays(nchans, 12.0, ndm)
+    assert _run(orc, nbits, d, nchans, nvalid + int(d.max()), seed=nvalid) >= 4
+
+
+@pytest.mark.parametrize("nbits,nchans", [(1, 8), (1, 24), (2, 36), (4, 38), (8, 7), (8, 21), (8, 34)])
+def test_partial_slabs(orc, nbits, nchans):
+    """Groups that do not fill the last slab read the zero row."""
+    d = _delays(nchans, 15.0, 12)
+    assert _run(orc, nbits, d, nchans, 3000 + int(d.max()), seed=nchans) >= 4
+
+
+@pytest.mark.parametrize("nbits", [1, 2, 4, 8])
+def test_rows_longer_than_32_runs(orc, nbits):
+    """300 outputs behind delays of 12000 samples: a row is 1500 words of which
+    16 carry outputs, so its words span dozens of 32-run blocks."""
+    nchans = 16
+    d = _delays(nchans, 800.0, 400)
+    assert int(d.max()) > 11000
+    assert _run(orc, nbits, d, nchans, 300 + int(d.max()), seed=5) >= 2
+
+
+@pytest.mark.parametrize("nbits", [2, 8])
+def test_negative_offsets_and_roll(orc, nbits):
+    """Delays about the band centre (rows start before sample 0 and wrap) and
+    circular rolls (offsets are -delay)."""
+    nchans, ndm = 40, 13
+    d = _delays(nchans, 25.0, ndm, ref="fcenter")
+    assert d.min() < 0 < d.max()
+    assert _run(orc, nbits, d, nchans, 5000, seed=1) >= 4
+    d = _delays(nchans, 25.0, ndm)
+    assert _run(orc, nbits, d, nchans, 4096, mode="roll", seed=2) >= 4
