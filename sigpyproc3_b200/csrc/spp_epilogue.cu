@@ -428,7 +428,7 @@ __global__ void k_snr_final(int64_t n, const SnrCfg cfg, int64_t nrows, int64_t 
   }
   double sd = cnt > 0 ? sqrt(m2 / cnt) : 0.0;
   if (sd == 0.0) sd = 1.0;
-  if (locscale) {  // median / IQR scale computed by k_row_quantiles
+  if (locscale) {  // median / IQR scale
     mean = locscale[rf * 2];
     sd = locscale[rf * 2 + 1];
   }
@@ -447,18 +447,26 @@ __global__ void k_snr_final(int64_t n, const SnrCfg cfg, int64_t nrows, int64_t 
 // ---------------------------------------------------------------------------
 // Median / IQR of each downsampled row (the S/N epilogue's robust z-score:
 // stats.estimate_zscore with loc "median" and scale "iqr", core/stats.py:
-// 418-502).  One CTA per (row, factor): the y values (the same float32
-// downsampled means as k_snr_chunk) are mapped to order-preserving 32-bit keys
-// and the needed order statistics are found exactly by radix selection, three
-// passes of 11/11/10-bit digits with one shared-memory histogram per distinct
-// key prefix (warp-aggregated increments).  Up to six ranks: the two middle
-// values (median) and the two neighbours of each quartile's index (q25, q75,
-// linear interpolation as numpy's percentile).
+// 418-502).  The y values (the same float32 downsampled means as k_snr_chunk)
+// are mapped to order-preserving 32-bit keys and the needed order statistics
+// are found exactly by radix selection.  Up to six ranks: the two middle values
+// (median) and the two neighbours of each quartile's index (q25, q75, linear
+// interpolation as numpy's percentile).
+//
+// A first pass finds the smallest and largest key, so that the 2048 bins of the
+// first histogram span the values present (rows of sums share their upper key
+// bits: bins by those bits would hold everything at once); two more passes of
+// up to 2048 bins per distinct prefix finish any 32-bit range, and passes stop
+// once a bin is one key wide.  Rows are split over gridDim.x CTAs whose
+// histograms are added in global memory, and the last CTA of a row to finish a
+// pass selects: one CTA per row took 2.1 ms for a single row of 262144 samples.
 // ---------------------------------------------------------------------------
-constexpr int kQThreads = 256;
+constexpr int kQThreads = 256;      // row MAD
 constexpr int kQBits = 11;
 constexpr int kQBins = 1 << kQBits;
 constexpr int kQRanks = 6;
+constexpr int kQPassThreads = 512;
+constexpr int kQSplitRows = 148;    // fewer rows than this are split over CTAs
 
 __device__ __forceinline__ uint32_t f32_key(float v) {
   const uint32_t b = __float_as_uint(v);
@@ -482,109 +490,222 @@ __device__ __forceinline__ double quantile_lerp(double a, double b, double g) {
   return g >= 0.5 ? b - diff * (1.0 - g) : a + diff * g;
 }
 
-__global__ void __launch_bounds__(kQThreads)
-k_row_quantiles(const void* __restrict__ in, int kind, int64_t n, int64_t in_stride,
-                const SnrCfg cfg, double* __restrict__ locscale) {
-  extern __shared__ uint32_t qhist[];  // kQRanks x kQBins
-  __shared__ uint32_t pre[kQRanks];    // key prefix per rank (bits above the digit)
-  __shared__ int64_t rnk[kQRanks];     // rank within the prefix
-  __shared__ uint32_t dpre[kQRanks];   // distinct prefixes this pass
-  __shared__ int slot[kQRanks];        // rank -> distinct-prefix histogram
-  __shared__ int ndist;
-  const int64_t row = blockIdx.x / cfg.nf;
-  const int fi = blockIdx.x % cfg.nf;
-  const int f = cfg.f[fi];
-  const int64_t m = n / f;
-  const char* base = static_cast<const char*>(in) + row * in_stride * 4;
+// State of one row's selection between passes.
+struct QState {
+  uint32_t kmin_inv, kmax;  // ~smallest key, largest key (both start at 0: atomicMax)
+  uint32_t shift;           // key bits below the bins chosen so far
+  uint32_t ndist;
+  uint32_t dpre[kQRanks];   // distinct bins (their smallest keys)
+  uint32_t slot[kQRanks];   // rank -> distinct bin
+  uint32_t left[kQRanks];   // rank within the bin
+  uint32_t ctr[4];          // CTAs done, per pass
+};
+
+struct QArgs {
+  const void* in;
+  int kind;
+  int64_t n, in_stride;
+  QState* st;
+  uint32_t* hist;  // per row: kQRanks x kQBins, zeroed per call (split rows only)
+  double* locscale;
+};
+
+// The row block's values, one per thread and step: f(key) for each.
+template <class F>
+__device__ __forceinline__ void q_each(const QArgs& a, const SnrCfg& cfg, F&& fn) {
+  const int64_t row = blockIdx.y / cfg.nf;
+  const int f = cfg.f[blockIdx.y % cfg.nf];
+  const int64_t m = a.n / f;
+  const char* base = static_cast<const char*>(a.in) + row * a.in_stride * 4;
   const bool pow2 = (f & (f - 1)) == 0;
   const double inv = 1.0 / (double)f;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // ranks: median pair, then q25 and q75 neighbours (0-based, in [0, m))
-  const double v25 = (double)(m - 1) * 0.25, v75 = (double)(m - 1) * 0.75;
-  const int64_t l25 = (int64_t)floor(v25), l75 = (int64_t)floor(v75);
-  if (threadIdx.x == 0) {
-    const int64_t r[kQRanks] = {(m - 1) / 2, m / 2, l25, l25 + 1 < m ? l25 + 1 : m - 1,
-                                l75, l75 + 1 < m ? l75 + 1 : m - 1};
-    for (int t = 0; t < kQRanks; ++t) { pre[t] = 0u; rnk[t] = r[t]; }
+  const int64_t per = (m + gridDim.x - 1) / gridDim.x;
+  const int64_t i1 = imin64(m, per * (blockIdx.x + 1));
+#pragma unroll 4
+  for (int64_t i = per * blockIdx.x + threadIdx.x; i < i1; i += blockDim.x)
+    fn(f32_key(f == 1 ? (float)row_val(base, a.kind, i) : snr_y(base, a.kind, i, f, pow2, inv)));
+}
+
+__device__ __forceinline__ void q_range(const QArgs& a, const SnrCfg& cfg, QState& st) {
+  uint32_t lo = 0xFFFFFFFFu, hi = 0u;
+  q_each(a, cfg, [&](uint32_t k) {
+    lo = min(lo, k);
+    hi = max(hi, k);
+  });
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if ((threadIdx.x & 31) == 0 && lo <= hi) {
+    atomicMax(&st.kmin_inv, ~lo);
+    atomicMax(&st.kmax, hi);
+  }
+}
+
+// One pass: histogram of the next key bits of the values in the chosen bins,
+// then (the row's last CTA) each rank's bin.
+template <int PASS>
+__device__ __forceinline__ void q_pass(const QArgs& a, const SnrCfg& cfg, QState& st) {
+  extern __shared__ uint32_t qhist[];  // (PASS == 0 ? 1 : kQRanks) x kQBins
+  __shared__ uint32_t dpre[kQRanks], pick[kQRanks], left[kQRanks];
+  __shared__ bool last;
+  const int f = cfg.f[blockIdx.y % cfg.nf];
+  const int64_t m = a.n / f;
+  const uint32_t kmin = ~st.kmin_inv;
+  const int old = PASS == 0 ? 32 - __clz(st.kmax - kmin) : (int)st.shift;  // bits still open
+  if (PASS > 0 && old == 0) return;                                       // selected already
+  const int sh = old > kQBits ? old - kQBits : 0;
+  const int nd = PASS == 0 ? 1 : (int)st.ndist;
+  if (threadIdx.x < kQRanks) dpre[threadIdx.x] = PASS == 0 ? kmin : st.dpre[threadIdx.x];
+  for (int i = threadIdx.x; i < nd * kQBins; i += blockDim.x) qhist[i] = 0u;
+  __syncthreads();
+  if (PASS == 0) {
+    q_each(a, cfg, [&](uint32_t k) { atomicAdd(&qhist[(k - kmin) >> sh], 1u); });
+  } else {
+    const uint32_t span = 1u << old;  // old <= 21
+    q_each(a, cfg, [&](uint32_t k) {
+      for (int d = 0; d < nd; ++d) {
+        const uint32_t r = k - dpre[d];
+        if (r < span) atomicAdd(&qhist[d * kQBins + (r >> sh)], 1u);
+      }
+    });
   }
   __syncthreads();
-  const int shifts[3] = {21, 10, 0};
-  const int widths[3] = {11, 11, 10};
-  for (int pass = 0; pass < 3; ++pass) {
-    const int sh = shifts[pass], wb = widths[pass];
-    const uint32_t hi_mask = (sh + wb >= 32) ? 0u : ~((1u << (sh + wb)) - 1u);
-    const uint32_t dmask = (1u << wb) - 1u;
-    if (threadIdx.x == 0) {
-      int nd = 0;
-      for (int t = 0; t < kQRanks; ++t) {
-        int k = 0;
-        while (k < nd && dpre[k] != pre[t]) ++k;
-        if (k == nd) dpre[nd++] = pre[t];
-        slot[t] = k;
-      }
-      ndist = nd;
-    }
-    for (int i = threadIdx.x; i < kQRanks * kQBins; i += kQThreads) qhist[i] = 0u;
+  const uint32_t* h = qhist;
+  if (gridDim.x > 1) {
+    uint32_t* gh = a.hist + ((int64_t)blockIdx.y * 3 + PASS) * kQRanks * kQBins;
+    for (int i = threadIdx.x; i < nd * kQBins; i += blockDim.x)
+      if (qhist[i]) atomicAdd(gh + i, qhist[i]);
+    __threadfence();
     __syncthreads();
-    const int nd = ndist;
-    const int64_t mr = (m + kQThreads - 1) / kQThreads * kQThreads;  // whole warps iterate
-    for (int64_t i = threadIdx.x; i < mr; i += kQThreads) {
-      int id = -1;
-      if (i < m) {
-        const uint32_t key = f32_key(snr_y(base, kind, i, f, pow2, inv));
-        const uint32_t hp = key & hi_mask;
-        for (int k = 0; k < nd; ++k)
-          if (dpre[k] == hp) { id = k * kQBins + (int)((key >> sh) & dmask); break; }
-      }
-      const unsigned peers = __match_any_sync(0xffffffffu, id);
-      if (id >= 0 && lane == __ffs(peers) - 1) atomicAdd(&qhist[id], (uint32_t)__popc(peers));
-    }
+    if (threadIdx.x == 0) last = atomicAdd(&st.ctr[PASS], 1u) == gridDim.x - 1;
     __syncthreads();
-    // one warp per rank: the digit whose cumulative count passes the rank
-    if (warp < kQRanks) {
-      const uint32_t* h = qhist + slot[warp] * kQBins;
-      constexpr int per = kQBins / 32;
-      uint32_t sum = 0;
-      for (int j = 0; j < per; ++j) sum += h[lane * per + j];
-      uint32_t incl = sum;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-      }
-      const int64_t r = rnk[warp];
-      const uint32_t excl = incl - sum;
-      const unsigned hit = __ballot_sync(0xffffffffu, (int64_t)excl <= r && r < (int64_t)incl);
-      const int src = __ffs(hit) - 1;
-      if (lane == src) {
-        int64_t c = excl;
-        int d = lane * per;
-        for (int j = 0; j < per; ++j, ++d) {
-          if (r < c + (int64_t)h[d]) break;
-          c += h[d];
-        }
-        rnk[warp] = r - c;
-        pre[warp] |= (uint32_t)d << sh;
-      }
-    }
+    if (!last) return;
+    __threadfence();
+    for (int i = threadIdx.x; i < nd * kQBins; i += blockDim.x) qhist[i] = __ldcg(gh + i);
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    float med;
-    if (m & 1) {
-      med = key_f32(pre[0]);
+  // one warp per rank: the bin whose cumulative count passes the rank
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const double v25 = (double)(m - 1) * 0.25, v75 = (double)(m - 1) * 0.75;
+  const int64_t l25 = (int64_t)floor(v25), l75 = (int64_t)floor(v75);
+  if (warp < kQRanks) {
+    int64_t r;
+    int slot = 0;
+    if (PASS == 0) {
+      r = warp == 0 ? (m - 1) / 2 : warp == 1 ? m / 2 : warp == 2 ? l25 : warp == 3 ? l25 + 1
+          : warp == 4 ? l75 : l75 + 1;
+      r = imin64(r, m - 1);
     } else {
-      med = __fmul_rn(__fadd_rn(key_f32(pre[0]), key_f32(pre[1])), 0.5f);
+      r = st.left[warp];
+      slot = (int)st.slot[warp];
     }
-    const double q25 = quantile_lerp((double)key_f32(pre[2]), (double)key_f32(pre[3]),
-                                     v25 - (double)l25);
-    const double q75 = quantile_lerp((double)key_f32(pre[4]), (double)key_f32(pre[5]),
-                                     v75 - (double)l75);
-    double sc = (q75 - q25) / 1.3489795003921634;
-    if (fabs(sc) <= 1e-8) sc = 1.0;  // np.isclose(scale, 0) -> 1
-    locscale[blockIdx.x * 2] = (double)med;
-    locscale[blockIdx.x * 2 + 1] = sc;
+    h = qhist + slot * kQBins;
+    constexpr int per = kQBins / 32;
+    uint32_t sum = 0;
+    for (int j = 0; j < per; ++j) sum += h[lane * per + j];
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    const uint32_t excl = incl - sum;
+    if ((int64_t)excl <= r && r < (int64_t)incl) {
+      int64_t c = excl;
+      int d = lane * per;
+      for (int j = 0; j < per; ++j, ++d) {
+        if (r < c + (int64_t)h[d]) break;
+        c += h[d];
+      }
+      pick[warp] = dpre[slot] + ((uint32_t)d << sh);
+      left[warp] = (uint32_t)(r - c);
+    }
   }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  st.shift = (uint32_t)sh;
+  int n = 0;
+  for (int t = 0; t < kQRanks; ++t) {
+    int k = 0;
+    while (k < n && st.dpre[k] != pick[t]) ++k;
+    if (k == n) st.dpre[n++] = pick[t];
+    st.slot[t] = (uint32_t)k;
+    st.left[t] = left[t];
+  }
+  st.ndist = (uint32_t)n;
+  if (sh > 0) return;
+  float med;
+  if (m & 1) {
+    med = key_f32(pick[0]);
+  } else {
+    med = __fmul_rn(__fadd_rn(key_f32(pick[0]), key_f32(pick[1])), 0.5f);
+  }
+  const double q25 = quantile_lerp((double)key_f32(pick[2]), (double)key_f32(pick[3]), v25 - (double)l25);
+  const double q75 = quantile_lerp((double)key_f32(pick[4]), (double)key_f32(pick[5]), v75 - (double)l75);
+  double sc = (q75 - q25) / 1.3489795003921634;
+  if (fabs(sc) <= 1e-8) sc = 1.0;  // np.isclose(scale, 0) -> 1
+  a.locscale[blockIdx.y * 2] = (double)med;
+  a.locscale[blockIdx.y * 2 + 1] = sc;
+}
+
+__global__ void __launch_bounds__(kQPassThreads) k_q_range(const QArgs a, const SnrCfg cfg) {
+  q_range(a, cfg, a.st[blockIdx.y]);
+}
+template <int PASS>
+__global__ void __launch_bounds__(kQPassThreads) k_q_pass(const QArgs a, const SnrCfg cfg) {
+  q_pass<PASS>(a, cfg, a.st[blockIdx.y]);
+}
+// All passes of a row in one CTA, its state in shared memory.
+__global__ void __launch_bounds__(kQPassThreads) k_row_quantiles(const QArgs a, const SnrCfg cfg) {
+  __shared__ QState st;
+  for (int i = threadIdx.x; i < (int)(sizeof(QState) / 4); i += blockDim.x)
+    reinterpret_cast<uint32_t*>(&st)[i] = 0u;
+  __syncthreads();
+  q_range(a, cfg, st);
+  __syncthreads();
+  q_pass<0>(a, cfg, st);
+  __syncthreads();
+  q_pass<1>(a, cfg, st);
+  __syncthreads();
+  q_pass<2>(a, cfg, st);
+}
+
+// CTAs per (row, factor): enough to fill the chip, 2048 values each at least.
+static int q_split(int64_t nrf, int64_t n) {
+  if (nrf >= kQSplitRows) return 1;
+  return (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(2 * 148, nrf), n / 2048));
+}
+
+static int64_t q_state_bytes(int64_t nrf) { return round_up(nrf * (int64_t)sizeof(QState), 256); }
+static int64_t q_workspace(int64_t nrf, int64_t n) {
+  return q_split(nrf, n) > 1 ? q_state_bytes(nrf) + nrf * 3 * kQRanks * kQBins * 4 : 0;
+}
+
+// Median / IQR scale of `nrf` (row, factor) series; `ws` of q_workspace bytes,
+// or nullptr for one CTA per series.
+static int launch_quantiles(const void* in, int kind, int64_t nrf, int64_t n, int64_t in_stride,
+                            const SnrCfg& cfg, double* locscale, void* ws, cudaStream_t st) {
+  const int64_t smem = (int64_t)kQRanks * kQBins * 4;
+  QArgs a{in, kind, n, in_stride, nullptr, nullptr, locscale};
+  const int split = ws ? q_split(nrf, n) : 1;
+  int rc = SPP_OK;
+  if (split == 1) {
+    rc = set_smem_attr(reinterpret_cast<const void*>(k_row_quantiles), smem);
+    if (rc) return rc;
+    k_row_quantiles<<<dim3(1, (unsigned)nrf), kQPassThreads, smem, st>>>(a, cfg);
+    return cuda_status(cudaGetLastError(), "row quantiles launch");
+  }
+  rc = cuda_status(cudaMemsetAsync(ws, 0, (size_t)q_workspace(nrf, n), st), "quantile state clear");
+  if (!rc) rc = set_smem_attr(reinterpret_cast<const void*>(k_q_pass<1>), smem);
+  if (!rc) rc = set_smem_attr(reinterpret_cast<const void*>(k_q_pass<2>), smem);
+  if (rc) return rc;
+  a.st = static_cast<QState*>(ws);
+  a.hist = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(ws) + q_state_bytes(nrf));
+  dim3 grid((unsigned)split, (unsigned)nrf);
+  k_q_range<<<grid, kQPassThreads, 0, st>>>(a, cfg);
+  k_q_pass<0><<<grid, kQPassThreads, kQBins * 4, st>>>(a, cfg);
+  k_q_pass<1><<<grid, kQPassThreads, smem, st>>>(a, cfg);
+  k_q_pass<2><<<grid, kQPassThreads, smem, st>>>(a, cfg);
+  return cuda_status(cudaGetLastError(), "row quantiles launch");
 }
 
 // ---------------------------------------------------------------------------
@@ -877,6 +998,11 @@ int64_t spp_boxcar_snr_workspace_bytes(int64_t nrows, int64_t n, int nfactors, i
 
 }  // extern "C"
 
+// Robust z-score: loc and scale per (row, factor), and the selection's state.
+static int64_t robust_ws(int64_t nrf, int64_t n) {
+  return round_up(nrf * 16, 256) + round_up(q_workspace(nrf, n), 256);
+}
+
 static int boxcar_snr_impl(const void* in, int in_kind, int64_t nrows, int64_t n,
                            int64_t in_stride, const int32_t* factors, int nfactors,
                            const int32_t* widths, int nwidths, float* snr, int32_t* peak_index,
@@ -902,7 +1028,7 @@ static int boxcar_snr_impl(const void* in, int in_kind, int64_t nrows, int64_t n
   }
   int64_t nck;
   const int64_t base_need = snr_ws(nrows, n, nfactors, nwidths, &nck);
-  const int64_t need = base_need + (robust ? round_up(nrows * nfactors * 16, 256) : 0);
+  const int64_t need = base_need + (robust ? robust_ws(nrows * nfactors, n) : 0);
   if (workspace_bytes < need)
     return fail(SPP_ERR_SIZE, "workspace %lld < %lld", (long long)workspace_bytes, (long long)need);
   cudaStream_t st = as_stream(stream);
@@ -926,12 +1052,8 @@ static int boxcar_snr_impl(const void* in, int in_kind, int64_t nrows, int64_t n
   double* locscale = nullptr;
   if (robust) {
     locscale = reinterpret_cast<double*>(ws + base_need);
-    const int64_t qsmem = (int64_t)kQRanks * kQBins * 4;
-    rc = set_smem_attr(reinterpret_cast<const void*>(k_row_quantiles), qsmem);
-    if (rc) return rc;
-    k_row_quantiles<<<(unsigned)(nrows * nfactors), kQThreads, qsmem, st>>>(in, in_kind, n,
-                                                                          in_stride, cfg, locscale);
-    rc = cuda_status(cudaGetLastError(), "row quantiles launch");
+    rc = launch_quantiles(in, in_kind, nrows * nfactors, n, in_stride, cfg, locscale,
+                          ws + base_need + round_up(nrows * nfactors * 16, 256), st);
     if (rc) return rc;
   }
   const int64_t nout = nrows * nfactors * nwidths;
@@ -1112,12 +1234,7 @@ int spp_row_loc_scale(const void* in, int in_kind, int64_t nrows, int64_t n, int
   SnrCfg cfg{};
   cfg.nf = 1;
   cfg.f[0] = 1;
-  const int64_t qsmem = (int64_t)kQRanks * kQBins * 4;
-  int rc = set_smem_attr(reinterpret_cast<const void*>(k_row_quantiles), qsmem);
-  if (rc) return rc;
-  k_row_quantiles<<<(unsigned)nrows, kQThreads, qsmem, st>>>(in, in_kind, n, in_stride, cfg,
-                                                             loc_scale);
-  return cuda_status(cudaGetLastError(), "row quantiles launch");
+  return launch_quantiles(in, in_kind, nrows, n, in_stride, cfg, loc_scale, nullptr, st);
 }
 
 int spp_zscore(const float* in, int64_t n, const double* loc_scale, float* out, void* stream) {
@@ -1160,7 +1277,7 @@ int spp_matched_filter(const float* z, int64_t n, int64_t nfft, const double* te
 int64_t spp_boxcar_snr_robust_workspace_bytes(int64_t nrows, int64_t n, int nfactors,
                                               int nwidths) {
   int64_t nck;
-  return snr_ws(nrows, n, nfactors, nwidths, &nck) + round_up(nrows * nfactors * 16, 256);
+  return snr_ws(nrows, n, nfactors, nwidths, &nck) + robust_ws(nrows * nfactors, n);
 }
 
 int spp_boxcar_snr_robust(const void* in, int in_kind, int64_t nrows, int64_t n,
