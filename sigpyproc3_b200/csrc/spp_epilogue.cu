@@ -211,13 +211,21 @@ __global__ void k_subband(const void* __restrict__ in, int64_t nchans, int64_t n
 
 // ---------------------------------------------------------------------------
 // Boxcar S/N.  Chunk pass: CTA (chunk k, row r, factor fi) builds the
-// downsampled series y over its chunk plus a halo of (wmax-1) samples in
-// shared memory as float64, scans it to prefix sums, and records per width the
-// best window sum starting inside the chunk (smallest start on ties) plus the
-// chunk's sum and second central moment.  Final pass merges chunks (Chan et
-// al. 1979 pairwise variance) and forms (best - w*mean) / (std*sqrt(w)).
+// downsampled series y over its chunk plus a halo of wmax samples in shared
+// memory, scans it to prefix sums, and records per width the best window sum
+// starting inside the chunk (smallest start on ties) plus the chunk's sum and
+// second central moment.  Final pass merges chunks (Chan et al. 1979 pairwise
+// variance) and forms (best - w*mean) / (std*sqrt(w)).
+//
+// Integer rows run on 32-bit integers wherever that is exact (see k_snr_chunk):
+// half the shared memory and no float64 in the window loop.  Threads keep the
+// largest window sum only; who holds the chunk's best looks its index up
+// afterwards, so a window costs a load, a subtraction and a maximum.  512 int32
+// rows x 250001, factors 1/2/4, 9 widths: 2057 -> 979 us (issue 59 %, shared
+// loads 48 %, the rest waits at the block's scans); 200 float32 rows x 300001,
+// factors 1/2: 875 -> 795 us.
 // ---------------------------------------------------------------------------
-constexpr int kSnrChunk = 6144;     // downsampled samples per CTA (24 per thread)
+constexpr int kSnrChunk = 6144;     // downsampled samples per CTA, most
 constexpr int kSnrThreads = 256;
 constexpr int kSnrMaxW = 4096;
 constexpr int kSnrMaxWidths = 32;
@@ -229,6 +237,8 @@ struct SnrPart {
 
 struct SnrCfg {
   int nf, nw, wmax;
+  int chunk;      // downsampled samples per CTA
+  int smem_words;
   int32_t f[8];
   int32_t w[kSnrMaxWidths];
 };
@@ -238,210 +248,386 @@ __device__ __forceinline__ double row_val(const void* in, int kind, int64_t i) {
                              : (double)static_cast<const float*>(in)[i];
 }
 
-// One CTA per (chunk of kSnrChunk downsampled samples, row, factor).  Chunk-
-// local indices are 32-bit; the width maxima keep per-thread candidates for up
-// to kSnrWGroup widths in registers over one pass of the chunk, then reduce
-// once (ties go to the smaller sample index, as the reference's argmax).
-constexpr int kSnrWGroup = 12;
+constexpr int kSnrWarps = kSnrThreads / 32;
 
-__global__ void __launch_bounds__(kSnrThreads)
-k_snr_chunk(const void* __restrict__ in, int kind, int64_t n, int64_t in_stride, const SnrCfg cfg,
-            int64_t nchunks, SnrPart* __restrict__ parts, double* __restrict__ stats) {
-  const int nfactors = cfg.nf, nwidths = cfg.nw, wmax = cfg.wmax;
-  extern __shared__ double sy[];  // kSnrChunk + wmax + 1
-  __shared__ double red_d[kSnrThreads / 32 * kSnrWGroup];
-  __shared__ int red_i[kSnrThreads / 32 * kSnrWGroup];
-  __shared__ int sw[kSnrMaxWidths];
-  __shared__ double carry;
-  const int64_t k = blockIdx.x;
-  const int64_t row = blockIdx.y / nfactors;
-  const int fi = blockIdx.y % nfactors;
-  const int f = cfg.f[fi];
-  const int64_t m = n / f;
-  const int64_t i0 = k * kSnrChunk;
-  if (i0 >= m) {
-    return;
-  }
-  const int own = (int)imin64(kSnrChunk, m - i0);
-  const int len = (int)imin64(own + wmax, m - i0);  // samples loaded
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x < nwidths) sw[threadIdx.x] = cfg.w[threadIdx.x];
-  const char* base = static_cast<const char*>(in) + row * in_stride * 4;
-  // y values (downsampled means rounded to float32 as the reference output
-  // dtype); a power-of-two factor divides exactly by multiplying
-  const bool pow2 = (f & (f - 1)) == 0;
-  const double inv = 1.0 / (double)f;
-  for (int j = threadIdx.x; j < len; j += blockDim.x) {
-    double s = 0.0;
-    const int64_t x0 = (i0 + j) * f;
-    for (int q = 0; q < f; ++q) s += row_val(base, kind, x0 + q);
-    sy[j + 1] = (double)(float)(pow2 ? s * inv : s / f);
-  }
-  if (threadIdx.x == 0) { sy[0] = 0.0; carry = 0.0; }
+__device__ __forceinline__ double block_sum(double v, double* red) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   __syncthreads();
-  // chunk sum and M2 over owned samples
-  {
-    double s = 0.0;
-    for (int j = threadIdx.x; j < own; j += blockDim.x) s += sy[j + 1];
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double t = 0.0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) red_d[warp] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double t = 0.0;
-      for (int w = 0; w < kSnrThreads / 32; ++w) t += red_d[w];
-      carry = t;
-    }
-    __syncthreads();
-    const double mu = carry / (double)own;
-    double q = 0.0;
-    for (int j = threadIdx.x; j < own; j += blockDim.x) {
-      const double d = sy[j + 1] - mu;
-      q += d * d;
-    }
+  for (int w = 0; w < kSnrWarps; ++w) t += red[w];
+  return t;
+}
+
+__device__ __forceinline__ long long block_sum(long long v, long long* red) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
-    __syncthreads();
-    if (lane == 0) red_d[warp] = q;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double t = 0.0;
-      for (int w = 0; w < kSnrThreads / 32; ++w) t += red_d[w];
-      double* st = stats + ((row * nfactors + fi) * nchunks + k) * 3;
-      st[0] = (double)own;
-      st[1] = carry;
-      st[2] = t;
-    }
-    __syncthreads();
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  long long t = 0;
+#pragma unroll
+  for (int w = 0; w < kSnrWarps; ++w) t += red[w];
+  return t;
+}
+
+// Window arithmetic of the two paths: prefix sums (T), the sum of a window
+// (V), and the warp's largest one.
+struct SnrInt {
+  typedef uint32_t T;
+  typedef int32_t V;
+  __device__ __forceinline__ static V lowest() { return INT_MIN; }
+  __device__ __forceinline__ static V window(T b, T a) { return (int32_t)(b - a); }
+  __device__ __forceinline__ static V larger(V a, V b) { return max(a, b); }
+  __device__ __forceinline__ static V warp_max(V v) { return __reduce_max_sync(0xffffffffu, v); }
+};
+struct SnrF64 {
+  typedef double T;
+  typedef double V;
+  __device__ __forceinline__ static V lowest() { return -DBL_MAX; }
+  __device__ __forceinline__ static V window(T b, T a) { return b - a; }
+  __device__ __forceinline__ static V larger(V a, V b) { return b > a ? b : a; }  // ignores NaN
+  __device__ __forceinline__ static V warp_max(V v) {
+    // ordered 64-bit key, largest high word first, then the low word among equals
+    long long k = __double_as_longlong(v);
+    k ^= (k >> 63) & 0x7fffffffffffffffll;
+    const int hi = (int)(k >> 32);
+    const int mh = __reduce_max_sync(0xffffffffu, hi);
+    const uint32_t ml = __reduce_max_sync(0xffffffffu, hi == mh ? (uint32_t)k : 0u);
+    long long m = ((long long)mh << 32) | ml;
+    m ^= (m >> 63) & 0x7fffffffffffffffll;
+    return __longlong_as_double(m);
   }
-  // inclusive scan of sy[1..len] (sequential per thread segment + warp/block scan)
-  {
-    const int per = (len + blockDim.x - 1) / blockDim.x;
-    const int a = 1 + threadIdx.x * per;
-    const int b = min(a + per, len + 1);
-    double s = 0.0;
-    for (int j = a; j < b; ++j) { s += sy[j]; sy[j] = s; }
-    double incl = s;
+};
+
+// Inclusive scan of s[1..len] in place (s[0] = 0): each thread a run of an odd
+// length (distinct banks), then warp and block offsets.
+template <typename T>
+__device__ __forceinline__ void snr_scan(T* s, int len, T* red) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int per = ((len + kSnrThreads - 1) / kSnrThreads) | 1;
+  const int a = min(1 + (int)threadIdx.x * per, len + 1), b = min(a + per, len + 1);
+  T sum = T(0);
+#pragma unroll 5
+  for (int j = a; j < b; ++j) sum += s[j];
+  T incl = sum;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const double v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    if (lane == 31) red_d[warp] = incl;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double acc = 0.0;
-      for (int w = 0; w < kSnrThreads / 32; ++w) { const double v = red_d[w]; red_d[w] = acc; acc += v; }
-    }
-    __syncthreads();
-    const double off = red_d[warp] + (incl - s);
-    for (int j = a; j < b; ++j) sy[j] += off;
-    __syncthreads();
+  for (int o = 1; o < 32; o <<= 1) {
+    const T v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
   }
-  // window maxima: widths in groups of kSnrWGroup, one pass over the chunk each
-  for (int w0 = 0; w0 < nwidths; w0 += kSnrWGroup) {
-    double best[kSnrWGroup];
-    int bt[kSnrWGroup], wv[kSnrWGroup];
+  __syncthreads();
+  if (lane == 31) red[warp] = incl;
+  __syncthreads();
+  T run = incl - sum;
+  for (int w = 0; w < warp; ++w) run += red[w];
+#pragma unroll 5
+  for (int j = a; j < b; ++j) {
+    run += s[j];
+    s[j] = run;
+  }
+  __syncthreads();
+}
+
+// Best window of NG widths (from w0) over starts 0..own-1 of the scanned chunk,
+// folded into the running best (best, idx) in shared memory; the chunk's first
+// sample is at `at` of the CTA's, values are scaled by `scale`.
+template <class A, int NG>
+__device__ __forceinline__ void snr_window_group(const typename A::T* s, int own, int len,
+                                                 const SnrCfg& cfg, int w0, int at, double scale,
+                                                 double* best, int* idx) {
+  typedef typename A::V V;
+  __shared__ V wbest[kSnrWarps][NG];
+  __shared__ V bbest[NG];
+  __shared__ int bidx[NG];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  V m[NG];
+  const typename A::T* sw[NG];
 #pragma unroll
-    for (int g = 0; g < kSnrWGroup; ++g) {
-      best[g] = -DBL_MAX;
-      bt[g] = INT_MAX;
-      wv[g] = (w0 + g < nwidths) ? sw[w0 + g] : INT_MAX / 2;
+  for (int g = 0; g < NG; ++g) {
+    m[g] = A::lowest();
+    sw[g] = s + cfg.w[w0 + g] + threadIdx.x;
+  }
+  const typename A::T* s0 = s + threadIdx.x;
+  // starts with every window loaded, four steps of the CTA at a time
+  const int full = len == own + cfg.wmax ? own : max(0, min(own, len - cfg.wmax + 1));
+  int t = 0;
+  for (; t + 4 * kSnrThreads <= full; t += 4 * kSnrThreads) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const typename A::T p0 = s0[t + i * kSnrThreads];
+#pragma unroll
+      for (int g = 0; g < NG; ++g)
+        m[g] = A::larger(m[g], A::window(sw[g][t + i * kSnrThreads], p0));
     }
-    const int ng = min(kSnrWGroup, nwidths - w0);
-    if (len == own + wmax) {
-      // interior chunk: every window of every owned sample is loaded
-      for (int t = threadIdx.x; t < own; t += blockDim.x) {
-        const double p0 = sy[t];
+  }
+  for (; t + (int)threadIdx.x < own; t += kSnrThreads) {
+    const typename A::T p0 = s0[t];
 #pragma unroll
-        for (int g = 0; g < kSnrWGroup; ++g) {
-          if (g < ng) {
-            const double v = sy[t + wv[g]] - p0;
-            if (v > best[g]) { best[g] = v; bt[g] = t; }
-          }
-        }
-      }
-    } else {
-      for (int t = threadIdx.x; t < own; t += blockDim.x) {
-        const double p0 = sy[t];
+    for (int g = 0; g < NG; ++g)
+      if (sw[g] + t <= s + len) m[g] = A::larger(m[g], A::window(sw[g][t], p0));
+  }
 #pragma unroll
-        for (int g = 0; g < kSnrWGroup; ++g) {
-          if (t + wv[g] <= len) {  // window inside the row
-            const double v = sy[t + wv[g]] - p0;
-            if (v > best[g]) { best[g] = v; bt[g] = t; }
-          }
-        }
-      }
+  for (int g = 0; g < NG; ++g) {
+    const V x = A::warp_max(m[g]);
+    if (lane == 0) wbest[warp][g] = x;
+  }
+  __syncthreads();
+  if (threadIdx.x < NG) {
+    V x = wbest[0][threadIdx.x];
+#pragma unroll
+    for (int w = 1; w < kSnrWarps; ++w) x = A::larger(x, wbest[w][threadIdx.x]);
+    bbest[threadIdx.x] = x;
+    bidx[threadIdx.x] = INT_MAX;
+  }
+  __syncthreads();
+  // the threads that hold a width's best find its first start
+#pragma unroll
+  for (int g = 0; g < NG; ++g) {
+    if (m[g] != bbest[g]) continue;
+    for (int j = 0; j + (int)threadIdx.x < own; j += kSnrThreads) {
+      if (sw[g] + j > s + len || A::window(sw[g][j], s0[j]) != m[g]) continue;
+      atomicMin(&bidx[g], j + (int)threadIdx.x);
+      break;
     }
-#pragma unroll
-    for (int g = 0; g < kSnrWGroup; ++g) {
-      if (g >= ng) break;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ov = __shfl_xor_sync(0xffffffffu, best[g], o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bt[g], o);
-        if (ov > best[g] || (ov == best[g] && oi < bt[g])) { best[g] = ov; bt[g] = oi; }
-      }
-      if (lane == 0) { red_d[warp * kSnrWGroup + g] = best[g]; red_i[warp * kSnrWGroup + g] = bt[g]; }
+  }
+  __syncthreads();
+  if (threadIdx.x < NG && bidx[threadIdx.x] != INT_MAX) {
+    const double v = (double)bbest[threadIdx.x] * scale;
+    const int i = w0 + threadIdx.x;
+    if (idx[i] == INT_MAX || v > best[i]) {
+      best[i] = v;
+      idx[i] = at + bidx[threadIdx.x];
     }
-    __syncthreads();
-    if (threadIdx.x < kSnrWGroup && w0 + (int)threadIdx.x < nwidths) {
-      const int g = threadIdx.x;
-      double bb = red_d[g];
-      int bi = red_i[g];
-      for (int w2 = 1; w2 < kSnrThreads / 32; ++w2) {
-        const double v = red_d[w2 * kSnrWGroup + g];
-        const int vi = red_i[w2 * kSnrWGroup + g];
-        if (v > bb || (v == bb && vi < bi)) { bb = v; bi = vi; }
-      }
-      SnrPart* p = parts + (((row * nfactors + fi) * nwidths + (w0 + g)) * nchunks + k);
-      p->best = bb;
-      p->idx = bi == INT_MAX ? LLONG_MAX : i0 + bi;
-    }
-    __syncthreads();
+  }
+  __syncthreads();
+}
+
+// All widths, ten at a time.
+template <class A>
+__device__ __forceinline__ void snr_windows(const typename A::T* s, int own, int len, const SnrCfg& cfg,
+                                            int at, double scale, double* best, int* idx) {
+  int w0 = 0;
+  for (; w0 + 10 <= cfg.nw; w0 += 10) snr_window_group<A, 10>(s, own, len, cfg, w0, at, scale, best, idx);
+  switch (cfg.nw - w0) {
+#define SPP_SNR_CASE(NG)                                                      \
+  case NG:                                                                    \
+    snr_window_group<A, NG>(s, own, len, cfg, w0, at, scale, best, idx);      \
+    break;
+    SPP_SNR_CASE(1) SPP_SNR_CASE(2) SPP_SNR_CASE(3) SPP_SNR_CASE(4) SPP_SNR_CASE(5)
+    SPP_SNR_CASE(6) SPP_SNR_CASE(7) SPP_SNR_CASE(8) SPP_SNR_CASE(9)
+#undef SPP_SNR_CASE
+    default: break;
   }
 }
 
-__global__ void k_snr_final(int64_t n, const SnrCfg cfg, int64_t nrows, int64_t nchunks, const SnrPart* __restrict__ parts,
-                            const double* __restrict__ stats, float* __restrict__ snr,
-                            int32_t* __restrict__ peak, const double* __restrict__ locscale) {
-  const int nfactors = cfg.nf, nwidths = cfg.nw;
-  const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= nrows * nfactors * nwidths) return;
-  const int wi = id % nwidths;
-  const int64_t rf = id / nwidths;  // row * nfactors + fi
-  const int fi = rf % nfactors;
-  const int64_t m = n / cfg.f[fi];
-  const int64_t nck = (m + kSnrChunk - 1) / kSnrChunk;
-  // merge moments
+// Sums of F consecutive samples (F = 0: f) for every start of the chunk: prefix
+// input, largest sample magnitude, and (of the owned ones) sum and sum of
+// squares.  Everything is exact where the caller goes on: f * big <= 2^24, and a
+// thread owns 24 sums at most.
+template <int F>
+__device__ __forceinline__ void snr_load_int(const int32_t* __restrict__ x, int f, int own, int len,
+                                             uint32_t* s, uint32_t& big, long long& s1, long long& s2) {
+  const int ff = F > 0 ? F : f;
+  auto get = [&](int j) {
+    const int32_t* p = x + (int64_t)j * ff;
+    int v = 0;
+#pragma unroll
+    for (int q = 0; q < (F > 0 ? F : ff); ++q) {
+      const int y = __ldg(p + q);
+      big = max(big, (uint32_t)(y < 0 ? 0u - (uint32_t)y : (uint32_t)y));
+      v = (int)((uint32_t)v + (uint32_t)y);
+    }
+    s[j + 1] = (uint32_t)v;
+    return v;
+  };
+  int a1 = 0;
+#pragma unroll 4
+  for (int j = threadIdx.x; j < own; j += kSnrThreads) {
+    const int v = get(j);
+    a1 = (int)((uint32_t)a1 + (uint32_t)v);
+    s2 += (long long)v * v;
+  }
+  s1 = a1;
+#pragma unroll 2
+  for (int j = own + threadIdx.x; j < len; j += kSnrThreads) get(j);
+}
+
+// KIND int32: for a power-of-two factor f, y = s / f with s the integer sum of f
+// samples.  Where f * |x| <= 2^24 the float32 rounding of y is exact, and where
+// f * |x| * wmax < 2^31 window sums are exact differences of prefix sums
+// modulo 2^32; the chunk's moments come from 64-bit sums (n * sum(s^2) -
+// sum(s)^2 in 128 bits).  Other chunks and float32 rows take float64, in pieces
+// that fit the shared memory.
+template <int KIND>
+__global__ void __launch_bounds__(kSnrThreads, 4)
+k_snr_chunk(const void* __restrict__ in, int64_t n, int64_t in_stride, const SnrCfg cfg,
+            int64_t nchunks, SnrPart* __restrict__ parts, double* __restrict__ stats) {
+  extern __shared__ __align__(16) uint32_t snr_sm[];
+  __shared__ double best[kSnrMaxWidths];
+  __shared__ int idx[kSnrMaxWidths];
+  __shared__ double red[kSnrWarps];
+  const int64_t k = blockIdx.x;
+  const int64_t row = blockIdx.y / cfg.nf;
+  const int fi = blockIdx.y % cfg.nf;
+  const int f = cfg.f[fi];
+  const int64_t m = n / f;
+  const int64_t i0 = k * cfg.chunk;
+  if (i0 >= m) return;
+  const int own = (int)imin64(cfg.chunk, m - i0);
+  const char* base = static_cast<const char*>(in) + row * in_stride * 4;
+  const bool pow2 = (f & (f - 1)) == 0;
+  if (threadIdx.x < cfg.nw) {
+    best[threadIdx.x] = -DBL_MAX;
+    idx[threadIdx.x] = INT_MAX;
+  }
+  double* st = stats + ((row * cfg.nf + fi) * nchunks + k) * 3;
+  bool done = false;
+  if constexpr (KIND == SPP_OUT_I32) {
+    if (pow2) {
+      const int len = (int)imin64(own + cfg.wmax, m - i0);
+      const int32_t* x = reinterpret_cast<const int32_t*>(base) + i0 * f;
+      uint32_t big = 0u;
+      long long s1 = 0, s2 = 0;
+      if (f == 1) snr_load_int<1>(x, f, own, len, snr_sm, big, s1, s2);
+      else if (f == 2) snr_load_int<2>(x, f, own, len, snr_sm, big, s1, s2);
+      else if (f == 4) snr_load_int<4>(x, f, own, len, snr_sm, big, s1, s2);
+      else snr_load_int<0>(x, f, own, len, snr_sm, big, s1, s2);
+      if (threadIdx.x == 0) snr_sm[0] = 0u;
+      const unsigned long long top = (unsigned long long)big * (unsigned)f;
+      const int wide = top * (unsigned)cfg.wmax >= (1ull << 31) || top > (1ull << 24);
+      if (__syncthreads_or(wide) == 0) {
+        const long long S1 = block_sum(s1, reinterpret_cast<long long*>(red));
+        const long long S2 = block_sum(s2, reinterpret_cast<long long*>(red));
+        if (threadIdx.x == 0) {
+          const __int128 num = (__int128)S2 * own - (__int128)S1 * S1;
+          st[0] = (double)own;
+          st[1] = (double)S1 / (double)f;
+          st[2] = (double)num / (double)own / ((double)f * (double)f);
+        }
+        snr_scan<uint32_t>(snr_sm, len, reinterpret_cast<uint32_t*>(red));
+        snr_windows<SnrInt>(snr_sm, own, len, cfg, 0, 1.0 / (double)f, best, idx);
+        done = true;
+      }
+    }
+  }
+  if (!done) {
+    double* sy = reinterpret_cast<double*>(snr_sm);
+    const int piece = min(cfg.chunk, cfg.smem_words / 2 - cfg.wmax - 1);
+    const double inv = 1.0 / (double)f;
+    double cnt = 0.0, mean = 0.0, m2 = 0.0;
+    for (int p0 = 0; p0 < own; p0 += piece) {
+      const int po = min(piece, own - p0);
+      const int len = (int)imin64(po + cfg.wmax, m - i0 - p0);
+      __syncthreads();
+      double s = 0.0;
+      for (int j = threadIdx.x; j < len; j += kSnrThreads) {
+        // downsampled means rounded to float32 as the reference output dtype; a
+        // power-of-two factor divides exactly by multiplying
+        double v = 0.0;
+        const int64_t x0 = (i0 + p0 + j) * f;
+        for (int q = 0; q < f; ++q) v += row_val(base, KIND, x0 + q);
+        v = (double)(float)(pow2 ? v * inv : v / f);
+        sy[j + 1] = v;
+        if (j < po) s += v;
+      }
+      if (threadIdx.x == 0) sy[0] = 0.0;
+      const double tot = block_sum(s, red);
+      const double mu = tot / (double)po;
+      double q = 0.0;
+      for (int j = threadIdx.x; j < po; j += kSnrThreads) {
+        const double d = sy[j + 1] - mu;
+        q += d * d;
+      }
+      q = block_sum(q, red);
+      // pairwise merge of the pieces' moments (every thread keeps them)
+      const double nb = (double)po, d = mu - mean, all = cnt + nb;
+      mean += d * nb / all;
+      m2 += q + d * d * cnt * nb / all;
+      cnt = all;
+      if (threadIdx.x == 0) {
+        st[0] = cnt;
+        st[1] = p0 == 0 ? tot : st[1] + tot;
+        st[2] = m2;
+      }
+      __syncthreads();
+      snr_scan<double>(sy, len, red);
+      snr_windows<SnrF64>(sy, po, len, cfg, p0, 1.0, best, idx);
+    }
+  }
+  if (threadIdx.x < cfg.nw) {
+    SnrPart* p = parts + (((row * cfg.nf + fi) * cfg.nw + threadIdx.x) * nchunks + k);
+    p->best = best[threadIdx.x];
+    p->idx = idx[threadIdx.x] == INT_MAX ? LLONG_MAX : i0 + idx[threadIdx.x];
+  }
+}
+
+// One warp per (row, factor, width): lanes take chunks, moments and maxima merge
+// pairwise.
+__global__ void k_snr_final(int64_t n, const SnrCfg cfg, int64_t nrows, int64_t nchunks,
+                            const SnrPart* __restrict__ parts, const double* __restrict__ stats,
+                            float* __restrict__ snr, int32_t* __restrict__ peak,
+                            const double* __restrict__ locscale) {
+  const int64_t id = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (id >= nrows * cfg.nf * cfg.nw) return;
+  const int wi = id % cfg.nw;
+  const int64_t rf = id / cfg.nw;  // row * nfactors + fi
+  const int64_t m = n / cfg.f[rf % cfg.nf];
+  const int64_t nck = (m + cfg.chunk - 1) / cfg.chunk;
   double cnt = 0.0, mean = 0.0, m2 = 0.0;
-  for (int64_t k = 0; k < nck; ++k) {
+  double best = -DBL_MAX;
+  long long bidx = LLONG_MAX;
+  for (int64_t k = lane; k < nck; k += 32) {
     const double* st = stats + (rf * nchunks + k) * 3;
-    const double nb = st[0];
-    if (nb <= 0) continue;
-    const double mb = st[1] / nb;
-    const double d = mb - mean;
-    const double tot = cnt + nb;
+    const double nb = st[0], mb = st[1] / nb;
+    const double d = mb - mean, tot = cnt + nb;
     mean += d * nb / tot;
     m2 += st[2] + d * d * cnt * nb / tot;
     cnt = tot;
+    const SnrPart p = parts[(rf * cfg.nw + wi) * nchunks + k];
+    if (p.idx != LLONG_MAX && (bidx == LLONG_MAX || p.best > best)) {
+      best = p.best;
+      bidx = p.idx;
+    }
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double nb = __shfl_xor_sync(0xffffffffu, cnt, o);
+    const double mb = __shfl_xor_sync(0xffffffffu, mean, o);
+    const double qb = __shfl_xor_sync(0xffffffffu, m2, o);
+    const double tot = cnt + nb;
+    if (nb > 0.0) {
+      if (cnt > 0.0) {
+        const double d = mb - mean;
+        mean += d * nb / tot;
+        m2 += qb + d * d * cnt * nb / tot;
+      } else {
+        mean = mb;
+        m2 = qb;
+      }
+      cnt = tot;
+    }
+    const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+    const long long oi = __shfl_xor_sync(0xffffffffu, bidx, o);
+    if (oi != LLONG_MAX && (bidx == LLONG_MAX || ob > best || (ob == best && oi < bidx))) {
+      best = ob;
+      bidx = oi;
+    }
+  }
+  if (lane != 0) return;
   double sd = cnt > 0 ? sqrt(m2 / cnt) : 0.0;
   if (sd == 0.0) sd = 1.0;
   if (locscale) {  // median / IQR scale
     mean = locscale[rf * 2];
     sd = locscale[rf * 2 + 1];
   }
-  double best = -DBL_MAX;
-  long long bidx = -1;
-  for (int64_t k = 0; k < nck; ++k) {
-    const SnrPart p = parts[(rf * nwidths + wi) * nchunks + k];
-    if (p.idx < 0 || p.idx == LLONG_MAX) continue;
-    if (p.best > best) { best = p.best; bidx = p.idx; }
-  }
   const int w = cfg.w[wi];
-  snr[id] = bidx < 0 ? NAN : (float)((best - (double)w * mean) / (sd * sqrt((double)w)));
-  if (peak) peak[id] = (int32_t)bidx;
+  snr[id] = bidx == LLONG_MAX ? NAN : (float)((best - (double)w * mean) / (sd * sqrt((double)w)));
+  if (peak) peak[id] = bidx == LLONG_MAX ? -1 : (int32_t)bidx;
 }
 
 // ---------------------------------------------------------------------------
@@ -980,9 +1166,18 @@ int spp_subband(const void* in, int nbits, int bitorder, int64_t nchans, int64_t
 
 }  // extern "C"
 
+// Samples per CTA of the chunk pass: the largest of 6144, 3072 and 1536 that
+// still gives eight CTAs per SM, so that few rows fill the chip too (one int32
+// series of 20001, factors 1/2/4: 38.6 -> 24.3 us with the warp-wide final pass).
+static int snr_chunk(int64_t nrf, int64_t n) {
+  for (int c = kSnrChunk; c > 1536; c /= 2)
+    if (nrf * ceil_div(n, c) >= 148 * 8) return c;
+  return 1536;
+}
+
 // Sizes the S/N workspace for `n` samples per row.
 int64_t snr_ws(int64_t nrows, int64_t n, int nfactors, int nwidths, int64_t* nchunks) {
-  const int64_t nck = ceil_div(std::max<int64_t>(n, 1), kSnrChunk);
+  const int64_t nck = ceil_div(std::max<int64_t>(n, 1), snr_chunk(nrows * nfactors, n));
   *nchunks = nck;
   const int64_t parts = nrows * nfactors * nwidths * nck * (int64_t)sizeof(SnrPart);
   const int64_t stats = nrows * nfactors * nck * 3 * (int64_t)sizeof(double);
@@ -1036,17 +1231,26 @@ static int boxcar_snr_impl(const void* in, int in_kind, int64_t nrows, int64_t n
   SnrPart* parts = reinterpret_cast<SnrPart*>(ws + kStatusBytes);
   double* stats = reinterpret_cast<double*>(
       ws + kStatusBytes + round_up(nrows * nfactors * nwidths * nck * (int64_t)sizeof(SnrPart), 256));
-  int rc = cuda_status(cudaMemsetAsync(parts, 0xFF, sizeof(SnrPart) * nrows * nfactors * nwidths * nck, st), "parts init");
-  if (rc) return rc;
-  rc = cuda_status(cudaMemsetAsync(stats, 0, sizeof(double) * 3 * nrows * nfactors * nck, st), "stats init");
-  if (rc) return rc;
-  const int64_t smem = (int64_t)(kSnrChunk + cfg.wmax + 1) * 8;
+  // chunks shorter than two halos would mostly load halo
+  cfg.chunk = snr_chunk(nrows * nfactors, n);
+  if (cfg.chunk < 2 * cfg.wmax) cfg.chunk = kSnrChunk;
+  const bool ints = in_kind == SPP_OUT_I32;
+  // float64 pieces of at least 512 starts fit beside the halo
+  cfg.smem_words = ints ? std::max(cfg.chunk + cfg.wmax + 2, 2 * (cfg.wmax + 513))
+                        : 2 * (cfg.chunk + cfg.wmax + 1);
+  const int64_t smem = (int64_t)cfg.smem_words * 4;
+  const void* fn = ints ? reinterpret_cast<const void*>(k_snr_chunk<SPP_OUT_I32>)
+                        : reinterpret_cast<const void*>(k_snr_chunk<SPP_OUT_F32>);
+  int rc = SPP_OK;
   if (smem > 48 * 1024) {
-    rc = set_smem_attr(reinterpret_cast<const void*>(k_snr_chunk), smem);
+    rc = set_smem_attr(fn, smem);
     if (rc) return rc;
   }
-  dim3 grid((unsigned)nck, (unsigned)(nrows * nfactors));
-  k_snr_chunk<<<grid, kSnrThreads, smem, st>>>(in, in_kind, n, in_stride, cfg, nck, parts, stats);
+  dim3 grid((unsigned)ceil_div(n, cfg.chunk), (unsigned)(nrows * nfactors));
+  if (ints)
+    k_snr_chunk<SPP_OUT_I32><<<grid, kSnrThreads, smem, st>>>(in, n, in_stride, cfg, nck, parts, stats);
+  else
+    k_snr_chunk<SPP_OUT_F32><<<grid, kSnrThreads, smem, st>>>(in, n, in_stride, cfg, nck, parts, stats);
   rc = cuda_status(cudaGetLastError(), "snr chunk launch");
   if (rc) return rc;
   double* locscale = nullptr;
@@ -1057,7 +1261,7 @@ static int boxcar_snr_impl(const void* in, int in_kind, int64_t nrows, int64_t n
     if (rc) return rc;
   }
   const int64_t nout = nrows * nfactors * nwidths;
-  k_snr_final<<<(unsigned)ceil_div(nout, 256), 256, 0, st>>>(n, cfg, nrows, nck, parts, stats, snr,
+  k_snr_final<<<(unsigned)ceil_div(nout, 8), 256, 0, st>>>(n, cfg, nrows, nck, parts, stats, snr,
                                                              peak_index, locscale);
   return cuda_status(cudaGetLastError(), "snr final launch");
 }

@@ -1,0 +1,53 @@
+"""Boxcar S/N chunks at the edges of their two paths: rows around the chunk
+sizes, widths up to the halo limit, integer rows inside the exact 32-bit path,
+past its window limit (|sum| * width >= 2^31) and past float32's exact integers
+(|x| > 2^24, factor 1: rounding as the float32 input of the oracle), many equal
+windows, float32 rows.  S/N within rtol 1e-5 of the float64 oracle, peak index
+equal (integer window sums are exact on both sides)."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(orc, x, widths, factors):
+    import torch
+
+    from sigpyproc3_b200.search import boxcar_snr
+
+    snr, idx = boxcar_snr(torch.from_numpy(x).cuda(), widths=widths, factors=factors)
+    esnr, eidx = orc.boxcar_snr(x.astype(np.float32), factors, widths)
+    np.testing.assert_allclose(snr.cpu().numpy(), esnr, rtol=1e-5)
+    np.testing.assert_array_equal(idx.cpu().numpy(), eidx)
+
+
+@pytest.mark.parametrize("rows,n", [(1, 300), (3, 1535), (2, 1537), (400, 6143), (399, 6145), (1, 40000)])
+def test_integer_rows(orc, rows, n):
+    rng = np.random.default_rng(n)
+    x = np.rint(rng.normal(3000.0, 40.0, size=(rows, n))).astype(np.int32)
+    x[0, n // 2:n // 2 + 20] += 200
+    _check(orc, x, [1, 2, 7, 33, 256], [1, 2, 4])
+
+
+@pytest.mark.parametrize("top", [1 << 20, 1 << 23, 1 << 26, (1 << 31) - 1])
+def test_integer_range(orc, top):
+    """Values up to `top` of both signs: the 32-bit path ends between the first
+    and second for widths of 4096."""
+    rng = np.random.default_rng(top)
+    x = rng.integers(-top, top, size=(2, 9001), endpoint=True).astype(np.int32)
+    _check(orc, x, [1, 16, 4096], [1])
+
+
+def test_equal_windows(orc):
+    """The first of many equal best windows, across chunks."""
+    x = np.full((2, 20000), 5, dtype=np.int32)
+    x[1, ::2] = 6
+    _check(orc, x, list(range(1, 33)), [1, 2, 8])
+
+
+@pytest.mark.parametrize("n", [1537, 30001])
+def test_float_rows(orc, n):
+    rng = np.random.default_rng(n)
+    x = np.rint(rng.normal(0.0, 500.0, size=(3, n)) * 8).astype(np.float32) / 8  # sums exact in float64
+    _check(orc, x, [1, 3, 64, 1000], [1, 2, 3])
