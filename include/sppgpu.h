@@ -119,6 +119,17 @@ int spp_dedisperse_hd(const void* in, int nbits, int64_t nchans, int64_t nsamps,
                       const int32_t* delays_host, float* out, int64_t out_len,
                       int64_t out_start, void* stream);
 
+/* The same computation for any sample width with `delays_host` in host memory
+ * (at most 4096 channels): one launch that reads each row of the block once, no
+ * workspace, no delay upload.  Integer input is summed exactly, float32 input
+ * in float64 in channel order.  Any alignment of `in` (float32: 4 bytes).
+ * Returns SPP_ERR_UNSUPPORTED (nothing launched) when a group of 32 bytes of
+ * channels has a delay spread that does not fit in shared memory; callers then
+ * use spp_dedisperse. */
+int spp_dedisperse_host(const void* in, int nbits, int bitorder, int64_t nchans,
+                        int64_t nsamps, const int32_t* delays_host, float* out,
+                        int64_t out_len, int64_t out_start, void* stream);
+
 /* ---- folding -------------------------------------------------------------
  * Replaces kernels.fold (core/kernels.py:403-445) for one read_plan block
  * (Filterbank.fold, base.py:1109-1207): sample t of the block (t < nsamps -

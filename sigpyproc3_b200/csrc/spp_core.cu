@@ -20,6 +20,8 @@ int launch_single8(const uint8_t* raw, int64_t nchans, int64_t nsamps, const int
                    uint32_t* status, cudaStream_t st);
 int launch_single8_hd(const uint8_t* raw, int64_t nchans, int64_t nsamps, const int32_t* delays_host,
                       float* out, int64_t out_start, int64_t nvalid, cudaStream_t st);
+int launch_single_stream(const void* in, int nbits, int bitorder, int64_t nchans, int64_t nsamps,
+                         const int32_t* delays_host, float* out, int64_t nvalid, cudaStream_t st);
 
 static thread_local char g_err[1024] = "";
 
@@ -462,6 +464,32 @@ int spp_dedisperse_hd(const void* in, int nbits, int64_t nchans, int64_t nsamps,
   if (rc == SPP_ERR_UNSUPPORTED)
     return fail(rc, "host-table path needs nchans %% 32 == 0, nchans <= 1024, a 16-B aligned "
                 "block and every slab resident in shared memory");
+  return rc;
+}
+
+int spp_dedisperse_host(const void* in, int nbits, int bitorder, int64_t nchans, int64_t nsamps,
+                        const int32_t* delays_host, float* out, int64_t out_len,
+                        int64_t out_start, void* stream) {
+  if (!in || !delays_host || !out) return fail(SPP_ERR_ARG, "spp_dedisperse_host: null pointer");
+  if (!valid_nbits(nbits)) return fail(SPP_ERR_ARG, "nbits must be 1, 2, 4, 8 or 32 (got %d)", nbits);
+  if (bitorder != SPP_BITORDER_BIG && bitorder != SPP_BITORDER_LITTLE)
+    return fail(SPP_ERR_ARG, "bad bitorder %d", bitorder);
+  if (nchans <= 0 || nsamps <= 0) return fail(SPP_ERR_ARG, "bad shape");
+  if (nbits < 8 && (nchans * nbits) % 8 != 0)
+    return fail(SPP_ERR_ARG, "nchans*nbits must be a multiple of 8");
+  const int32_t dmin = *std::min_element(delays_host, delays_host + nchans);
+  const int32_t dmax = *std::max_element(delays_host, delays_host + nchans);
+  const int64_t nvalid = nsamps - std::max<int64_t>(std::llabs(dmin), std::llabs(dmax));
+  if (nvalid <= 0) return SPP_OK;  // reference: prange over a non-positive count
+  if (-(int64_t)dmin > nsamps)
+    return fail(SPP_ERR_DELAY, "negative delay %d reaches before the block", dmin);
+  if (out_start < 0 || out_start + nvalid > out_len)
+    return fail(SPP_ERR_SIZE, "output too small: out_start %lld + %lld samples > out_len %lld",
+                (long long)out_start, (long long)nvalid, (long long)out_len);
+  const int rc = launch_single_stream(in, nbits, bitorder, nchans, nsamps, delays_host,
+                                      out + out_start, nvalid, as_stream(stream));
+  if (rc == SPP_ERR_UNSUPPORTED)
+    return fail(rc, "streaming path needs nchans <= 4096 and every slab's delay spread in shared memory");
   return rc;
 }
 

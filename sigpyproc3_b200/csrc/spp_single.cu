@@ -429,4 +429,361 @@ int launch_single8_hd(const uint8_t* raw, int64_t nchans, int64_t nsamps, const 
   return SPP_ERR_UNSUPPORTED;
 }
 
+
+// ---------------------------------------------------------------------------
+// Streaming single-DM kernel, every sample width (spp_dedisperse_host): the
+// block is read once, straight from its time-major rows, whatever its length,
+// channel count and alignment.
+//
+// CTA = T outputs over all channels, walked in slabs of 32 bytes of each row
+// (256 / NB channels; 64 bytes of float32).  Slab s needs rows [t0 + min delay, t0 + T + max delay)
+// of its channels; a ring of them is filled ahead of the adds: 16-byte cp.async
+// where rows are so aligned (up to six slabs), else aligned words shifted into
+// place and stored.  Staged rows are dense 32-byte
+// rows: lane (i = lane & 3, j = lane >> 2) reads a byte of word j in row
+// t + i + delay, which hits 32 different banks for any delays; 1-, 2- and
+// 4-bit fields are masked in place, summed per position within the byte and
+// shifted once per word, so a channel costs a byte load and one and a half
+// logic operations.  Float32 rows (16 channels, pitch 17 words) give each lane an
+// output and are added in channel order in float64.
+//
+// Bound by the byte loads (32 adds per shared-memory wavefront) next to the row
+// copies.  Against the planar path (corner turn, then the DM-time kernel on one
+// row): 8-bit 1024 ch x 262144, DM 300: 392 -> 92 us (2.9 TB/s); 2-bit 1024 ch x
+// 200000: 138 -> 46 us, 1020 ch (rows at odd addresses): 198 -> 78 us; 1-bit
+// 1024 ch x 300000: 140 -> 55 us; float32 256 ch x 100000: 112 -> 53 us.
+// ---------------------------------------------------------------------------
+constexpr int kSdWarps = 16;
+constexpr int kSdThreads = 32 * kSdWarps;
+constexpr int kSdSeg = 32;  // bytes of a row per slab (integers)
+// float32: 64 bytes (16 channels) at an odd word pitch
+__host__ __device__ constexpr int sd_seg(int nb) { return nb == 32 ? 64 : kSdSeg; }
+__host__ __device__ constexpr int sd_pitch(int nb) { return nb == 32 ? 68 : kSdSeg; }
+
+template <int MAXC>
+struct SdArgs {
+  const uint8_t* raw;
+  int64_t rowbytes, nsamps;
+  float* out;           // output of sample 0
+  int64_t nvalid;
+  int32_t nslab, T, stages, stage_bytes;
+  int32_t bitorder;
+  int32_t align;        // of the rows: 16, 4 or 1 bytes
+  int32_t mn[MAXC / 8];    // per slab: smallest delay (float32: 16 channels each)
+  uint16_t rows[MAXC / 8]; // per slab: rows beyond T
+  uint16_t off[MAXC];      // per channel: delay - the slab's smallest
+};
+
+// Aligned words of a row segment that starts at any byte: word k of the 32
+// bytes from byte `seg` of row `row`, zero past the row's end.  Only words that
+// hold a wanted byte are loaded.
+__device__ __forceinline__ uint32_t row_word(const uint8_t* raw, int64_t rowbytes, int64_t row,
+                                             int64_t seg, int k) {
+  const int64_t left = rowbytes - seg - 4 * k;  // bytes of the row from this word on
+  if (left <= 0) return 0u;
+  const uint8_t* p = raw + row * rowbytes + seg + 4 * k;
+  const int sh = (int)(reinterpret_cast<uintptr_t>(p) & 3);
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(p - sh);
+  const uint32_t lo = __ldg(w);
+  const uint32_t hi = (sh && left > 4 - sh) ? __ldg(w + 1) : 0u;
+  uint32_t v = __funnelshift_r(lo, hi, 8 * sh);
+  if (left < 4) v &= (1u << (8 * left)) - 1u;
+  return v;
+}
+
+template <int NB, int MAXC>
+__device__ __forceinline__ void sd_stage(const SdArgs<MAXC>& a, uint8_t* buf, int64_t t0, int s) {
+  const int64_t seg = (int64_t)s * sd_seg(NB);
+  const int64_t r0 = t0 + a.mn[s];
+  const int nrows = a.T + a.rows[s];
+  auto wrap = [&](int64_t row) {  // rows outside the block wrap once or read zero
+    if (row < 0) row += a.nsamps;
+    else if (row >= a.nsamps) row -= a.nsamps;
+    return (row >= 0 && row < a.nsamps) ? row : (int64_t)-1;
+  };
+  if (NB == 32) {
+    // float rows keep an odd pitch for the adds, so they pass through registers:
+    // 16-byte loads where rows allow, four in flight
+    constexpr int PW = sd_pitch(NB) / 4;
+    float* dst = reinterpret_cast<float*>(buf);
+    if (a.align == 16) {
+      constexpr int Q = sd_seg(NB) / 16;  // loads per row
+      const int h = threadIdx.x % Q;
+      const bool col = seg + 16 * h < a.rowbytes;
+      for (int r = threadIdx.x / Q; r < nrows; r += 4 * (kSdThreads / Q)) {
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int rr = r + u * (kSdThreads / Q);
+          const int64_t row = col && rr < nrows ? wrap(r0 + rr) : -1;
+          v[u] = row >= 0 ? __ldg(reinterpret_cast<const float4*>(a.raw + row * a.rowbytes + seg) + h)
+                          : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int rr = r + u * (kSdThreads / Q);
+          if (rr >= nrows) break;
+          float* q = dst + rr * PW + 4 * h;
+          q[0] = v[u].x; q[1] = v[u].y; q[2] = v[u].z; q[3] = v[u].w;
+        }
+      }
+    } else {
+      constexpr int Q = sd_seg(NB) / 4;
+      const int k = threadIdx.x % Q;
+      const bool col = seg + 4 * k < a.rowbytes;
+      for (int r = threadIdx.x / Q; r < nrows; r += 4 * (kSdThreads / Q)) {
+        float v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int rr = r + u * (kSdThreads / Q);
+          const int64_t row = col && rr < nrows ? wrap(r0 + rr) : -1;
+          v[u] = row >= 0 ? __ldg(reinterpret_cast<const float*>(a.raw + row * a.rowbytes + seg) + k) : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int rr = r + u * (kSdThreads / Q);
+          if (rr < nrows) dst[rr * PW + k] = v[u];
+        }
+      }
+    }
+  } else if (a.align == 16) {
+    const int h = threadIdx.x & 1;
+    const bool col = seg + 16 * h < a.rowbytes;
+    for (int r = threadIdx.x >> 1; r < nrows; r += kSdThreads / 2) {
+      const int64_t row = col ? wrap(r0 + r) : -1;
+      cp_async16(buf + r * kSdSeg + 16 * h, row >= 0 ? a.raw + row * a.rowbytes + seg + 16 * h : a.raw,
+                 row >= 0);
+    }
+  } else {
+    const int k = threadIdx.x & 7;
+    const int left = (int)min(a.rowbytes - seg - 4 * k, (int64_t)4);  // bytes wanted of this word
+    if (r0 >= 0 && r0 + nrows <= a.nsamps) {
+      // whole rows of the block: the aligned words of four rows in flight
+      const uint32_t keep = left >= 4 ? 0xFFFFFFFFu : left > 0 ? (1u << (8 * left)) - 1u : 0u;
+      const uint8_t* p = a.raw + (r0 + (threadIdx.x >> 3)) * a.rowbytes + seg + 4 * k;
+      const int64_t step = (int64_t)(kSdThreads / 8) * a.rowbytes;
+      for (int r = threadIdx.x >> 3; r < nrows; r += kSdThreads / 2) {
+        uint32_t lo[4], hi[4], sh[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          sh[u] = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 3);
+          const uint32_t* w = reinterpret_cast<const uint32_t*>(p - sh[u]);
+          const bool on = left > 0 && r + u * (kSdThreads / 8) < nrows;
+          lo[u] = on ? __ldg(w) : 0u;
+          hi[u] = on && left + (int)sh[u] > 4 ? __ldg(w + 1) : 0u;
+          p += step;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int row = r + u * (kSdThreads / 8);
+          if (row < nrows)
+            *reinterpret_cast<uint32_t*>(buf + row * kSdSeg + 4 * k) = __funnelshift_r(lo[u], hi[u], 8 * sh[u]) & keep;
+        }
+      }
+    } else {
+      for (int r = threadIdx.x >> 3; r < nrows; r += kSdThreads / 8) {
+        const int64_t row = wrap(r0 + r);
+        *reinterpret_cast<uint32_t*>(buf + r * kSdSeg + 4 * k) =
+            row >= 0 ? row_word(a.raw, a.rowbytes, row, seg, k) : 0u;
+      }
+    }
+  }
+}
+
+template <int NB, int G, int MAXC>
+__global__ void __launch_bounds__(kSdThreads, 2)
+k_dedisp_stream(const __grid_constant__ SdArgs<MAXC> a) {
+  extern __shared__ __align__(16) uint8_t sm[];
+  constexpr int CH = 8 * sd_seg(NB) / NB;  // channels per slab
+  const int64_t t0 = (int64_t)blockIdx.x * a.T;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // byte offset of every channel's first row and byte (float32: of its word)
+  int32_t* tab = reinterpret_cast<int32_t*>(sm + (int64_t)a.stages * a.stage_bytes);
+  for (int c = threadIdx.x; c < a.nslab * CH; c += kSdThreads)
+    tab[c] = NB == 32 ? a.off[c] * sd_pitch(NB) + 4 * (c % CH) : a.off[c] * kSdSeg + (c % CH) * NB / 8;
+  const int ahead = a.stages - 1;
+  for (int s = 0; s < ahead; ++s) {
+    if (s < a.nslab) sd_stage<NB, MAXC>(a, sm + (int64_t)s * a.stage_bytes, t0, s);
+    cp_async_commit();
+  }
+  const int i = lane & 3, j = lane >> 2;
+  const int obase = NB == 32 ? warp * 32 * G + lane : warp * 4 * G + i;  // first output row
+  int32_t acc[G];
+  double dacc[G];
+#pragma unroll
+  for (int g = 0; g < G; ++g) { acc[g] = 0; dacc[g] = 0.0; }
+  int buf = 0, fill = ahead;
+  for (int s = 0; s < a.nslab; ++s) {
+    cp_async_wait_n(ahead - 1);  // slab s has landed
+    __syncthreads();
+    if (s + ahead < a.nslab) sd_stage<NB, MAXC>(a, sm + (int64_t)fill * a.stage_bytes, t0, s + ahead);
+    cp_async_commit();
+    const uint8_t* base = sm + (int64_t)buf * a.stage_bytes;
+    if (++buf == a.stages) buf = 0;
+    if (++fill == a.stages) fill = 0;
+    if constexpr (NB == 32) {
+      const uint8_t* p = base + obase * sd_pitch(NB);
+#pragma unroll
+      for (int c = 0; c < CH; ++c) {
+        const uint8_t* q = p + tab[s * CH + c];
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+          dacc[g] += (double)*reinterpret_cast<const float*>(q + g * 32 * sd_pitch(NB));
+      }
+    } else {
+      constexpr int CPW = 32 / NB;             // channels per 4-byte word
+      constexpr int KG = CPW < 16 ? CPW : 16;  // taken at a time
+      constexpr int PB = 8 / NB;               // channels per byte
+      uint32_t mask[PB], sh[PB];
+#pragma unroll
+      for (int p = 0; p < PB; ++p) {
+        sh[p] = (a.bitorder == SPP_BITORDER_BIG) ? 8 - (p + 1) * NB : p * NB;
+        mask[p] = ((1u << NB) - 1u) << sh[p];
+      }
+      const uint8_t* p0 = base + obase * kSdSeg;
+#pragma unroll
+      for (int kg = 0; kg < CPW; kg += KG) {
+        const uint8_t* q[KG];
+#pragma unroll
+        for (int k = 0; k < KG; k += 4) {
+          const int4 o = *reinterpret_cast<const int4*>(tab + s * CH + j * CPW + kg + k);
+          q[k] = p0 + o.x;
+          q[k + 1] = p0 + o.y;
+          q[k + 2] = p0 + o.z;
+          q[k + 3] = p0 + o.w;
+        }
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          uint32_t part[PB];
+#pragma unroll
+          for (int p = 0; p < PB; ++p) part[p] = 0u;
+#pragma unroll
+          for (int k = 0; k < KG; ++k) {
+            const uint32_t b = q[k][g * 4 * kSdSeg];
+            part[k % PB] += NB == 8 ? b : b & mask[k % PB];
+          }
+#pragma unroll
+          for (int p = 0; p < PB; ++p) acc[g] += (int32_t)(NB == 8 ? part[p] : part[p] >> sh[p]);
+        }
+      }
+    }
+  }
+  if constexpr (NB == 32) {
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      const int64_t t = t0 + obase + 32 * g;
+      if (t < a.nvalid) a.out[t] = (float)dacc[g];
+    }
+  } else {
+    // sum over the eight words (lanes with equal i); lane (i, j) writes groups j, j + 8
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      acc[g] += __shfl_xor_sync(0xffffffffu, acc[g], 4);
+      acc[g] += __shfl_xor_sync(0xffffffffu, acc[g], 8);
+      acc[g] += __shfl_xor_sync(0xffffffffu, acc[g], 16);
+      const int64_t t = t0 + obase + 4 * g;
+      if ((g & 7) == j && t < a.nvalid) a.out[t] = (float)acc[g];
+    }
+  }
+}
+
+template <int NB, int MAXC>
+static void (*sd_kernel(int G))(const SdArgs<MAXC>) {
+  if (NB == 32) return G <= 1 ? k_dedisp_stream<NB, 1, MAXC> : G <= 2 ? k_dedisp_stream<NB, 2, MAXC> : k_dedisp_stream<NB, 4, MAXC>;
+  return G <= 2 ? k_dedisp_stream<NB, 2, MAXC> : G <= 4 ? k_dedisp_stream<NB, 4, MAXC>
+         : G <= 8 ? k_dedisp_stream<NB, 8, MAXC> : G <= 12 ? k_dedisp_stream<NB, 12, MAXC>
+                                                           : k_dedisp_stream<NB, 16, MAXC>;
+}
+
+template <int NB, int MAXC>
+static int launch_stream(const uint8_t* raw, int bitorder, int64_t nchans, int64_t nsamps,
+                         const int32_t* d, float* out, int64_t nvalid, cudaStream_t st) {
+  constexpr int CH = 8 * sd_seg(NB) / NB;
+  constexpr int pitch = sd_pitch(NB);
+  constexpr int unit = NB == 32 ? 32 * kSdWarps : 4 * kSdWarps;  // outputs per G
+  static const int kG[] = {1, 2, 4, 8, 12, 16};
+  SdArgs<MAXC> a{};
+  a.nslab = (int32_t)ceil_div(nchans, CH);
+  int32_t spread = 0;
+  for (int s = 0; s < a.nslab; ++s) {
+    const int64_t c0 = (int64_t)s * CH, c1 = std::min<int64_t>(nchans, c0 + CH);
+    const int32_t mn = *std::min_element(d + c0, d + c1), mx = *std::max_element(d + c0, d + c1);
+    if (mx - mn > 60000) return SPP_ERR_UNSUPPORTED;
+    spread = std::max(spread, mx - mn);
+    a.mn[s] = mn;
+    a.rows[s] = (uint16_t)(mx - mn);
+    // channels past the last read zeros: offset 0 of a zero-filled byte
+    for (int64_t c = c0; c < c1; ++c) a.off[c] = (uint16_t)(d[c] - mn);
+  }
+  // outputs per CTA: two CTAs per SM where they fit, and the least estimated
+  // time: waves x slabs x the longer of a slab's rows (2.7 ns each at two CTAs
+  // per SM) and a copy's latency (1.5 us) over the slabs in flight, or both in
+  // part where the copies go through registers
+  const int64_t tab = (int64_t)a.nslab * CH * 4;
+  a.rowbytes = NB == 32 ? nchans * 4 : nchans * NB / 8;
+  const uintptr_t both = (uintptr_t)a.rowbytes | reinterpret_cast<uintptr_t>(raw);
+  a.align = both % 16 == 0 ? 16 : both % 4 == 0 ? 4 : 1;
+  const bool async = NB != 32 && a.align == 16;
+  int G = 0;
+  int64_t smem = 0;
+  for (int cps = 2; cps >= 1 && G == 0; --cps) {
+    const int64_t room = (cps == 2 ? 113 : 226) * 1024 - tab;
+    double best = 0.0;
+    for (int g : kG) {
+      if (NB == 32 ? g > 4 : g < 2) continue;
+      const int64_t T = (int64_t)unit * g;
+      const int64_t stage = round_up((T + spread) * pitch, 16);
+      if (2 * stage > room) break;
+      const int64_t stages = std::min<int64_t>(async ? 6 : 2, room / stage);
+      const double rows_us = 2.7e-3 * (double)(T + spread);
+      const double slab_us = async ? std::max(rows_us, 1.5 / (double)(stages - 1)) : rows_us + 0.7;
+      const double t = (double)ceil_div(ceil_div(nvalid, T), 148 * cps) * slab_us;
+      if (G == 0 || t < best) {
+        best = t;
+        G = g;
+        a.T = (int32_t)T;
+        a.stage_bytes = (int32_t)stage;
+        a.stages = (int32_t)stages;
+        smem = stages * stage + tab;
+      }
+    }
+  }
+  if (G == 0) return SPP_ERR_UNSUPPORTED;
+  a.raw = raw;
+  a.nsamps = nsamps;
+  a.out = out;
+  a.nvalid = nvalid;
+  a.bitorder = bitorder;
+  const int64_t gx = ceil_div(nvalid, a.T);
+  if (gx > INT32_MAX) return SPP_ERR_UNSUPPORTED;
+  auto fn = sd_kernel<NB, MAXC>(G);
+  int rc = set_smem_attr(reinterpret_cast<const void*>(fn), smem);
+  if (rc) return rc;
+  fn<<<(unsigned)gx, kSdThreads, smem, st>>>(a);
+  return cuda_status(cudaGetLastError(), "single-DM stream launch");
+}
+
+// Any width, up to 4096 channels, delays in host memory; SPP_ERR_UNSUPPORTED
+// (nothing launched) outside that or where a slab's delay spread does not fit.
+int launch_single_stream(const void* in, int nbits, int bitorder, int64_t nchans, int64_t nsamps,
+                         const int32_t* delays_host, float* out, int64_t nvalid, cudaStream_t st) {
+  if (nchans > 4096 || (nbits == 32 && (reinterpret_cast<uintptr_t>(in) & 3) != 0))
+    return SPP_ERR_UNSUPPORTED;
+  const uint8_t* raw = static_cast<const uint8_t*>(in);
+#define SPP_SD(NB)                                                                              \
+  case NB:                                                                                      \
+    return nchans <= 1024                                                                       \
+               ? launch_stream<NB, 1024>(raw, bitorder, nchans, nsamps, delays_host, out, nvalid, st) \
+               : launch_stream<NB, 4096>(raw, bitorder, nchans, nsamps, delays_host, out, nvalid, st)
+  switch (nbits) {
+    SPP_SD(1);
+    SPP_SD(2);
+    SPP_SD(4);
+    SPP_SD(8);
+    SPP_SD(32);
+    default: return SPP_ERR_UNSUPPORTED;
+  }
+#undef SPP_SD
+}
+
 }  // namespace spp

@@ -97,8 +97,10 @@ def dedisperse_block(raw: torch.Tensor, delays: np.ndarray, nchans: int, nsamps:
     (uint8 packed or float32).  ``delays`` is the host int32 table (its range
     bounds the kernel's checks); ``delays_dev`` may carry a device copy.
     8-bit blocks go through ``spp_dedisperse_hd`` (offsets precomputed from the
-    host table) when their shape allows, else through ``spp_dedisperse``;
-    ``host_table`` True/False forces one of the two.
+    host table) when their shape allows; other blocks through
+    ``spp_dedisperse_host`` (any width, the host table in its parameters), else
+    through ``spp_dedisperse``.  ``host_table`` True/False forces the first or
+    the last.
     """
     raw = _as_raw(raw)
     nb = _nbits_of(raw, nbits)
@@ -122,6 +124,18 @@ def dedisperse_block(raw: torch.Tensor, delays: np.ndarray, nchans: int, nsamps:
             _lib.check(rc)
     elif host_table:
         raise NotImplementedError("the host-table path covers 8-bit data")
+    # 8-bit rows aligned to 4 bytes only, over a short delay range: the device-
+    # table kernel copies them in one pass without touching registers (1020
+    # channels x 100000 samples, DM 100: 91 us against 125 us)
+    narrow = nb == 8 and nchans % 4 == 0 and nchans % 16 != 0 and dmax - dmin <= 2600
+    if host_table is None and not narrow and (nb != 32 or acc == _lib.ACC_F64):
+        rc = lib.spp_dedisperse_host(raw.data_ptr(), nb, bitorder_code(bitorder), nchans, nsamps,
+                                     delays.ctypes.data, out.data_ptr(), out.numel(), out_start,
+                                     st)
+        if rc == _lib.SPP_OK:
+            return nvalid
+        if rc != _lib.SPP_ERR_UNSUPPORTED:
+            _lib.check(rc)
     need = lib.spp_dedisperse_workspace_bytes(nb, nchans, nsamps, dmin, dmax)
     if need < 0:
         _lib.check(_lib.SPP_ERR_ARG)
