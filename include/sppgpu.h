@@ -414,7 +414,7 @@ typedef struct spp_dmt_item {
   int32_t dlo, dhi;       /* range of sign*delay (checked on the device)     */
   int32_t span_max;       /* max over channels of the tile's delay spread    */
   int32_t out_kind;       /* SPP_OUT_F32 / _I32 / _U16                       */
-  int32_t reserved;
+  int32_t pack_rows;      /* 16-bit rows: so many rows sum below 65536 (0: 1) */
 } spp_dmt_item;           /* 112 bytes */
 
 int spp_wl_num_variants(int nbits, int acc);

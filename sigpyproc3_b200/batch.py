@@ -18,7 +18,7 @@ from . import _lib
 ITEM_DTYPE = np.dtype({
     "names": ["planar", "pitch_w", "halo", "delays", "dpitch", "out", "out_stride", "out_start",
               "nvalid", "t0", "nchans", "nrows", "sign", "dlo", "dhi", "span_max", "out_kind",
-              "reserved"],
+              "pack_rows"],
     "formats": ["<u8", "<i8", "<i8", "<u8", "<i8", "<u8", "<i8", "<i8", "<i8", "<i8", "<i4", "<i4",
                 "<i4", "<i4", "<i4", "<i4", "<i4", "<i4"],
     "offsets": [0, 8, 16, 24, 32, 40, 48, 56, 64, 72, 80, 84, 88, 92, 96, 100, 104, 108],
@@ -93,12 +93,14 @@ class WorkList:
     def add_job(self, *, planar_ptr: int, pitch_w: int, halo: int, nchans: int,
                 delays_dev: torch.Tensor, delays_host: np.ndarray, out_ptr: int, out_stride: int,
                 out_start: int, out_elem: int, nvalid: int, out_kind: int, sign: int = 1,
-                row_stride_out: int | None = None, span: int | None = None) -> None:
+                row_stride_out: int | None = None, span: int | None = None,
+                max_value: int = 65535) -> None:
         """One DM-time job: rows of ``delays`` (ndm x >= nchans, row pitch =
         delays_dev.stride(0)) against ``nchans`` planar rows; output row r at
         out_ptr + r * out_stride * out_elem.  ``span``: the job's tile span
         (``tile_span`` of the signed delays for this variant's DW), when the
-        caller has it cached."""
+        caller has it cached.  ``max_value``: largest value in 16-bit rows (rows
+        whose sum stays below 65536 are added two samples at a time)."""
         if not counter_fits(self.cfg, self.nbits, nchans):
             raise ValueError(f"work-list variant {self.variant}: sums of {nchans} {self.nbits}-bit "
                              "samples overflow its bit-sliced counter")
@@ -134,6 +136,7 @@ class WorkList:
         rec["dlo"] = dlo
         rec["dhi"] = dhi
         rec["out_kind"] = out_kind
+        rec["pack_rows"] = max(1, 65535 // max(1, int(max_value)))
         self._rows.append(rec)
 
     def layout(self, nvalid: int, omin: int, omax: int, slot_w: int | None = None):

@@ -40,12 +40,24 @@ static const std::vector<WlVariant>& wl_variants() {
       mkwlb<1, 2, 8, 1, 2, 64>(), mkwlb<1, 2, 8, 1, 3, 32>(),
       mkwlb<2, 2, 8, 1, 2, 32, 80, 4>(), mkwlb<2, 2, 8, 1, 2, 32, 128, 4>(),
       mkwlb<2, 2, 8, 1, 2, 64>(), mkwlb<2, 2, 8, 1, 3, 32>(),
-      // bit-sliced 4- and 8-bit ahead of the SIMD kernels (faster at every span)
+      // bit-sliced 4-bit ahead of the SIMD kernels (faster at every span)
       mkwlb<4, 2, 8, 1, 2, 16, 96, 3>(), mkwlb<4, 2, 8, 1, 2, 16, 128, 3>(),
       mkwlb<4, 2, 8, 1, 2, 16>(),
+      // 8-bit byte lanes, eight words per thread: an item of 8 trials x 1024
+      // samples is long enough to hide the next one's claim and delay reads
+      // (two words per thread, 256 samples: 2.54 ms for the first stage of two
+      // beams, 32 groups x 1024 channels; 1.17 ms here, 3.48 ms bit-sliced; 512
+      // trials x 1024 channels x 63616 outputs: 2.74 against 3.26 ms).  The bit-
+      // sliced shapes take spreads beyond its shared memory.
+      mkwl<8, 8, 8, 1, 32, 2, 0>(),
       mkwlb<8, 2, 8, 1, 2, 16, 96, 2>(), mkwlb<8, 2, 8, 1, 2, 16, 0, 2>(),
       mkwlb<8, 1, 8, 1, 2, 16>(),
-      SPP_WL_INT(1), SPP_WL_INT(2), SPP_WL_INT(4), SPP_WL_INT(8), SPP_WL_INT(16),
+      mkwl<8, 4, 8, 1, 32, 2, 0>(), mkwl<8, 8, 4, 2, 32, 2, 0>(), mkwl<8, 4, 8, 1, 32, 3, 0>(),
+      SPP_WL_INT(1), SPP_WL_INT(2), SPP_WL_INT(4),
+      // 16-bit rows (second subband stage): 8 trials x 512 samples per item, 0.89
+      // ms for two beams x 512 trials x 32 subbands against 3.80 ms with 128
+      mkwl<16, 8, 8, 1, 32, 2, 0>(), mkwl<16, 16, 8, 1, 32, 2, 0>(), mkwl<16, 4, 8, 1, 32, 2, 0>(),
+      mkwl<16, 2, 4, 2, 64, 3, 0>(),
       mkwl<32, 8, 8, 1, 32, 2, SPP_ACC_KAHAN32>(), mkwl<32, 4, 8, 2, 32, 2, SPP_ACC_KAHAN32>(),
       mkwl<32, 8, 8, 1, 32, 2, SPP_ACC_F64>(),     mkwl<32, 4, 8, 2, 32, 2, SPP_ACC_F64>(),
   };

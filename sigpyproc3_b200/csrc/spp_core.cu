@@ -126,7 +126,9 @@ static const std::vector<Variant>& variants() {
       // within a third of shared memory
       mkb<4, 2, 8, 1, 2, 16, 96, 3>(), mkb<4, 2, 8, 1, 2, 16>(),
       SPP_INT_VARIANTS(4),
-      // eight plane rows per channel, 20-level counters
+      // byte lanes, eight words per thread: 1.2e13 channel-adds/s, also on wide
+      // spreads; then eight plane rows per channel (1.0e13) for the widest
+      mk<8, 8, 8, 1, 32, 2, 0>(0),
       mkb<8, 2, 8, 1, 2, 16, 96, 2>(), mkb<8, 2, 8, 1, 2, 16, 0, 2>(), mkb<8, 1, 8, 1, 2, 16>(),
       SPP_INT_VARIANTS(8),
       mk<8, 4, 1, 4, 16, 3, 0>(1),
@@ -748,7 +750,7 @@ static int first_choice(const spp_dmt_plan* p) {
     }
     return pick;
   }
-  const double adds_per_us = p->nbits == 1 ? 8.2e7 : p->nbits == 2 ? 5.0e7 : p->nbits == 4 ? 2.2e7 : 1.0e7;
+  const double adds_per_us = p->nbits == 1 ? 8.2e7 : p->nbits == 2 ? 5.0e7 : p->nbits == 4 ? 2.2e7 : 1.2e7;
   double best = 1.5 * (double)p->ndm * nvalid * p->nchans / adds_per_us + 20.0;
   const int64_t prows = p->ilv_rows[1].nrows;
   const bool shared_pairs = p->nbits == 2 && prows > 0 && p->ndm * (p->nchans / 2) >= 100 * prows;

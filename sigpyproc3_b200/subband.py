@@ -154,7 +154,8 @@ class SubbandSearch:
                 planar_ptr=b.sub.data_ptr() + g * p.nsub * b.pitch2 * 4, pitch_w=b.pitch2, halo=0,
                 nchans=p.nsub, delays_dev=self.dsub_dev[i0:i1], delays_host=p.dsub[i0:i1],
                 out_ptr=b.dmt.data_ptr() + i0 * b.dmt.stride(0) * 4, out_stride=b.dmt.stride(0),
-                out_start=0, out_elem=4, nvalid=b.nvalid, out_kind=_lib.OUT_I32)
+                out_start=0, out_elem=4, nvalid=b.nvalid, out_kind=_lib.OUT_I32,
+                max_value=min(65535, 255 * p.cps))
 
     def run(self, stream: torch.cuda.Stream | None = None, snr: bool = True) -> None:
         """Enqueue the whole batch on `stream` (no host synchronisation)."""
