@@ -80,6 +80,19 @@ int spp_status_clear(void* workspace, void* stream);
 int spp_host_register(void* ptr, int64_t bytes);
 int spp_host_unregister(void* ptr);
 
+/* Copies of a block stream through two device buffers.  spp_blocks_put copies
+ * `halo_bytes` device bytes and then `bytes` host bytes to `dst` (buffer k) on
+ * the copy stream: after the work that the compute stream had when the next
+ * block after buffer k's last was put (on first use: when the handle was
+ * created), and before whatever the compute stream is given next.
+ * spp_blocks_wait blocks until the last copy into buffer k has left the host
+ * memory; spp_blocks_destroy (null is fine) waits for every copy first. */
+int spp_blocks_create(void** handle, void* copy_stream, void* compute_stream);
+int spp_blocks_put(void* handle, int k, void* dst, const void* halo, int64_t halo_bytes,
+                   const void* src, int64_t bytes);
+int spp_blocks_wait(void* handle, int k);
+int spp_blocks_destroy(void* handle);
+
 /* ---- R4: unpack -------------------------------------------------------------
  * Replaces kernels.unpack{1,2,4}_8_{big,little} (core/kernels.py:20-69) and
  * io/bits.py unpack (:19-70): `nbytes` packed bytes -> nbytes*8/nbits uint8
@@ -130,6 +143,15 @@ int spp_dedisperse_host(const void* in, int nbits, int bitorder, int64_t nchans,
                         int64_t nsamps, const int32_t* delays_host, float* out,
                         int64_t out_len, int64_t out_start, void* stream);
 
+/* The faster of spp_dedisperse_hd and spp_dedisperse_host for the block: the
+ * number of samples written (0 for a block no longer than the largest delay),
+ * or a status (SPP_ERR_UNSUPPORTED, nothing launched: callers then use
+ * spp_dedisperse; float32 with SPP_ACC_KAHAN32 is one such case, a negative
+ * bit order on a block that spp_dedisperse_hd does not take another). */
+int64_t spp_dedisperse_block(const void* in, int nbits, int bitorder, int64_t nchans,
+                             int64_t nsamps, const int32_t* delays_host, int acc, float* out,
+                             int64_t out_len, int64_t out_start, void* stream);
+
 /* ---- folding -------------------------------------------------------------
  * Replaces kernels.fold (core/kernels.py:403-445) for one read_plan block
  * (Filterbank.fold, base.py:1109-1207): sample t of the block (t < nsamps -
@@ -160,6 +182,12 @@ int spp_fold_exact(const void* in, int64_t nchans, int64_t nsamps,
                    int32_t nbins, int32_t nints, int32_t nsubs, int64_t index,
                    const int32_t* band_start, unsigned long long* fold_sums,
                    int32_t* count_ar, int64_t cells, void* stream);
+
+/* Cells to means in float32: sums (64-bit if `sums64` is given, else the float32
+ * `fold`) rounded to float32, divided by the counts in float64 and rounded, as
+ * numpy divides float32 sums by int32 counts (0 / 0 is NaN). */
+int spp_fold_finish(const float* fold, const unsigned long long* sums64, const int32_t* count,
+                    int64_t cells, float* out, void* stream);
 
 /* Same computation as spp_dedisperse, but allocating nothing and taking no
  * workspace.  No counterpart in the reference.  It serves callers that must not

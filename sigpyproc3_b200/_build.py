@@ -40,7 +40,7 @@ def _stale() -> bool:
     if not LIB.exists():
         return True
     t = LIB.stat().st_mtime
-    deps = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(INCLUDE.glob("*.h"))
+    deps = [p for pat in ("*.cu", "*.cuh", "*.h") for p in CSRC.glob(pat)] + list(INCLUDE.glob("*.h"))
     return any(p.stat().st_mtime > t for p in deps)
 
 

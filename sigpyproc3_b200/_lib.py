@@ -50,6 +50,12 @@ SIGNATURES: dict[str, tuple[list, object]] = {
     "spp_dedisperse": ([_p, _int, _int, _i64, _i64, _p, _i32, _i32, _p, _i64, _i64, _int, _p,
                         _i64, _p], _int),
     "spp_dedisperse_hd": ([_p, _int, _i64, _i64, _p, _p, _i64, _i64, _p], _int),
+    "spp_dedisperse_block": ([_p, _int, _int, _i64, _i64, _p, _int, _p, _i64, _i64, _p], _i64),
+    "spp_blocks_create": ([_p, _p, _p], _int),
+    "spp_blocks_put": ([_p, _int, _p, _p, _i64, _p, _i64], _int),
+    "spp_blocks_wait": ([_p, _int], _int),
+    "spp_blocks_destroy": ([_p], _int),
+    "spp_fold_finish": ([_p, _p, _p, _i64, _p, _p], _int),
     "spp_dedisperse_host": ([_p, _int, _int, _i64, _i64, _p, _p, _i64, _i64, _p], _int),
     "spp_fold": ([_p, _int, _i64, _i64, _p, _i32, ctypes.c_float, ctypes.c_float, ctypes.c_float,
                   _i64, _i32, _i32, _i32, _i64, _p, _p, _p, _i64, _p], _int),

@@ -97,6 +97,16 @@ __global__ void k_fold(const FoldArgs a) {
   atomicAdd(a.count_ar + pos2, c1 - c0);
 }
 
+// The cube leaves the device once, as the 4-byte means, in place of 12 bytes of
+// sums and counts per cell and three host passes over them.
+__global__ void k_fold_finish(const float* __restrict__ fold, const unsigned long long* __restrict__ sums,
+                              const int32_t* __restrict__ count, int64_t cells, float* __restrict__ out) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= cells) return;
+  const float s = sums ? __ll2float_rn((long long)sums[i]) : fold[i];
+  out[i] = __double2float_rn(__ddiv_rn((double)s, (double)count[i]));
+}
+
 }  // namespace spp
 
 using namespace spp;
@@ -167,4 +177,13 @@ extern "C" int spp_fold_exact(const void* in, int64_t nchans, int64_t nsamps,
   return fold_impl(in, 8, nchans, nsamps, delays, maxdelay, tsamp, period, accel, total_nsamps,
                    nbins, nints, nsubs, index, band_start, nullptr, fold_sums, count_ar, cells,
                    stream);
+}
+
+extern "C" int spp_fold_finish(const float* fold, const unsigned long long* sums64,
+                               const int32_t* count, int64_t cells, float* out, void* stream) {
+  if ((!fold && !sums64) || !count || !out) return fail(SPP_ERR_ARG, "spp_fold_finish: null pointer");
+  if (cells <= 0) return fail(SPP_ERR_ARG, "spp_fold_finish: no cells");
+  k_fold_finish<<<(unsigned)ceil_div(cells, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+      fold, sums64, count, cells, out);
+  return cuda_status(cudaGetLastError(), "fold finish launch");
 }

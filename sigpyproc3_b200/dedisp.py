@@ -107,35 +107,37 @@ def dedisperse_block(raw: torch.Tensor, delays: np.ndarray, nchans: int, nsamps:
     delays = np.ascontiguousarray(delays, dtype=np.int32)
     if delays.size != nchans:
         raise ValueError(f"delays has {delays.size} entries for {nchans} channels")
+    if not delays.size:
+        raise ValueError("no channels")
+    if out.dtype != torch.float32 or not out.is_cuda:
+        # a block no longer than its largest delay writes nothing, whatever `out` is
+        if nsamps <= max(abs(int(delays.min())), abs(int(delays.max()))):
+            return 0
+        raise TypeError("out must be a CUDA float32 tensor")
+    lib = _lib.load()
+    st = stream_handle(stream, raw.device)
+    if host_table is None:
+        # spp_dedisperse_hd asks for no bit order; an unknown one keeps the
+        # block from the other kernels, and is refused further down
+        known = bitorder in ("big", "b", "little", "l")
+        order = bitorder_code(bitorder) if nb != 8 or known else -1
+        rc = lib.spp_dedisperse_block(raw.data_ptr(), nb, order, nchans, nsamps,
+                                      delays.ctypes.data, acc, out.data_ptr(), out.numel(),
+                                      out_start, st)
+        if rc >= 0:
+            return rc
+        if rc != _lib.SPP_ERR_UNSUPPORTED:
+            _lib.check(rc)
     dmin, dmax = int(delays.min()), int(delays.max())
     nvalid = nsamps - max(abs(dmin), abs(dmax))
     if nvalid <= 0:
         return 0
-    if out.dtype != torch.float32 or not out.is_cuda:
-        raise TypeError("out must be a CUDA float32 tensor")
-    lib = _lib.load()
-    st = stream_handle(stream, raw.device)
-    if nb == 8 and host_table is not False:
-        rc = lib.spp_dedisperse_hd(raw.data_ptr(), nb, nchans, nsamps, delays.ctypes.data,
-                                   out.data_ptr(), out.numel(), out_start, st)
-        if rc == _lib.SPP_OK:
-            return nvalid
-        if rc != _lib.SPP_ERR_UNSUPPORTED or host_table:
-            _lib.check(rc)
-    elif host_table:
-        raise NotImplementedError("the host-table path covers 8-bit data")
-    # 8-bit rows aligned to 4 bytes only, over a short delay range: the device-
-    # table kernel copies them in one pass without touching registers (1020
-    # channels x 100000 samples, DM 100: 91 us against 125 us)
-    narrow = nb == 8 and nchans % 4 == 0 and nchans % 16 != 0 and dmax - dmin <= 2600
-    if host_table is None and not narrow and (nb != 32 or acc == _lib.ACC_F64):
-        rc = lib.spp_dedisperse_host(raw.data_ptr(), nb, bitorder_code(bitorder), nchans, nsamps,
-                                     delays.ctypes.data, out.data_ptr(), out.numel(), out_start,
-                                     st)
-        if rc == _lib.SPP_OK:
-            return nvalid
-        if rc != _lib.SPP_ERR_UNSUPPORTED:
-            _lib.check(rc)
+    if host_table:
+        if nb != 8:
+            raise NotImplementedError("the host-table path covers 8-bit data")
+        _lib.check(lib.spp_dedisperse_hd(raw.data_ptr(), nb, nchans, nsamps, delays.ctypes.data,
+                                         out.data_ptr(), out.numel(), out_start, st))
+        return nvalid
     need = lib.spp_dedisperse_workspace_bytes(nb, nchans, nsamps, dmin, dmax)
     if need < 0:
         _lib.check(_lib.SPP_ERR_ARG)

@@ -5,12 +5,13 @@
 ``FilReader.read_plan`` (src/sigpyproc/readers.py:171-233).  Blocks travel
 as raw bytes: file -> pinned host buffer -> async H2D (copy stream) -> HBM,
 double-buffered, and the GPU kernels unpack them in their load path.  The
-``skipback`` halo is re-read exactly as the reference does, so results are
-identical block for block.
+``skipback`` halo leads every block as in the reference (read again, or copied
+on the device where it is long), so results are identical block for block.
 """
 
 from __future__ import annotations
 
+import ctypes
 import warnings
 from collections.abc import Callable, Iterator
 from pathlib import Path
@@ -51,6 +52,12 @@ def plan_blocks(nsamples: int, gulp: int, start: int, nsamps: int | None,
 # In-memory filterbanks up to this size are page-locked in place on first use.
 REGISTER_MAX_BYTES = 8 << 30
 
+# A halo of this size or more is copied from the previous block on the device:
+# that copy, between two from the host, holds the copy stream up by 27 us
+# whatever its size, in which the host link moves 1.5 MB (8-bit, 64 MB in 16384-row
+# blocks or longer: 2.3 ms either way at 1.5 MB, 2.80 -> 2.23 ms at 2.5 MB).
+KEEP_HALO_MIN_BYTES = 3 << 19
+
 
 def pinned_allocator(nbytes: int) -> torch.Tensor:
     return torch.empty(nbytes, dtype=torch.uint8, pin_memory=True)
@@ -75,6 +82,26 @@ def _allocate(allocator: Callable[[int], object], nbytes: int):
         raise ValueError(f"Allocated buffer is not the expected size: {view.nbytes} (actual) "
                          f"!= {nbytes} (expected)")
     return buf
+
+
+class _DelayTable:
+    """Delays on the device, uploaded (and the workspace's status words cleared)
+    when a kernel that reads them is first launched: most blocks go through
+    kernels that take the delays from the host."""
+
+    def __init__(self, delays: np.ndarray, dev: torch.device, ws: torch.Tensor):
+        self._delays, self._dev, self._ws = delays, dev, ws
+        self._t: torch.Tensor | None = None
+
+    @property
+    def used(self) -> bool:
+        return self._t is not None
+
+    def data_ptr(self) -> int:
+        if self._t is None:
+            self._t = torch.from_numpy(self._delays).to(self._dev)
+            status_clear(self._ws)
+        return self._t.data_ptr()
 
 
 class Filterbank:
@@ -111,12 +138,15 @@ class Filterbank:
     # --- streaming (R5) ---
     def stream_blocks(self, gulp: int = 16384, start: int = 0, nsamps: int | None = None,
                       skipback: int = 0, *, allocator: Callable[[int], object] | None = None,
-                      description: str | None = None, quiet: bool = False
-                      ) -> Iterator[tuple[int, int, torch.Tensor]]:
+                      description: str | None = None, quiet: bool = False,
+                      keep_halo: bool = False) -> Iterator[tuple[int, int, torch.Tensor]]:
         """Yields ``(nsamps_read, ii, raw)``: ``raw`` is a CUDA uint8 tensor of
         the block's raw bytes, valid until the next iteration.  Work the
         consumer enqueues on the current stream is ordered before the buffer
-        is refilled."""
+        is refilled.  ``keep_halo``: a consumer that leaves ``raw`` as it is
+        lets each block take its first ``skipback`` rows from the previous
+        block on the device, where they are many (the same bytes; a caller's
+        allocator always sees whole blocks)."""
         gulp, blocks = plan_blocks(self.header.nsamples, gulp, start, nsamps, skipback)
         rb = self.row_bytes
         if self.header.nbits < 8 and (self.header.nchans * self.header.nbits) % 8:
@@ -133,38 +163,43 @@ class Filterbank:
             hviews = [_host_view(h) for h in host]
         devbuf = [torch.empty(nbytes, dtype=torch.uint8, device=dev) for _ in range(2)]
         copy_stream = torch.cuda.Stream(dev)
-        compute = torch.cuda.current_stream(dev)
-        copied = [torch.cuda.Event() for _ in range(2)]
-        consumed = [torch.cuda.Event() for _ in range(2)]
-        used = [False, False]
+        lib = _lib.load()
+        handle = ctypes.c_void_p()
+        _lib.check(lib.spp_blocks_create(ctypes.byref(handle), copy_stream.cuda_stream,
+                                         stream_handle(None, dev)))
+        dptr = [d.data_ptr() for d in devbuf]
         pos = start * rb
-        for ii, nsamp_blk, skip in blocks:
-            k = ii & 1
-            want = nsamp_blk * rb
-            src = self._device_source(pos, want) if direct else None
-            if src is None:
-                if direct:
-                    got = self._bytes_available(pos, want)
-                    raise ValueError(f"Unexpected number of bytes read from file {got} (actual) "
-                                     f"!= {want} (expected)")
-                if used[k]:
-                    copied[k].synchronize()  # host buffer k is free once its copy landed
-                got = self._read_bytes(pos, hviews[k][:want])
-                if got != want:
-                    raise ValueError(f"Unexpected number of bytes read from file {got} (actual) "
-                                     f"!= {want} (expected)")
-                src = (host[k] if torch.is_tensor(host[k]) else torch.from_numpy(hviews[k]))[:want]
-            pos += want + skip * rb
-            with torch.cuda.stream(copy_stream):
-                if used[k]:
-                    copy_stream.wait_event(consumed[k])
-                devbuf[k][:want].copy_(src, non_blocking=True)
-                copied[k].record(copy_stream)
-            compute.wait_event(copied[k])
-            used[k] = True
-            yield nsamp_blk, ii, devbuf[k][:want]
-            consumed[k].record(compute)
-        torch.cuda.current_stream(dev).synchronize()
+        back = abs(skipback) * rb if keep_halo and allocator is None else 0
+        if back < KEEP_HALO_MIN_BYTES:
+            back = 0
+        try:
+            for n, (ii, nsamp_blk, skip) in enumerate(blocks):
+                k = n & 1
+                want = nsamp_blk * rb
+                # already on the device: only the last block is shorter than the gulp
+                old = min(back, want) if n else 0
+                src = self._device_source(pos + old, want - old) if direct else None
+                if src is None:
+                    if direct:
+                        got = self._bytes_available(pos, want)
+                        raise ValueError(f"Unexpected number of bytes read from file {got} "
+                                         f"(actual) != {want} (expected)")
+                    if n > 1:  # host buffer k is free once its copy landed
+                        _lib.check(lib.spp_blocks_wait(handle, k))
+                    got = old + self._read_bytes(pos + old, hviews[k][:want - old])
+                    if got != want:
+                        raise ValueError(f"Unexpected number of bytes read from file {got} "
+                                         f"(actual) != {want} (expected)")
+                    sptr = hviews[k].ctypes.data
+                else:
+                    sptr = src.data_ptr()
+                pos += want + skip * rb
+                _lib.check(lib.spp_blocks_put(handle, k, dptr[k], dptr[1 - k] + nbytes - back, old,
+                                              sptr, want - old))
+                yield nsamp_blk, ii, devbuf[k][:want]
+            torch.cuda.current_stream(dev).synchronize()
+        finally:
+            _lib.check(lib.spp_blocks_destroy(handle))
 
     def read_plan(self, gulp: int = 16384, start: int = 0, nsamps: int | None = None,
                   skipback: int = 0, description: str | None = None, *, quiet: bool = False,
@@ -200,20 +235,20 @@ class Filterbank:
         tim_len = h.nsamples - max_delay
         dev = torch.device("cuda", torch.cuda.current_device())
         tim = torch.zeros(max(tim_len, 0), dtype=torch.float32, device=dev)
-        ddev = torch.from_numpy(chan_delays).to(dev)
         # one workspace for every block (a block never exceeds the gulp); its
         # device status words collect any kernel-side error over the whole run
         need = _lib.load().spp_dedisperse_workspace_bytes(
             h.nbits, h.nchans, min(gulp, h.nsamples), int(chan_delays.min()),
             int(chan_delays.max()))
         ws = workspace(max(int(need), 256), dev)
-        status_clear(ws)
+        table = _DelayTable(chan_delays, dev, ws)
         for nsamps_r, ii, raw in self.stream_blocks(gulp, start, nsamps, skipback=max_delay,
-                                                    **plan_kwargs):
+                                                    keep_halo=True, **plan_kwargs):
             dedisperse_block(raw, chan_delays, h.nchans, nsamps_r, tim, ii * (gulp - max_delay),
                              nbits=h.nbits, bitorder=self.bitorder, acc=_lib.ACC_F64,
-                             delays_dev=ddev, ws=ws)
-        status_check(ws)
+                             delays_dev=table, ws=ws)
+        if table.used:  # only kernels that read the table record a device status
+            status_check(ws)
         return TimeSeries(tim, h.new_header({"nchans": 1, "dm": dm, "nsamples": tim_len}))
 
     # --- R3: DM-trial batch ---
@@ -248,7 +283,7 @@ class Filterbank:
             ws = workspace(plan.workspace_bytes(min(gulp, span)), dev)
             status_clear(ws)
             for nsamps_r, ii, raw in self.stream_blocks(gulp, start, nsamps, skipback=max_delay,
-                                                        **plan_kwargs):
+                                                        keep_halo=True, **plan_kwargs):
                 plan.execute(raw, nsamps_r, out, out_start=ii * (gulp - max_delay), ws=ws)
             status_check(ws)
         finally:
@@ -399,7 +434,8 @@ class Filterbank:
         st = stream_handle(None, dev)
         with h.prep_outfile(outfile_name, updates=updates, nbits=32) as out_file:
             for nsamps_r, _ii, raw in self.stream_blocks(gulp, start, nsamps,
-                                                        skipback=max_delay, **plan_kwargs):
+                                                        skipback=max_delay, keep_halo=True,
+                                                        **plan_kwargs):
                 nout = nsamps_r - max_delay
                 if nout <= 0:
                     continue
@@ -447,12 +483,12 @@ class Filterbank:
         exact = h.nbits != 32  # integer samples: 64-bit integer cells, rounded once at the end
         fold_ar = torch.zeros(cells, dtype=torch.int64 if exact else torch.float32, device=dev)
         count_ar = torch.zeros(cells, dtype=torch.int32, device=dev)
-        ddev = torch.from_numpy(chan_delays).to(dev)
-        bdev = torch.from_numpy(band_start).to(dev)
+        tables = torch.from_numpy(np.concatenate([chan_delays, band_start])).to(dev)  # one upload
+        ddev, bdev = tables[:h.nchans], tables[h.nchans:]
         lib = _lib.load()
         st = stream_handle(None, dev)
         for nsamps_r, ii, raw in self.stream_blocks(gulp, start, nsamps, skipback=max_delay,
-                                                    **plan_kwargs):
+                                                    keep_halo=True, **plan_kwargs):
             if h.nbits < 8:
                 x, nb = gpu_unpack(raw[:nsamps_r * self.row_bytes], h.nbits, self.bitorder), 8
             else:
@@ -469,10 +505,11 @@ class Filterbank:
                                         max_delay, h.tsamp, period, accel, h.nsamples, nbins,
                                         nints, nbands, ii * (gulp - max_delay), bdev.data_ptr(),
                                         fold_ar.data_ptr(), count_ar.data_ptr(), cells, st))
-        f = fold_ar.cpu().numpy().astype(np.float32)
-        c = count_ar.cpu().numpy()
-        with np.errstate(divide="ignore", invalid="ignore"):
-            f /= c
+        mean = torch.empty(cells, dtype=torch.float32, device=dev)
+        _lib.check(lib.spp_fold_finish(None if exact else fold_ar.data_ptr(),
+                                       fold_ar.data_ptr() if exact else None, count_ar.data_ptr(),
+                                       cells, mean.data_ptr(), st))
+        f = mean.cpu().numpy()
         return FoldedData(f.reshape(nints, nbands, nbins), h.new_header(), period, dm, accel)
 
 
@@ -560,6 +597,7 @@ class ArrayFilterbank(Filterbank):
         self._raw = np.ascontiguousarray(raw).view(np.uint8).ravel()
         self._header = header
         self._registered: bool | None = None  # None: not tried yet
+        self._whole: torch.Tensor | None = None  # _raw as a tensor, once registered
 
     @property
     def header(self) -> Header:
@@ -580,9 +618,11 @@ class ArrayFilterbank(Filterbank):
                                 _lib.load().spp_host_register(self._raw.ctypes.data, n) == 0)
         if not self._registered or offset + nbytes > self._raw.nbytes:
             return None
-        with warnings.catch_warnings():  # read-only arrays: the view is only read
-            warnings.simplefilter("ignore", UserWarning)
-            return torch.from_numpy(self._raw[offset:offset + nbytes])
+        if self._whole is None:
+            with warnings.catch_warnings():  # read-only arrays: the view is only read
+                warnings.simplefilter("ignore", UserWarning)
+                self._whole = torch.from_numpy(self._raw)
+        return self._whole[offset:offset + nbytes]
 
     def __del__(self):
         if getattr(self, "_registered", False):
