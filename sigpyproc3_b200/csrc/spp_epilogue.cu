@@ -222,8 +222,10 @@ __global__ void k_subband(const void* __restrict__ in, int64_t nchans, int64_t n
 // largest window sum only; who holds the chunk's best looks its index up
 // afterwards, so a window costs a load, a subtraction and a maximum.  512 int32
 // rows x 250001, factors 1/2/4, 9 widths: 2057 -> 979 us (issue 59 %, shared
-// loads 48 %, the rest waits at the block's scans); 200 float32 rows x 300001,
-// factors 1/2: 875 -> 795 us.
+// loads 48 %, a third of the warps' time at the block's barriers); with the scan's
+// runs kept in registers between its passes, the moments' 128-bit arithmetic
+// moved past the windows and the index search without dependent steps: 805 us.
+// 200 float32 rows x 300001, factors 1/2: 875 -> 795 us.
 // ---------------------------------------------------------------------------
 constexpr int kSnrChunk = 6144;     // downsampled samples per CTA, most
 constexpr int kSnrThreads = 256;
@@ -262,16 +264,12 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
   return t;
 }
 
-__device__ __forceinline__ long long block_sum(long long v, long long* red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  long long t = 0;
-#pragma unroll
-  for (int w = 0; w < kSnrWarps; ++w) t += red[w];
-  return t;
+// Sum over the warp modulo 2^64, in three pieces whose sums fit 32 bits.
+__device__ __forceinline__ long long warp_sum64(long long v) {
+  const uint32_t lo = __reduce_add_sync(0xffffffffu, (uint32_t)v & 0x3ffffffu);
+  const uint32_t mid = __reduce_add_sync(0xffffffffu, (uint32_t)(v >> 26) & 0x3ffffffu);
+  const int hi = __reduce_add_sync(0xffffffffu, (int)(v >> 52));
+  return (long long)lo + ((long long)mid << 26) + ((long long)hi << 52);
 }
 
 // Window arithmetic of the two paths: prefix sums (T), the sum of a window
@@ -332,6 +330,39 @@ __device__ __forceinline__ void snr_scan(T* s, int len, T* red) {
   __syncthreads();
 }
 
+// The same for words, each thread's run of PER (odd) held in registers between
+// the two passes.  s has 1 + PER * kSnrThreads words; those past the chunk are
+// scanned along and mean nothing.
+template <int PER>
+__device__ __forceinline__ void snr_scan_regs(uint32_t* s, uint32_t* red) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t* p = s + 1 + (int)threadIdx.x * PER;
+  uint32_t v[PER];
+  uint32_t sum = 0u;
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    v[j] = p[j];
+    sum += v[j];
+  }
+  uint32_t incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += x;
+  }
+  if (lane == 31) red[warp] = incl;
+  __syncthreads();
+  uint32_t run = incl - sum;
+#pragma unroll
+  for (int w = 0; w < kSnrWarps - 1; ++w) run += w < warp ? red[w] : 0u;
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    run += v[j];
+    p[j] = run;
+  }
+  __syncthreads();
+}
+
 // Best window of NG widths (from w0) over starts 0..own-1 of the scanned chunk,
 // folded into the running best (best, idx) in shared memory; the chunk's first
 // sample is at `at` of the CTA's, values are scaled by `scale`.
@@ -388,11 +419,12 @@ __device__ __forceinline__ void snr_window_group(const typename A::T* s, int own
 #pragma unroll
   for (int g = 0; g < NG; ++g) {
     if (m[g] != bbest[g]) continue;
-    for (int j = 0; j + (int)threadIdx.x < own; j += kSnrThreads) {
-      if (sw[g] + j > s + len || A::window(sw[g][j], s0[j]) != m[g]) continue;
-      atomicMin(&bidx[g], j + (int)threadIdx.x);
-      break;
-    }
+    const int last = min(own - 1, len - cfg.w[w0 + g]) - (int)threadIdx.x;  // its last start
+    int hit = INT_MAX;
+#pragma unroll 8
+    for (int j = 0; j <= last; j += kSnrThreads)
+      hit = min(hit, A::window(sw[g][j], s0[j]) == m[g] ? j : INT_MAX);
+    if (hit != INT_MAX) atomicMin(&bidx[g], hit + (int)threadIdx.x);
   }
   __syncthreads();
   if (threadIdx.x < NG && bidx[threadIdx.x] != INT_MAX) {
@@ -470,6 +502,8 @@ k_snr_chunk(const void* __restrict__ in, int64_t n, int64_t in_stride, const Snr
   __shared__ double best[kSnrMaxWidths];
   __shared__ int idx[kSnrMaxWidths];
   __shared__ double red[kSnrWarps];
+  __shared__ long long wsum[2][kSnrWarps];
+  __shared__ uint32_t scan_red[kSnrWarps];
   const int64_t k = blockIdx.x;
   const int64_t row = blockIdx.y / cfg.nf;
   const int fi = blockIdx.y % cfg.nf;
@@ -499,18 +533,31 @@ k_snr_chunk(const void* __restrict__ in, int64_t n, int64_t in_stride, const Snr
       if (threadIdx.x == 0) snr_sm[0] = 0u;
       const unsigned long long top = (unsigned long long)big * (unsigned)f;
       const int wide = top * (unsigned)cfg.wmax >= (1ull << 31) || top > (1ull << 24);
+      // a thread's sums are below 24 * 2^24 and 24 * 2^48 unless its values are wide
+      s1 = warp_sum64(s1);
+      s2 = warp_sum64(s2);
+      if ((threadIdx.x & 31) == 0) {
+        wsum[0][threadIdx.x >> 5] = s1;
+        wsum[1][threadIdx.x >> 5] = s2;
+      }
       if (__syncthreads_or(wide) == 0) {
-        const long long S1 = block_sum(s1, reinterpret_cast<long long*>(red));
-        const long long S2 = block_sum(s2, reinterpret_cast<long long*>(red));
-        if (threadIdx.x == 0) {
+        if (len <= 7 * kSnrThreads) snr_scan_regs<7>(snr_sm, scan_red);
+        else if (len <= 13 * kSnrThreads) snr_scan_regs<13>(snr_sm, scan_red);
+        else if (len <= 25 * kSnrThreads) snr_scan_regs<25>(snr_sm, scan_red);
+        else snr_scan<uint32_t>(snr_sm, len, scan_red);
+        snr_windows<SnrInt>(snr_sm, own, len, cfg, 0, 1.0 / (double)f, best, idx);
+        done = true;
+        if (threadIdx.x == 32) {  // beside the threads that write the widths' bests
+          long long S1 = 0, S2 = 0;
+          for (int w = 0; w < kSnrWarps; ++w) {
+            S1 += wsum[0][w];
+            S2 += wsum[1][w];
+          }
           const __int128 num = (__int128)S2 * own - (__int128)S1 * S1;
           st[0] = (double)own;
           st[1] = (double)S1 / (double)f;
           st[2] = (double)num / (double)own / ((double)f * (double)f);
         }
-        snr_scan<uint32_t>(snr_sm, len, reinterpret_cast<uint32_t*>(red));
-        snr_windows<SnrInt>(snr_sm, own, len, cfg, 0, 1.0 / (double)f, best, idx);
-        done = true;
       }
     }
   }
@@ -1235,8 +1282,11 @@ static int boxcar_snr_impl(const void* in, int in_kind, int64_t nrows, int64_t n
   cfg.chunk = snr_chunk(nrows * nfactors, n);
   if (cfg.chunk < 2 * cfg.wmax) cfg.chunk = kSnrChunk;
   const bool ints = in_kind == SPP_OUT_I32;
-  // float64 pieces of at least 512 starts fit beside the halo
-  cfg.smem_words = ints ? std::max(cfg.chunk + cfg.wmax + 2, 2 * (cfg.wmax + 513))
+  // float64 pieces of at least 512 starts fit beside the halo; whole runs of the
+  // scan in registers
+  const int most = cfg.chunk + cfg.wmax;
+  const int runs = most <= 7 * kSnrThreads ? 7 : most <= 13 * kSnrThreads ? 13 : most <= 25 * kSnrThreads ? 25 : 0;
+  cfg.smem_words = ints ? std::max({most + 2, 1 + runs * kSnrThreads, 2 * (cfg.wmax + 513)})
                         : 2 * (cfg.chunk + cfg.wmax + 1);
   const int64_t smem = (int64_t)cfg.smem_words * 4;
   const void* fn = ints ? reinterpret_cast<const void*>(k_snr_chunk<SPP_OUT_I32>)

@@ -51,3 +51,13 @@ def test_float_rows(orc, n):
     rng = np.random.default_rng(n)
     x = np.rint(rng.normal(0.0, 500.0, size=(3, n)) * 8).astype(np.float32) / 8  # sums exact in float64
     _check(orc, x, [1, 3, 64, 1000], [1, 2, 3])
+
+
+@pytest.mark.parametrize("rows,n", [(1, 1536), (2, 5000), (400, 6500)])
+@pytest.mark.parametrize("wmax", [255, 256, 257, 512, 1024])
+def test_scan_runs(orc, rows, n, wmax):
+    """Chunk and halo at the ends of the scan's run lengths (7, 13 and 25 words per
+    thread, and past them)."""
+    rng = np.random.default_rng(n + wmax)
+    x = rng.integers(-2000, 2000, size=(rows, n), endpoint=True).astype(np.int32)
+    _check(orc, x, [1, 5, wmax], [1, 2])
