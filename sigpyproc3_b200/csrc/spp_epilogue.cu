@@ -220,12 +220,14 @@ __global__ void k_subband(const void* __restrict__ in, int64_t nchans, int64_t n
 // Integer rows run on 32-bit integers wherever that is exact (see k_snr_chunk):
 // half the shared memory and no float64 in the window loop.  Threads keep the
 // largest window sum only; who holds the chunk's best looks its index up
-// afterwards, so a window costs a load, a subtraction and a maximum.  512 int32
+// afterwards, so a window costs a load and a subtract-and-maximum.  512 int32
 // rows x 250001, factors 1/2/4, 9 widths: 2057 -> 979 us (issue 59 %, shared
 // loads 48 %, a third of the warps' time at the block's barriers); with the scan's
 // runs kept in registers between its passes, the moments' 128-bit arithmetic
-// moved past the windows and the index search without dependent steps: 805 us.
-// 200 float32 rows x 300001, factors 1/2: 875 -> 795 us.
+// moved past the windows and the index search without dependent steps: 805 us;
+// twelve to sixteen loads of a thread in flight, and the subtraction and maximum
+// of a window in one instruction: 772 us (one factor: 409 -> 366 us, of them 209
+// for loads and scan).  200 float32 rows x 300001, factors 1/2: 875 -> 795 us.
 // ---------------------------------------------------------------------------
 constexpr int kSnrChunk = 6144;     // downsampled samples per CTA, most
 constexpr int kSnrThreads = 256;
@@ -280,6 +282,8 @@ struct SnrInt {
   __device__ __forceinline__ static V lowest() { return INT_MIN; }
   __device__ __forceinline__ static V window(T b, T a) { return (int32_t)(b - a); }
   __device__ __forceinline__ static V larger(V a, V b) { return max(a, b); }
+  // the sum wraps modulo 2^32 as the prefix sums do
+  __device__ __forceinline__ static V fold(V m, T b, T a) { return __viaddmax_s32((int32_t)b, (int32_t)(0u - a), m); }
   __device__ __forceinline__ static V warp_max(V v) { return __reduce_max_sync(0xffffffffu, v); }
 };
 struct SnrF64 {
@@ -288,6 +292,7 @@ struct SnrF64 {
   __device__ __forceinline__ static V lowest() { return -DBL_MAX; }
   __device__ __forceinline__ static V window(T b, T a) { return b - a; }
   __device__ __forceinline__ static V larger(V a, V b) { return b > a ? b : a; }  // ignores NaN
+  __device__ __forceinline__ static V fold(V m, T b, T a) { return larger(m, window(b, a)); }
   __device__ __forceinline__ static V warp_max(V v) {
     // ordered 64-bit key, largest high word first, then the low word among equals
     long long k = __double_as_longlong(v);
@@ -392,7 +397,7 @@ __device__ __forceinline__ void snr_window_group(const typename A::T* s, int own
       const typename A::T p0 = s0[t + i * kSnrThreads];
 #pragma unroll
       for (int g = 0; g < NG; ++g)
-        m[g] = A::larger(m[g], A::window(sw[g][t + i * kSnrThreads], p0));
+        m[g] = A::fold(m[g], sw[g][t + i * kSnrThreads], p0);
     }
   }
   for (; t + (int)threadIdx.x < own; t += kSnrThreads) {
@@ -464,28 +469,48 @@ template <int F>
 __device__ __forceinline__ void snr_load_int(const int32_t* __restrict__ x, int f, int own, int len,
                                              uint32_t* s, uint32_t& big, long long& s1, long long& s2) {
   const int ff = F > 0 ? F : f;
-  auto get = [&](int j) {
-    const int32_t* p = x + (int64_t)j * ff;
-    int v = 0;
-#pragma unroll
-    for (int q = 0; q < (F > 0 ? F : ff); ++q) {
-      const int y = __ldg(p + q);
-      big = max(big, (uint32_t)(y < 0 ? 0u - (uint32_t)y : (uint32_t)y));
-      v = (int)((uint32_t)v + (uint32_t)y);
-    }
+  auto put = [&](int j, int v) {
     s[j + 1] = (uint32_t)v;
     return v;
   };
+  auto sum = [&](const int32_t* p, auto load) {
+    int v = 0;
+#pragma unroll
+    for (int q = 0; q < (F > 0 ? F : ff); ++q) {
+      const int y = load(p, q);
+      big = max(big, (uint32_t)(y < 0 ? 0u - (uint32_t)y : (uint32_t)y));
+      v = (int)((uint32_t)v + (uint32_t)y);
+    }
+    return v;
+  };
+  auto get = [&](int j) {
+    return put(j, sum(x + (int64_t)j * ff, [](const int32_t* p, int q) { return __ldg(p + q); }));
+  };
   int a1 = 0;
-#pragma unroll 4
-  for (int j = threadIdx.x; j < own; j += kSnrThreads) {
-    const int v = get(j);
+  auto add = [&](int v) {
     a1 = (int)((uint32_t)a1 + (uint32_t)v);
     s2 += (long long)v * v;
+  };
+  int j = threadIdx.x;
+  if constexpr (F > 0) {
+    // twelve or sixteen loads of a thread in flight
+    constexpr int B = F == 1 ? 12 : F == 2 ? 8 : 4;
+    for (; j - (int)threadIdx.x + B * kSnrThreads <= own; j += B * kSnrThreads) {
+      int y[B][F];
+#pragma unroll
+      for (int i = 0; i < B; ++i)
+#pragma unroll
+        for (int q = 0; q < F; ++q) y[i][q] = __ldg(x + (int64_t)(j + i * kSnrThreads) * F + q);
+#pragma unroll
+      for (int i = 0; i < B; ++i)
+        add(put(j + i * kSnrThreads, sum(nullptr, [&](const int32_t*, int q) { return y[i][q]; })));
+    }
   }
+#pragma unroll 4
+  for (; j < own; j += kSnrThreads) add(get(j));
   s1 = a1;
 #pragma unroll 2
-  for (int j = own + threadIdx.x; j < len; j += kSnrThreads) get(j);
+  for (j = own + threadIdx.x; j < len; j += kSnrThreads) get(j);
 }
 
 // KIND int32: for a power-of-two factor f, y = s / f with s the integer sum of f
