@@ -61,3 +61,12 @@ def test_scan_runs(orc, rows, n, wmax):
     rng = np.random.default_rng(n + wmax)
     x = rng.integers(-2000, 2000, size=(rows, n), endpoint=True).astype(np.int32)
     _check(orc, x, [1, 5, wmax], [1, 2])
+
+
+@pytest.mark.parametrize("sign", [1, -1])
+def test_prefix_sums_wrap(orc, sign):
+    """Large samples of one sign: a chunk's prefix sums pass 2^32 several times while
+    every window stays below 2^31."""
+    rng = np.random.default_rng(22)
+    x = (sign * rng.integers((1 << 22) - 900, 1 << 22, size=(2, 13000))).astype(np.int32)
+    _check(orc, x, [1, 3, 100, 256], [1, 2])
