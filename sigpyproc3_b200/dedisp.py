@@ -117,10 +117,9 @@ def dedisperse_block(raw: torch.Tensor, delays: np.ndarray, nchans: int, nsamps:
     lib = _lib.load()
     st = stream_handle(stream, raw.device)
     if host_table is None:
-        # spp_dedisperse_hd asks for no bit order; an unknown one keeps the
-        # block from the other kernels, and is refused further down
-        known = bitorder in ("big", "b", "little", "l")
-        order = bitorder_code(bitorder) if nb != 8 or known else -1
+        # an unknown bit order is no matter to a block that writes nothing nor to
+        # spp_dedisperse_hd; it keeps others from these kernels, to be refused below
+        order = bitorder_code(bitorder) if bitorder in ("big", "b", "little", "l") else -1
         rc = lib.spp_dedisperse_block(raw.data_ptr(), nb, order, nchans, nsamps,
                                       delays.ctypes.data, acc, out.data_ptr(), out.numel(),
                                       out_start, st)

@@ -90,3 +90,20 @@ def test_wide_spreads_fall_back(orc):
     out = torch.zeros(nsamps - 9000, dtype=torch.float32, device="cuda")
     assert dedisperse_block(raw, d, nchans, nsamps, out) == nsamps - 9000
     np.testing.assert_array_equal(out.cpu().numpy(), orc.dedisperse(x, d, nchans, nsamps)[:3000])
+
+
+@pytest.mark.parametrize("nbits", [8, 2])
+def test_unknown_bit_order(nbits):
+    """A block that writes nothing returns 0 whatever the order; a packed one
+    that does is refused."""
+    import torch
+
+    from sigpyproc3_b200.dedisp import dedisperse_block
+
+    d = np.array([0, 1, 2, 3], dtype=np.int32)
+    raw = torch.zeros(64, dtype=torch.uint8, device="cuda")
+    out = torch.zeros(8, dtype=torch.float32, device="cuda")
+    assert dedisperse_block(raw, d, 4, 3, out, nbits=nbits, bitorder="x") == 0
+    if nbits < 8:
+        with pytest.raises(ValueError):
+            dedisperse_block(raw, d, 4, 8, out, nbits=nbits, bitorder="x")
