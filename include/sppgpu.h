@@ -232,6 +232,10 @@ int spp_dmt_plan_create(spp_dmt_plan** plan, int nbits, int bitorder,
                         int64_t nchans, int64_t nsamps_max, int64_t ndm,
                         const int32_t* delays_host, int mode, int out_kind,
                         int acc);
+/* device bytes that creating such a plan allocates for its delay table and, from
+ * *work_offset (a multiple of 256) on, the words its row tables are made in */
+int spp_dmt_plan_layout(int nbits, int64_t nchans, int64_t ndm, int64_t* work_offset,
+                        int64_t* total_bytes);
 int spp_dmt_plan_destroy(spp_dmt_plan* plan);
 /* valid output samples per row for an input of `nsamps` samples */
 int64_t spp_dmt_plan_nvalid(const spp_dmt_plan* plan, int64_t nsamps);

@@ -68,6 +68,7 @@ SIGNATURES: dict[str, tuple[list, object]] = {
     "spp_dedisperse_noalloc_status_read": ([_p, _p], _int),
     "spp_dmt_plan_create": ([ctypes.POINTER(_p), _int, _int, _i64, _i64, _i64, _p, _int, _int,
                              _int], _int),
+    "spp_dmt_plan_layout": ([_int, _i64, _i64, _p, _p], _int),
     "spp_dmt_plan_destroy": ([_p], _int),
     "spp_dmt_plan_nvalid": ([_p, _i64], _i64),
     "spp_dmt_plan_workspace_bytes": ([_p, _i64], _i64),

@@ -697,6 +697,19 @@ static void free_device(spp_dmt_plan* p) {
 // Pair rows a plan may hold, per channel.
 constexpr int64_t kPairRowsPerChan = 12;
 
+// Device words of a plan: the delay table, then (for interleaved shapes) the
+// words that make their rows, from a 256-byte boundary on: the range passes
+// store pairs of words there, whatever the table's size.
+struct PlanWords {
+  int64_t work, total;
+};
+static PlanWords plan_words(int nbits, int64_t nchans, int64_t ndm) {
+  const int64_t table = ndm * nchans;
+  if (ndm <= 1 || nbits > 8) return {table, table};
+  const int64_t work = round_up(table, 64);
+  return {work, work + ilv_plan_words(nchans, kPairRowsPerChan * nchans)};
+}
+
 // Interleaved bit-plane shapes this table and sample width can use.  `words`:
 // plan-owned device words after the delay table.
 static int add_ilv_candidates(spp_dmt_plan* p, int32_t* words) {
@@ -877,12 +890,12 @@ int spp_dmt_plan_create(spp_dmt_plan** plan, int nbits, int bitorder, int64_t nc
   }
   p->dpitch = nchans;
   const bool ilv = ndm > 1 && nbits <= 8;
-  const int64_t more = ilv ? ilv_plan_words(nchans, kPairRowsPerChan * nchans) : 0;
-  cudaError_t e = cudaMalloc(&p->d_delays, sizeof(int32_t) * (ndm * nchans + more));
+  const PlanWords words = plan_words(nbits, nchans, ndm);
+  cudaError_t e = cudaMalloc(&p->d_delays, sizeof(int32_t) * words.total);
   if (e != cudaSuccess) { delete p; return cuda_status(e, "plan cudaMalloc"); }
   e = cudaMemcpy(p->d_delays, delays_host, sizeof(int32_t) * ndm * nchans, cudaMemcpyHostToDevice);
   int rc = cuda_status(e, "plan upload");
-  if (rc == SPP_OK && ilv) rc = add_ilv_candidates(p, p->d_delays + ndm * nchans);
+  if (rc == SPP_OK && ilv) rc = add_ilv_candidates(p, p->d_delays + words.work);
   if (rc == SPP_OK && p->cands.empty())
     rc = fail(SPP_ERR_UNSUPPORTED, "no kernel variant fits this delay table");
   if (rc == SPP_OK) {
@@ -895,6 +908,18 @@ int spp_dmt_plan_create(spp_dmt_plan** plan, int nbits, int bitorder, int64_t nc
     return rc;
   }
   *plan = p;
+  return SPP_OK;
+}
+
+int spp_dmt_plan_layout(int nbits, int64_t nchans, int64_t ndm, int64_t* work_offset,
+                        int64_t* total_bytes) {
+  if (!work_offset || !total_bytes) return fail(SPP_ERR_ARG, "spp_dmt_plan_layout: null pointer");
+  if (!valid_nbits(nbits)) return fail(SPP_ERR_ARG, "nbits must be 1, 2, 4, 8 or 32 (got %d)", nbits);
+  if (nchans <= 0 || ndm <= 0 || nchans > INT32_MAX || ndm > INT32_MAX)
+    return fail(SPP_ERR_ARG, "bad shape");
+  const PlanWords w = plan_words(nbits, nchans, ndm);
+  *work_offset = 4 * w.work;
+  *total_bytes = 4 * w.total;
   return SPP_OK;
 }
 

@@ -817,6 +817,8 @@ int64_t ilv_plan_words(int64_t nchans, int64_t max_rows) {
 int ilv_make_rows(const IlvDelays& d, int G, int64_t max_rows, IlvArena* ar, IlvRows* out) {
   const int64_t ng = d.nchans / G;
   if (d.nchans % G || ng <= 0) return SPP_ERR_UNSUPPORTED;
+  if (reinterpret_cast<uintptr_t>(ar->scratch) % sizeof(int2))  // k_ilv_ranges stores int2
+    return fail(SPP_ERR_ARG, "interleaved rows: misaligned scratch");
   IlvRows r{};
   r.G = G;
   int32_t* scratch = ar->scratch;
