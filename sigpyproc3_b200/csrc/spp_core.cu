@@ -120,6 +120,8 @@ static const std::vector<Variant>& variants() {
       mkb<2, 2, 8, 1, 2, 32, 80, 4>(), mkb<2, 2, 8, 1, 2, 32, 128>(), mkb<2, 2, 8, 1, 2, 32>(),
       mkb<2, 4, 8, 1, 2, 32>(),
       mkb<1, 2, 8, 1, 2, 32, 80>(), mkb<1, 2, 8, 1, 2, 32, 128>(), mkb<1, 2, 8, 1, 3, 32>(),
+      // widest spreads of 1-bit rows (8 trials: up to 24000 samples, 14000 above)
+      mkb<1, 4, 8, 1, 2, 32>(),
       SPP_INT_VARIANTS(1),
       SPP_INT_VARIANTS(2),
       // four plane rows per channel; 16-channel slabs keep a stage's planes
@@ -656,6 +658,8 @@ struct spp_dmt_plan {
   size_t evused = 0;
 };
 
+constexpr int64_t kMaxTimeTiles = 65535;  // gridDim.y
+
 // Candidate codes at or above this name an interleaved bit-plane shape.
 constexpr int kIlvCode = 1 << 20;
 static int ilv_index(const spp_dmt_plan* p, int cand) {
@@ -765,14 +769,21 @@ static int add_ilv_candidates(spp_dmt_plan* p, int32_t* words) {
 static int first_choice(const spp_dmt_plan* p) {
   constexpr int64_t kIlvDefaultBytes = 16ll << 30;
   const int64_t nvalid = std::max<int64_t>(1, plan_nvalid(p, p->nsamps_max));
+  // Time tiles are a grid's y extent: shapes of short tiles cannot run the
+  // longest blocks (256-sample tiles: 16.8 million outputs).
+  auto tiles_fit = [&](int i) {
+    return ilv_index(p, i) >= 0 || ceil_div(nvalid, tile_T(variants()[p->cands[i]])) <= kMaxTimeTiles;
+  };
+  int first = 0;
+  while (first + 1 < (int)p->cands.size() && !tiles_fit(first)) ++first;
   if (p->nbits == 32) {
     // float64 sums: waves of the CTAs an SM holds (shared memory, 64 warps)
     // times a tile's adds over its rate, which falls below 12 adding warps per SM
-    int pick = 0;
+    int pick = first;
     double best = 0.0;
     for (int i = 0; i < (int)p->cands.size(); ++i) {
       const Variant& v = variants()[p->cands[i]];
-      if (v.rate <= 0.0) continue;
+      if (v.rate <= 0.0 || !tiles_fit(i)) continue;
       const int64_t smem = smem_bytes(v, slot_words(v, p->spans[i])) + 1024;
       const int64_t per_sm = std::min<int64_t>((228 << 10) / smem, 64 / (v.DW * v.TW + 1));
       const int64_t ctas = ceil_div(p->ndm, v.DW) * ceil_div(nvalid, tile_T(v));
@@ -790,8 +801,8 @@ static int first_choice(const spp_dmt_plan* p) {
   double best = 1.5 * (double)p->ndm * nvalid * p->nchans / adds_per_us + 20.0;
   const int64_t prows = p->ilv_rows[1].nrows;
   const bool shared_pairs = p->nbits == 2 && prows > 0 && p->ndm * (p->nchans / 2) >= 100 * prows;
-  int pick = 0;
-  bool any = p->cands[0] < kIlvCode;  // candidate 0 is taken unless a better one follows
+  int pick = first;
+  bool any = p->cands[first] < kIlvCode;  // `first` is taken unless a better one follows
   bool paired = false;
   for (int i = 0; i < (int)p->cands.size(); ++i) {
     const int iv = ilv_index(p, i);
@@ -1045,7 +1056,7 @@ static int dmt_run(const spp_dmt_plan* p, const void* in, int64_t nsamps, void* 
   if (ws_bytes < kStatusBytes + g.bytes)
     return fail(SPP_ERR_SIZE, "workspace %lld B < required %lld B", (long long)ws_bytes,
                 (long long)(kStatusBytes + g.bytes));
-  if (g.ntiles_t > 65535)
+  if (g.ntiles_t > kMaxTimeTiles)
     return fail(SPP_ERR_UNSUPPORTED, "%lld time tiles exceed the grid limit", (long long)g.ntiles_t);
   const Variant& v = variants()[p->cands[p->cur]];
   void* planar = ws + kStatusBytes;
