@@ -75,8 +75,11 @@ constexpr int kCtWords = 16;
 __host__ __device__ constexpr int planes_ct_chans(int nb) { return 256 / nb; }
 constexpr int kPlaneWords = 8;
 
+// Eight CTAs per SM for 8-bit rows (others: as compiled): the 16-byte branch below took 48 registers
+// where rows that miss it need 32 and lost a fifth of their rate (336 channels at
+// an address that is 4 mod 16, 26967 rows: 105 us with 32 registers, 126 with 48).
 template <int NB>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, NB == 8 ? 8 : 0)
 k_corner_turn_int(const uint8_t* __restrict__ raw, int64_t nchans, int64_t nsamps,
                   int bitorder, int64_t halo, uint32_t* __restrict__ planar,
                   int64_t pitch_w) {
