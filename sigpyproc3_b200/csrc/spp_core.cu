@@ -4,6 +4,7 @@
 #include <atomic>
 #include <climits>
 #include <cstring>
+#include <limits>
 #include <mutex>
 #include <new>
 #include <tuple>
@@ -21,7 +22,8 @@ int launch_single8(const uint8_t* raw, int64_t nchans, int64_t nsamps, const int
 int launch_single8_hd(const uint8_t* raw, int64_t nchans, int64_t nsamps, const int32_t* delays_host,
                       float* out, int64_t out_start, int64_t nvalid, cudaStream_t st);
 int launch_single_stream(const void* in, int nbits, int bitorder, int64_t nchans, int64_t nsamps,
-                         const int32_t* delays_host, float* out, int64_t nvalid, cudaStream_t st);
+                         const int32_t* delays_host, float* out, int64_t nvalid, double limit_us,
+                         cudaStream_t st);
 
 static thread_local char g_err[1024] = "";
 
@@ -471,9 +473,9 @@ int spp_dedisperse_hd(const void* in, int nbits, int64_t nchans, int64_t nsamps,
   return rc;
 }
 
-int spp_dedisperse_host(const void* in, int nbits, int bitorder, int64_t nchans, int64_t nsamps,
-                        const int32_t* delays_host, float* out, int64_t out_len,
-                        int64_t out_start, void* stream) {
+static int dedisperse_host(const void* in, int nbits, int bitorder, int64_t nchans, int64_t nsamps,
+                           const int32_t* delays_host, float* out, int64_t out_len,
+                           int64_t out_start, double limit_us, void* stream) {
   if (!in || !delays_host || !out) return fail(SPP_ERR_ARG, "spp_dedisperse_host: null pointer");
   if (!valid_nbits(nbits)) return fail(SPP_ERR_ARG, "nbits must be 1, 2, 4, 8 or 32 (got %d)", nbits);
   if (bitorder != SPP_BITORDER_BIG && bitorder != SPP_BITORDER_LITTLE)
@@ -491,10 +493,30 @@ int spp_dedisperse_host(const void* in, int nbits, int bitorder, int64_t nchans,
     return fail(SPP_ERR_SIZE, "output too small: out_start %lld + %lld samples > out_len %lld",
                 (long long)out_start, (long long)nvalid, (long long)out_len);
   const int rc = launch_single_stream(in, nbits, bitorder, nchans, nsamps, delays_host,
-                                      out + out_start, nvalid, as_stream(stream));
+                                      out + out_start, nvalid, limit_us, as_stream(stream));
   if (rc == SPP_ERR_UNSUPPORTED)
     return fail(rc, "streaming path needs nchans <= 4096 and every slab's delay spread in shared memory");
   return rc;
+}
+
+int spp_dedisperse_host(const void* in, int nbits, int bitorder, int64_t nchans, int64_t nsamps,
+                        const int32_t* delays_host, float* out, int64_t out_len,
+                        int64_t out_start, void* stream) {
+  return dedisperse_host(in, nbits, bitorder, nchans, nsamps, delays_host, out, out_len, out_start,
+                         std::numeric_limits<double>::infinity(), stream);
+}
+
+// What spp_dedisperse takes for a block, in us: launches, the DM-time kernel's walk
+// over the channels, and both kernels' traffic, which bytes moved one at a time
+// (rows at odd addresses) slow down.  Fitted with the estimate of
+// launch_single_stream: mostly within 20 %.
+static double planar_us(int nbits, int64_t nchans, int64_t nsamps, uintptr_t align) {
+  const double mb = (double)nsamps * (double)(nchans * nbits) / 8e6;
+  const bool a16 = align % 16 == 0, a4 = align % 4 == 0;
+  if (nbits == 32) return 12.0 + 0.0455 * nchans + 0.94 * mb;
+  if (nbits == 8)
+    return a16 ? 8.0 + 0.032 * nchans + 0.57 * mb : 12.0 + 0.047 * nchans + (a4 ? 1.14 : 2.66) * mb;
+  return 13.3 + 0.05 * nchans + (a16 ? 1.51 : a4 ? 1.57 : 2.93) * mb;
 }
 
 int64_t spp_dedisperse_block(const void* in, int nbits, int bitorder, int64_t nchans,
@@ -513,10 +535,17 @@ int64_t spp_dedisperse_block(const void* in, int nbits, int bitorder, int64_t nc
     rc = spp_dedisperse_hd(in, nbits, nchans, nsamps, delays_host, out, out_len, out_start, stream);
   // 8-bit rows aligned to 4 bytes only, over a short delay range: the device-
   // table kernel copies them in one pass without touching registers (1020
-  // channels x 100000 samples, DM 100: 91 us against 125 us)
-  const bool narrow = nbits == 8 && nchans % 4 == 0 && nchans % 16 != 0 && (int64_t)dmax - dmin <= 2600;
+  // channels x 100000 samples, DM 100: 91 us against 125 us; 336 channels at an
+  // address that is 4 mod 16, 106670 samples: 33 against 54 us)
+  const uintptr_t rows = reinterpret_cast<uintptr_t>(in) | (uintptr_t)(nchans * nbits / 8);
+  const bool narrow = nbits == 8 && rows % 4 == 0 && rows % 16 != 0 && (int64_t)dmax - dmin <= 2600;
+  // one CTA walks all channels of its outputs, so short blocks and wide delay
+  // spreads can take longer than two passes over the whole block (float32, 2048
+  // channels, 4147 outputs: 288 us against 149 us; 8-bit, 512 channels, 3148
+  // samples within a slab, 97385 outputs: 277 against 112 us)
   if (rc == SPP_ERR_UNSUPPORTED && !narrow && bitorder >= 0 && (nbits != 32 || acc == SPP_ACC_F64))
-    rc = spp_dedisperse_host(in, nbits, bitorder, nchans, nsamps, delays_host, out, out_len, out_start, stream);
+    rc = dedisperse_host(in, nbits, bitorder, nchans, nsamps, delays_host, out, out_len, out_start,
+                         planar_us(nbits, nchans, nsamps, rows), stream);
   return rc == SPP_OK ? nvalid : rc;
 }
 

@@ -697,7 +697,8 @@ static void (*sd_kernel(int G))(const SdArgs<MAXC>) {
 
 template <int NB, int MAXC>
 static int launch_stream(const uint8_t* raw, int bitorder, int64_t nchans, int64_t nsamps,
-                         const int32_t* d, float* out, int64_t nvalid, cudaStream_t st) {
+                         const int32_t* d, float* out, int64_t nvalid, double limit_us,
+                         cudaStream_t st) {
   constexpr int CH = 8 * sd_seg(NB) / NB;
   constexpr int pitch = sd_pitch(NB);
   constexpr int unit = NB == 32 ? 32 * kSdWarps : 4 * kSdWarps;  // outputs per G
@@ -708,7 +709,7 @@ static int launch_stream(const uint8_t* raw, int bitorder, int64_t nchans, int64
   for (int s = 0; s < a.nslab; ++s) {
     const int64_t c0 = (int64_t)s * CH, c1 = std::min<int64_t>(nchans, c0 + CH);
     const int32_t mn = *std::min_element(d + c0, d + c1), mx = *std::max_element(d + c0, d + c1);
-    if (mx - mn > 60000) return SPP_ERR_UNSUPPORTED;
+    if ((int64_t)mx - mn > 60000) return SPP_ERR_UNSUPPORTED;
     spread = std::max(spread, mx - mn);
     a.mn[s] = mn;
     a.rows[s] = (uint16_t)(mx - mn);
@@ -749,6 +750,19 @@ static int launch_stream(const uint8_t* raw, int bitorder, int64_t nchans, int64
     }
   }
   if (G == 0) return SPP_ERR_UNSUPPORTED;
+  // Estimated time: a launch, then slab after slab: a fixed part, its rows (a part
+  // alone, a part shared with the other CTAs in flight) and its adds; where copies
+  // go through registers nothing hides the first slab's.  Fitted to 850 blocks of
+  // 16-4096 channels, 500-300000 outputs, cold caches: mostly within 20 %.
+  const int64_t ctas = ceil_div(nvalid, a.T), full = 148 * (smem > 113 * 1024 ? 1 : 2);
+  const double conc = std::max((double)std::min(ctas, full) / 148.0, 0.25);
+  const double rows = 1e-3 * (double)(a.T + spread), add = G * std::max(conc, 1.0);
+  const double slab = async       ? 0.30 + (0.38 + 0.11 * conc) * rows + 0.10 * add
+                      : NB != 32  ? 0.87 + (0.87 + 0.42 * conc) * rows + 0.25 * add
+                      : a.align == 16 ? 1.45 + (1.32 + 0.63 * conc) * rows
+                                      : (2.93 + 0.41 * conc) * rows + 2.53 * add;
+  const double first = async || (NB == 32 && a.align == 16) ? 0.0 : 3.2 * rows;
+  if (6.0 + first + (double)ceil_div(ctas, full) * a.nslab * slab > limit_us) return SPP_ERR_UNSUPPORTED;
   a.raw = raw;
   a.nsamps = nsamps;
   a.out = out;
@@ -764,17 +778,19 @@ static int launch_stream(const uint8_t* raw, int bitorder, int64_t nchans, int64
 }
 
 // Any width, up to 4096 channels, delays in host memory; SPP_ERR_UNSUPPORTED
-// (nothing launched) outside that or where a slab's delay spread does not fit.
+// (nothing launched) outside that, where a slab's delay spread does not fit, or
+// where the estimated time is above `limit_us`.
 int launch_single_stream(const void* in, int nbits, int bitorder, int64_t nchans, int64_t nsamps,
-                         const int32_t* delays_host, float* out, int64_t nvalid, cudaStream_t st) {
+                         const int32_t* delays_host, float* out, int64_t nvalid, double limit_us,
+                         cudaStream_t st) {
   if (nchans > 4096 || (nbits == 32 && (reinterpret_cast<uintptr_t>(in) & 3) != 0))
     return SPP_ERR_UNSUPPORTED;
   const uint8_t* raw = static_cast<const uint8_t*>(in);
 #define SPP_SD(NB)                                                                              \
   case NB:                                                                                      \
     return nchans <= 1024                                                                       \
-               ? launch_stream<NB, 1024>(raw, bitorder, nchans, nsamps, delays_host, out, nvalid, st) \
-               : launch_stream<NB, 4096>(raw, bitorder, nchans, nsamps, delays_host, out, nvalid, st)
+               ? launch_stream<NB, 1024>(raw, bitorder, nchans, nsamps, delays_host, out, nvalid, limit_us, st) \
+               : launch_stream<NB, 4096>(raw, bitorder, nchans, nsamps, delays_host, out, nvalid, limit_us, st)
   switch (nbits) {
     SPP_SD(1);
     SPP_SD(2);

@@ -107,3 +107,32 @@ def test_unknown_bit_order(nbits):
     if nbits < 8:
         with pytest.raises(ValueError):
             dedisperse_block(raw, d, 4, 8, out, nbits=nbits, bitorder="x")
+
+
+@pytest.mark.parametrize("nbits,nchans,nvalid,step,shift", [(32, 2048, 4147, 0, 0), (8, 512, 3001, 100, 4),
+                                                            (8, 336, 20000, 1, 4), (2, 64, 20000, 60, 4)])
+def test_blocks_left_to_two_passes(orc, nbits, nchans, nvalid, step, shift):
+    """Short float32 blocks, delays `step` apart per channel (wide slabs) and
+    8-bit rows aligned to 4 bytes: nothing is launched, and dedisperse_block
+    takes them through spp_dedisperse."""
+    import torch
+
+    from sigpyproc3_b200 import _lib
+    from sigpyproc3_b200.dedisp import dedisperse_block
+
+    rng = np.random.default_rng(nchans)
+    d = (step * np.arange(nchans)).astype(np.int32)
+    nsamps = nvalid + int(d.max())
+    if nbits == 32:
+        x = rng.normal(0.0, 1.0, size=nsamps * nchans).astype(np.float32)
+        raw = torch.from_numpy(x).cuda()
+    else:
+        x = rng.integers(0, 1 << nbits, size=nsamps * nchans, dtype=np.uint8)
+        raw = torch.from_numpy(np.concatenate([np.zeros(shift, np.uint8), _pack(x, nbits)])).cuda()[shift:]
+    out = torch.full((nvalid,), -5.0, dtype=torch.float32, device="cuda")
+    args = (raw.data_ptr(), nbits, 0, nchans, nsamps, d.ctypes.data, _lib.ACC_F64, out.data_ptr(),
+            out.numel(), 0, torch.cuda.current_stream().cuda_stream)
+    assert _lib.load().spp_dedisperse_block(*args) == _lib.SPP_ERR_UNSUPPORTED
+    assert bool((out == -5.0).all())
+    assert dedisperse_block(raw, d, nchans, nsamps, out, nbits=nbits) == nvalid
+    np.testing.assert_array_equal(out.cpu().numpy(), orc.dedisperse(x, d, nchans, nsamps))
