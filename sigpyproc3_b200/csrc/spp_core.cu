@@ -696,7 +696,7 @@ static int ilv_index(const spp_dmt_plan* p, int cand) {
 }
 static int plan_sign(const spp_dmt_plan* p) { return p->mode == SPP_MODE_ROLL ? -1 : 1; }
 static IlvDelays ilv_delays(const spp_dmt_plan* p) {
-  return IlvDelays{p->d_delays, p->ndm, p->nchans, plan_sign(p)};
+  return IlvDelays{p->d_delays, p->ndm, p->nchans, plan_sign(p), p->nbits};
 }
 
 static cudaEvent_t plan_event(spp_dmt_plan* p) {

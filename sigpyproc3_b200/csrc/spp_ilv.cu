@@ -349,9 +349,13 @@ k_ilv(const IlvArgs a) {
 // one funnel-shifted by q mod 32, so every raw row is read and transposed once
 // however long the rows are.  Each channel's 8 words x NB planes leave as one
 // contiguous run.  Bound by the transposes (shuffles and logic) and the row
-// stores.
+// stores.  LONG: rows of more than 32 M words beside the outputs', whose further
+// blocks are loaded as the first two are, one ahead (2-bit, 4096 channels, delays
+// to 32402: 128 words 232 -> 180 us, 32 words 699 -> 185 us when they were read
+// byte by byte); a kernel of its own, since its registers cost the others a
+// fifth of their rate.
 // ---------------------------------------------------------------------------
-template <int NB>
+template <int NB, bool LONG>
 __global__ void __launch_bounds__(256)
 k_ilv_turn(const uint8_t* __restrict__ raw, int64_t nchans, int64_t nsamps, int bitorder,
            int64_t M, int64_t mp, const int32_t* __restrict__ lo, const int32_t* __restrict__ ext,
@@ -467,7 +471,9 @@ k_ilv_turn(const uint8_t* __restrict__ raw, int64_t nchans, int64_t nsamps, int 
       if (qm > 0) fill(s_raw[1], w0, 1, rows_of(qm, 1));
     }
     __syncthreads();
-    if (vec16 && tile + gridDim.y < ntile) {
+    if (LONG && vec16 && qm >= 32) {
+      fetch(pre0, w0, 2, rows_of(qm, 2));
+    } else if (vec16 && tile + gridDim.y < ntile) {
       const int64_t w1 = w0 + 8 * (int64_t)gridDim.y;
       fetch(pre0, w1, 0, 32);
       fetch(pre1, w1, 1, rows_of(qmax(w1), 1));
@@ -499,7 +505,18 @@ k_ilv_turn(const uint8_t* __restrict__ raw, int64_t nchans, int64_t nsamps, int 
       if (qm < 32 * (b + 1)) break;
       // rows longer than 32 M words: the next block of 32 raw rows per word
       __syncthreads();
-      fill(s_raw[0], w0, b + 2, rows_of(qm, b + 2));
+      if (LONG && vec16) {
+        put(pre0, s_raw[0]);
+        if (qm >= 32 * (b + 2)) {
+          fetch(pre0, w0, b + 3, rows_of(qm, b + 3));
+        } else if (tile + gridDim.y < ntile) {
+          const int64_t w1 = w0 + 8 * (int64_t)gridDim.y;
+          fetch(pre0, w1, 0, 32);
+          fetch(pre1, w1, 1, rows_of(qmax(w1), 1));
+        }
+      } else {
+        fill(s_raw[0], w0, b + 2, rows_of(qm, b + 2));
+      }
       __syncthreads();
       turn(s_raw[0], s_out[b & 1]);
       __syncthreads();
@@ -881,6 +898,17 @@ int ilv_make_rows(const IlvDelays& d, int G, int64_t max_rows, IlvArena* ar, Ilv
     if (total > (1 << 30)) return SPP_ERR_UNSUPPORTED;
   }
   ext[r.nrows] = (int32_t)total;
+  if (G == 1) {
+    const int64_t cc = planes_ct_chans(d.nb);
+    for (int64_t c0 = 0; c0 < ng; c0 += cc) {
+      int64_t first = INT64_MAX, last = INT64_MIN;
+      for (int64_t c = c0; c < std::min(ng, c0 + cc); ++c) {
+        first = std::min<int64_t>(first, lo[c]);
+        last = std::max<int64_t>(last, (int64_t)lo[c] + ext[c + 1] - ext[c]);
+      }
+      r.max_group = std::max(r.max_group, last - first);
+    }
+  }
   r.ext_total = total;
   r.d_lo = ar->take(2 * r.nrows + 1);
   r.d_ext = r.d_lo + r.nrows;
@@ -961,12 +989,17 @@ int ilv_corner_turn(const IlvCfg& c, const IlvRows& chan, const IlvGeom& g, cons
                                                         ceil_div(g.M, 8)));
   const uint8_t* raw = static_cast<const uint8_t*>(in);
   uint32_t* rows = static_cast<uint32_t*>(ws);
+  const bool lng = chan.max_group > 31 * g.M;  // (M + max_group - 1) / M >= 32
+#define SPP_ILV_TURN(NB)                                                                            \
+  (lng ? k_ilv_turn<NB, true> : k_ilv_turn<NB, false>)<<<grid, 256, 0, st>>>(                       \
+      raw, nchans, nsamps, bitorder, g.M, g.mp, chan.d_lo, chan.d_ext, rows)
   switch (c.nb) {
-    case 1: k_ilv_turn<1><<<grid, 256, 0, st>>>(raw, nchans, nsamps, bitorder, g.M, g.mp, chan.d_lo, chan.d_ext, rows); break;
-    case 2: k_ilv_turn<2><<<grid, 256, 0, st>>>(raw, nchans, nsamps, bitorder, g.M, g.mp, chan.d_lo, chan.d_ext, rows); break;
-    case 4: k_ilv_turn<4><<<grid, 256, 0, st>>>(raw, nchans, nsamps, bitorder, g.M, g.mp, chan.d_lo, chan.d_ext, rows); break;
-    default: k_ilv_turn<8><<<grid, 256, 0, st>>>(raw, nchans, nsamps, bitorder, g.M, g.mp, chan.d_lo, chan.d_ext, rows); break;
+    case 1: SPP_ILV_TURN(1); break;
+    case 2: SPP_ILV_TURN(2); break;
+    case 4: SPP_ILV_TURN(4); break;
+    default: SPP_ILV_TURN(8); break;
   }
+#undef SPP_ILV_TURN
   return cuda_status(cudaGetLastError(), "interleaved corner turn launch");
 }
 

@@ -33,6 +33,7 @@ struct IlvRows {
   int64_t nrows = 0;       // rows over all groups
   int64_t ext_total = 0;   // words beyond the common row length, all rows
   int64_t max_ext = 0;     // the same, widest row
+  int64_t max_group = 0;   // G = 1: words beside M that the rows a turning CTA owns span, most
   int32_t* d_lo = nullptr;     // device, nrows: first word of the row (multiple of 8)
   int32_t* d_ext = nullptr;    // device, nrows + 1: prefix sums of the extra words
   int max_offsets = 0;         // G = 2: relative offsets of one pair, most
@@ -55,6 +56,7 @@ struct IlvDelays {
   const int32_t* d_delays;  // ndm x nchans
   int64_t ndm, nchans;
   int sign;
+  int nb;  // sample width, bits
 };
 
 // Plan-owned device words (beside the delay table): rows are taken from it,

@@ -99,3 +99,33 @@ def test_negative_offsets_and_roll(orc, nbits):
     assert _run(orc, nbits, d, nchans, 5000, seed=1) >= 4
     d = _delays(nchans, 25.0, ndm)
     assert _run(orc, nbits, d, nchans, 4096, mode="roll", seed=2) >= 4
+
+
+@pytest.mark.parametrize("nbits,nchans", [(1, 512), (2, 128), (4, 192), (8, 64)])
+def test_long_rows_in_whole_sectors(orc, nbits, nchans):
+    """The same where raw rows are read 32 bytes at a time: further blocks of 32
+    runs are loaded one ahead."""
+    d = _delays(nchans, 800.0, 400)
+    assert _run(orc, nbits, d, nchans, 300 + int(d.max()), seed=6) >= 2
+
+
+def test_long_rows_before_another_tile(orc):
+    """69 channel groups x 70 word tiles of rows that just pass 32 runs: one CTA
+    per group turns two tiles, the first of them with a further block."""
+    import torch
+
+    from sigpyproc3_b200.dedisp import DMTPlan
+
+    nchans, nvalid, ndm, step = 4368, 17900, 400, 44
+    d = np.repeat(step * np.arange(ndm, dtype=np.int32)[:, None], nchans, axis=1)
+    nsamps = nvalid + step * (ndm - 1)
+    g = torch.Generator(device="cuda").manual_seed(4)
+    raw = torch.randint(0, 256, (nsamps * nchans // 2,), device="cuda", dtype=torch.uint8, generator=g)
+    b = raw.view(nsamps, nchans // 2).to(torch.int32)
+    s = ((b >> 4) + (b & 15)).sum(1, dtype=torch.int32)
+    del b
+    expect = s.unfold(0, nvalid, step)
+    plan = DMTPlan(d, nchans, nsamps, nbits=4, out_dtype=torch.int32)
+    assert plan.describe()["bit_sliced"] and plan.describe()["T"] > 2048  # interleaved
+    assert torch.equal(plan.execute(raw, nsamps, check=True), expect)
+    plan.close()
