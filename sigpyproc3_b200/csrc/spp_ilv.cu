@@ -547,11 +547,10 @@ __device__ __forceinline__ void load_planes(const uint32_t* __restrict__ row, in
   } else if constexpr (NB == 4) {
     const uint4 a = __ldg(reinterpret_cast<const uint4*>(row + w * 4));
     x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
-  } else if constexpr (NB == 2) {
+  } else {
+    static_assert(NB == 2, "pair rows are sums of 2-, 4- and 8-bit channels");
     const uint2 a = __ldg(reinterpret_cast<const uint2*>(row + w * 2));
     x[0] = a.x; x[1] = a.y;
-  } else {
-    x[0] = __ldg(row + w);
   }
 }
 
@@ -568,11 +567,9 @@ __device__ __forceinline__ void load_planes_shared(const uint32_t* row, int w, u
   } else if constexpr (NB == 4) {
     const uint4 a = *reinterpret_cast<const uint4*>(row + w * 4);
     x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
-  } else if constexpr (NB == 2) {
+  } else {
     const uint2 a = *reinterpret_cast<const uint2*>(row + w * 2);
     x[0] = a.x; x[1] = a.y;
-  } else {
-    x[0] = row[w];
   }
 }
 
@@ -1020,7 +1017,6 @@ int ilv_group_rows(const IlvCfg& c, const IlvRows& chan, const IlvRows& rows, co
   k_ilv_pairs<NB><<<grid, 256, smem, st>>>(ch, g.mp, chan.d_lo, chan.d_ext, g.M, rows.d_rbase,     \
                                            rows.d_rlo, g.mp, rows.d_lo, rows.d_ext, rows.max_offsets, out)
   switch (c.nb) {
-    case 1: SPP_ILV_PAIRS(1); break;
     case 2: SPP_ILV_PAIRS(2); break;
     case 4: SPP_ILV_PAIRS(4); break;
     default: SPP_ILV_PAIRS(8); break;
