@@ -526,15 +526,17 @@ k_ilv_turn(const uint8_t* __restrict__ raw, int64_t nchans, int64_t nsamps, int 
 
 // ---------------------------------------------------------------------------
 // Pair rows: S[w] = x[2k][w] + x[2k+1][w + r] (ripple add of NB planes into
-// NB + 1).  A CTA takes one pair and 512 words and makes all of the pair's rows
-// there: channel 2k's words stay in registers (two per thread), channel
-// 2k+1's window in shared memory, so the channel rows are read once per pair
-// and not once per row.  Each warp gathers its 64 words in shared memory to
-// store whole 16-byte units in order.  The rows' bounds are read into shared
+// NB + 1).  A CTA takes one pair and 512 words (1024 of 2-bit rows) and makes all of
+// the pair's rows there: channel 2k's words stay in registers (two or four per
+// thread), channel 2k+1's window in shared memory, so the channel rows are read
+// once per pair and not once per row.  Each warp gathers its words in shared
+// memory to store whole 16-byte units in order.  The rows' bounds are read into shared
 // memory beside the window: read row by row they put a global load's latency
 // into every step (4-bit, 1024 channels, 9553 rows of 1632 words: 138 -> 125 us;
 // 2-bit, 4096 channels, 19038 rows of 31768 words: 1.98 -> 1.92 ms).  Bound by
-// the row stores.
+// the row stores where rows are long; short blocks behind long delays are mostly
+// CTAs that hold two rows or none, and twice the words per CTA of 2-bit rows takes
+// 347 -> 270 us there (4096 outputs, delays to 32402; 262144 outputs: 750 -> 630).
 // ---------------------------------------------------------------------------
 template <int NB>
 __device__ __forceinline__ void load_planes(const uint32_t* __restrict__ row, int64_t w, uint32_t (&x)[NB]) {
@@ -554,7 +556,8 @@ __device__ __forceinline__ void load_planes(const uint32_t* __restrict__ row, in
   }
 }
 
-constexpr int kPairWords = 512;     // words per CTA: two per thread
+// words per thread: 4-bit and wider windows would leave fewer CTAs per SM
+__host__ __device__ constexpr int pair_wpt(int nb) { return nb <= 2 ? 4 : 2; }
 constexpr int kPairMaxOffsets = 512;  // distinct relative offsets of one pair, most
 template <int NB>
 __device__ __forceinline__ void load_planes_shared(const uint32_t* row, int w, uint32_t (&x)[NB]) {
@@ -580,8 +583,9 @@ k_ilv_pairs(const uint32_t* __restrict__ chan, int64_t mpc, const int32_t* __res
             const int32_t* __restrict__ roff, int64_t mpr, const int32_t* __restrict__ rlo,
             const int32_t* __restrict__ rext, int max_rows, uint32_t* __restrict__ rows) {
   constexpr int NP = NB + 1;
+  constexpr int WPT = pair_wpt(NB), kPairWords = 256 * WPT, WW = 32 * WPT;  // words per thread, CTA, warp
   extern __shared__ __align__(16) uint32_t sm[];
-  uint32_t* st = sm + (threadIdx.x >> 5) * 64 * NP;  // this warp's 64 words
+  uint32_t* st = sm + (threadIdx.x >> 5) * WW * NP;  // this warp's words
   uint32_t* sy = sm + kPairWords * NP;               // channel 2k+1's window
   int3* srow = reinterpret_cast<int3*>(sy + (kPairWords + max_rows + 16) * NB);  // first word, end, extra words before
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -590,7 +594,7 @@ k_ilv_pairs(const uint32_t* __restrict__ chan, int64_t mpc, const int32_t* __res
   const int r0 = roff[k];
   const int64_t alo = clo[c], alen = M + cext[c + 1] - cext[c];
   const int64_t blo = clo[c + 1], blen = M + cext[c + 2] - cext[c + 1];
-  // words [w0, w0 + 512) of channel 2k's grid; all offsets lie in its row
+  // words [w0, w0 + kPairWords) of channel 2k's grid; all offsets lie in its row
   const int64_t w0 = alo + (int64_t)blockIdx.y * kPairWords;
   if (w0 >= alo + alen) return;
   const uint32_t* a = chan + ((int64_t)c * mpc + cext[c]) * NB;
@@ -608,10 +612,10 @@ k_ilv_pairs(const uint32_t* __restrict__ chan, int64_t mpc, const int32_t* __res
     if (w >= 0 && w < blen) v = __ldg(reinterpret_cast<const uint4*>(b + (y0 - blo) * NB) + u);
     reinterpret_cast<uint4*>(sy)[u] = v;
   }
-  uint32_t x[2][NB];
+  uint32_t x[WPT][NB];
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int64_t w = w0 - alo + warp * 64 + 32 * i + lane;
+  for (int i = 0; i < WPT; ++i) {
+    const int64_t w = w0 - alo + warp * WW + 32 * i + lane;
     if (w < alen) {
       load_planes<NB>(a, w, x[i]);
     } else {
@@ -620,14 +624,14 @@ k_ilv_pairs(const uint32_t* __restrict__ chan, int64_t mpc, const int32_t* __res
     }
   }
   __syncthreads();
-  const int64_t ww = w0 + warp * 64;  // this warp's first word
+  const int64_t ww = w0 + warp * WW;  // this warp's first word
   for (int e = e0; e < e1; ++e) {
     const int3 row = srow[e - e0];
     const int64_t lo = row.x, hi = row.y;
-    if (lo >= ww + 64 || hi <= ww) continue;
+    if (lo >= ww + WW || hi <= ww) continue;
     const int ys = (int)(ww + r0 + (e - e0) - y0);
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < WPT; ++i) {
       uint32_t y[NB], o[NP];
       load_planes_shared<NB>(sy, ys + 32 * i + lane, y);
       uint32_t cy = 0u;
@@ -643,7 +647,7 @@ k_ilv_pairs(const uint32_t* __restrict__ chan, int64_t mpc, const int32_t* __res
     __syncwarp();
     // row bounds are multiples of 8 words = 2 NP units
     uint4* dst = reinterpret_cast<uint4*>(rows + (e * mpr + row.z + ww - lo) * NP);
-    for (int u = lane; u < 16 * NP; u += 32) {
+    for (int u = lane; u < WW / 4 * NP; u += 32) {
       const int64_t w = ww + 8 * (u / (2 * NP));
       if (w >= lo && w < hi) dst[u] = reinterpret_cast<const uint4*>(st)[u];
     }
@@ -1005,10 +1009,11 @@ int ilv_group_rows(const IlvCfg& c, const IlvRows& chan, const IlvRows& rows, co
   if (c.G == 1) return SPP_OK;
   const uint32_t* ch = static_cast<const uint32_t*>(ws);
   uint32_t* out = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(ws) + g.chan_bytes);
-  const int64_t gy = ceil_div(g.M + chan.max_ext, kPairWords), ng = nchans / 2;
+  const int pair_words = 256 * pair_wpt(c.nb);
+  const int64_t gy = ceil_div(g.M + chan.max_ext, pair_words), ng = nchans / 2;
   if (gy > 65535) return fail(SPP_ERR_UNSUPPORTED, "pair rows of %lld words", (long long)g.M);
   dim3 grid((unsigned)ng, (unsigned)gy);
-  const int64_t smem = (int64_t)kPairWords * c.np * 4 + (int64_t)(kPairWords + rows.max_offsets + 16) * c.nb * 4 +
+  const int64_t smem = (int64_t)pair_words * c.np * 4 + (int64_t)(pair_words + rows.max_offsets + 16) * c.nb * 4 +
                        (int64_t)rows.max_offsets * 12;
   int rc = SPP_OK;
 #define SPP_ILV_PAIRS(NB)                                                                          \
