@@ -245,7 +245,9 @@ int64_t spp_dmt_plan_workspace_bytes(const spp_dmt_plan* plan, int64_t nsamps);
  * bit_sliced = 1 when the kernel counts over bit-plane rows (R = words per
  * thread); paired = 1 when its rows are sums of channel pairs (SLAB counts
  * pairs; the workspace then also holds one row per pair and relative delay,
- * which spp_dmt_plan_workspace_bytes includes) */
+ * which spp_dmt_plan_workspace_bytes includes).  Unless spp_dmt_plan_set_variant
+ * was called, blocks of less than half the plan's longest may run another shape,
+ * within the same workspace. */
 int spp_dmt_plan_describe(const spp_dmt_plan* plan, int32_t* cfg);
 /* override the tile shape (autotuner); variant index in [0, n) */
 int spp_dmt_plan_num_variants(const spp_dmt_plan* plan);

@@ -676,6 +676,8 @@ struct spp_dmt_plan {
   std::vector<int> cands;      // candidate variant indices
   std::vector<int32_t> spans;  // span per candidate
   int cur = 0;                 // index into cands
+  int packed[2] = {-1, -1};    // of these the packed shapes that estimates consider
+  bool chosen = false;         // cur was set by the caller
   // interleaved bit-plane kernels: rows of channels and of channel pairs, and
   // per kernel shape the staging tables (sized at creation, built when first
   // selected)
@@ -778,24 +780,72 @@ static int add_ilv_candidates(spp_dmt_plan* p, int32_t* words) {
   return SPP_OK;
 }
 
+// Byte lanes, four trials x two warps: the packed shape with the shortest walk
+// over the channels.
+static bool short_walk(const Variant& v) { return !v.planes && v.R == 2 && v.DW == 4 && v.TW == 2; }
+
+// Estimated time (us) of a block by a packed kernel over 32 consecutive samples
+// per word.  Few tiles: one CTA's walk over all channels, whatever the trials
+// (1024 channels: 170-330 us bit-sliced, 115 us by byte lanes of four trials).
+// Many: channel-adds at the measured rate, half as much again on coarse grids.
+// Either way the corner turn.
+static double packed_us(const spp_dmt_plan* p, int cand, int64_t nsamps, int64_t nvalid) {
+  const Variant& v = variants()[p->cands[cand]];
+  const int32_t span = p->spans[cand];
+  const int k = p->nbits == 1 ? 0 : p->nbits == 2 ? 1 : p->nbits == 4 ? 2 : 3;
+  const double adds = (double)p->ndm * nvalid * p->nchans;
+  const double mb = (double)nsamps * (double)(p->nchans * p->nbits) / 8e6;
+  if (short_walk(v)) {
+    static const double rate[] = {1.7e7, 1.9e7, 1.25e7, 0.75e7};  // adds per us
+    const double two = 1.2 + 3e-4 * p->nchans;  // walks of two CTAs on an SM over one alone
+    const int64_t ctas = ceil_div(p->ndm, v.DW) * ceil_div(nvalid, tile_T(v));
+    const int64_t per_sm = (228 << 10) / (smem_bytes(v, slot_words(v, span)) + 1024) >= 2 ? 2 : 1;
+    const double walk = 15.0 + (k == 0 ? 0.112 : 0.098) * p->nchans;
+    const double waves = (double)ceil_div(ctas, 148 * per_sm) * (per_sm == 2 && ctas > 148 ? two : 1.0);
+    return std::max(adds / rate[k] + 20.0, walk * waves) + (k == 3 ? 0.5 : 2.0) * mb;
+  }
+  static const double rate[] = {5.0e7, 5.2e7, 2.2e7, 0.95e7}, us0[] = {10, 14, 25, 25},
+                      chan[] = {0.158, 0.19, 0.305, 0.44};
+  const bool lanes = !v.planes;  // 8-bit, eight words per thread
+  const double fill = 0.35 + 0.65 * std::min(1.0, (double)p->ndm / v.DW);  // warps without a trial
+  const double walk = (lanes ? 12.0 : us0[k]) + (lanes ? 0.15 : chan[k]) * fill * p->nchans;
+  return std::max(1.5 * adds / (lanes ? 1.2e7 : rate[k]) + 20.0, walk) + (lanes ? 0.5 : 1.2) * mb;
+}
+
+// The same by an interleaved shape: per wave of 148 CTAs a fixed part (start,
+// first copies, stores) and a part per group of channels, both measured per shape
+// (IlvCfg::us_wave, ns_group), 0.3 us per MB of what its rows hold beyond the
+// block itself, 5.5 us per further block of 32 runs that a turning CTA goes
+// through, and the pair rows' CTAs where those are many and short.  Raw rows that
+// are no whole number of 16-byte units, and a last group of channels that is no
+// whole 32 bytes, are turned byte by byte (5.5 us per MB, 22 us per block).
+static double interleaved_us(const spp_dmt_plan* p, const IlvCfg& c, int64_t nsamps, const IlvGeom& g) {
+  const int64_t ctas = ceil_div(p->ndm, c.DW) * ceil_div(g.M, c.words());
+  const double ng = (double)round_up(p->nchans / c.G, 4 * c.nq);
+  double t = 10.0 + (double)ceil_div(ctas, 148) * (c.us_wave + ng * c.ns_group * 1e-3);
+  t += (double)(g.chan_bytes - p->nchans * g.M * c.nb * 4) * 3e-7;
+  const int64_t rowbytes = p->nchans * c.nb / 8, odd = rowbytes % 16 ? rowbytes : rowbytes % 32;
+  const int64_t blocks = p->ilv_rows[0].max_group / (32 * g.M);
+  t += odd ? 10.0 + 5.5e-6 * (double)nsamps * (double)odd + 22.0 * blocks : 5.5 * blocks;
+  if (c.G == 2) {
+    const double pair_ctas = (double)(p->nchans / 2) * (double)ceil_div(g.M + p->ilv_rows[0].max_ext, 512);
+    t += std::max((double)g.row_bytes * 3e-7, 2.3e-3 * pair_ctas);
+  }
+  return t;
+}
+
 // The shape a plan starts from (without autotuning): the least estimated time
-// at nsamps_max.  An interleaved shape takes, per wave of 148 CTAs, a fixed
-// part (start, first copies, stores) and a part per group of channels, both
-// measured per shape (IlvCfg::us_wave, ns_group: within 4 % of 20 measured
-// geometries of 256-4096 channels and 64-1024 trials), plus 0.3 us per MB of
-// what its rows hold beyond the block itself.  The kernels over 32 consecutive
-// samples per word run at the rates below (channel-adds per us on fine trial
-// grids); coarse grids and short blocks cost them half as much again and a
-// launch (8-bit, 1024 channels, 64 trials to DM 600, 40289 outputs: 0.56 ms
-// against 0.40 ms interleaved; 2-bit, 100 trials to DM 1500, 35724 outputs:
-// 0.18 against 0.22 ms).  Rows above kIlvDefaultBytes leave a shape to explicit
-// choice: they grow with the block and the delay range.
-// 2-bit grids so fine that a pair row serves 100 trials or more start from
-// pairs at every block length, so that the blocks of one observation run one
-// kernel (4096 channels, 1024 trials to DM 2000: 45.9 ms against 52.6 ms
-// without pairs at 1016174 outputs, 3.5 against 3.7 ms at 65536, 1.3 against
-// 1.0 ms at 16384).
-static int first_choice(const spp_dmt_plan* p) {
+// at nsamps_max, over the interleaved shapes, the first packed one and the one of
+// the shortest walk.  Over 190 measured plans (64-4096 channels, 2-1024 trials,
+// 50-100000 outputs) the choice is within 15 % of the fastest shape for all but
+// 12, and within 45 % for those.  Rows above kIlvDefaultBytes leave a shape to
+// explicit choice: they grow with the block and the delay range.
+// 2-bit grids so fine that a pair row serves 100 trials or more start from pairs
+// from 4096 outputs on (a pair shape's shortest tile), so that the blocks of one
+// observation run one kernel (4096 channels, 1024 trials to DM 2000: 45.9 ms
+// against 52.6 ms without pairs at 1016174 outputs, 3.5 against 3.7 ms at 65536,
+// 1.2 against 1.0 ms at 16384, 0.84 against 0.63 ms at 4096).
+static int first_choice(spp_dmt_plan* p) {
   constexpr int64_t kIlvDefaultBytes = 16ll << 30;
   const int64_t nvalid = std::max<int64_t>(1, plan_nvalid(p, p->nsamps_max));
   // Time tiles are a grid's y extent: shapes of short tiles cannot run the
@@ -826,31 +876,37 @@ static int first_choice(const spp_dmt_plan* p) {
     }
     return pick;
   }
-  const double adds_per_us = p->nbits == 1 ? 8.2e7 : p->nbits == 2 ? 5.0e7 : p->nbits == 4 ? 2.2e7 : 1.2e7;
-  double best = 1.5 * (double)p->ndm * nvalid * p->nchans / adds_per_us + 20.0;
+  for (int i = 0, n = 0; i < (int)p->cands.size() && n < 2; ++i)
+    if (ilv_index(p, i) < 0 && tiles_fit(i) && (n == 0 ? i >= first : short_walk(variants()[p->cands[i]])))
+      p->packed[n++] = i;
   const int64_t prows = p->ilv_rows[1].nrows;
-  const bool shared_pairs = p->nbits == 2 && prows > 0 && p->ndm * (p->nchans / 2) >= 100 * prows;
+  const bool shared_pairs = p->nbits == 2 && prows > 0 && nvalid >= 4096 &&
+                            p->ndm * (p->nchans / 2) >= 100 * prows;
   int pick = first;
-  bool any = p->cands[first] < kIlvCode;  // `first` is taken unless a better one follows
+  bool any = false;
   bool paired = false;
+  double best = 0.0;
   for (int i = 0; i < (int)p->cands.size(); ++i) {
     const int iv = ilv_index(p, i);
-    if (iv < 0) continue;
-    const IlvCfg& c = ilv_cfgs()[iv];
-    const IlvRows& rows = p->ilv_rows[c.G - 1];
-    const IlvGeom g = ilv_geometry(c, p->ilv_rows[0], rows, p->nchans, nvalid);
-    if (g.chan_bytes + g.row_bytes > kIlvDefaultBytes && any) continue;
-    const int64_t ctas = ceil_div(p->ndm, c.DW) * ceil_div(g.M, c.words());
-    const double ng = (double)round_up(p->nchans / c.G, 4 * c.nq);
-    double t = (double)ceil_div(ctas, 148) * (c.us_wave + ng * c.ns_group * 1e-3);
-    t += (double)(g.chan_bytes - p->nchans * g.M * c.nb * 4 + g.row_bytes) * 3e-7;
-    const bool first_pair = shared_pairs && c.G == 2 && !paired;
-    if (shared_pairs && paired && c.G == 1) continue;
-    if (t < best || !any || first_pair) {
+    double t;
+    bool pairs = false;
+    if (iv < 0) {
+      if (i != p->packed[0] && i != p->packed[1]) continue;
+      t = packed_us(p, i, p->nsamps_max, nvalid);
+      if (i == p->packed[0]) t *= 0.95;  // near ties stay with the smaller workspace
+    } else {
+      const IlvCfg& c = ilv_cfgs()[iv];
+      const IlvGeom g = ilv_geometry(c, p->ilv_rows[0], p->ilv_rows[c.G - 1], p->nchans, nvalid);
+      if (g.chan_bytes + g.row_bytes > kIlvDefaultBytes && any) continue;
+      t = interleaved_us(p, c, p->nsamps_max, g);
+      pairs = c.G == 2;
+    }
+    if (paired && shared_pairs && !pairs) continue;
+    if (t < best || !any || (shared_pairs && pairs && !paired)) {
       best = t;
       pick = i;
       any = true;
-      paired = paired || c.G == 2;
+      paired = pairs;
     }
   }
   return pick;
@@ -987,6 +1043,7 @@ int spp_dmt_plan_set_variant(spp_dmt_plan* p, int variant) {
   const int rc = ensure_tables(p, variant);
   if (rc != SPP_OK) return rc;
   p->cur = variant;
+  p->chosen = true;
   return SPP_OK;
 }
 
@@ -1011,9 +1068,9 @@ int spp_dmt_plan_describe(const spp_dmt_plan* p, int32_t* cfg) {
   return SPP_OK;
 }
 
-static Geometry plan_geometry(const spp_dmt_plan* p, int64_t nsamps, int* slot) {
-  const Variant& v = variants()[p->cands[p->cur]];
-  *slot = slot_words(v, p->spans[p->cur]);
+static Geometry plan_geometry(const spp_dmt_plan* p, int cand, int64_t nsamps, int* slot) {
+  const Variant& v = variants()[p->cands[cand]];
+  *slot = slot_words(v, p->spans[cand]);
   return geometry(v, p->nchans, nsamps, plan_nvalid(p, nsamps), p->omin, p->omax, *slot);
 }
 
@@ -1030,7 +1087,7 @@ int64_t spp_dmt_plan_workspace_bytes(const spp_dmt_plan* p, int64_t nsamps) {
     return kStatusBytes + g.chan_bytes + g.row_bytes;
   }
   int slot;
-  Geometry g = plan_geometry(p, nsamps, &slot);
+  Geometry g = plan_geometry(p, p->cur, nsamps, &slot);
   return kStatusBytes + g.bytes;
 }
 
@@ -1065,6 +1122,30 @@ static int ilv_run(const spp_dmt_plan* p, int iv, const void* in, int64_t nsamps
   return rc;
 }
 
+// The shape that a block runs.  Interleaved rows carry the whole delay range
+// whatever the block's length, so a block much shorter than the plan's longest (the
+// last of a stream) goes to a packed shape where that is estimated to take less and
+// the workspace, sized for the plan's own shape, holds its rows (1-bit, 336
+// channels, 639 trials to DM 1877, 1012 of 16205 outputs: 501 us against 79 us).
+// A shape that the caller set runs every block.
+static int block_shape(const spp_dmt_plan* p, int64_t nsamps, int64_t ws_bytes) {
+  const int iv = ilv_index(p, p->cur);
+  const int64_t nvalid = plan_nvalid(p, nsamps);
+  if (iv < 0 || p->chosen || 2 * nvalid > plan_nvalid(p, p->nsamps_max)) return p->cur;
+  int pick = p->cur;
+  double best = interleaved_us(p, ilv_cfgs()[iv], nsamps, plan_ilv_geometry(p, iv, nsamps));
+  for (int i : p->packed) {
+    if (i < 0) continue;
+    int slot;
+    const double t = packed_us(p, i, nsamps, nvalid);
+    if (t < best && kStatusBytes + plan_geometry(p, i, nsamps, &slot).bytes <= ws_bytes) {
+      best = t;
+      pick = i;
+    }
+  }
+  return pick;
+}
+
 static int dmt_run(const spp_dmt_plan* p, const void* in, int64_t nsamps, void* out,
                    int64_t out_stride, int64_t out_start, uint8_t* ws, int64_t ws_bytes,
                    cudaStream_t st, const float* zd_bpass = nullptr,
@@ -1078,16 +1159,17 @@ static int dmt_run(const spp_dmt_plan* p, const void* in, int64_t nsamps, void* 
   if (out_start < 0 || (p->ndm > 1 && out_stride < out_start + nvalid))
     return fail(SPP_ERR_SIZE, "out_stride %lld < out_start %lld + nvalid %lld",
                 (long long)out_stride, (long long)out_start, (long long)nvalid);
-  const int iv = ilv_index(p, p->cur);
+  const int cand = block_shape(p, nsamps, ws_bytes);
+  const int iv = ilv_index(p, cand);
   if (iv >= 0) return ilv_run(p, iv, in, nsamps, out, out_stride, out_start, ws, ws_bytes, st);
   int slot;
-  Geometry g = plan_geometry(p, nsamps, &slot);
+  Geometry g = plan_geometry(p, cand, nsamps, &slot);
   if (ws_bytes < kStatusBytes + g.bytes)
     return fail(SPP_ERR_SIZE, "workspace %lld B < required %lld B", (long long)ws_bytes,
                 (long long)(kStatusBytes + g.bytes));
   if (g.ntiles_t > kMaxTimeTiles)
     return fail(SPP_ERR_UNSUPPORTED, "%lld time tiles exceed the grid limit", (long long)g.ntiles_t);
-  const Variant& v = variants()[p->cands[p->cur]];
+  const Variant& v = variants()[p->cands[cand]];
   void* planar = ws + kStatusBytes;
   spp_dmt_plan* pm = const_cast<spp_dmt_plan*>(p);
   cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
@@ -1128,7 +1210,7 @@ static int dmt_run(const spp_dmt_plan* p, const void* in, int64_t nsamps, void* 
   a.sign = plan_sign(p);
   a.dlo = p->omin;
   a.dhi = p->omax;
-  a.span_max = p->spans[p->cur];
+  a.span_max = p->spans[cand];
   a.slot_w = slot;
   a.out = out;
   a.out_kind = p->out_kind;

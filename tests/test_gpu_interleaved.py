@@ -129,3 +129,33 @@ def test_long_rows_before_another_tile(orc):
     assert plan.describe()["bit_sliced"] and plan.describe()["T"] > 2048  # interleaved
     assert torch.equal(plan.execute(raw, nsamps, check=True), expect)
     plan.close()
+
+
+@pytest.mark.parametrize("nbits,nchans", [(1, 336), (2, 256), (4, 340), (8, 65)])
+def test_short_blocks_of_a_long_plan(orc, nbits, nchans):
+    """Blocks far shorter than nsamps_max may run another shape than the plan's:
+    the same sums, in the workspace that the plan asks for at that length or at
+    its longest, from an aligned address and the next."""
+    import torch
+
+    from sigpyproc3_b200.dedisp import DMTPlan
+
+    d = _delays(nchans, 600.0, 130)
+    longest = 20000 + int(d.max())
+    plan = DMTPlan(d, nchans, longest, nbits=nbits, bitorder="little" if nbits == 1 else "big",
+                   out_dtype=torch.int32)
+    for nvalid in (1, 257, 1900, 9999, 10001):
+        nsamps = nvalid + int(d.max())
+        vals = np.random.default_rng(nvalid).integers(0, 1 << nbits, nsamps * nchans, dtype=np.uint8)
+        expect = orc.dmt(vals, d, nchans, nsamps).astype(np.int64)
+        for shift, ws_samps in ((0, nsamps), (1, longest)):
+            raw = torch.from_numpy(np.concatenate([np.zeros(shift, np.uint8), _pack(vals, nbits)])).cuda()[shift:]
+            ws = torch.zeros(plan.workspace_bytes(ws_samps), dtype=torch.uint8, device="cuda")
+            out = torch.full((plan.ndm, nvalid + 2), -7, dtype=torch.int32, device="cuda")
+            got = plan.execute(raw, nsamps, out, out_start=1, ws=ws, check=True).cpu().numpy()
+            np.testing.assert_array_equal(got[:, 1:-1].astype(np.int64), expect)
+            assert (got[:, 0] == -7).all() and (got[:, -1] == -7).all()
+        small = torch.zeros(256, dtype=torch.uint8, device="cuda")
+        with pytest.raises(ValueError):
+            plan.execute(raw, nsamps, out, out_start=1, ws=small)
+    plan.close()
