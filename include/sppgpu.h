@@ -337,7 +337,8 @@ int spp_downsample_2d_mean_u8(const uint8_t* in, int64_t dim1, int64_t dim2,
  * argmax t to peak_index[row][fi][wi] (int32).  Semantics follow
  * TimeSeries.downsample + apply_boxcar (timeseries.py:107-132, :296-325) on a
  * z-scored series (stats.estimate_zscore, core/stats.py:418-477, loc=mean,
- * scale=std). */
+ * scale=std).  Scratch for (nrows, n, nfactors, nwidths) serves every call with
+ * none of the four larger. */
 int64_t spp_boxcar_snr_workspace_bytes(int64_t nrows, int64_t n, int nfactors,
                                        int nwidths);
 int spp_boxcar_snr(const void* in, int in_kind, int64_t nrows, int64_t n,
@@ -363,7 +364,8 @@ int spp_boxcar_filter(const float* in, int64_t n, int width, float* out,
  *   scale = (q75 - q25) / 1.3489795003921634 (float64; numpy's linear
  *           percentile interpolation; 1 when ~0)
  *   snr   = max_t (sum_{k<w} y[t+k] - w*loc) / (scale * sqrt(w)).
- * The order statistics are exact (radix selection over the float32 y). */
+ * The order statistics are exact (radix selection over the float32 y).  Scratch
+ * as above. */
 int64_t spp_boxcar_snr_robust_workspace_bytes(int64_t nrows, int64_t n,
                                               int nfactors, int nwidths);
 int spp_boxcar_snr_robust(const void* in, int in_kind, int64_t nrows,

@@ -1247,13 +1247,18 @@ static int snr_chunk(int64_t nrf, int64_t n) {
   return 1536;
 }
 
-// Sizes the S/N workspace for `n` samples per row.
+// Sizes the S/N workspace for `n` samples per row, and sets the chunks per series.
+// The size is for any shorter series and any fewer of them too: scratch reserved
+// for the largest call serves all.  Chunks shorter than kSnrChunk are taken while
+// longer ones number below 148 * 8, so they number below twice that.
 int64_t snr_ws(int64_t nrows, int64_t n, int nfactors, int nwidths, int64_t* nchunks) {
-  const int64_t nck = ceil_div(std::max<int64_t>(n, 1), snr_chunk(nrows * nfactors, n));
-  *nchunks = nck;
-  const int64_t parts = nrows * nfactors * nwidths * nck * (int64_t)sizeof(SnrPart);
-  const int64_t stats = nrows * nfactors * nck * 3 * (int64_t)sizeof(double);
-  return kStatusBytes + round_up(parts, 256) + round_up(stats, 256);
+  const int64_t nrf = nrows * nfactors;
+  n = std::max<int64_t>(n, 1);
+  *nchunks = ceil_div(n, snr_chunk(nrf, n));
+  const int64_t most = std::max(nrf * ceil_div(n, kSnrChunk),
+                                std::min<int64_t>(nrf * ceil_div(n, 1536), 2 * 148 * 8));
+  return kStatusBytes + round_up(most * nwidths * (int64_t)sizeof(SnrPart), 256) +
+         round_up(most * 3 * (int64_t)sizeof(double), 256);
 }
 
 extern "C" {
@@ -1265,9 +1270,10 @@ int64_t spp_boxcar_snr_workspace_bytes(int64_t nrows, int64_t n, int nfactors, i
 
 }  // extern "C"
 
-// Robust z-score: loc and scale per (row, factor), and the selection's state.
+// Robust z-score: loc and scale per (row, factor), and the selection's state, for
+// any fewer series too (from kQSplitRows on they are not split and need none).
 static int64_t robust_ws(int64_t nrf, int64_t n) {
-  return round_up(nrf * 16, 256) + round_up(q_workspace(nrf, n), 256);
+  return round_up(nrf * 16, 256) + round_up(q_workspace(std::min<int64_t>(nrf, kQSplitRows - 1), n), 256);
 }
 
 static int boxcar_snr_impl(const void* in, int in_kind, int64_t nrows, int64_t n,
