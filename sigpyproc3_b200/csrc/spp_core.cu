@@ -683,6 +683,8 @@ struct spp_dmt_plan {
   // selected)
   IlvRows ilv_rows[2];
   std::vector<IlvTables> ilv_tabs;
+  void* room = nullptr;        // within the allocation of d_delays
+  int64_t room_bytes = 0;
   // optional per-kernel timing: events (start, after corner turn, end) per execute
   bool timing = false;
   std::vector<cudaEvent_t> evpool;
@@ -720,7 +722,11 @@ static int ensure_tables(spp_dmt_plan* p, int i) {
   const int iv = ilv_index(p, i);
   if (iv < 0) return SPP_OK;
   const IlvCfg& c = ilv_cfgs()[iv];
-  return ilv_build_tables(c, ilv_delays(p), p->ilv_rows[c.G - 1], &p->ilv_tabs[iv]);
+  // the plan's room serves the first shape
+  bool taken = false;
+  for (const IlvTables& t : p->ilv_tabs) taken = taken || (t.d_off && !t.own);
+  return ilv_build_tables(c, ilv_delays(p), p->ilv_rows[c.G - 1], p->room, taken ? 0 : p->room_bytes,
+                          &p->ilv_tabs[iv]);
 }
 
 static void free_device(spp_dmt_plan* p) {
@@ -732,22 +738,26 @@ static void free_device(spp_dmt_plan* p) {
 // Pair rows a plan may hold, per channel.
 constexpr int64_t kPairRowsPerChan = 12;
 
-// Device words of a plan: the delay table, then (for interleaved shapes) the
-// words that make their rows, from a 256-byte boundary on: the range passes
-// store pairs of words there, whatever the table's size.
+// Device words of a plan, one allocation (a second one of some MB takes 0.4 ms): the
+// delay table, then (for interleaved shapes) the words that make their rows, from
+// a 256-byte boundary on: the range pass stores pairs of words there, whatever
+// the table's size; then room for the staging tables of the shape that the plan
+// starts from, unless they may be large.
 struct PlanWords {
-  int64_t work, total;
+  int64_t work, room, total;
 };
 static PlanWords plan_words(int nbits, int64_t nchans, int64_t ndm) {
   const int64_t table = ndm * nchans;
-  if (ndm <= 1 || nbits > 8) return {table, table};
+  if (ndm <= 1 || nbits > 8) return {table, table, table};
   const int64_t work = round_up(table, 64);
-  return {work, work + ilv_plan_words(nchans, kPairRowsPerChan * nchans)};
+  const int64_t room = round_up(work + ilv_plan_words(nchans, kPairRowsPerChan * nchans), 64);
+  const int64_t bytes = ilv_table_room(nbits, nchans, ndm);
+  return {work, room, room + (bytes <= 64ll << 20 ? bytes / 4 : 0)};
 }
 
 // Interleaved bit-plane shapes this table and sample width can use.  `words`:
 // plan-owned device words after the delay table.
-static int add_ilv_candidates(spp_dmt_plan* p, int32_t* words) {
+static int add_ilv_candidates(spp_dmt_plan* p, const IlvScan& scan, int32_t* words) {
   const auto& cfgs = ilv_cfgs();
   p->ilv_tabs.resize(cfgs.size());
   const IlvDelays d = ilv_delays(p);
@@ -761,7 +771,7 @@ static int add_ilv_candidates(spp_dmt_plan* p, int32_t* words) {
     for (int G = 1; G <= c.G; ++G) {
       IlvRows& r = p->ilv_rows[G - 1];
       if (r.G != 0) continue;
-      const int rc = ilv_make_rows(d, G, max_rows, &ar, &r);
+      const int rc = ilv_make_rows(d, scan, G, max_rows, &ar, &r);
       r.G = G;
       if (rc == SPP_ERR_UNSUPPORTED) continue;  // no rows: shapes of this grouping are skipped
       if (rc) return rc;
@@ -935,23 +945,55 @@ int spp_dmt_plan_create(spp_dmt_plan** plan, int nbits, int bitorder, int64_t nc
   if (!p) return fail(SPP_ERR_ARG, "out of host memory");
   p->nbits = nbits; p->bitorder = bitorder; p->mode = mode; p->out_kind = out_kind; p->acc = acc;
   p->nchans = nchans; p->nsamps_max = nsamps_max; p->ndm = ndm;
-  int32_t dmin = INT32_MAX, dmax = INT32_MIN;
-  for (int64_t i = 0; i < ndm * nchans; ++i) {
-    dmin = std::min(dmin, delays_host[i]);
-    dmax = std::max(dmax, delays_host[i]);
-  }
-  p->dmin = dmin; p->dmax = dmax;
-  p->maxabs = (int32_t)std::max<int64_t>(std::llabs(dmin), std::llabs(dmax));
+  const bool ilv = ndm > 1 && nbits <= 8;
   const int sign = plan_sign(p);
-  p->omin = sign > 0 ? dmin : -dmax;
-  p->omax = sign > 0 ? dmax : -dmin;
+  auto set_range = [&](int32_t omin, int32_t omax) {
+    p->omin = omin; p->omax = omax;
+    p->dmin = sign > 0 ? omin : -omax;
+    p->dmax = sign > 0 ? omax : -omin;
+    p->maxabs = (int32_t)std::max<int64_t>(std::llabs(omin), std::llabs(omax));
+  };
+  if (!ilv || mode == SPP_MODE_ROLL) {
+    int32_t dmin = INT32_MAX, dmax = INT32_MIN;
+    for (int64_t i = 0; i < ndm * nchans; ++i) {
+      dmin = std::min(dmin, delays_host[i]);
+      dmax = std::max(dmax, delays_host[i]);
+    }
+    set_range(sign > 0 ? dmin : -dmax, sign > 0 ? dmax : -dmin);
+  }
   if (mode == SPP_MODE_ROLL && p->maxabs >= nsamps_max) {
     delete p;
     return fail(SPP_ERR_DELAY, "roll mode needs |delay| < nsamps");
   }
+  p->dpitch = nchans;
+  const PlanWords words = plan_words(nbits, nchans, ndm);
+  cudaError_t e = cudaMalloc(&p->d_delays, sizeof(int32_t) * words.total);
+  if (e != cudaSuccess) { delete p; return cuda_status(e, "plan cudaMalloc"); }
+  e = cudaMemcpy(p->d_delays, delays_host, sizeof(int32_t) * ndm * nchans, cudaMemcpyHostToDevice);
+  int rc = cuda_status(e, "plan upload");
+  p->room = p->d_delays + words.room;
+  p->room_bytes = 4 * (words.total - words.room);
+  // Ranges and the spreads of trial tiles, of four and eight trials for all packed
+  // integer shapes: found on the device beside the interleaved rows' ranges (the
+  // host took 0.14 ms per tile height and as much for the range over 512 trials x
+  // 1024 channels).
+  IlvScan scan;
+  if (rc == SPP_OK && ilv) {
+    IlvArena ar{nullptr, p->d_delays + words.work};
+    rc = ilv_scan(ilv_delays(p), &ar, &scan);
+    if (rc == SPP_OK) {
+      int32_t omin = INT32_MAX, omax = INT32_MIN;
+      for (const int2& r : scan.range[0]) {
+        omin = std::min(omin, r.x);
+        omax = std::max(omax, r.y);
+      }
+      set_range(omin, omax);
+    }
+  }
   // candidates; the delay spread of DM tiles is computed once per tile height
   const auto& vs = variants();
   std::vector<std::pair<int, int32_t>> span_of_dw;
+  if (ilv) span_of_dw = {{4, scan.span4}, {8, scan.span8}};
   auto tile_span = [&](int dw) -> int32_t {
     for (auto& e : span_of_dw)
       if (e.first == dw) return e.second;
@@ -984,14 +1026,7 @@ int spp_dmt_plan_create(spp_dmt_plan** plan, int nbits, int bitorder, int64_t nc
     p->cands.push_back(i);
     p->spans.push_back(span);
   }
-  p->dpitch = nchans;
-  const bool ilv = ndm > 1 && nbits <= 8;
-  const PlanWords words = plan_words(nbits, nchans, ndm);
-  cudaError_t e = cudaMalloc(&p->d_delays, sizeof(int32_t) * words.total);
-  if (e != cudaSuccess) { delete p; return cuda_status(e, "plan cudaMalloc"); }
-  e = cudaMemcpy(p->d_delays, delays_host, sizeof(int32_t) * ndm * nchans, cudaMemcpyHostToDevice);
-  int rc = cuda_status(e, "plan upload");
-  if (rc == SPP_OK && ilv) rc = add_ilv_candidates(p, p->d_delays + words.work);
+  if (rc == SPP_OK && ilv) rc = add_ilv_candidates(p, scan, p->d_delays + words.work);
   if (rc == SPP_OK && p->cands.empty())
     rc = fail(SPP_ERR_UNSUPPORTED, "no kernel variant fits this delay table");
   if (rc == SPP_OK) {

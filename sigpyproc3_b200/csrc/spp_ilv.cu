@@ -658,32 +658,62 @@ k_ilv_pairs(const uint32_t* __restrict__ chan, int64_t mpc, const int32_t* __res
 // ---------------------------------------------------------------------------
 // Plan tables, from the delay table on the device.
 // ---------------------------------------------------------------------------
-// Smallest and largest signed offset of every channel; for pairs the same of
-// the relative offsets.  A CTA takes 32 groups, its eight warps the trials.
+// One pass over the table: smallest and largest signed offset of every channel and
+// relative offset of every pair, and the widest spread of a channel over tiles of
+// four and of eight trials (per CTA).  A CTA takes 32 channels, its eight warps
+// the tiles.
 __global__ void __launch_bounds__(256)
-k_ilv_ranges(IlvDelays d, int G, int2* __restrict__ out) {
-  __shared__ int2 red[8][32];
+k_ilv_scan(IlvDelays d, int2* __restrict__ chan, int2* __restrict__ pair, int2* __restrict__ spans) {
+  __shared__ int2 red[8][32], redp[8][32], reds[8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t g = (int64_t)blockIdx.x * 32 + lane;
-  int mn = INT_MAX, mx = INT_MIN;
-  if (g < d.nchans / G) {
-#pragma unroll 4
-    for (int64_t i = warp; i < d.ndm; i += 8) {
-      const int32_t* row = d.d_delays + i * d.nchans;
-      const int o = G == 1 ? d.sign * row[g] : d.sign * (row[2 * g + 1] - row[2 * g]);
-      mn = min(mn, o);
-      mx = max(mx, o);
+  const int64_t c = (int64_t)blockIdx.x * 32 + lane;
+  const bool on = c < d.nchans, two = !(lane & 1) && c + 1 < d.nchans;
+  int mn = INT_MAX, mx = INT_MIN, pmn = INT_MAX, pmx = INT_MIN, s4 = 0, s8 = 0;
+  for (int64_t t = warp; t * 8 < d.ndm; t += 8) {
+    int o[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      o[i] = on ? d.sign * __ldg(d.d_delays + min(t * 8 + i, d.ndm - 1) * d.nchans + c) : 0;
+    int tn[2], tx[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      tn[h] = tx[h] = o[4 * h];
+#pragma unroll
+      for (int i = 1; i < 4; ++i) {
+        tn[h] = min(tn[h], o[4 * h + i]);
+        tx[h] = max(tx[h], o[4 * h + i]);
+      }
+      s4 = max(s4, tx[h] - tn[h]);
+    }
+    const int n8 = min(tn[0], tn[1]), x8 = max(tx[0], tx[1]);
+    s8 = max(s8, x8 - n8);
+    mn = min(mn, n8);
+    mx = max(mx, x8);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = __shfl_down_sync(0xffffffffu, o[i], 1) - o[i];
+      pmn = min(pmn, r);
+      pmx = max(pmx, r);
     }
   }
+  s4 = __reduce_max_sync(0xffffffffu, s4);
+  s8 = __reduce_max_sync(0xffffffffu, s8);
   red[warp][lane] = make_int2(mn, mx);
+  redp[warp][lane] = make_int2(pmn, pmx);
+  if (lane == 0) reds[warp] = make_int2(s4, s8);
   __syncthreads();
-  if (warp == 0 && g < d.nchans / G) {
-    for (int w = 1; w < 8; ++w) {
-      mn = min(mn, red[w][lane].x);
-      mx = max(mx, red[w][lane].y);
-    }
-    out[g] = make_int2(mn, mx);
+  if (warp != 0) return;
+  for (int w = 1; w < 8; ++w) {
+    mn = min(mn, red[w][lane].x);
+    mx = max(mx, red[w][lane].y);
+    pmn = min(pmn, redp[w][lane].x);
+    pmx = max(pmx, redp[w][lane].y);
+    s4 = max(s4, reds[w].x);
+    s8 = max(s8, reds[w].y);
   }
+  if (on) chan[c] = make_int2(mn, mx);
+  if (two) pair[c / 2] = make_int2(pmn, pmx);
+  if (lane == 0) spans[blockIdx.x] = make_int2(s4, s8);
 }
 
 __device__ __forceinline__ int ilv_row_of(const IlvDelays& d, int G, const int32_t* rbase,
@@ -695,6 +725,14 @@ __device__ __forceinline__ int ilv_row_of(const IlvDelays& d, int G, const int32
   }
   *o = d.sign * row[2 * g];
   return rbase[g] + (d.sign * row[2 * g + 1] - *o) - rlo[g];
+}
+
+__global__ void k_ilv_row_init(int64_t n, int32_t* __restrict__ mn, int32_t* __restrict__ mx) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) {
+    mn[i] = INT_MAX;
+    mx[i] = INT_MIN;
+  }
 }
 
 // Offset range of every pair row over the trials that read it.
@@ -714,13 +752,17 @@ __global__ void k_ilv_row_ranges(IlvDelays d, const int32_t* __restrict__ rbase,
 
 // Staging tables: one thread per (trial tile, slab).  Without `off` only the
 // largest entry count and stage size are taken (stats[0], stats[1] in words).
-__global__ void k_ilv_tables(IlvDelays d, int G, int np, int DW, int W, int nq, int emax,
-                             int64_t ntile, int64_t nslab, const int32_t* __restrict__ lo,
-                             const int32_t* __restrict__ ext, const int32_t* __restrict__ rbase,
-                             const int32_t* __restrict__ rlo, int32_t* __restrict__ off,
-                             int4* __restrict__ ent, int* __restrict__ stats) {
-  const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= ntile * nslab) return;
+struct IlvTableShape {
+  int G, np, DW, W, nq;
+  int64_t ntile, nslab;
+  const int32_t *lo, *ext, *rbase, *rlo;
+};
+__device__ __forceinline__ void ilv_table(const IlvDelays& d, const IlvTableShape& sh, int64_t id, int emax,
+                                          int32_t* __restrict__ off, int4* __restrict__ ent,
+                                          int* __restrict__ stats) {
+  const int G = sh.G, np = sh.np, DW = sh.DW, W = sh.W, nq = sh.nq;
+  const int64_t nslab = sh.nslab;
+  const int32_t *lo = sh.lo, *ext = sh.ext, *rbase = sh.rbase, *rlo = sh.rlo;
   const int64_t tile = id / nslab, k = id - tile * nslab;
   const int64_t ng = d.nchans / G;
   int pos = 0, e = 0, zpos = -1;
@@ -773,6 +815,21 @@ __global__ void k_ilv_tables(IlvDelays d, int G, int np, int DW, int W, int nq, 
     atomicMax(&stats[1], pos);
   }
 }
+__global__ void k_ilv_tables(IlvDelays d, IlvTableShape sh, int emax, int32_t* __restrict__ off,
+                             int4* __restrict__ ent) {
+  const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (id < sh.ntile * sh.nslab) ilv_table(d, sh, id, emax, off, ent, nullptr);
+}
+// The sizes of several shapes at once (shape blockIdx.y).
+constexpr int kIlvMaxShapes = 8;
+struct IlvTableShapes {
+  IlvTableShape s[kIlvMaxShapes];
+};
+__global__ void k_ilv_table_sizes(IlvDelays d, const __grid_constant__ IlvTableShapes sh, int* __restrict__ stats) {
+  const IlvTableShape& s = sh.s[blockIdx.y];
+  const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (id < s.ntile * s.nslab) ilv_table(d, s, id, kIlvMaxEnt, nullptr, nullptr, stats + 2 * blockIdx.y);
+}
 
 template <int NB, int G, int P, int DW, int TW, int NQ, int LR, int MINB>
 IlvCfg mki(double us_wave, double ns_group) {
@@ -821,22 +878,62 @@ const std::vector<IlvCfg>& ilv_cfgs() {
 }
 
 void ilv_free_tables(IlvTables* t) {
-  cudaFree(t->d_off);
+  if (t->own) cudaFree(t->d_off);
   t->d_off = nullptr;
   t->d_ent = nullptr;
+  t->own = false;
 }
 
 // Device words a plan keeps beside its delay table: the rows of both
 // groupings, and scratch for the range passes and table sizes.
 int64_t ilv_plan_words(int64_t nchans, int64_t max_rows) {
-  return 2 * (nchans + 1) + 2 * (max_rows + 1) + (nchans + 2) + 2 * nchans + 2 * max_rows + 64;
+  return 2 * (nchans + 1) + 2 * (max_rows + 1) + (nchans + 2) + 4 * nchans + 2 * max_rows + 64;
 }
 
-int ilv_make_rows(const IlvDelays& d, int G, int64_t max_rows, IlvArena* ar, IlvRows* out) {
+static IlvTableShape table_shape(const IlvCfg& c, const IlvDelays& d, const IlvRows& r) {
+  return IlvTableShape{c.G, c.np, c.DW, c.words(), c.nq, ceil_div(d.ndm, c.DW),
+                       ceil_div(d.nchans / c.G, 4 * c.nq), r.d_lo, r.d_ext, r.d_rbase, r.d_rlo};
+}
+
+static int64_t table_off_bytes(const IlvCfg& c, int64_t nchans, int64_t ndm) {
+  return round_up(ceil_div(ndm, c.DW) * ceil_div(nchans / c.G, 4 * c.nq) * c.DW * 4 * c.nq * 4, 256);
+}
+static int64_t table_bytes(const IlvCfg& c, int64_t nchans, int64_t ndm, int emax) {
+  return table_off_bytes(c, nchans, ndm) +
+         ceil_div(ndm, c.DW) * ceil_div(nchans / c.G, 4 * c.nq) * emax * (int64_t)sizeof(int4);
+}
+
+// Room for the staging tables of whichever shape a plan starts from: a slab's
+// groups read a row each, pairs up to kIlvMaxEnt together.
+int64_t ilv_table_room(int nb, int64_t nchans, int64_t ndm) {
+  int64_t most = 0;
+  for (const IlvCfg& c : ilv_cfgs())
+    if (c.nb == nb && nchans % c.G == 0)
+      most = std::max(most, table_bytes(c, nchans, ndm, c.G == 1 ? 4 * c.nq + 1 : kIlvMaxEnt));
+  return most;
+}
+
+int ilv_scan(const IlvDelays& d, IlvArena* ar, IlvScan* out) {
+  if (reinterpret_cast<uintptr_t>(ar->scratch) % sizeof(int2))  // ranges are stored as int2
+    return fail(SPP_ERR_ARG, "interleaved rows: misaligned scratch");
+  const int64_t np = d.nchans / 2, nblk = ceil_div(d.nchans, 32);
+  int2* base = reinterpret_cast<int2*>(ar->scratch);
+  std::vector<int2> h(d.nchans + np + nblk);
+  k_ilv_scan<<<(unsigned)nblk, 256>>>(d, base, base + d.nchans, base + d.nchans + np);
+  const int rc = cuda_status(cudaMemcpy(h.data(), base, sizeof(int2) * h.size(), cudaMemcpyDeviceToHost), "offset ranges");
+  if (rc) return rc;
+  out->range[0].assign(h.begin(), h.begin() + d.nchans);
+  out->range[1].assign(h.begin() + d.nchans, h.begin() + d.nchans + np);
+  for (int64_t b = d.nchans + np; b < (int64_t)h.size(); ++b) {
+    out->span4 = std::max(out->span4, h[b].x);
+    out->span8 = std::max(out->span8, h[b].y);
+  }
+  return SPP_OK;
+}
+
+int ilv_make_rows(const IlvDelays& d, const IlvScan& scan, int G, int64_t max_rows, IlvArena* ar, IlvRows* out) {
   const int64_t ng = d.nchans / G;
   if (d.nchans % G || ng <= 0) return SPP_ERR_UNSUPPORTED;
-  if (reinterpret_cast<uintptr_t>(ar->scratch) % sizeof(int2))  // k_ilv_ranges stores int2
-    return fail(SPP_ERR_ARG, "interleaved rows: misaligned scratch");
   IlvRows r{};
   r.G = G;
   int32_t* scratch = ar->scratch;
@@ -847,10 +944,7 @@ int ilv_make_rows(const IlvDelays& d, int G, int64_t max_rows, IlvArena* ar, Ilv
   auto down = [&](void* dst, const void* s, int64_t words) {
     if (!rc) rc = cuda_status(cudaMemcpy(dst, s, 4 * words, cudaMemcpyDeviceToHost), "row ranges");
   };
-  std::vector<int2> rng(ng);
-  k_ilv_ranges<<<(unsigned)ceil_div(ng, 32), 256>>>(d, G, reinterpret_cast<int2*>(scratch));
-  down(rng.data(), scratch, 2 * ng);
-  if (rc) return rc;
+  const std::vector<int2>& rng = scan.range[G - 1];
   std::vector<int32_t> mn, mx;
   if (G == 1) {
     r.nrows = ng;
@@ -872,12 +966,11 @@ int ilv_make_rows(const IlvDelays& d, int G, int64_t max_rows, IlvArena* ar, Ilv
     r.d_rbase = ar->take(2 * ng + 1);
     r.d_rlo = r.d_rbase + ng + 1;
     up(r.d_rbase, head.data(), 2 * ng + 1);
-    mn.assign(2 * n, INT_MAX);
-    std::fill(mn.begin() + n, mn.end(), INT_MIN);
-    up(scratch, mn.data(), 2 * n);
     if (rc) return rc;
+    k_ilv_row_init<<<(unsigned)ceil_div(n, 256), 256>>>(n, scratch, scratch + n);
     k_ilv_row_ranges<<<dim3((unsigned)ceil_div(ng, 128), (unsigned)std::min<int64_t>(d.ndm, 64)), 128>>>(
         d, r.d_rbase, r.d_rlo, scratch, scratch + n);
+    mn.resize(2 * n);
     down(mn.data(), scratch, 2 * n);
     if (rc) return rc;
     mx.assign(mn.begin() + n, mn.end());
@@ -919,25 +1012,22 @@ int ilv_make_rows(const IlvDelays& d, int G, int64_t max_rows, IlvArena* ar, Ilv
   return SPP_OK;
 }
 
-static int table_pass(const IlvCfg& c, const IlvDelays& d, const IlvRows& r, int emax, int32_t* off,
-                      int4* ent, int* stats) {
-  const int64_t ntile = ceil_div(d.ndm, c.DW), nslab = ceil_div(d.nchans / c.G, 4 * c.nq);
-  k_ilv_tables<<<(unsigned)ceil_div(ntile * nslab, 64), 64>>>(d, c.G, c.np, c.DW, c.words(), c.nq, emax, ntile,
-                                                             nslab, r.d_lo, r.d_ext, r.d_rbase,
-                                                             r.d_rlo, off, ent, stats);
-  return cuda_status(cudaGetLastError(), "staging tables");
-}
-
 int ilv_size_tables(const std::vector<int>& which, const IlvDelays& d, const IlvRows* rows,
                     IlvArena* ar, std::vector<IlvTables>* tabs) {
   const int n = (int)which.size();
-  std::vector<int> st(2 * n + 1, 0);
-  int rc = cuda_status(cudaMemset(ar->scratch, 0, sizeof(int) * 2 * n), "stats clear");
-  for (int i = 0; i < n && !rc; ++i) {
+  if (n > kIlvMaxShapes) return fail(SPP_ERR_ARG, "more than %d interleaved shapes", kIlvMaxShapes);
+  std::vector<int> st(2 * n, 0);
+  IlvTableShapes sh{};
+  int64_t most = 1;
+  for (int i = 0; i < n; ++i) {
     const IlvCfg& c = ilv_cfgs()[which[i]];
-    rc = table_pass(c, d, rows[c.G - 1], kIlvMaxEnt, nullptr, nullptr, ar->scratch + 2 * i);
+    sh.s[i] = table_shape(c, d, rows[c.G - 1]);
+    most = std::max(most, sh.s[i].ntile * sh.s[i].nslab);
   }
-  if (!rc) rc = cuda_status(cudaMemcpy(st.data(), ar->scratch, sizeof(int) * 2 * n, cudaMemcpyDeviceToHost), "stats");
+  int rc = cuda_status(cudaMemsetAsync(ar->scratch, 0, sizeof(int) * 2 * n), "stats clear");
+  if (rc) return rc;
+  k_ilv_table_sizes<<<dim3((unsigned)ceil_div(most, 64), (unsigned)n), 64>>>(d, sh, ar->scratch);
+  rc = cuda_status(cudaMemcpy(st.data(), ar->scratch, sizeof(int) * 2 * n, cudaMemcpyDeviceToHost), "table sizes");
   if (rc) return rc;
   for (int i = 0; i < n; ++i) {
     const IlvCfg& c = ilv_cfgs()[which[i]];
@@ -957,16 +1047,23 @@ int ilv_size_tables(const std::vector<int>& which, const IlvDelays& d, const Ilv
   return SPP_OK;
 }
 
-int ilv_build_tables(const IlvCfg& c, const IlvDelays& d, const IlvRows& r, IlvTables* t) {
+int ilv_build_tables(const IlvCfg& c, const IlvDelays& d, const IlvRows& r, void* room, int64_t room_bytes,
+                     IlvTables* t) {
   if (t->d_off) return SPP_OK;
-  const int64_t n = ceil_div(d.ndm, c.DW) * ceil_div(d.nchans / c.G, 4 * c.nq);
-  const int64_t off_bytes = round_up(n * c.DW * 4 * c.nq * 4, 256);
-  void* p = nullptr;
-  int rc = cuda_status(cudaMalloc(&p, (size_t)(off_bytes + n * t->emax * (int64_t)sizeof(int4))), "plan table alloc");
-  if (rc) return rc;
+  const int64_t bytes = table_bytes(c, d.nchans, d.ndm, t->emax);
+  void* p = room;
+  int rc = SPP_OK;
+  if (bytes > room_bytes) {
+    rc = cuda_status(cudaMalloc(&p, (size_t)bytes), "plan table alloc");
+    if (rc) return rc;
+    t->own = true;
+  }
+  t->bytes = bytes;
   t->d_off = static_cast<int32_t*>(p);
-  t->d_ent = reinterpret_cast<int4*>(static_cast<uint8_t*>(p) + off_bytes);
-  rc = table_pass(c, d, r, t->emax, t->d_off, t->d_ent, nullptr);
+  t->d_ent = reinterpret_cast<int4*>(static_cast<uint8_t*>(p) + table_off_bytes(c, d.nchans, d.ndm));
+  const IlvTableShape sh = table_shape(c, d, r);
+  k_ilv_tables<<<(unsigned)ceil_div(sh.ntile * sh.nslab, 64), 64>>>(d, sh, t->emax, t->d_off, t->d_ent);
+  rc = cuda_status(cudaGetLastError(), "staging tables");
   if (!rc) rc = cuda_status(cudaStreamSynchronize(nullptr), "staging tables");
   if (rc) ilv_free_tables(t);
   return rc;

@@ -47,8 +47,10 @@ struct IlvTables {
   int64_t stage_bytes = 0;
   int stages = 0;
   int64_t smem = 0;
-  int32_t* d_off = nullptr;  // (tile, slab, trial, group): byte offset in the stage (owns both)
+  int32_t* d_off = nullptr;  // (tile, slab, trial, group): byte offset in the stage
   int4* d_ent = nullptr;     // (tile, slab, entry): row, word offset, words, stage position
+  bool own = false;          // d_off is an allocation (of both), not a plan's room
+  int64_t bytes = 0;         // of both
 };
 
 // A delay table on the device.
@@ -71,16 +73,27 @@ struct IlvArena {
   }
 };
 int64_t ilv_plan_words(int64_t nchans, int64_t max_rows);
+// Bytes that the tables of any shape of this width may take.
+int64_t ilv_table_room(int nb, int64_t nchans, int64_t ndm);
+
+// What one pass over a delay table finds.
+struct IlvScan {
+  std::vector<int2> range[2];        // per channel, per pair: smallest and largest (relative) offset
+  int32_t span4 = 0, span8 = 0;      // widest spread over tiles of four, of eight trials
+};
+int ilv_scan(const IlvDelays& d, IlvArena* ar, IlvScan* out);
 
 void ilv_free_tables(IlvTables* t);
 // Rows of grouping G (1 or 2); more than `max_rows` pair rows:
 // SPP_ERR_UNSUPPORTED.
-int ilv_make_rows(const IlvDelays& d, int G, int64_t max_rows, IlvArena* ar, IlvRows* out);
+int ilv_make_rows(const IlvDelays& d, const IlvScan& scan, int G, int64_t max_rows, IlvArena* ar, IlvRows* out);
 // Sizes the staging of the shapes `which` (stages = 0: the table's spreads do
 // not fit) from the rows of G = 1 and 2.
 int ilv_size_tables(const std::vector<int>& which, const IlvDelays& d, const IlvRows* rows,
                     IlvArena* ar, std::vector<IlvTables>* tabs);
-int ilv_build_tables(const IlvCfg& c, const IlvDelays& d, const IlvRows& r, IlvTables* t);
+// Builds them in `room` where it is large enough, else in memory of their own.
+int ilv_build_tables(const IlvCfg& c, const IlvDelays& d, const IlvRows& r, void* room, int64_t room_bytes,
+                     IlvTables* t);
 
 struct IlvGeom {
   int64_t M;        // words per row that carry outputs (32 * M >= nvalid)
