@@ -275,8 +275,11 @@ __device__ __forceinline__ long long warp_sum64(long long v) {
 }
 
 // Window arithmetic of the two paths: prefix sums (T), the sum of a window
-// (V), and the warp's largest one.
+// (V), the warp's largest one, and the widths taken at a time (kGroup: float64
+// twelve, as 256 rows x 100001 and 11 or 24 widths take 7 and 2 % longer by tens;
+// integer ten, as twelve cost banks of up to ten widths 2 %).
 struct SnrInt {
+  static constexpr int kGroup = 10;
   typedef uint32_t T;
   typedef int32_t V;
   __device__ __forceinline__ static V lowest() { return INT_MIN; }
@@ -287,6 +290,7 @@ struct SnrInt {
   __device__ __forceinline__ static V warp_max(V v) { return __reduce_max_sync(0xffffffffu, v); }
 };
 struct SnrF64 {
+  static constexpr int kGroup = 12;
   typedef double T;
   typedef double V;
   __device__ __forceinline__ static V lowest() { return -DBL_MAX; }
@@ -368,17 +372,28 @@ __device__ __forceinline__ void snr_scan_regs(uint32_t* s, uint32_t* red) {
   __syncthreads();
 }
 
+// Shared words of the widths' search, one set for every group size: a set of its
+// own per group size left three float32 CTAs per SM where four fit (100 rows x
+// 30000, widths 1 to 512: 51.1 -> 38.2 us; 256 x 100001: 288 -> 241 us).
+template <class A>
+struct SnrBest {
+  typename A::V wbest[kSnrWarps][A::kGroup];
+  typename A::V bbest[A::kGroup];
+  int bidx[A::kGroup];
+};
+
 // Best window of NG widths (from w0) over starts 0..own-1 of the scanned chunk,
 // folded into the running best (best, idx) in shared memory; the chunk's first
 // sample is at `at` of the CTA's, values are scaled by `scale`.
 template <class A, int NG>
 __device__ __forceinline__ void snr_window_group(const typename A::T* s, int own, int len,
                                                  const SnrCfg& cfg, int w0, int at, double scale,
-                                                 double* best, int* idx) {
+                                                 double* best, int* idx, SnrBest<A>& sh) {
   typedef typename A::V V;
-  __shared__ V wbest[kSnrWarps][NG];
-  __shared__ V bbest[NG];
-  __shared__ int bidx[NG];
+  static_assert(NG <= A::kGroup, "widths of a group");
+  auto& wbest = sh.wbest;
+  auto& bbest = sh.bbest;
+  auto& bidx = sh.bidx;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   V m[NG];
   const typename A::T* sw[NG];
@@ -443,19 +458,23 @@ __device__ __forceinline__ void snr_window_group(const typename A::T* s, int own
   __syncthreads();
 }
 
-// All widths, ten at a time.
+// All widths, kGroup at a time.
 template <class A>
 __device__ __forceinline__ void snr_windows(const typename A::T* s, int own, int len, const SnrCfg& cfg,
                                             int at, double scale, double* best, int* idx) {
+  __shared__ SnrBest<A> sh;
   int w0 = 0;
-  for (; w0 + 10 <= cfg.nw; w0 += 10) snr_window_group<A, 10>(s, own, len, cfg, w0, at, scale, best, idx);
+  for (; w0 + A::kGroup <= cfg.nw; w0 += A::kGroup)
+    snr_window_group<A, A::kGroup>(s, own, len, cfg, w0, at, scale, best, idx, sh);
   switch (cfg.nw - w0) {
-#define SPP_SNR_CASE(NG)                                                      \
-  case NG:                                                                    \
-    snr_window_group<A, NG>(s, own, len, cfg, w0, at, scale, best, idx);      \
+#define SPP_SNR_CASE(NG)                                                         \
+  case NG:                                                                       \
+    if constexpr (NG < A::kGroup)                                                \
+      snr_window_group<A, NG>(s, own, len, cfg, w0, at, scale, best, idx, sh);   \
     break;
     SPP_SNR_CASE(1) SPP_SNR_CASE(2) SPP_SNR_CASE(3) SPP_SNR_CASE(4) SPP_SNR_CASE(5)
-    SPP_SNR_CASE(6) SPP_SNR_CASE(7) SPP_SNR_CASE(8) SPP_SNR_CASE(9)
+    SPP_SNR_CASE(6) SPP_SNR_CASE(7) SPP_SNR_CASE(8) SPP_SNR_CASE(9) SPP_SNR_CASE(10)
+    SPP_SNR_CASE(11)
 #undef SPP_SNR_CASE
     default: break;
   }
@@ -1239,11 +1258,15 @@ int spp_subband(const void* in, int nbits, int bitorder, int64_t nchans, int64_t
 }  // extern "C"
 
 // Samples per CTA of the chunk pass: the largest of 6144, 3072 and 1536 that
-// still gives eight CTAs per SM, so that few rows fill the chip too (one int32
+// still gives three CTAs per two SMs, so that few rows fill the chip too (one int32
 // series of 20001, factors 1/2/4: 38.6 -> 24.3 us with the warp-wide final pass).
+// Shorter chunks than that spend more on halos, barriers and the search of each
+// width's first best than they gain (32 float32 rows x 100003, 9 widths / 24
+// widths: 37 / 61 us in chunks of 6144, 58 / 110 us in chunks of 1536).
+constexpr int64_t kSnrFill = 148 * 3 / 2;
 static int snr_chunk(int64_t nrf, int64_t n) {
   for (int c = kSnrChunk; c > 1536; c /= 2)
-    if (nrf * ceil_div(n, c) >= 148 * 8) return c;
+    if (nrf * ceil_div(n, c) >= kSnrFill) return c;
   return 1536;
 }
 
@@ -1256,7 +1279,7 @@ int64_t snr_ws(int64_t nrows, int64_t n, int nfactors, int nwidths, int64_t* nch
   n = std::max<int64_t>(n, 1);
   *nchunks = ceil_div(n, snr_chunk(nrf, n));
   const int64_t most = std::max(nrf * ceil_div(n, kSnrChunk),
-                                std::min<int64_t>(nrf * ceil_div(n, 1536), 2 * 148 * 8));
+                                std::min<int64_t>(nrf * ceil_div(n, 1536), 2 * kSnrFill));
   return kStatusBytes + round_up(most * nwidths * (int64_t)sizeof(SnrPart), 256) +
          round_up(most * 3 * (int64_t)sizeof(double), 256);
 }
@@ -1311,7 +1334,7 @@ static int boxcar_snr_impl(const void* in, int in_kind, int64_t nrows, int64_t n
       ws + kStatusBytes + round_up(nrows * nfactors * nwidths * nck * (int64_t)sizeof(SnrPart), 256));
   // chunks shorter than two halos would mostly load halo
   cfg.chunk = snr_chunk(nrows * nfactors, n);
-  if (cfg.chunk < 2 * cfg.wmax) cfg.chunk = kSnrChunk;
+  while (cfg.chunk < kSnrChunk && cfg.chunk < 2 * cfg.wmax) cfg.chunk *= 2;
   const bool ints = in_kind == SPP_OUT_I32;
   // float64 pieces of at least 512 starts fit beside the halo; whole runs of the
   // scan in registers

@@ -70,3 +70,14 @@ def test_prefix_sums_wrap(orc, sign):
     rng = np.random.default_rng(22)
     x = (sign * rng.integers((1 << 22) - 900, 1 << 22, size=(2, 13000))).astype(np.int32)
     _check(orc, x, [1, 3, 100, 256], [1, 2])
+
+
+@pytest.mark.parametrize("rows", [111, 110, 74, 73])
+@pytest.mark.parametrize("wmax", [256, 1024])
+def test_chunk_rule(orc, rows, wmax):
+    """222 chunks of 6144 samples, fewer (3072), 222 of 3072, fewer (1536; 3072 with
+    halos of 1024); a last chunk of one sample."""
+    rng = np.random.default_rng(rows)
+    x = rng.integers(-2000, 2000, size=(rows, 6145), endpoint=True).astype(np.int32)
+    _check(orc, x, [1, 5, wmax], [1])
+    _check(orc, x.astype(np.float32), [1, 5, wmax], [1])

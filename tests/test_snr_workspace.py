@@ -22,6 +22,19 @@ def test_scratch_monotone(robust):
         assert size(200, n, 1, 9) <= size(200, n, 2, 9) and size(200, n, 1, 8) <= size(200, n, 1, 9)
 
 
+def test_few_rows_keep_long_chunks():
+    """544 chunks of 6144 samples fill the chip: 32 rows of 100003 samples are not cut
+    shorter, which took up to 1.8 times as long."""
+    from sigpyproc3_b200 import _lib
+
+    def up(v):
+        return -(-v // 256) * 256
+
+    chunks = 32 * 17
+    assert _lib.load().spp_boxcar_snr_workspace_bytes(32, 100003, 1, 9) == \
+        256 + up(chunks * 9 * 16) + up(chunks * 3 * 8)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("robust,rows,n,most_rows,most_n", [(False, 200, 30720, 200, 36864),
                                                            (False, 100, 20000, 1300, 20000),
