@@ -755,39 +755,16 @@ static PlanWords plan_words(int nbits, int64_t nchans, int64_t ndm) {
   return {work, room, room + (bytes <= 64ll << 20 ? bytes / 4 : 0)};
 }
 
-// Interleaved bit-plane shapes this table and sample width can use.  `words`:
-// plan-owned device words after the delay table.
-static int add_ilv_candidates(spp_dmt_plan* p, const IlvScan& scan, int32_t* words) {
+// Interleaved bit-plane shapes that channel count and sample width allow.
+static std::vector<int> ilv_shapes(int nbits, int64_t nchans) {
   const auto& cfgs = ilv_cfgs();
-  p->ilv_tabs.resize(cfgs.size());
-  const IlvDelays d = ilv_delays(p);
-  const int64_t max_rows = kPairRowsPerChan * p->nchans;
-  IlvArena ar{words + 2 * p->nchans + 2 * max_rows + 64, words};
   std::vector<int> which;
   for (int i = 0; i < (int)cfgs.size(); ++i) {
     const IlvCfg& c = cfgs[i];
-    if (c.nb != p->nbits || p->nchans % c.G) continue;
-    if (p->nchans * ((1ll << c.nb) - 1) >= (1ll << c.levels)) continue;
-    for (int G = 1; G <= c.G; ++G) {
-      IlvRows& r = p->ilv_rows[G - 1];
-      if (r.G != 0) continue;
-      const int rc = ilv_make_rows(d, scan, G, max_rows, &ar, &r);
-      r.G = G;
-      if (rc == SPP_ERR_UNSUPPORTED) continue;  // no rows: shapes of this grouping are skipped
-      if (rc) return rc;
-    }
-    if (p->ilv_rows[0].nrows == 0 || p->ilv_rows[c.G - 1].nrows == 0) continue;
-    which.push_back(i);
+    if (c.nb == nbits && nchans % c.G == 0 && nchans * ((1ll << c.nb) - 1) < (1ll << c.levels))
+      which.push_back(i);
   }
-  if (which.empty()) return SPP_OK;
-  const int rc = ilv_size_tables(which, d, p->ilv_rows, &ar, &p->ilv_tabs);
-  if (rc) return rc;
-  for (int i : which) {
-    if (p->ilv_tabs[i].stages == 0) continue;
-    p->cands.push_back(kIlvCode + i);
-    p->spans.push_back(0);
-  }
-  return SPP_OK;
+  return which;
 }
 
 // Byte lanes, four trials x two warps: the packed shape with the shortest walk
@@ -922,6 +899,39 @@ static int first_choice(spp_dmt_plan* p) {
   return pick;
 }
 
+// Range of a host table and the widest spread of a channel over tiles of two, four
+// and eight trials, in one sweep (float32 plan of 1024 trials x 4096 channels: 7.1
+// ms with a sweep per tile height and one for the range, 4.2 ms).
+static void table_range(const int32_t* d, int64_t ndm, int64_t nchans, int32_t* dmin, int32_t* dmax,
+                        int32_t (&span)[3]) {
+  int32_t mn = INT32_MAX, mx = INT32_MIN, s2 = 0, s4 = 0, s8 = 0;
+  for (int64_t t = 0; t < ndm; t += 8) {
+    const int32_t* row[8];
+    for (int i = 0; i < 8; ++i) row[i] = d + std::min(t + i, ndm - 1) * nchans;
+    for (int64_t c = 0; c < nchans; ++c) {
+      int32_t lo[4], hi[4];
+      for (int i = 0; i < 4; ++i) {
+        const int32_t x = row[2 * i][c], y = row[2 * i + 1][c];
+        lo[i] = std::min(x, y);
+        hi[i] = std::max(x, y);
+        s2 = std::max(s2, hi[i] - lo[i]);
+      }
+      const int32_t la = std::min(lo[0], lo[1]), ha = std::max(hi[0], hi[1]);
+      const int32_t lb = std::min(lo[2], lo[3]), hb = std::max(hi[2], hi[3]);
+      const int32_t l8 = std::min(la, lb), h8 = std::max(ha, hb);
+      s4 = std::max(s4, std::max(ha - la, hb - lb));
+      s8 = std::max(s8, h8 - l8);
+      mn = std::min(mn, l8);
+      mx = std::max(mx, h8);
+    }
+  }
+  *dmin = mn;
+  *dmax = mx;
+  span[0] = s2;
+  span[1] = s4;
+  span[2] = s8;
+}
+
 extern "C" {
 
 int spp_dmt_plan_create(spp_dmt_plan** plan, int nbits, int bitorder, int64_t nchans,
@@ -953,7 +963,13 @@ int spp_dmt_plan_create(spp_dmt_plan** plan, int nbits, int bitorder, int64_t nc
     p->dmax = sign > 0 ? omax : -omin;
     p->maxabs = (int32_t)std::max<int64_t>(std::llabs(omin), std::llabs(omax));
   };
-  if (!ilv || mode == SPP_MODE_ROLL) {
+  std::vector<std::pair<int, int32_t>> span_of_dw;  // widest spread of a channel over tiles of so many trials
+  if (nbits == 32 && ndm > 1) {
+    int32_t omin, omax, span[3];
+    table_range(delays_host, ndm, nchans, &omin, &omax, span);
+    set_range(sign > 0 ? omin : -omax, sign > 0 ? omax : -omin);
+    span_of_dw = {{2, span[0]}, {4, span[1]}, {8, span[2]}};
+  } else if (!ilv || mode == SPP_MODE_ROLL) {
     int32_t dmin = INT32_MAX, dmax = INT32_MIN;
     for (int64_t i = 0; i < ndm * nchans; ++i) {
       dmin = std::min(dmin, delays_host[i]);
@@ -974,26 +990,20 @@ int spp_dmt_plan_create(spp_dmt_plan** plan, int nbits, int bitorder, int64_t nc
   p->room = p->d_delays + words.room;
   p->room_bytes = 4 * (words.total - words.room);
   // Ranges and the spreads of trial tiles, of four and eight trials for all packed
-  // integer shapes: found on the device beside the interleaved rows' ranges (the
-  // host took 0.14 ms per tile height and as much for the range over 512 trials x
-  // 1024 channels).
-  IlvScan scan;
+  // integer shapes: found on the device beside the interleaved rows (the host took
+  // 0.14 ms per tile height and as much for the range over 512 trials x 1024
+  // channels).
+  IlvRange range{};
+  const std::vector<int> shapes = ilv ? ilv_shapes(nbits, nchans) : std::vector<int>();
   if (rc == SPP_OK && ilv) {
-    IlvArena ar{nullptr, p->d_delays + words.work};
-    rc = ilv_scan(ilv_delays(p), &ar, &scan);
-    if (rc == SPP_OK) {
-      int32_t omin = INT32_MAX, omax = INT32_MIN;
-      for (const int2& r : scan.range[0]) {
-        omin = std::min(omin, r.x);
-        omax = std::max(omax, r.y);
-      }
-      set_range(omin, omax);
-    }
+    p->ilv_tabs.resize(ilv_cfgs().size());
+    rc = ilv_find(shapes, ilv_delays(p), kPairRowsPerChan * nchans, p->d_delays + words.work, &range,
+                  p->ilv_rows, &p->ilv_tabs);
+    set_range(range.omin, range.omax);
   }
   // candidates; the delay spread of DM tiles is computed once per tile height
   const auto& vs = variants();
-  std::vector<std::pair<int, int32_t>> span_of_dw;
-  if (ilv) span_of_dw = {{4, scan.span4}, {8, scan.span8}};
+  if (ilv) span_of_dw = {{4, range.span4}, {8, range.span8}};
   auto tile_span = [&](int dw) -> int32_t {
     for (auto& e : span_of_dw)
       if (e.first == dw) return e.second;
@@ -1026,7 +1036,11 @@ int spp_dmt_plan_create(spp_dmt_plan** plan, int nbits, int bitorder, int64_t nc
     p->cands.push_back(i);
     p->spans.push_back(span);
   }
-  if (rc == SPP_OK && ilv) rc = add_ilv_candidates(p, scan, p->d_delays + words.work);
+  for (int i : shapes) {
+    if (p->ilv_tabs.empty() || p->ilv_tabs[i].stages == 0) continue;
+    p->cands.push_back(kIlvCode + i);
+    p->spans.push_back(0);
+  }
   if (rc == SPP_OK && p->cands.empty())
     rc = fail(SPP_ERR_UNSUPPORTED, "no kernel variant fits this delay table");
   if (rc == SPP_OK) {

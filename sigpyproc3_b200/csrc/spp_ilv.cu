@@ -727,18 +727,155 @@ __device__ __forceinline__ int ilv_row_of(const IlvDelays& d, int G, const int32
   return rbase[g] + (d.sign * row[2 * g + 1] - *o) - rlo[g];
 }
 
-__global__ void k_ilv_row_init(int64_t n, int32_t* __restrict__ mn, int32_t* __restrict__ mx) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    mn[i] = INT_MAX;
-    mx[i] = INT_MIN;
+// What plan creation reads back, in one copy.
+constexpr int kIlvMaxShapes = 8;
+struct IlvFoundRows {
+  long long nrows, ext_total, max_ext, max_group;
+  int max_offsets, ok;
+};
+struct IlvFound {
+  IlvFoundRows rows[2];
+  int omin, omax, span4, span8;
+  int stats[2 * kIlvMaxShapes];  // per shape: most entries, most stage words
+};
+
+// Sum of the values of the threads before this one (1024 threads), and of all.
+__device__ __forceinline__ long long block_before(long long v, long long* red, long long* all) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto scan = [&](long long x) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    return x;
+  };
+  const long long incl = scan(v);
+  __syncthreads();
+  if (lane == 31) red[warp] = incl;
+  __syncthreads();
+  const long long warps = scan(red[lane]);
+  *all = __shfl_sync(0xffffffffu, warps, 31);
+  const long long before = __shfl_sync(0xffffffffu, warps, warp - 1);
+  return (warp ? before : 0) + incl - v;
+}
+// Largest value of the block in *to (shared, set before), once all threads pass a barrier.
+__device__ __forceinline__ void block_largest(int v, int* to) {
+  v = __reduce_max_sync(0xffffffffu, v);
+  if ((threadIdx.x & 31) == 0) atomicMax(to, v);
+}
+
+// First word of a row of offsets mn..mx and its words beyond the common length.
+__device__ __forceinline__ int row_first(int mn) { return mn & ~7; }
+__device__ __forceinline__ long long row_extra(int mn, int mx) {
+  return ((long long)mx - row_first(mn) + 8) & ~7ll;
+}
+constexpr long long kIlvMaxExtra = 1 << 30;  // of all rows of a grouping
+
+// Words of a table's rows: where each part of a plan's words behind its delay
+// table lies.
+struct IlvWords {
+  int2 *chan, *pair, *spans;  // k_ilv_scan's ranges
+  int32_t *rmn, *rmx;         // offset ranges of pair rows
+  IlvFound* found;
+  int32_t *lo[2], *ext[2], *rbase, *rlo;
+};
+
+// One CTA of 1024 threads: channel rows, each pair's first row, and cleared ranges
+// and sizes for the kernels that follow.  A thread takes a run of channels.  Row
+// lengths are offsets' spreads plus up to 15 words: a spread above 2^30 counts as
+// that, which is too many words in any case.
+__global__ void __launch_bounds__(1024)
+k_ilv_rows(int64_t nchans, int64_t nblk, int group, int64_t max_rows, int max_offsets, IlvWords w) {
+  __shared__ long long red[32], redp[32];
+  __shared__ int top[7];  // row words beyond the common length, -offset, offset, group span, spreads, pair rows
+  const int tid = threadIdx.x;
+  if (tid < 7) top[tid] = INT_MIN;
+  __syncthreads();
+  auto cap = [](long long v) { return (int)min(v, kIlvMaxExtra + 1); };
+  const int64_t per = (nchans + 1023) / 1024;
+  const int64_t a = min(tid * per, nchans), b = min(a + per, nchans);
+  long long sum = 0;
+  int most = 0, mn = INT_MAX, mx = INT_MIN;
+  for (int64_t c = a; c < b; ++c) {
+    const int2 r = w.chan[c];
+    const long long x = row_extra(r.x, r.y);
+    sum += x;
+    most = max(most, cap(x));
+    mn = min(mn, r.x);
+    mx = max(mx, r.y);
   }
+  long long total, run = block_before(sum, red, &total);
+  for (int64_t c = a; c < b; ++c) {
+    const int2 r = w.chan[c];
+    w.lo[0][c] = row_first(r.x);
+    w.ext[0][c] = (int32_t)run;
+    run += row_extra(r.x, r.y);
+  }
+  int span = 0;  // words beside the common length that the rows of a turning CTA's channels cover
+  for (int64_t g = tid; g * group < nchans; g += 1024) {
+    long long first = LLONG_MAX, last = LLONG_MIN;
+    for (int64_t c = g * group; c < min(nchans, (g + 1) * group); ++c) {
+      const int2 r = w.chan[c];
+      first = min(first, (long long)row_first(r.x));
+      last = max(last, row_first(r.x) + row_extra(r.x, r.y));
+    }
+    span = max(span, cap(last - first));
+  }
+  int s4 = 0, s8 = 0;
+  for (int64_t i = tid; i < nblk; i += 1024) {
+    s4 = max(s4, w.spans[i].x);
+    s8 = max(s8, w.spans[i].y);
+  }
+  // pairs: a row per relative offset
+  const int64_t np = nchans % 2 ? 0 : nchans / 2;
+  const int64_t pper = (np + 1023) / 1024;
+  const int64_t pa = min(tid * pper, np), pb = min(pa + pper, np);
+  long long rows = 0;
+  int widest = 0;
+  for (int64_t k = pa; k < pb; ++k) {
+    const long long cnt = (long long)w.pair[k].y - w.pair[k].x + 1;
+    rows += cnt;
+    widest = max(widest, cap(cnt));
+  }
+  block_largest(most, top);
+  block_largest(~mn, top + 1);
+  block_largest(mx, top + 2);
+  block_largest(span, top + 3);
+  block_largest(s4, top + 4);
+  block_largest(s8, top + 5);
+  block_largest(widest, top + 6);
+  long long nrows, first = block_before(rows, redp, &nrows);  // its barriers complete `top`
+  const bool pairs = np > 0 && nrows <= max_rows && top[6] <= max_offsets;
+  if (pairs) {
+    for (int64_t k = pa; k < pb; ++k) {
+      w.rbase[k] = (int32_t)first;
+      w.rlo[k] = w.pair[k].x;
+      first += (long long)w.pair[k].y - w.pair[k].x + 1;
+    }
+    for (int64_t i = tid; i < nrows; i += 1024) {
+      w.rmn[i] = INT_MAX;
+      w.rmx[i] = INT_MIN;
+    }
+  }
+  if (tid < 2 * kIlvMaxShapes) w.found->stats[tid] = 0;
+  if (tid != 0) return;
+  w.ext[0][nchans] = (int32_t)total;
+  if (pairs) w.rbase[np] = (int32_t)nrows;
+  IlvFound* f = w.found;
+  f->rows[0] = IlvFoundRows{nchans, total, top[0], top[3], 0, total <= kIlvMaxExtra};
+  f->rows[1] = IlvFoundRows{pairs ? nrows : 0, 0, 0, 0, pairs ? top[6] : 0, pairs};
+  f->omin = ~top[1];
+  f->omax = top[2];
+  f->span4 = top[4];
+  f->span8 = top[5];
 }
 
 // Offset range of every pair row over the trials that read it.
 __global__ void k_ilv_row_ranges(IlvDelays d, const int32_t* __restrict__ rbase,
                                  const int32_t* __restrict__ rlo, int32_t* __restrict__ mn,
-                                 int32_t* __restrict__ mx) {
+                                 int32_t* __restrict__ mx, const IlvFound* __restrict__ found) {
+  if (!found->rows[1].ok) return;
   const int64_t np = d.nchans / 2;
   const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= np) return;
@@ -750,41 +887,74 @@ __global__ void k_ilv_row_ranges(IlvDelays d, const int32_t* __restrict__ rbase,
   }
 }
 
-// Staging tables: one thread per (trial tile, slab).  Without `off` only the
-// largest entry count and stage size are taken (stats[0], stats[1] in words).
+// Pair rows from their offset ranges, as k_ilv_rows makes channel rows.
+__global__ void __launch_bounds__(1024) k_ilv_pair_rows(IlvWords w) {
+  __shared__ long long red[32];
+  if (!w.found->rows[1].ok) return;
+  const int tid = threadIdx.x;
+  const int64_t n = w.found->rows[1].nrows, per = (n + 1023) / 1024;
+  const int64_t a = min(tid * per, n), b = min(a + per, n);
+  // an offset between two used ones that no trial has is never made
+  auto extra = [](int mn, int mx) { return mn > mx ? 0ll : row_extra(mn, mx); };
+  __shared__ int most;
+  if (tid == 0) most = 0;
+  long long sum = 0;
+  int top = 0;
+#pragma unroll 4
+  for (int64_t i = a; i < b; ++i) {
+    const long long x = extra(w.rmn[i], w.rmx[i]);
+    sum += x;
+    top = max(top, (int)min(x, kIlvMaxExtra + 1));
+  }
+  __syncthreads();
+  block_largest(top, &most);
+  long long total, run = block_before(sum, red, &total);  // its barriers complete `most`
+#pragma unroll 4
+  for (int64_t i = a; i < b; ++i) {
+    const int mn = w.rmn[i], mx = w.rmx[i];
+    w.lo[1][i] = mn > mx ? 1 << 30 : row_first(mn);
+    w.ext[1][i] = (int32_t)run;
+    run += extra(mn, mx);
+  }
+  if (tid != 0) return;
+  w.ext[1][n] = (int32_t)total;
+  w.found->rows[1].ext_total = total;
+  w.found->rows[1].max_ext = most;
+  w.found->rows[1].ok = total <= kIlvMaxExtra;
+}
+
+// Staging tables: a lane per group of a (trial tile, slab), whose 4 nq lanes sit in
+// one warp and place their rows by a scan over it.  A thread per slab walked its
+// groups one after the other: 15 to 37 us for the sizes of plans of any size, 17 to
+// 30 us for the tables; 8 to 10 and 7 to 14 us.  Without `off` only the largest entry count and
+// stage size are taken (stats[0], stats[1] in words).
 struct IlvTableShape {
   int G, np, DW, W, nq;
   int64_t ntile, nslab;
   const int32_t *lo, *ext, *rbase, *rlo;
 };
-__device__ __forceinline__ void ilv_table(const IlvDelays& d, const IlvTableShape& sh, int64_t id, int emax,
+__device__ __forceinline__ void ilv_table(const IlvDelays& d, const IlvTableShape& sh, int64_t thread, int emax,
                                           int32_t* __restrict__ off, int4* __restrict__ ent,
                                           int* __restrict__ stats) {
-  const int G = sh.G, np = sh.np, DW = sh.DW, W = sh.W, nq = sh.nq;
-  const int64_t nslab = sh.nslab;
-  const int32_t *lo = sh.lo, *ext = sh.ext, *rbase = sh.rbase, *rlo = sh.rlo;
-  const int64_t tile = id / nslab, k = id - tile * nslab;
-  const int64_t ng = d.nchans / G;
-  int pos = 0, e = 0, zpos = -1;
-  for (int j = 0; j < 4 * nq; ++j) {
-    const int64_t g = k * 4 * nq + j;
-    if (g >= ng) {
-      if (zpos < 0) {
-        zpos = pos;
-        if (ent && e < emax) ent[id * emax + e] = make_int4(-2, 0, W, pos);
-        ++e;
-        pos += W * np;
-      }
-      if (off) for (int i = 0; i < DW; ++i) off[(id * DW + i) * 4 * nq + j] = zpos * 4;
-      continue;
-    }
-    int o[16], rr[16];
-    uint32_t left = 0;
-    for (int i = 0; i < DW; ++i) {
-      const int64_t dm = min(tile * DW + i, d.ndm - 1);
-      rr[i] = ilv_row_of(d, G, rbase, rlo, dm, g, &o[i]);
-      left |= 1u << i;
-    }
+  const int np = sh.np, DW = sh.DW, W = sh.W, nl = 4 * sh.nq;  // 4, 8 or 16 lanes
+  const int32_t *lo = sh.lo, *ext = sh.ext;
+  const int64_t id = thread / nl;
+  if (id >= sh.ntile * sh.nslab) return;
+  const int j = (int)(thread - id * nl), lane = threadIdx.x & 31;
+  const uint32_t slab_lanes = ((1u << nl) - 1u) << (lane - j);
+  const int64_t tile = id / sh.nslab, k = id - tile * sh.nslab;
+  const int64_t ng = d.nchans / sh.G, g = k * nl + j;
+  const bool on = g < ng, pad = !on && (j == 0 || g - 1 < ng);  // the slab's one zero row
+  int o[16], rr[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    o[i] = rr[i] = 0;
+    if (on && i < DW)
+      rr[i] = ilv_row_of(d, sh.G, sh.rbase, sh.rlo, min(tile * DW + i, d.ndm - 1), g, &o[i]);
+  }
+  // rows of the group, in the order of their first trial: fn(trials, row, word, words)
+  auto each_row = [&](auto&& fn) {
+    uint32_t left = on ? (1u << DW) - 1u : 0u;
     while (left) {
       const int f = __ffs(left) - 1;
       const int r = rr[f];
@@ -798,37 +968,63 @@ __device__ __forceinline__ void ilv_table(const IlvDelays& d, const IlvTableShap
       }
       left &= ~same;
       const int start = (mn - lo[r]) & ~7;  // words from the row's first, 8-word groups
-      const int len = (W + (mx - lo[r] - start) + 7) & ~7;
-      if (ent && e < emax) ent[id * emax + e] = make_int4(r, ext[r] + start, len, pos);
-      if (off)
-        for (int i = f; i < DW; ++i)
-          if (same >> i & 1) off[(id * DW + i) * 4 * nq + j] = (pos + (o[i] - lo[r] - start) * np) * 4;
-      ++e;
-      // a spread no stage can hold: stop before the sum overflows
-      pos = min(pos, 1 << 28) + min(len, 1 << 20) * np;
+      fn(same, r, start, (W + (mx - lo[r] - start) + 7) & ~7);
+    }
+  };
+  // a spread that no stage can hold: the sum stays below overflow
+  auto words_of = [&](int len) { return min(len, 1 << 20) * np; };
+  int e = pad ? 1 : 0, pos = pad ? W * np : 0;
+  each_row([&](uint32_t, int, int, int len) {
+    ++e;
+    pos = min(pos + words_of(len), 1 << 24);
+  });
+  const int own_e = e, own_pos = pos;
+  for (int s = 1; s < nl; s <<= 1) {
+    const int xe = __shfl_up_sync(slab_lanes, e, s, nl), xp = __shfl_up_sync(slab_lanes, pos, s, nl);
+    if (j >= s) {
+      e += xe;
+      pos += xp;
     }
   }
-  if (ent)
-    for (; e < emax; ++e) ent[id * emax + e] = make_int4(-1, 0, 0, 0);
-  if (stats) {
-    atomicMax(&stats[0], e);
-    atomicMax(&stats[1], pos);
+  if (stats && j == nl - 1) {  // the values only grow: most slabs find theirs no larger
+    if (e > __ldcg(&stats[0])) atomicMax(&stats[0], e);
+    if (pos > __ldcg(&stats[1])) atomicMax(&stats[1], pos);
   }
+  if (!off) return;
+  const int all = __shfl_sync(slab_lanes, e, nl - 1, nl);
+  e -= own_e;
+  pos -= own_pos;
+  int32_t* to = off + id * DW * nl + j;
+  int4* en = ent + id * emax;
+  if (!on) {
+    const int zpos = pad ? pos : pos - W * np;
+    if (pad && e < emax) en[e] = make_int4(-2, 0, W, zpos);
+    for (int i = 0; i < DW; ++i) to[i * nl] = zpos * 4;
+  }
+  each_row([&](uint32_t same, int r, int start, int len) {
+    if (e < emax) en[e] = make_int4(r, ext[r] + start, len, pos);
+    for (int i = 0; i < DW; ++i)
+      if (same >> i & 1) to[i * nl] = (pos + (o[i] - lo[r] - start) * np) * 4;
+    ++e;
+    pos += words_of(len);
+  });
+  for (int i = all + j; i < emax; i += nl) en[i] = make_int4(-1, 0, 0, 0);
 }
-__global__ void k_ilv_tables(IlvDelays d, IlvTableShape sh, int emax, int32_t* __restrict__ off,
-                             int4* __restrict__ ent) {
-  const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (id < sh.ntile * sh.nslab) ilv_table(d, sh, id, emax, off, ent, nullptr);
+constexpr int kIlvTableThreads = 128;
+__global__ void __launch_bounds__(kIlvTableThreads)
+k_ilv_tables(IlvDelays d, IlvTableShape sh, int emax, int32_t* __restrict__ off, int4* __restrict__ ent) {
+  ilv_table(d, sh, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, emax, off, ent, nullptr);
 }
 // The sizes of several shapes at once (shape blockIdx.y).
-constexpr int kIlvMaxShapes = 8;
 struct IlvTableShapes {
   IlvTableShape s[kIlvMaxShapes];
 };
-__global__ void k_ilv_table_sizes(IlvDelays d, const __grid_constant__ IlvTableShapes sh, int* __restrict__ stats) {
+__global__ void __launch_bounds__(kIlvTableThreads)
+k_ilv_table_sizes(IlvDelays d, const __grid_constant__ IlvTableShapes sh, IlvFound* found) {
   const IlvTableShape& s = sh.s[blockIdx.y];
-  const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (id < s.ntile * s.nslab) ilv_table(d, s, id, kIlvMaxEnt, nullptr, nullptr, stats + 2 * blockIdx.y);
+  if (!found->rows[0].ok || !found->rows[s.G - 1].ok) return;
+  ilv_table(d, s, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, kIlvMaxEnt, nullptr, nullptr,
+            found->stats + 2 * blockIdx.y);
 }
 
 template <int NB, int G, int P, int DW, int TW, int NQ, int LR, int MINB>
@@ -884,11 +1080,27 @@ void ilv_free_tables(IlvTables* t) {
   t->own = false;
 }
 
-// Device words a plan keeps beside its delay table: the rows of both
-// groupings, and scratch for the range passes and table sizes.
-int64_t ilv_plan_words(int64_t nchans, int64_t max_rows) {
-  return 2 * (nchans + 1) + 2 * (max_rows + 1) + (nchans + 2) + 4 * nchans + 2 * max_rows + 64;
-}
+// Device words a plan keeps behind its delay table: scratch of the passes that
+// make its rows (ranges, sizes), and the rows of both groupings.
+struct IlvWordOffsets {
+  int64_t pair, spans, rmn, rmx, found, lo0, ext0, rbase, rlo, lo1, ext1, total;
+  IlvWordOffsets(int64_t nchans, int64_t max_rows) {
+    const int64_t np = nchans / 2;
+    pair = 2 * nchans;
+    spans = pair + 2 * np;
+    rmn = spans + 2 * ceil_div(nchans, 32);
+    rmx = rmn + max_rows;
+    found = round_up(rmx + max_rows, 2);
+    lo0 = found + (int64_t)(sizeof(IlvFound) / 4);
+    ext0 = lo0 + nchans;
+    rbase = ext0 + nchans + 1;
+    rlo = rbase + np + 1;
+    lo1 = rlo + np;
+    ext1 = lo1 + max_rows;
+    total = ext1 + max_rows + 1;
+  }
+};
+int64_t ilv_plan_words(int64_t nchans, int64_t max_rows) { return IlvWordOffsets(nchans, max_rows).total; }
 
 static IlvTableShape table_shape(const IlvCfg& c, const IlvDelays& d, const IlvRows& r) {
   return IlvTableShape{c.G, c.np, c.DW, c.words(), c.nq, ceil_div(d.ndm, c.DW),
@@ -913,133 +1125,81 @@ int64_t ilv_table_room(int nb, int64_t nchans, int64_t ndm) {
   return most;
 }
 
-int ilv_scan(const IlvDelays& d, IlvArena* ar, IlvScan* out) {
-  if (reinterpret_cast<uintptr_t>(ar->scratch) % sizeof(int2))  // ranges are stored as int2
+// Five kernels and one copy back: with the ranges on the host between them, plans
+// of few channels and trials took 70 (8-bit) to 130 us (2-bit) longer than the
+// allocation and the upload (256 channels x 64 trials: 480 us of 370 us, 441 us
+// here; 1024 x 300: 640 -> 560 us).
+int ilv_find(const std::vector<int>& which, const IlvDelays& d, int64_t max_rows, int32_t* words,
+             IlvRange* range, IlvRows* rows, std::vector<IlvTables>* tabs) {
+  if (reinterpret_cast<uintptr_t>(words) % sizeof(int2))  // ranges are stored as int2
     return fail(SPP_ERR_ARG, "interleaved rows: misaligned scratch");
-  const int64_t np = d.nchans / 2, nblk = ceil_div(d.nchans, 32);
-  int2* base = reinterpret_cast<int2*>(ar->scratch);
-  std::vector<int2> h(d.nchans + np + nblk);
-  k_ilv_scan<<<(unsigned)nblk, 256>>>(d, base, base + d.nchans, base + d.nchans + np);
-  const int rc = cuda_status(cudaMemcpy(h.data(), base, sizeof(int2) * h.size(), cudaMemcpyDeviceToHost), "offset ranges");
-  if (rc) return rc;
-  out->range[0].assign(h.begin(), h.begin() + d.nchans);
-  out->range[1].assign(h.begin() + d.nchans, h.begin() + d.nchans + np);
-  for (int64_t b = d.nchans + np; b < (int64_t)h.size(); ++b) {
-    out->span4 = std::max(out->span4, h[b].x);
-    out->span8 = std::max(out->span8, h[b].y);
-  }
-  return SPP_OK;
-}
-
-int ilv_make_rows(const IlvDelays& d, const IlvScan& scan, int G, int64_t max_rows, IlvArena* ar, IlvRows* out) {
-  const int64_t ng = d.nchans / G;
-  if (d.nchans % G || ng <= 0) return SPP_ERR_UNSUPPORTED;
-  IlvRows r{};
-  r.G = G;
-  int32_t* scratch = ar->scratch;
-  int rc = SPP_OK;
-  auto up = [&](void* dst, const void* s, int64_t words) {
-    if (!rc) rc = cuda_status(cudaMemcpy(dst, s, 4 * words, cudaMemcpyHostToDevice), "row table upload");
-  };
-  auto down = [&](void* dst, const void* s, int64_t words) {
-    if (!rc) rc = cuda_status(cudaMemcpy(dst, s, 4 * words, cudaMemcpyDeviceToHost), "row ranges");
-  };
-  const std::vector<int2>& rng = scan.range[G - 1];
-  std::vector<int32_t> mn, mx;
-  if (G == 1) {
-    r.nrows = ng;
-    mn.resize(ng); mx.resize(ng);
-    for (int64_t i = 0; i < ng; ++i) { mn[i] = rng[i].x; mx[i] = rng[i].y; }
-  } else {
-    std::vector<int32_t> head(2 * ng + 1);  // first row of each pair (and the end), smallest offset
-    int64_t n = 0;
-    for (int64_t k = 0; k < ng; ++k) {
-      head[k] = (int32_t)n;
-      head[ng + 1 + k] = rng[k].x;
-      const int64_t cnt = (int64_t)rng[k].y - rng[k].x + 1;
-      n += cnt;
-      if (n > max_rows || cnt > kPairMaxOffsets) return SPP_ERR_UNSUPPORTED;
-      r.max_offsets = std::max(r.max_offsets, (int)cnt);
-    }
-    head[ng] = (int32_t)n;
-    r.nrows = n;
-    r.d_rbase = ar->take(2 * ng + 1);
-    r.d_rlo = r.d_rbase + ng + 1;
-    up(r.d_rbase, head.data(), 2 * ng + 1);
-    if (rc) return rc;
-    k_ilv_row_init<<<(unsigned)ceil_div(n, 256), 256>>>(n, scratch, scratch + n);
-    k_ilv_row_ranges<<<dim3((unsigned)ceil_div(ng, 128), (unsigned)std::min<int64_t>(d.ndm, 64)), 128>>>(
-        d, r.d_rbase, r.d_rlo, scratch, scratch + n);
-    mn.resize(2 * n);
-    down(mn.data(), scratch, 2 * n);
-    if (rc) return rc;
-    mx.assign(mn.begin() + n, mn.end());
-  }
-  std::vector<int32_t> tab(2 * r.nrows + 1);  // first word of each row, then prefix sums of the extra words
-  int32_t* lo = tab.data();
-  int32_t* ext = tab.data() + r.nrows;
-  int64_t total = 0;
-  for (int64_t i = 0; i < r.nrows; ++i) {
-    ext[i] = (int32_t)total;
-    if (mn[i] > mx[i]) {  // an offset between two used ones that no trial has: never made
-      lo[i] = 1 << 30;
-      continue;
-    }
-    lo[i] = mn[i] & ~7;
-    const int64_t w = round_up((int64_t)mx[i] - lo[i] + 1, 8);
-    total += w;
-    r.max_ext = std::max(r.max_ext, w);
-    if (total > (1 << 30)) return SPP_ERR_UNSUPPORTED;
-  }
-  ext[r.nrows] = (int32_t)total;
-  if (G == 1) {
-    const int64_t cc = planes_ct_chans(d.nb);
-    for (int64_t c0 = 0; c0 < ng; c0 += cc) {
-      int64_t first = INT64_MAX, last = INT64_MIN;
-      for (int64_t c = c0; c < std::min(ng, c0 + cc); ++c) {
-        first = std::min<int64_t>(first, lo[c]);
-        last = std::max<int64_t>(last, (int64_t)lo[c] + ext[c + 1] - ext[c]);
-      }
-      r.max_group = std::max(r.max_group, last - first);
-    }
-  }
-  r.ext_total = total;
-  r.d_lo = ar->take(2 * r.nrows + 1);
-  r.d_ext = r.d_lo + r.nrows;
-  up(r.d_lo, tab.data(), 2 * r.nrows + 1);
-  if (rc) return rc;
-  *out = r;
-  return SPP_OK;
-}
-
-int ilv_size_tables(const std::vector<int>& which, const IlvDelays& d, const IlvRows* rows,
-                    IlvArena* ar, std::vector<IlvTables>* tabs) {
   const int n = (int)which.size();
   if (n > kIlvMaxShapes) return fail(SPP_ERR_ARG, "more than %d interleaved shapes", kIlvMaxShapes);
-  std::vector<int> st(2 * n, 0);
+  const int64_t np = d.nchans / 2, nblk = ceil_div(d.nchans, 32);
+  const IlvWordOffsets at(d.nchans, max_rows);
+  IlvWords w{};
+  w.chan = reinterpret_cast<int2*>(words);
+  w.pair = reinterpret_cast<int2*>(words + at.pair);
+  w.spans = reinterpret_cast<int2*>(words + at.spans);
+  w.rmn = words + at.rmn;
+  w.rmx = words + at.rmx;
+  w.found = reinterpret_cast<IlvFound*>(words + at.found);
+  w.lo[0] = words + at.lo0;
+  w.ext[0] = words + at.ext0;
+  w.rbase = words + at.rbase;
+  w.rlo = words + at.rlo;
+  w.lo[1] = words + at.lo1;
+  w.ext[1] = words + at.ext1;
+  for (int g = 0; g < 2; ++g) {
+    rows[g].G = g + 1;
+    rows[g].d_lo = w.lo[g];
+    rows[g].d_ext = w.ext[g];
+  }
+  rows[1].d_rbase = w.rbase;
+  rows[1].d_rlo = w.rlo;
+  k_ilv_scan<<<(unsigned)nblk, 256>>>(d, w.chan, w.pair, w.spans);
+  k_ilv_rows<<<1, 1024>>>(d.nchans, nblk, planes_ct_chans(d.nb), max_rows, kPairMaxOffsets, w);
+  bool pairs = false;
   IlvTableShapes sh{};
   int64_t most = 1;
   for (int i = 0; i < n; ++i) {
     const IlvCfg& c = ilv_cfgs()[which[i]];
+    pairs = pairs || c.G == 2;
     sh.s[i] = table_shape(c, d, rows[c.G - 1]);
-    most = std::max(most, sh.s[i].ntile * sh.s[i].nslab);
+    most = std::max(most, sh.s[i].ntile * sh.s[i].nslab * 4 * c.nq);
   }
-  int rc = cuda_status(cudaMemsetAsync(ar->scratch, 0, sizeof(int) * 2 * n), "stats clear");
+  if (pairs) {
+    k_ilv_row_ranges<<<dim3((unsigned)ceil_div(np, 128), (unsigned)std::min<int64_t>(d.ndm, 64)), 128>>>(
+        d, w.rbase, w.rlo, w.rmn, w.rmx, w.found);
+    k_ilv_pair_rows<<<1, 1024>>>(w);
+  }
+  if (n > 0)
+    k_ilv_table_sizes<<<dim3((unsigned)ceil_div(most, kIlvTableThreads), (unsigned)n), kIlvTableThreads>>>(d, sh, w.found);
+  int rc = cuda_status(cudaGetLastError(), "row tables launch");
+  IlvFound f{};
+  if (!rc) rc = cuda_status(cudaMemcpy(&f, w.found, sizeof f, cudaMemcpyDeviceToHost), "row tables");
   if (rc) return rc;
-  k_ilv_table_sizes<<<dim3((unsigned)ceil_div(most, 64), (unsigned)n), 64>>>(d, sh, ar->scratch);
-  rc = cuda_status(cudaMemcpy(st.data(), ar->scratch, sizeof(int) * 2 * n, cudaMemcpyDeviceToHost), "table sizes");
-  if (rc) return rc;
+  *range = IlvRange{f.omin, f.omax, f.span4, f.span8};
+  for (int g = 0; g < (pairs ? 2 : 1); ++g) {
+    if (!f.rows[g].ok) continue;  // no rows: shapes of this grouping are not offered
+    rows[g].nrows = f.rows[g].nrows;
+    rows[g].ext_total = f.rows[g].ext_total;
+    rows[g].max_ext = f.rows[g].max_ext;
+    rows[g].max_group = f.rows[g].max_group;
+    rows[g].max_offsets = f.rows[g].max_offsets;
+  }
   for (int i = 0; i < n; ++i) {
     const IlvCfg& c = ilv_cfgs()[which[i]];
     IlvTables& t = (*tabs)[which[i]];
     t.stages = 0;  // does not fit
-    if (st[2 * i] > kIlvMaxEnt || st[2 * i + 1] >= 1 << 18) continue;
-    const int64_t stage = round_up((int64_t)st[2 * i + 1] * 4, 256);
+    if (rows[0].nrows == 0 || rows[c.G - 1].nrows == 0) continue;
+    if (f.stats[2 * i] > kIlvMaxEnt || f.stats[2 * i + 1] >= 1 << 18) continue;
+    const int64_t stage = round_up((int64_t)f.stats[2 * i + 1] * 4, 256);
     const int64_t per = stage + (int64_t)c.DW * 4 * c.nq * 4 + 16;
     const int64_t avail = kIlvMaxSmem - c.hi_bytes - 16;
     const int64_t stages = std::min<int64_t>(4, avail / per);
     if (stages < 2) continue;
-    t.emax = st[2 * i];
+    t.emax = f.stats[2 * i];
     t.stage_bytes = stage;
     t.stages = (int)stages;
     t.smem = stages * per + c.hi_bytes + 16;
@@ -1062,7 +1222,8 @@ int ilv_build_tables(const IlvCfg& c, const IlvDelays& d, const IlvRows& r, void
   t->d_off = static_cast<int32_t*>(p);
   t->d_ent = reinterpret_cast<int4*>(static_cast<uint8_t*>(p) + table_off_bytes(c, d.nchans, d.ndm));
   const IlvTableShape sh = table_shape(c, d, r);
-  k_ilv_tables<<<(unsigned)ceil_div(sh.ntile * sh.nslab, 64), 64>>>(d, sh, t->emax, t->d_off, t->d_ent);
+  k_ilv_tables<<<(unsigned)ceil_div(sh.ntile * sh.nslab * 4 * c.nq, kIlvTableThreads), kIlvTableThreads>>>(
+      d, sh, t->emax, t->d_off, t->d_ent);
   rc = cuda_status(cudaGetLastError(), "staging tables");
   if (!rc) rc = cuda_status(cudaStreamSynchronize(nullptr), "staging tables");
   if (rc) ilv_free_tables(t);

@@ -61,36 +61,23 @@ struct IlvDelays {
   int nb;  // sample width, bits
 };
 
-// Plan-owned device words (beside the delay table): rows are taken from it,
-// `scratch` serves the passes that make them.
-struct IlvArena {
-  int32_t* next = nullptr;
-  int32_t* scratch = nullptr;
-  int32_t* take(int64_t words) {
-    int32_t* p = next;
-    next += words;
-    return p;
-  }
-};
+// Device words that ilv_find needs for at most `max_rows` pair rows.
 int64_t ilv_plan_words(int64_t nchans, int64_t max_rows);
 // Bytes that the tables of any shape of this width may take.
 int64_t ilv_table_room(int nb, int64_t nchans, int64_t ndm);
 
-// What one pass over a delay table finds.
-struct IlvScan {
-  std::vector<int2> range[2];        // per channel, per pair: smallest and largest (relative) offset
-  int32_t span4 = 0, span8 = 0;      // widest spread over tiles of four, of eight trials
-};
-int ilv_scan(const IlvDelays& d, IlvArena* ar, IlvScan* out);
-
 void ilv_free_tables(IlvTables* t);
-// Rows of grouping G (1 or 2); more than `max_rows` pair rows:
-// SPP_ERR_UNSUPPORTED.
-int ilv_make_rows(const IlvDelays& d, const IlvScan& scan, int G, int64_t max_rows, IlvArena* ar, IlvRows* out);
-// Sizes the staging of the shapes `which` (stages = 0: the table's spreads do
-// not fit) from the rows of G = 1 and 2.
-int ilv_size_tables(const std::vector<int>& which, const IlvDelays& d, const IlvRows* rows,
-                    IlvArena* ar, std::vector<IlvTables>* tabs);
+// Range of a table's offsets, and the widest spread over tiles of four and of
+// eight trials.
+struct IlvRange {
+  int32_t omin, omax, span4, span8;
+};
+// One pass over a delay table: its range, the rows of both groupings (nrows = 0:
+// none, as more than `max_rows` pair rows) and the staging sizes of the shapes
+// `which` (stages = 0: the spreads do not fit).  `words`: device words that the
+// rows live in, on an 8-byte boundary.
+int ilv_find(const std::vector<int>& which, const IlvDelays& d, int64_t max_rows, int32_t* words,
+             IlvRange* range, IlvRows* rows, std::vector<IlvTables>* tabs);
 // Builds them in `room` where it is large enough, else in memory of their own.
 int ilv_build_tables(const IlvCfg& c, const IlvDelays& d, const IlvRows& r, void* room, int64_t room_bytes,
                      IlvTables* t);
