@@ -159,3 +159,49 @@ def test_short_blocks_of_a_long_plan(orc, nbits, nchans):
         with pytest.raises(ValueError):
             plan.execute(raw, nsamps, out, out_start=1, ws=small)
     plan.close()
+
+
+def _shapes(nbits, d, nchans, nsamps, mode="dedisperse"):
+    """Whether channel and channel-pair rows are offered: interleaved tiles are of 3, 7,
+    9, 11 or 15 trials, the others' of 1, 4 or 8."""
+    from sigpyproc3_b200.dedisp import DMTPlan
+
+    plan = DMTPlan(d, nchans, nsamps, nbits=nbits, mode=mode, bitorder="little" if nbits == 1 else "big")
+    kinds = set()
+    for v in range(plan.num_variants):
+        plan.set_variant(v)
+        if plan.describe()["DW"] not in (1, 4, 8):
+            kinds.add(plan.describe()["paired"])
+    plan.close()
+    return kinds
+
+
+@pytest.mark.parametrize("nbits,nchans,dm,ndm,nvalid,mode,ref", [
+    (1, 64, 12.0, 16, 7941, "dedisperse", "fch1"), (2, 64, 12.0, 2, 1, "dedisperse", "fch1"),
+    (4, 64, 12.0, 15, 8192, "dedisperse", "fch1"), (8, 64, 12.0, 19, 8449, "dedisperse", "fch1"),
+    (1, 8, 15.0, 12, 3000, "dedisperse", "fch1"), (2, 36, 15.0, 12, 3000, "dedisperse", "fch1"),
+    (4, 38, 15.0, 12, 3000, "dedisperse", "fch1"), (8, 7, 15.0, 12, 3000, "dedisperse", "fch1"),
+    (8, 34, 15.0, 12, 3000, "dedisperse", "fch1"), (1, 16, 800.0, 400, 300, "dedisperse", "fch1"),
+    (2, 16, 800.0, 400, 300, "dedisperse", "fch1"), (4, 16, 800.0, 400, 300, "dedisperse", "fch1"),
+    (8, 16, 800.0, 400, 300, "dedisperse", "fch1"), (2, 40, 25.0, 13, 4096, "roll", "fch1"),
+    (8, 40, 25.0, 13, 4096, "roll", "fch1"), (2, 40, 25.0, 13, 4500, "dedisperse", "fcenter"),
+    (8, 40, 25.0, 13, 4500, "dedisperse", "fcenter")])
+def test_tables_are_offered(nbits, nchans, dm, ndm, nvalid, mode, ref):
+    """The tables above reach the interleaved kernels, those of 64 channels (few distinct
+    offsets within a pair) the pairs' too."""
+    d = _delays(nchans, dm, ndm, ref=ref)
+    nsamps = nvalid + (0 if mode == "roll" else int(np.abs(d).max()))
+    kinds = _shapes(nbits, d, nchans, nsamps, mode)
+    assert 0 in kinds
+    if nchans == 64:
+        assert (1 in kinds) == (nbits > 1)
+
+
+@pytest.mark.parametrize("nbits,nchans,mode", [(2, 36, "dedisperse"), (2, 68, "roll"), (4, 38, "dedisperse"),
+                                               (8, 34, "roll"), (8, 66, "dedisperse")])
+def test_partial_slabs_of_pairs(orc, nbits, nchans, mode):
+    """Pairs that do not fill the last slab read the zero row of pair planes."""
+    d = _delays(nchans, 2.0, 25)
+    nsamps = 3000 + int(d.max())
+    assert _shapes(nbits, d, nchans, nsamps, mode) == {0, 1}
+    assert _run(orc, nbits, d, nchans, nsamps, mode=mode, seed=nchans) >= 4
