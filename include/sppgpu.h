@@ -226,7 +226,11 @@ int spp_dedisperse_noalloc_status_read(uint32_t* host_out, void* stream);
  *   SPP_MODE_ROLL:       out[i][t] = sum_c x[(t - D[i][c]) mod nsamps][c], t < nsamps
  * writing rows of `out` with row stride `out_stride` elements starting at
  * column `out_start`.  delays_host is a host int32 array (ndm x nchans,
- * row-major), read once at plan creation. */
+ * row-major), read once at plan creation.  Beside the workspace a plan holds device
+ * memory of its own: the table, the words spp_dmt_plan_layout reports, and staging
+ * tables of about 0.4 KB per 15 trials and 4 channels (1- to 8-bit data, more than
+ * one trial) for the shape it starts from and each that spp_dmt_plan_set_variant
+ * chooses; where those find no memory at creation, it starts from a shape without. */
 typedef struct spp_dmt_plan spp_dmt_plan;
 int spp_dmt_plan_create(spp_dmt_plan** plan, int nbits, int bitorder,
                         int64_t nchans, int64_t nsamps_max, int64_t ndm,

@@ -825,8 +825,9 @@ static double interleaved_us(const spp_dmt_plan* p, const IlvCfg& c, int64_t nsa
 // at nsamps_max, over the interleaved shapes, the first packed one and the one of
 // the shortest walk.  Over 190 measured plans (64-4096 channels, 2-1024 trials,
 // 50-100000 outputs) the choice is within 15 % of the fastest shape for all but
-// 12, and within 45 % for those.  Rows above kIlvDefaultBytes leave a shape to
-// explicit choice: they grow with the block and the delay range.
+// 12, and within 45 % for those.  Rows and staging tables above kIlvDefaultBytes
+// leave a shape to explicit choice: they grow with the block and the delay range,
+// and with the trials.
 // 2-bit grids so fine that a pair row serves 100 trials or more start from pairs
 // from 4096 outputs on (a pair shape's shortest tile), so that the blocks of one
 // observation run one kernel (4096 channels, 1024 trials to DM 2000: 45.9 ms
@@ -884,7 +885,8 @@ static int first_choice(spp_dmt_plan* p) {
     } else {
       const IlvCfg& c = ilv_cfgs()[iv];
       const IlvGeom g = ilv_geometry(c, p->ilv_rows[0], p->ilv_rows[c.G - 1], p->nchans, nvalid);
-      if (g.chan_bytes + g.row_bytes > kIlvDefaultBytes && any) continue;
+      const int64_t own = ilv_table_bytes(c, ilv_delays(p), p->ilv_tabs[iv]);
+      if (g.chan_bytes + g.row_bytes + own > kIlvDefaultBytes && any) continue;
       t = interleaved_us(p, c, p->nsamps_max, g);
       pairs = c.G == 2;
     }
@@ -982,8 +984,13 @@ int spp_dmt_plan_create(spp_dmt_plan** plan, int nbits, int bitorder, int64_t nc
     return fail(SPP_ERR_DELAY, "roll mode needs |delay| < nsamps");
   }
   p->dpitch = nchans;
-  const PlanWords words = plan_words(nbits, nchans, ndm);
+  PlanWords words = plan_words(nbits, nchans, ndm);
   cudaError_t e = cudaMalloc(&p->d_delays, sizeof(int32_t) * words.total);
+  if (e == cudaErrorMemoryAllocation && words.room < words.total) {  // the rest may still fit
+    cudaGetLastError();
+    words.total = words.room;
+    e = cudaMalloc(&p->d_delays, sizeof(int32_t) * words.total);
+  }
   if (e != cudaSuccess) { delete p; return cuda_status(e, "plan cudaMalloc"); }
   e = cudaMemcpy(p->d_delays, delays_host, sizeof(int32_t) * ndm * nchans, cudaMemcpyHostToDevice);
   int rc = cuda_status(e, "plan upload");
@@ -1046,6 +1053,12 @@ int spp_dmt_plan_create(spp_dmt_plan** plan, int nbits, int bitorder, int64_t nc
   if (rc == SPP_OK) {
     p->cur = first_choice(p);
     rc = ensure_tables(p, p->cur);
+    // staging tables of a very fine grid may be larger than what is left of the
+    // device memory; the packed shapes need none
+    if (rc != SPP_OK && p->ilv_tabs[ilv_index(p, p->cur)].no_memory && p->packed[0] >= 0) {
+      p->cur = p->packed[0];
+      rc = SPP_OK;
+    }
   }
   if (rc != SPP_OK) {
     free_device(p);

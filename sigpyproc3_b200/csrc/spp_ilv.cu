@@ -1115,6 +1115,10 @@ static int64_t table_bytes(const IlvCfg& c, int64_t nchans, int64_t ndm, int ema
          ceil_div(ndm, c.DW) * ceil_div(nchans / c.G, 4 * c.nq) * emax * (int64_t)sizeof(int4);
 }
 
+int64_t ilv_table_bytes(const IlvCfg& c, const IlvDelays& d, const IlvTables& t) {
+  return table_bytes(c, d.nchans, d.ndm, t.emax);
+}
+
 // Room for the staging tables of whichever shape a plan starts from: a slab's
 // groups read a row each, pairs up to kIlvMaxEnt together.
 int64_t ilv_table_room(int nb, int64_t nchans, int64_t ndm) {
@@ -1214,7 +1218,10 @@ int ilv_build_tables(const IlvCfg& c, const IlvDelays& d, const IlvRows& r, void
   void* p = room;
   int rc = SPP_OK;
   if (bytes > room_bytes) {
-    rc = cuda_status(cudaMalloc(&p, (size_t)bytes), "plan table alloc");
+    const cudaError_t e = cudaMalloc(&p, (size_t)bytes);
+    t->no_memory = e == cudaErrorMemoryAllocation;
+    if (t->no_memory) cudaGetLastError();  // left for no later launch to report
+    rc = cuda_status(e, "plan table alloc");
     if (rc) return rc;
     t->own = true;
   }

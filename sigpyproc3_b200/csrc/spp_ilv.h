@@ -51,6 +51,7 @@ struct IlvTables {
   int4* d_ent = nullptr;     // (tile, slab, entry): row, word offset, words, stage position
   bool own = false;          // d_off is an allocation (of both), not a plan's room
   int64_t bytes = 0;         // of both
+  bool no_memory = false;    // the last attempt found no memory for them
 };
 
 // A delay table on the device.
@@ -78,6 +79,8 @@ struct IlvRange {
 // rows live in, on an 8-byte boundary.
 int ilv_find(const std::vector<int>& which, const IlvDelays& d, int64_t max_rows, int32_t* words,
              IlvRange* range, IlvRows* rows, std::vector<IlvTables>* tabs);
+// Device bytes that the tables of a sized shape take.
+int64_t ilv_table_bytes(const IlvCfg& c, const IlvDelays& d, const IlvTables& t);
 // Builds them in `room` where it is large enough, else in memory of their own.
 int ilv_build_tables(const IlvCfg& c, const IlvDelays& d, const IlvRows& r, void* room, int64_t room_bytes,
                      IlvTables* t);

@@ -55,3 +55,33 @@ def test_more_tiles_than_a_grid(nbits, nchans, tile, step):
     out = plan.execute(raw, nsamps, check=True)
     assert torch.equal(out[0], s[:nvalid]) and torch.equal(out[1], s[step:])
     plan.close()
+
+
+def test_no_memory_for_staging_tables(orc):
+    """A grid whose staging tables (some 90 MB) do not fit what the delay table (66 MB)
+    leaves of the device memory."""
+    import torch
+
+    from sigpyproc3_b200.dedisp import DMTPlan
+
+    nchans, ndm, nvalid = 2048, 8000, 4096
+    d = (np.arange(ndm)[:, None] * np.arange(nchans)[None, :] // (1 << 19)).astype(np.int32)
+    nsamps = nvalid + int(d.max())
+    rng = np.random.default_rng(8)
+    vals = rng.integers(0, 256, nsamps * nchans, dtype=np.uint8)
+    rows = np.concatenate([np.arange(0, ndm, 997), [ndm - 1]])
+    expect = orc.dmt(vals, np.ascontiguousarray(d[rows]), nchans, nsamps).astype(np.int64)
+    raw = torch.from_numpy(vals).cuda()
+    out = torch.zeros((ndm, nvalid), dtype=torch.int32, device="cuda")
+    ws = torch.zeros(256 << 20, dtype=torch.uint8, device="cuda")
+    torch.cuda.empty_cache()
+    rest = torch.empty(torch.cuda.mem_get_info()[0] - (100 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        assert torch.cuda.mem_get_info()[0] < 130 << 20
+        plan = DMTPlan(d, nchans, nsamps, nbits=8, out_dtype=torch.int32)
+    finally:
+        del rest
+        torch.cuda.empty_cache()
+    plan.execute(raw, nsamps, out, ws=ws, check=True)
+    np.testing.assert_array_equal(out.cpu().numpy()[rows].astype(np.int64), expect)
+    plan.close()
