@@ -498,8 +498,7 @@ k_dmt(const DmtArgs a) {
 #pragma unroll
           for (int r = 0; r < R; ++r) {
             const float x = row[32 * r];
-            if (ACC != SPP_ACC_F64) p_acc[r] = __fadd_rn(p_acc[r], x);
-            else if (decltype(sp)::value && (r & 1)) d_acc[r] = add_finite_f32(d_acc[r], x);
+            if (decltype(sp)::value && (r & 1)) d_acc[r] = add_finite_f32(d_acc[r], x);
             else d_acc[r] += (double)x;
           }
         };
@@ -516,8 +515,20 @@ k_dmt(const DmtArgs a) {
         }
         for (; j < nc; ++j) add_row(sd + j * a.slot_w + (wbase + dl[j]));
       };
-      if (split) add_slab(std::true_type{});
-      else add_slab(std::false_type{});
+      if constexpr (ACC != SPP_ACC_F64) {
+        // offsets one by one: by fours the 16-word shapes take 1.3 to 2 times as
+        // long (4096 channels, 64 trials, 2^17 outputs: 7.4 -> 9.3 ms)
+#pragma unroll 4
+        for (int j = 0; j < nc; ++j) {
+          const float* row = sd + j * a.slot_w + (wbase + dl[j]);
+#pragma unroll
+          for (int r = 0; r < R; ++r) p_acc[r] = __fadd_rn(p_acc[r], row[32 * r]);
+        }
+      } else if (split) {
+        add_slab(std::true_type{});
+      } else {
+        add_slab(std::false_type{});
+      }
       if (ACC != SPP_ACC_F64) {
 #pragma unroll
         for (int r = 0; r < R; ++r) {
