@@ -47,8 +47,10 @@ static const std::vector<WlVariant>& wl_variants() {
       // samples is long enough to hide the next one's claim and delay reads
       // (two words per thread, 256 samples: 2.54 ms for the first stage of two
       // beams, 32 groups x 1024 channels; 1.17 ms here, 3.48 ms bit-sliced; 512
-      // trials x 1024 channels x 63616 outputs: 2.74 against 3.26 ms).  The bit-
-      // sliced shapes take spreads beyond its shared memory.
+      // trials x 1024 channels x 63616 outputs: 2.74 against 3.26 ms; seven served
+      // beams of 256-4096 channels, 400-1942 trials 13-72 samples apart, chunks of
+      // 2^14-2^18: bit-sliced 1.14-1.54 times as long, every other shape longer
+      // too).  The bit-sliced shapes take spreads beyond its shared memory.
       mkwl<8, 8, 8, 1, 32, 2, 0>(),
       mkwlb<8, 2, 8, 1, 2, 16, 96, 2>(), mkwlb<8, 2, 8, 1, 2, 16, 0, 2>(),
       mkwlb<8, 1, 8, 1, 2, 16>(),

@@ -227,7 +227,7 @@ __global__ void k_subband(const void* __restrict__ in, int64_t nchans, int64_t n
 // moved past the windows and the index search without dependent steps: 805 us;
 // twelve to sixteen loads of a thread in flight, and the subtraction and maximum
 // of a window in one instruction: 772 us (one factor: 409 -> 366 us, of them 209
-// for loads and scan).  200 float32 rows x 300001, factors 1/2: 875 -> 795 us.
+// for loads and scan).  200 float32 rows x 300001, factors 1/2: 867 -> 694 us.
 // ---------------------------------------------------------------------------
 constexpr int kSnrChunk = 6144;     // downsampled samples per CTA, most
 constexpr int kSnrThreads = 256;
@@ -819,9 +819,10 @@ __device__ __forceinline__ void q_range(const QArgs& a, const SnrCfg& cfg, QStat
 
 // One pass: histogram of the next key bits of the values in the chosen bins,
 // then (the row's last CTA) each rank's bin.
-template <int PASS>
+template <int PASS, int BITS>
 __device__ __forceinline__ void q_pass(const QArgs& a, const SnrCfg& cfg, QState& st) {
-  extern __shared__ uint32_t qhist[];  // (PASS == 0 ? 1 : kQRanks) x kQBins
+  constexpr int kBins = 1 << BITS;
+  extern __shared__ uint32_t qhist[];  // (PASS == 0 ? 1 : kQRanks) x kBins
   __shared__ uint32_t dpre[kQRanks], pick[kQRanks], left[kQRanks];
   __shared__ bool last;
   const int f = cfg.f[blockIdx.y % cfg.nf];
@@ -829,27 +830,27 @@ __device__ __forceinline__ void q_pass(const QArgs& a, const SnrCfg& cfg, QState
   const uint32_t kmin = ~st.kmin_inv;
   const int old = PASS == 0 ? 32 - __clz(st.kmax - kmin) : (int)st.shift;  // bits still open
   if (PASS > 0 && old == 0) return;                                       // selected already
-  const int sh = old > kQBits ? old - kQBits : 0;
+  const int sh = old > BITS ? old - BITS : 0;
   const int nd = PASS == 0 ? 1 : (int)st.ndist;
   if (threadIdx.x < kQRanks) dpre[threadIdx.x] = PASS == 0 ? kmin : st.dpre[threadIdx.x];
-  for (int i = threadIdx.x; i < nd * kQBins; i += blockDim.x) qhist[i] = 0u;
+  for (int i = threadIdx.x; i < nd * kBins; i += blockDim.x) qhist[i] = 0u;
   __syncthreads();
   if (PASS == 0) {
     q_each(a, cfg, [&](uint32_t k) { atomicAdd(&qhist[(k - kmin) >> sh], 1u); });
   } else {
-    const uint32_t span = 1u << old;  // old <= 21
+    const uint32_t span = 1u << old;  // old <= 32 - BITS
     q_each(a, cfg, [&](uint32_t k) {
       for (int d = 0; d < nd; ++d) {
         const uint32_t r = k - dpre[d];
-        if (r < span) atomicAdd(&qhist[d * kQBins + (r >> sh)], 1u);
+        if (r < span) atomicAdd(&qhist[d * kBins + (r >> sh)], 1u);
       }
     });
   }
   __syncthreads();
   const uint32_t* h = qhist;
   if (gridDim.x > 1) {
-    uint32_t* gh = a.hist + ((int64_t)blockIdx.y * 3 + PASS) * kQRanks * kQBins;
-    for (int i = threadIdx.x; i < nd * kQBins; i += blockDim.x)
+    uint32_t* gh = a.hist + ((int64_t)blockIdx.y * 3 + PASS) * kQRanks * kBins;
+    for (int i = threadIdx.x; i < nd * kBins; i += blockDim.x)
       if (qhist[i]) atomicAdd(gh + i, qhist[i]);
     __threadfence();
     __syncthreads();
@@ -857,7 +858,7 @@ __device__ __forceinline__ void q_pass(const QArgs& a, const SnrCfg& cfg, QState
     __syncthreads();
     if (!last) return;
     __threadfence();
-    for (int i = threadIdx.x; i < nd * kQBins; i += blockDim.x) qhist[i] = __ldcg(gh + i);
+    for (int i = threadIdx.x; i < nd * kBins; i += blockDim.x) qhist[i] = __ldcg(gh + i);
     __syncthreads();
   }
   // one warp per rank: the bin whose cumulative count passes the rank
@@ -875,8 +876,8 @@ __device__ __forceinline__ void q_pass(const QArgs& a, const SnrCfg& cfg, QState
       r = st.left[warp];
       slot = (int)st.slot[warp];
     }
-    h = qhist + slot * kQBins;
-    constexpr int per = kQBins / 32;
+    h = qhist + slot * kBins;
+    constexpr int per = kBins / 32;
     uint32_t sum = 0;
     for (int j = 0; j < per; ++j) sum += h[lane * per + j];
     uint32_t incl = sum;
@@ -929,9 +930,15 @@ __global__ void __launch_bounds__(kQPassThreads) k_q_range(const QArgs a, const 
 }
 template <int PASS>
 __global__ void __launch_bounds__(kQPassThreads) k_q_pass(const QArgs a, const SnrCfg cfg) {
-  q_pass<PASS>(a, cfg, a.st[blockIdx.y]);
+  q_pass<PASS, kQBits>(a, cfg, a.st[blockIdx.y]);
 }
-// All passes of a row in one CTA, its state in shared memory.
+// All passes of a row in one CTA, its state in shared memory.  Short rows take 256
+// bins and, where their keys span all 32 bits, four passes: clearing and scanning
+// 2048 bins costs more than a pass over few samples (60000 float32 rows x 200, log-
+// normal: 4.62 ms with 2048 bins, 2.83 ms with 256; 1000 x 3000: 111 and 101 us;
+// one row of 5000: 22 and 25 us).
+constexpr int kQShortRow = 4096;
+template <int BITS>
 __global__ void __launch_bounds__(kQPassThreads) k_row_quantiles(const QArgs a, const SnrCfg cfg) {
   __shared__ QState st;
   for (int i = threadIdx.x; i < (int)(sizeof(QState) / 4); i += blockDim.x)
@@ -939,11 +946,15 @@ __global__ void __launch_bounds__(kQPassThreads) k_row_quantiles(const QArgs a, 
   __syncthreads();
   q_range(a, cfg, st);
   __syncthreads();
-  q_pass<0>(a, cfg, st);
+  q_pass<0, BITS>(a, cfg, st);
   __syncthreads();
-  q_pass<1>(a, cfg, st);
+  q_pass<1, BITS>(a, cfg, st);
   __syncthreads();
-  q_pass<2>(a, cfg, st);
+  q_pass<2, BITS>(a, cfg, st);
+  if constexpr (3 * BITS < 32) {
+    __syncthreads();
+    q_pass<3, BITS>(a, cfg, st);
+  }
 }
 
 // CTAs per (row, factor): enough to fill the chip, 2048 values each at least.
@@ -966,9 +977,14 @@ static int launch_quantiles(const void* in, int kind, int64_t nrf, int64_t n, in
   const int split = ws ? q_split(nrf, n) : 1;
   int rc = SPP_OK;
   if (split == 1) {
-    rc = set_smem_attr(reinterpret_cast<const void*>(k_row_quantiles), smem);
-    if (rc) return rc;
-    k_row_quantiles<<<dim3(1, (unsigned)nrf), kQPassThreads, smem, st>>>(a, cfg);
+    const dim3 grid(1, (unsigned)nrf);
+    if (n <= kQShortRow) {
+      k_row_quantiles<8><<<grid, kQPassThreads, kQRanks * 256 * 4, st>>>(a, cfg);
+    } else {
+      rc = set_smem_attr(reinterpret_cast<const void*>(k_row_quantiles<kQBits>), smem);
+      if (rc) return rc;
+      k_row_quantiles<kQBits><<<grid, kQPassThreads, smem, st>>>(a, cfg);
+    }
     return cuda_status(cudaGetLastError(), "row quantiles launch");
   }
   rc = cuda_status(cudaMemsetAsync(ws, 0, (size_t)q_workspace(nrf, n), st), "quantile state clear");
@@ -1259,7 +1275,7 @@ int spp_subband(const void* in, int nbits, int bitorder, int64_t nchans, int64_t
 
 // Samples per CTA of the chunk pass: the largest of 6144, 3072 and 1536 that
 // still gives three CTAs per two SMs, so that few rows fill the chip too (one int32
-// series of 20001, factors 1/2/4: 38.6 -> 24.3 us with the warp-wide final pass).
+// series of 20001, factors 1/2/4: 37 -> 12 us with the warp-wide final pass).
 // Shorter chunks than that spend more on halos, barriers and the search of each
 // width's first best than they gain (32 float32 rows x 100003, 9 widths / 24
 // widths: 37 / 61 us in chunks of 6144, 58 / 110 us in chunks of 1536).

@@ -119,7 +119,7 @@ class Server:
     # ---- sizing ----
     def _pick(self, st: BeamState) -> tuple[int, int]:
         """Work-list kernel for a beam: ``variant`` if given, else the first
-        variant (fixed-slot kernels come first) whose shared-memory slot holds
+        variant (they are listed fastest first) whose shared-memory slot holds
         the beam's tile span within the per-CTA limit.  Returns (variant, slot)."""
         if st.pick is None:
             lib = _lib.load()

@@ -35,3 +35,38 @@ def test_split_selection(orc, kind, rows, n):
                           loc_scale="median_iqr")
     esnr, _ = orc.boxcar_snr(x.astype(np.float32), factors, widths, "median_iqr")
     np.testing.assert_allclose(snr.cpu().numpy(), esnr, rtol=1e-5)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 31, 255, 256, 257, 4095, 4096, 4097])
+@pytest.mark.parametrize("kind", ["wide", "ties", "int"])
+def test_short_rows(n, kind):
+    """The shortest rows, and both sides of the length up to which 256 bins are taken
+    (4096): the same values as numpy's sorted row gives."""
+    import torch
+
+    from sigpyproc3_b200 import _lib
+
+    rng = np.random.default_rng(n)
+    rows = 7
+    if kind == "wide":  # every exponent, both signs, zeros
+        x = (np.exp(rng.uniform(-80, 80, (rows, n))) * rng.choice([-1, 1], (rows, n))).astype(np.float32)
+        x[:, ::5] = 0.0
+    elif kind == "ties":
+        x = rng.integers(-2, 3, (rows, n)).astype(np.float32)
+    else:
+        x = rng.integers(-(1 << 31), 1 << 31, (rows, n)).astype(np.int32)
+    dev = torch.from_numpy(x).cuda()
+    out = torch.zeros((rows, 2), dtype=torch.float64, device="cuda")
+    _lib.check(_lib.load().spp_row_loc_scale(
+        dev.data_ptr(), _lib.OUT_I32 if kind == "int" else _lib.OUT_F32, rows, n, n, 1, out.data_ptr(),
+        torch.cuda.current_stream().cuda_stream))
+    y = x.astype(np.float32)
+    loc = np.median(y, axis=1)
+    q25, q75 = np.percentile(y.astype(np.float64), [25, 75], axis=1)
+    scale = (q75 - q25) / 1.3489795003921634
+    scale = np.where(np.abs(scale) <= 1e-8, 1.0, scale)
+    got = out.cpu().numpy()
+    # the median of an even row is the float32 mean of two float32 values, either way round
+    np.testing.assert_allclose(got[:, 0], loc, rtol=2.0 ** -23, atol=0)
+    # two interpolations and a difference in float64; differences of values up to |y|
+    np.testing.assert_allclose(got[:, 1], scale, rtol=0, atol=8 * 2.0 ** -52 * (np.abs(q25) + np.abs(q75)).max() + 1e-300)
