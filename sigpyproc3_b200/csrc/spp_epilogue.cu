@@ -532,13 +532,13 @@ __device__ __forceinline__ void snr_load_int(const int32_t* __restrict__ x, int 
   for (j = own + threadIdx.x; j < len; j += kSnrThreads) get(j);
 }
 
-// KIND int32: for a power-of-two factor f, y = s / f with s the integer sum of f
+// SUMS (int32 rows): for a power-of-two factor f, y = s / f with s the integer sum of f
 // samples.  Where f * |x| <= 2^24 the float32 rounding of y is exact, and where
 // f * |x| * wmax < 2^31 window sums are exact differences of prefix sums
 // modulo 2^32; the chunk's moments come from 64-bit sums (n * sum(s^2) -
 // sum(s)^2 in 128 bits).  Other chunks and float32 rows take float64, in pieces
 // that fit the shared memory.
-template <int KIND>
+template <int KIND, bool SUMS>
 __global__ void __launch_bounds__(kSnrThreads, 4)
 k_snr_chunk(const void* __restrict__ in, int64_t n, int64_t in_stride, const SnrCfg cfg,
             int64_t nchunks, SnrPart* __restrict__ parts, double* __restrict__ stats) {
@@ -564,7 +564,7 @@ k_snr_chunk(const void* __restrict__ in, int64_t n, int64_t in_stride, const Snr
   }
   double* st = stats + ((row * cfg.nf + fi) * nchunks + k) * 3;
   bool done = false;
-  if constexpr (KIND == SPP_OUT_I32) {
+  if constexpr (SUMS) {
     if (pow2) {
       const int len = (int)imin64(own + cfg.wmax, m - i0);
       const int32_t* x = reinterpret_cast<const int32_t*>(base) + i0 * f;
@@ -634,11 +634,19 @@ k_snr_chunk(const void* __restrict__ in, int64_t n, int64_t in_stride, const Snr
         q += d * d;
       }
       q = block_sum(q, red);
-      // pairwise merge of the pieces' moments (every thread keeps them)
-      const double nb = (double)po, d = mu - mean, all = cnt + nb;
-      mean += d * nb / all;
-      m2 += q + d * d * cnt * nb / all;
-      cnt = all;
+      // pairwise merge of the pieces' moments (every thread keeps them); nearly all
+      // chunks are one piece, and float64 divisions by every thread are a tenth of a
+      // short row's time
+      if (p0 == 0) {
+        cnt = (double)po;
+        mean = mu;
+        m2 = q;
+      } else {
+        const double nb = (double)po, d = mu - mean, all = cnt + nb;
+        mean += d * nb / all;
+        m2 += q + d * d * cnt * nb / all;
+        cnt = all;
+      }
       if (threadIdx.x == 0) {
         st[0] = cnt;
         st[1] = p0 == 0 ? tot : st[1] + tot;
@@ -656,15 +664,18 @@ k_snr_chunk(const void* __restrict__ in, int64_t n, int64_t in_stride, const Snr
   }
 }
 
-// One warp per (row, factor, width): lanes take chunks, moments and maxima merge
-// pairwise.
-__global__ void k_snr_final(int64_t n, const SnrCfg cfg, int64_t nrows, int64_t nchunks,
+// `lanes` lanes (a power of two up to the warp) per (row, factor, width): they take
+// chunks, moments and maxima merge pairwise.  As many as there are chunks: a warp
+// each for rows of one chunk took 390 us for 60000 rows and 8 widths, a third of the
+// call (12 us with a lane each).
+__global__ void k_snr_final(int64_t n, const SnrCfg cfg, int64_t nrows, int64_t nchunks, int lanes,
                             const SnrPart* __restrict__ parts, const double* __restrict__ stats,
                             float* __restrict__ snr, int32_t* __restrict__ peak,
                             const double* __restrict__ locscale) {
-  const int64_t id = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (id >= nrows * cfg.nf * cfg.nw) return;
+  const int64_t all = nrows * cfg.nf * cfg.nw;
+  const int64_t own = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / lanes;
+  const int64_t id = imin64(own, all - 1);  // whole warps merge
+  const int lane = threadIdx.x & (lanes - 1);
   const int wi = id % cfg.nw;
   const int64_t rf = id / cfg.nw;  // row * nfactors + fi
   const int64_t m = n / cfg.f[rf % cfg.nf];
@@ -672,7 +683,7 @@ __global__ void k_snr_final(int64_t n, const SnrCfg cfg, int64_t nrows, int64_t 
   double cnt = 0.0, mean = 0.0, m2 = 0.0;
   double best = -DBL_MAX;
   long long bidx = LLONG_MAX;
-  for (int64_t k = lane; k < nck; k += 32) {
+  for (int64_t k = lane; k < nck; k += lanes) {
     const double* st = stats + (rf * nchunks + k) * 3;
     const double nb = st[0], mb = st[1] / nb;
     const double d = mb - mean, tot = cnt + nb;
@@ -685,8 +696,7 @@ __global__ void k_snr_final(int64_t n, const SnrCfg cfg, int64_t nrows, int64_t 
       bidx = p.idx;
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
+  for (int o = lanes / 2; o > 0; o >>= 1) {
     const double nb = __shfl_xor_sync(0xffffffffu, cnt, o);
     const double mb = __shfl_xor_sync(0xffffffffu, mean, o);
     const double qb = __shfl_xor_sync(0xffffffffu, m2, o);
@@ -709,7 +719,7 @@ __global__ void k_snr_final(int64_t n, const SnrCfg cfg, int64_t nrows, int64_t 
       bidx = oi;
     }
   }
-  if (lane != 0) return;
+  if (lane != 0 || own >= all) return;
   double sd = cnt > 0 ? sqrt(m2 / cnt) : 0.0;
   if (sd == 0.0) sd = 1.0;
   if (locscale) {  // median / IQR scale
@@ -978,7 +988,7 @@ static int launch_quantiles(const void* in, int kind, int64_t nrf, int64_t n, in
   int rc = SPP_OK;
   if (split == 1) {
     const dim3 grid(1, (unsigned)nrf);
-    if (n <= kQShortRow) {
+    if (n / *std::min_element(cfg.f, cfg.f + cfg.nf) <= kQShortRow) {
       k_row_quantiles<8><<<grid, kQPassThreads, kQRanks * 256 * 4, st>>>(a, cfg);
     } else {
       rc = set_smem_attr(reinterpret_cast<const void*>(k_row_quantiles<kQBits>), smem);
@@ -1359,18 +1369,16 @@ static int boxcar_snr_impl(const void* in, int in_kind, int64_t nrows, int64_t n
   cfg.smem_words = ints ? std::max({most + 2, 1 + runs * kSnrThreads, 2 * (cfg.wmax + 513)})
                         : 2 * (cfg.chunk + cfg.wmax + 1);
   const int64_t smem = (int64_t)cfg.smem_words * 4;
-  const void* fn = ints ? reinterpret_cast<const void*>(k_snr_chunk<SPP_OUT_I32>)
-                        : reinterpret_cast<const void*>(k_snr_chunk<SPP_OUT_F32>);
+  // integer rows without a power-of-two factor have no use for the integer path
+  const bool sums = ints && std::any_of(cfg.f, cfg.f + nfactors, [](int f) { return (f & (f - 1)) == 0; });
+  auto fn = !ints ? k_snr_chunk<SPP_OUT_F32, false> : sums ? k_snr_chunk<SPP_OUT_I32, true> : k_snr_chunk<SPP_OUT_I32, false>;
   int rc = SPP_OK;
   if (smem > 48 * 1024) {
-    rc = set_smem_attr(fn, smem);
+    rc = set_smem_attr(reinterpret_cast<const void*>(fn), smem);
     if (rc) return rc;
   }
   dim3 grid((unsigned)ceil_div(n, cfg.chunk), (unsigned)(nrows * nfactors));
-  if (ints)
-    k_snr_chunk<SPP_OUT_I32><<<grid, kSnrThreads, smem, st>>>(in, n, in_stride, cfg, nck, parts, stats);
-  else
-    k_snr_chunk<SPP_OUT_F32><<<grid, kSnrThreads, smem, st>>>(in, n, in_stride, cfg, nck, parts, stats);
+  fn<<<grid, kSnrThreads, smem, st>>>(in, n, in_stride, cfg, nck, parts, stats);
   rc = cuda_status(cudaGetLastError(), "snr chunk launch");
   if (rc) return rc;
   double* locscale = nullptr;
@@ -1381,8 +1389,10 @@ static int boxcar_snr_impl(const void* in, int in_kind, int64_t nrows, int64_t n
     if (rc) return rc;
   }
   const int64_t nout = nrows * nfactors * nwidths;
-  k_snr_final<<<(unsigned)ceil_div(nout, 8), 256, 0, st>>>(n, cfg, nrows, nck, parts, stats, snr,
-                                                             peak_index, locscale);
+  int lanes = 1;
+  while (lanes < 32 && lanes < ceil_div(n, cfg.chunk)) lanes *= 2;
+  k_snr_final<<<(unsigned)ceil_div(nout * lanes, 256), 256, 0, st>>>(n, cfg, nrows, nck, lanes, parts, stats,
+                                                                    snr, peak_index, locscale);
   return cuda_status(cudaGetLastError(), "snr final launch");
 }
 

@@ -81,3 +81,13 @@ def test_chunk_rule(orc, rows, wmax):
     x = rng.integers(-2000, 2000, size=(rows, 6145), endpoint=True).astype(np.int32)
     _check(orc, x, [1, 5, wmax], [1])
     _check(orc, x.astype(np.float32), [1, 5, wmax], [1])
+
+
+@pytest.mark.parametrize("rows,n,factors", [(1500, 130, [3]), (1500, 131, [1, 3]), (3, 3073, [1]), (1, 60001, [1, 2])])
+@pytest.mark.parametrize("dtype", [np.int32, np.float32])
+def test_chunks_per_row(orc, rows, n, factors, dtype):
+    """One chunk a row (a lane each in the final pass), three and forty (four lanes, a
+    warp); integer rows without a power-of-two factor."""
+    rng = np.random.default_rng(rows + n)
+    x = rng.integers(-2000, 2000, size=(rows, n), endpoint=True).astype(dtype)
+    _check(orc, x, [1, 5, 32], factors)
