@@ -1,6 +1,7 @@
 // libsppgpu core: error state, unpack (R4), single-DM dedispersion (R2) and
 // the DM-trial batch plan (R3).  Host code for the kernels in spp_dmt.cuh.
 #include <algorithm>
+#include <cmath>
 #include <atomic>
 #include <climits>
 #include <cstring>
@@ -83,19 +84,25 @@ __global__ void k_unpack(const uint8_t* __restrict__ in, int64_t nbytes, int bit
 // ---------------------------------------------------------------------------
 // DMT kernel variants
 // ---------------------------------------------------------------------------
+// Estimated time (us) of a CTA's walk over the channels: alone, and per tile of those
+// an SM runs beside one another.
+struct WalkTime {
+  double walk0, walk, tile, few;
+};
+
 struct Variant {
   int nb, acc, R, DW, TW, SLAB, STAGES;
   void (*fn)(const DmtArgs);
   int single;  // 1: meant for one DM (time-split warps)
   int planes;  // 1: bit-sliced kernel over bit-plane rows (R = words per thread)
   int slot;    // > 0: kernel compiled for exactly this slot width (words)
-  double rate = 0.0;  // float32 shapes: measured rate relative to the fastest
+  WalkTime time = {};  // float64 sums
 };
 
 template <int NB, int R, int DW, int TW, int SLAB, int STAGES, int ACC>
-static Variant mk(int single, double rate = 0.0) {
+static Variant mk(int single, WalkTime time = {}) {
   return Variant{NB, ACC, R, DW, TW, SLAB, STAGES, &k_dmt<NB, R, DW, TW, SLAB, STAGES, ACC>,
-                 single, 0, 0, rate};
+                 single, 0, 0, time};
 }
 
 // Bit-sliced counters hold sums below 2^bit_levels(nbits).
@@ -147,17 +154,20 @@ static const std::vector<Variant>& variants() {
       mk<32, 8, 2, 1, 16, 2, SPP_ACC_KAHAN32>(0),
       mk<32, 16, 2, 1, 16, 2, SPP_ACC_KAHAN32>(0),
       // float32 input, fp64 accumulator (channel-ordered sums: the reference's).
-      // The argument is the shape's measured rate with the SMs full, relative to
-      // the first (1024 channels, 256 trials to DM 500, 57444 outputs: 2.98 ms;
-      // 16 words x 4 trials, the choice before, 4.14 ms: three CTAs of four
-      // warps per SM leave the adders waiting on slab hand-overs).  16 words per
-      // thread leave few registers for loads in flight: 8 trials x 2 warps of
-      // them took 2.9 to 4.1 ms from one compilation to the next and are not used.
-      // Wide delay spreads fit only the small tiles.
-      mk<32, 8, 8, 2, 16, 2, SPP_ACC_F64>(0, 1.0), mk<32, 16, 5, 3, 16, 2, SPP_ACC_F64>(0, 0.97),
-      mk<32, 8, 4, 1, 16, 2, SPP_ACC_F64>(0, 0.95), mk<32, 8, 4, 2, 16, 2, SPP_ACC_F64>(0, 0.9),
-      mk<32, 16, 4, 1, 16, 2, SPP_ACC_F64>(0, 0.8), mk<32, 16, 2, 1, 16, 2, SPP_ACC_F64>(0, 0.6),
-      mk<32, 8, 2, 1, 16, 2, SPP_ACC_F64>(0, 0.75),
+      // With the SMs full, 8 words x 8 trials x 2 warps were the fastest (1024
+      // channels, 256 trials to DM 500, 57444 outputs: 2.98 ms; 16 words x 4 trials,
+      // the choice before, 4.14 ms: three CTAs of four warps per SM leave the adders
+      // waiting on slab hand-overs).  16 words per thread leave few registers for
+      // loads in flight: 8 trials x 2 warps of them took 2.9 to 4.1 ms from one
+      // compilation to the next and are not used.  Wide delay spreads fit only the
+      // small tiles.  The arguments are fitted beside float64_us.
+      mk<32, 8, 8, 2, 16, 2, SPP_ACC_F64>(0, {15.8, 0.147, 0.127, 1.9}),
+      mk<32, 16, 5, 3, 16, 2, SPP_ACC_F64>(0, {17.8, 0.144, 0.213, 13.1}),
+      mk<32, 8, 4, 1, 16, 2, SPP_ACC_F64>(0, {15.6, 0.0924, 0.0322, 1.28}),
+      mk<32, 8, 4, 2, 16, 2, SPP_ACC_F64>(0, {15.5, 0.0968, 0.0624, 1.71}),
+      mk<32, 16, 4, 1, 16, 2, SPP_ACC_F64>(0, {15.3, 0.111, 0.0589, 0.578}),
+      mk<32, 16, 2, 1, 16, 2, SPP_ACC_F64>(0, {15.3, 0.123, 0.0289, 0.799}),
+      mk<32, 8, 2, 1, 16, 2, SPP_ACC_F64>(0, {16.2, 0.0732, 0.0192, 0.785}),
       mk<32, 4, 1, 4, 32, 2, SPP_ACC_F64>(1),
       mk<32, 2, 1, 4, 32, 2, SPP_ACC_F64>(1),
   };
@@ -771,63 +781,103 @@ static std::vector<int> ilv_shapes(int nbits, int64_t nchans) {
 // over the channels.
 static bool short_walk(const Variant& v) { return !v.planes && v.R == 2 && v.DW == 4 && v.TW == 2; }
 
-// Estimated time (us) of a block by a packed kernel over 32 consecutive samples
-// per word.  Few tiles: one CTA's walk over all channels, whatever the trials
-// (1024 channels: 170-330 us bit-sliced, 115 us by byte lanes of four trials).
-// Many: channel-adds at the measured rate, half as much again on coarse grids.
-// Either way the corner turn.
+// Estimated times (us), fitted to 1573 plans measured with every shape they offer
+// (16-4096 channels, 2-1024 trials, 1000-250000 outputs, trial grids from fine to
+// thousands of samples apart; the logarithms' deviation is 0.08 to 0.2).
+
+// A block by a packed kernel over 32 consecutive samples per word.  Few tiles: one
+// CTA's walk over all channels, shorter where warps have no trial.  Many: tiles over
+// 148 SMs, each slower the fewer CTAs an SM holds beside it.  Between the two the sum
+// of fourth powers; then the corner turn, per MB of raw rows.
+struct PackedTime {
+  double walk0, walk, fill, full0, tile, few, mb;
+};
 static double packed_us(const spp_dmt_plan* p, int cand, int64_t nsamps, int64_t nvalid) {
+  static const PackedTime first[] = {{15.7, 0.0909, 0.57, 20.6, 0.0543, 1.42, 2.69},
+                                     {16.9, 0.126, 0.687, 24.0, 0.0716, 0.366, 1.98},
+                                     {14.8, 0.25, 0.745, 23.6, 0.137, 2.01, 1.49},
+                                     {14.4, 0.407, 0.819, 26.2, 0.0954, 3.79, 1.09}};
+  static const PackedTime lanes8 = {10.3, 0.132, 0.95, 17.6, 0.0952, 0.59, 0.836};
+  static const PackedTime brief[] = {{15.1, 0.106, 1.0, 24.4, 0.132, 0.173, 3.38},
+                                     {11.7, 0.0686, 1.0, 20.5, 0.0595, 0.531, 2.3},
+                                     {9.3, 0.0666, 1.0, 18.1, 0.0325, 1.89, 1.51},
+                                     {6.43, 0.0649, 1.0, 18.1, 0.0299, 1.72, 0.649}};
   const Variant& v = variants()[p->cands[cand]];
-  const int32_t span = p->spans[cand];
   const int k = p->nbits == 1 ? 0 : p->nbits == 2 ? 1 : p->nbits == 4 ? 2 : 3;
-  const double adds = (double)p->ndm * nvalid * p->nchans;
-  const double mb = (double)nsamps * (double)(p->nchans * p->nbits) / 8e6;
-  if (short_walk(v)) {
-    static const double rate[] = {1.7e7, 1.9e7, 1.25e7, 0.75e7};  // adds per us
-    const double two = 1.2 + 3e-4 * p->nchans;  // walks of two CTAs on an SM over one alone
-    const int64_t ctas = ceil_div(p->ndm, v.DW) * ceil_div(nvalid, tile_T(v));
-    const int64_t per_sm = (228 << 10) / (smem_bytes(v, slot_words(v, span)) + 1024) >= 2 ? 2 : 1;
-    const double walk = 15.0 + (k == 0 ? 0.112 : 0.098) * p->nchans;
-    const double waves = (double)ceil_div(ctas, 148 * per_sm) * (per_sm == 2 && ctas > 148 ? two : 1.0);
-    return std::max(adds / rate[k] + 20.0, walk * waves) + (k == 3 ? 0.5 : 2.0) * mb;
-  }
-  static const double rate[] = {5.0e7, 5.2e7, 2.2e7, 0.95e7}, us0[] = {10, 14, 25, 25},
-                      chan[] = {0.158, 0.19, 0.305, 0.44};
-  const bool lanes = !v.planes;  // 8-bit, eight words per thread
-  const double fill = 0.35 + 0.65 * std::min(1.0, (double)p->ndm / v.DW);  // warps without a trial
-  const double walk = (lanes ? 12.0 : us0[k]) + (lanes ? 0.15 : chan[k]) * fill * p->nchans;
-  return std::max(1.5 * adds / (lanes ? 1.2e7 : rate[k]) + 20.0, walk) + (lanes ? 0.5 : 1.2) * mb;
+  const PackedTime& c = short_walk(v) ? brief[k] : k == 3 && !v.planes ? lanes8 : first[k];
+  const double fill = c.fill + (1.0 - c.fill) * std::min(1.0, (double)p->ndm / v.DW);
+  const double ctas = (double)ceil_div(p->ndm, v.DW) * (double)ceil_div(nvalid, tile_T(v));
+  const int64_t per_sm = std::max<int64_t>(1, (228 << 10) / (smem_bytes(v, slot_words(v, p->spans[cand])) + 1024));
+  const double tile = c.tile * (1.0 + c.few * std::max(0.0, 1.0 / (double)per_sm - 0.25));
+  const double walk = c.walk0 + c.walk * fill * (double)p->nchans;
+  const double full = c.full0 + tile * fill * (double)p->nchans * ctas / 148.0;
+  const double w2 = walk * walk, f2 = full * full;
+  return std::sqrt(std::sqrt(w2 * w2 + f2 * f2)) +
+         c.mb * (double)nsamps * (double)(p->nchans * p->nbits) / 8e6;
 }
 
-// The same by an interleaved shape: per wave of 148 CTAs a fixed part (start,
-// first copies, stores) and a part per group of channels, both measured per shape
-// (IlvCfg::us_wave, ns_group), 0.3 us per MB of what its rows hold beyond the
-// block itself, 5.5 us per further block of 32 runs that a turning CTA goes
-// through, and the pair rows' CTAs where those are many and short.  Raw rows that
-// are no whole number of 16-byte units, and a last group of channels that is no
-// whole 32 bytes, are turned byte by byte (5.5 us per MB, 22 us per block).
+// The same by an interleaved shape: per wave of 148 CTAs a fixed part (start, first
+// copies, stores) and a part per group of channels, both measured per shape
+// (IlvCfg::us_wave, ns_group) and scaled; the corner turn per MB of raw rows and per
+// byte of what its rows hold beyond the block; its further blocks of 32 runs; and the
+// pair rows, by their bytes or, where those are many and short, their CTAs.  Raw rows
+// that are no whole number of 16-byte units, and a last group of channels that is no
+// whole 32 bytes, are turned byte by byte.
+struct IlvTime {
+  double us0, wave, group, mb, extra, odd_mb, odd0, block, row, pair_cta;
+};
 static double interleaved_us(const spp_dmt_plan* p, const IlvCfg& c, int64_t nsamps, const IlvGeom& g) {
+  static const IlvTime chans[] = {{7.54, 0.847, 0.901, 1.77, 14e-7, 3.46, 5.32, 1.94, 0, 0},
+                                  {6.87, 0.75, 0.904, 2.34, 9.14e-7, 2.88, 9.12, 1.93, 0, 0},
+                                  {4.13, 0.75, 0.95, 1.56, 4.78e-7, 3.21, 6.82, 2.49, 0, 0},
+                                  {6.25, 0.947, 0.974, 1.16, 1.59e-7, 3.08, 5.91, 3.24, 0, 0}};
+  static const IlvTime pairs[] = {{},
+                                  {8.0, 1.0, 1.0, 1.4, 7e-7, 3.41, 4.6, 2.01, 3.65e-7, 0.312e-3},
+                                  {7.38, 0.75, 0.899, 1.53, 8.79e-7, 3.31, 8.73, 2.2, 2.1e-7, 0.814e-3},
+                                  {9.84, 0.759, 0.937, 1.16, 0.06e-7, 3.29, 7.63, 1.54, 3.07e-7, 7.98e-3}};
+  const int k = p->nbits == 1 ? 0 : p->nbits == 2 ? 1 : p->nbits == 4 ? 2 : 3;
+  const IlvTime& e = c.G == 2 ? pairs[k] : chans[k];
   const int64_t ctas = ceil_div(p->ndm, c.DW) * ceil_div(g.M, c.words());
   const double ng = (double)round_up(p->nchans / c.G, 4 * c.nq);
-  double t = 10.0 + (double)ceil_div(ctas, 148) * (c.us_wave + ng * c.ns_group * 1e-3);
-  t += (double)(g.chan_bytes - p->nchans * g.M * c.nb * 4) * 3e-7;
   const int64_t rowbytes = p->nchans * c.nb / 8, odd = rowbytes % 16 ? rowbytes : rowbytes % 32;
-  const int64_t blocks = p->ilv_rows[0].max_group / (32 * g.M);
-  t += odd ? 10.0 + 5.5e-6 * (double)nsamps * (double)odd + 22.0 * blocks : 5.5 * blocks;
+  const double blocks = (double)(p->ilv_rows[0].max_group / (32 * g.M));
+  double t = e.us0 + (double)ceil_div(ctas, 148) * (e.wave * c.us_wave + ng * e.group * c.ns_group * 1e-3);
+  t += e.mb * (double)nsamps * (double)rowbytes * 1e-6;
+  t += e.extra * (double)(g.chan_bytes - p->nchans * g.M * c.nb * 4);
+  t += odd ? e.odd0 + e.odd_mb * 1e-6 * (double)nsamps * (double)odd + 4.0 * e.block * blocks : e.block * blocks;
   if (c.G == 2) {
     const double pair_ctas = (double)(p->nchans / 2) * (double)ceil_div(g.M + p->ilv_rows[0].max_ext, 512);
-    t += std::max((double)g.row_bytes * 3e-7, 2.3e-3 * pair_ctas);
+    t += std::max(e.row * (double)g.row_bytes, e.pair_cta * pair_ctas);
   }
   return t;
 }
 
+// Float64 sums of float32 rows, without the corner turn that all shapes share: one
+// CTA's walk where few tiles run, else the SM's share of the tiles (whole ones: the
+// fullest SM counts), slower below 12 adding warps per SM; the sum of fourth powers
+// between.  Over 629 plans (16-4096 channels, 2-500 trials) the shape of least
+// estimate takes 1.3 % longer than the fastest on average; a rate per shape over waves
+// of full SMs, 5.1 %.
+static double float64_us(const spp_dmt_plan* p, int cand, int64_t nvalid) {
+  const Variant& v = variants()[p->cands[cand]];
+  const int64_t smem = smem_bytes(v, slot_words(v, p->spans[cand])) + 1024;
+  const int64_t per_sm = std::max<int64_t>(1, std::min<int64_t>((228 << 10) / smem, 64 / (v.DW * v.TW + 1)));
+  const int64_t ctas = ceil_div(p->ndm, v.DW) * ceil_div(nvalid, tile_T(v));
+  const double few = 1.0 + v.time.few * std::max(0.0, 12.0 / (double)(per_sm * v.DW * v.TW) - 1.0);
+  const double walk = v.time.walk0 + v.time.walk * (double)p->nchans;
+  const double full = v.time.tile * few * (double)p->nchans * (double)ceil_div(ctas, 148);
+  const double w2 = walk * walk, f2 = full * full;
+  return std::sqrt(std::sqrt(w2 * w2 + f2 * f2));
+}
+
 // The shape a plan starts from (without autotuning): the least estimated time
 // at nsamps_max, over the interleaved shapes, the first packed one and the one of
-// the shortest walk.  Over 190 measured plans (64-4096 channels, 2-1024 trials,
-// 50-100000 outputs) the choice is within 15 % of the fastest shape for all but
-// 12, and within 45 % for those.  Rows and staging tables above kIlvDefaultBytes
-// leave a shape to explicit choice: they grow with the block and the delay range,
-// and with the trials.
+// the shortest walk.  Over the 1573 plans that the estimates are fitted to the choice
+// takes 3.3 % longer than the fastest shape on average, and some 20 take more than 8 %
+// longer than before the interleaved shapes (2-bit plans of few tiles, where a kernel
+// over channel pairs had been the fastest, and blocks of 20 to 40 us).  Rows and
+// staging tables above kIlvDefaultBytes leave a shape to explicit choice: they grow
+// with the block and the delay range, and with the trials.
 // 2-bit grids so fine that a pair row serves 100 trials or more start from pairs
 // from 4096 outputs on (a pair shape's shortest tile), so that the blocks of one
 // observation run one kernel (4096 channels, 1024 trials to DM 2000: 45.9 ms
@@ -844,19 +894,11 @@ static int first_choice(spp_dmt_plan* p) {
   int first = 0;
   while (first + 1 < (int)p->cands.size() && !tiles_fit(first)) ++first;
   if (p->nbits == 32) {
-    // float64 sums: waves of the CTAs an SM holds (shared memory, 64 warps)
-    // times a tile's adds over its rate, which falls below 12 adding warps per SM
     int pick = first;
     double best = 0.0;
     for (int i = 0; i < (int)p->cands.size(); ++i) {
-      const Variant& v = variants()[p->cands[i]];
-      if (v.rate <= 0.0 || !tiles_fit(i)) continue;
-      const int64_t smem = smem_bytes(v, slot_words(v, p->spans[i])) + 1024;
-      const int64_t per_sm = std::min<int64_t>((228 << 10) / smem, 64 / (v.DW * v.TW + 1));
-      const int64_t ctas = ceil_div(p->ndm, v.DW) * ceil_div(nvalid, tile_T(v));
-      const double full = std::min(1.0, (double)(per_sm * v.DW * v.TW) / 12.0);
-      const double t =
-          (double)(ceil_div(ctas, 148 * per_sm) * per_sm * v.DW * tile_T(v)) / (v.rate * full);
+      if (variants()[p->cands[i]].time.tile <= 0.0 || !tiles_fit(i)) continue;
+      const double t = float64_us(p, i, nvalid);
       if (best == 0.0 || t < best) {
         best = t;
         pick = i;
@@ -881,7 +923,7 @@ static int first_choice(spp_dmt_plan* p) {
     if (iv < 0) {
       if (i != p->packed[0] && i != p->packed[1]) continue;
       t = packed_us(p, i, p->nsamps_max, nvalid);
-      if (i == p->packed[0]) t *= 0.95;  // near ties stay with the smaller workspace
+      if (i == p->packed[0]) t *= 0.92;  // near ties stay with the smaller workspace
     } else {
       const IlvCfg& c = ilv_cfgs()[iv];
       const IlvGeom g = ilv_geometry(c, p->ilv_rows[0], p->ilv_rows[c.G - 1], p->nchans, nvalid);

@@ -1057,8 +1057,8 @@ const std::vector<IlvCfg>& ilv_cfgs() {
       mki<1, 1, 4, 11, 2, 4, 10, 1>(32, 97), mki<1, 1, 4, 9, 2, 4, 14, 1>(29, 86),
       mki<1, 1, 4, 15, 1, 4, 14, 1>(19, 81), mki<1, 1, 4, 3, 5, 4, 14, 1>(22, 83),
       mki<1, 1, 4, 3, 5, 2, 14, 1>(22, 95),
-      mki<2, 2, 4, 9, 2, 2, 14, 1>(44, 195), mki<2, 2, 4, 15, 1, 2, 14, 1>(72, 148),
-      mki<2, 2, 4, 7, 2, 2, 14, 1>(26, 164),
+      mki<2, 2, 4, 9, 2, 2, 14, 1>(32, 190), mki<2, 2, 4, 15, 1, 2, 14, 1>(24, 160),
+      mki<2, 2, 4, 7, 2, 2, 14, 1>(30, 150),
       mki<2, 1, 4, 15, 1, 4, 14, 1>(30, 101), mki<2, 1, 4, 9, 2, 4, 14, 1>(33, 141),
       mki<2, 1, 4, 3, 5, 4, 14, 1>(21, 103), mki<2, 1, 4, 3, 5, 2, 14, 1>(21, 115),
       mki<4, 2, 3, 7, 2, 2, 16, 1>(18, 174), mki<4, 2, 4, 9, 2, 1, 13, 1>(40, 312),
