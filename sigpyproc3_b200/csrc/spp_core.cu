@@ -748,11 +748,16 @@ static void free_device(spp_dmt_plan* p) {
 // Pair rows a plan may hold, per channel.
 constexpr int64_t kPairRowsPerChan = 12;
 
-// Device words of a plan, one allocation (a second one of some MB takes 0.4 ms): the
-// delay table, then (for interleaved shapes) the words that make their rows, from
-// a 256-byte boundary on: the range pass stores pairs of words there, whatever
-// the table's size; then room for the staging tables of the shape that the plan
-// starts from, unless they may be large.
+// Device words of a plan: the delay table, then (for interleaved shapes) the words
+// that make their rows, from a 256-byte boundary on: the range pass stores pairs of
+// words there, whatever the table's size; then room for the staging tables of the
+// shape that the plan starts from, of the most that they may need (some four times
+// what they take).  The driver hands out chunks of 2 MB: a new chunk or a larger
+// allocation takes 0.38 ms and its release 0.3, a part of a chunk 2 us.  So tables have
+// room here where all of it is small or where words and tables would not share a
+// chunk, unless they may be large; else they are allocated as they turn out (8-bit,
+// beside other plans, 256 channels x 228 trials: creation 870 us with room of 1.4 MB,
+// 450 us without; 1024 x 300: 920 us in two allocations, 560 us in one).
 struct PlanWords {
   int64_t work, room, total;
 };
@@ -762,7 +767,9 @@ static PlanWords plan_words(int nbits, int64_t nchans, int64_t ndm) {
   const int64_t work = round_up(table, 64);
   const int64_t room = round_up(work + ilv_plan_words(nchans, kPairRowsPerChan * nchans), 64);
   const int64_t bytes = ilv_table_room(nbits, nchans, ndm);
-  return {work, room, room + (bytes <= 64ll << 20 ? bytes / 4 : 0)};
+  const bool one_chunk = 4 * room + bytes / 4 < 7ll << 18;  // 1.75 MB
+  const bool here = one_chunk ? 4 * room + bytes <= 512ll << 10 : bytes <= 64ll << 20;
+  return {work, room, room + (here ? bytes / 4 : 0)};
 }
 
 // Interleaved bit-plane shapes that channel count and sample width allow.
